@@ -38,6 +38,7 @@ using tc5::smem_desc;
 constexpr int TN = 128;          // N columns per CTA (MMA M)
 constexpr int TOK = 64;          // token slots (MMA N)
 constexpr int MAX_KB = 8;        // k-blocks of 64 per CTA
+constexpr int ACC_COLS = 2 * TOK;   // one accumulator per issuing thread
 
 enum Epi { EPI_QKV_ROPE = 0, EPI_RESIDUAL = 1, EPI_GEGLU = 2, EPI_BIAS = 3 };
 
@@ -138,7 +139,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     if (tid == 32) { tc5::prefetch_tensormap(&tmW); if (EPI == EPI_GEGLU) tc5::prefetch_tensormap(&tmW2); }
     if (tid == 64 && x_by_tma) tc5::prefetch_tensormap(&tmX);
     if (tid == 0) {
-        mbar_init(done_bar, 1);
+        mbar_init(done_bar, 2);                              // one commit from each issuing thread
         mbar_init(in_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -161,7 +162,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     }
     __syncwarp();
     if (warp == 0) {
-        tc5::tmem_alloc(base + off_bar + (MAX_KB + 2) * 8, 64);
+        tc5::tmem_alloc(base + off_bar + (MAX_KB + 2) * 8, ACC_COLS);
         tc5::tmem_relinquish();
     }
     // Programmatic dependent launch: everything above touched only weights and this CTA's own
@@ -262,19 +263,21 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     const uint32_t tmem = *tmem_slot;
     FVLA_STAMP(2);
 
-    if (tid == 0) {
+    // Two threads issue the MMAs, k-blocks in turn, each into an accumulator of its own. One thread needs 46 clk per MMA and
+    // another 110 - 290 per k-block for its wait, the descriptors and the next address, so that 8 k-blocks took 2 400 clk
+    // against 1 540 of tensor pipe (N = 64: 48 clk per MMA); two hide that from one another.
+    if (warp < 2 && lane == 0) {
         constexpr uint32_t idesc = skinny_idesc();
+        const uint64_t ad = smem_desc(sW, 8192, 1024), bd = smem_desc(sX, 16, 1024);
         bool ok = true;
-        for (int kb = 0; kb < KB && ok; ++kb) {
+        for (int kb = warp; kb < KB && ok; kb += 2) {
             ok = mbar_wait(bars + kb * 8, 0, abort_flag);
             tc5::tc_fence_after();
             if (!ok) break;
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) {
-                const uint64_t adesc = smem_desc(sW + kb * 16384 + k16 * 2048, 8192, 1024);
-                const uint64_t bdesc = smem_desc(sX + kb * 8192 + k16 * 32, 16, 1024);
-                tc5::umma_bf16(tmem, adesc, bdesc, idesc, (kb > 0 || k16 > 0) ? 1u : 0u);
-            }
+            for (int k16 = 0; k16 < 4; ++k16)
+                tc5::umma_bf16(tmem + warp * TOK, ad + kb * (16384 >> 4) + k16 * (2048 >> 4), bd + kb * (8192 >> 4) + k16 * (32 >> 4), idesc,
+                               (kb > 1 || k16 > 0) ? 1u : 0u);
         }
         tc5::umma_commit(done_bar);
     }
@@ -305,6 +308,12 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         const int q = warp & 3, g = warp >> 2;
         float part[16];
         tc5::tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + g * 16, part);
+        if (KB > 1) {
+            float odd[16];
+            tc5::tmem_ld16(tmem + TOK + ((uint32_t)(q * 32) << 16) + g * 16, odd);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) part[t] += odd[t];
+        }
 #pragma unroll
         for (int t = 0; t < 16; ++t) stage[(g * 16 + t) * TN + q * 32 + lane] = done ? part[t] : 0.f;
     }
@@ -314,18 +323,18 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     tc5::tc_fence_before();
     __syncthreads();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has initialised its barriers
-    if (tid == 0) {
-        // one bulk copy per owner: its slice of tokens goes to slot [src = my rank] of its RED buffer
-        for (int r = 0; r < owners; ++r) {
-            if (r == (int)rank) continue;                    // the owner reads its own slice where it was staged
-            bulk_copy_to_cta(map_to_cta(base + off_red + (uint32_t)(rank * TS) * 512u, (uint32_t)r),
-                             base + (uint32_t)(r * TS) * 512u, (uint32_t)TS * 512u, map_to_cta(in_bar, (uint32_t)r));
-            if (p.need_factor)
-                bulk_copy_to_cta(map_to_cta(base + off_red + 32768 + (uint32_t)(rank * TS) * 4u, (uint32_t)r),
-                                 base + (uint32_t)(TOK * TN) * 4u + (uint32_t)(r * TS) * 4u, (uint32_t)TS * 4u,
-                                 map_to_cta(in_bar, (uint32_t)r));
-        }
+    if (tid < owners && tid != (int)rank) {
+        // one bulk copy per owner, issued by a lane of its own: its slice of tokens goes to slot [src = my rank] of its RED
+        // buffer (an owner reads its own slice where it was staged)
+        const int r = tid;
+        bulk_copy_to_cta(map_to_cta(base + off_red + (uint32_t)(rank * TS) * 512u, (uint32_t)r),
+                         base + (uint32_t)(r * TS) * 512u, (uint32_t)TS * 512u, map_to_cta(in_bar, (uint32_t)r));
+        if (p.need_factor)
+            bulk_copy_to_cta(map_to_cta(base + off_red + 32768 + (uint32_t)(rank * TS) * 4u, (uint32_t)r),
+                             base + (uint32_t)(TOK * TN) * 4u + (uint32_t)(r * TS) * 4u, (uint32_t)TS * 4u,
+                             map_to_cta(in_bar, (uint32_t)r));
     }
+    __syncwarp();
 
     FVLA_STAMP(4);
     // Owner phase: this CTA finishes tokens [rank*TS, rank*TS + TS), summing partials in rank order.
@@ -404,7 +413,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     if (warp == 0) {
         tc5::tc_fence_after();
-        tc5::tmem_dealloc(tmem, 64);
+        tc5::tmem_dealloc(tmem, ACC_COLS);
     }
     FVLA_STAMP(7);
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 2);
@@ -482,7 +491,8 @@ inline int launch_skinny(SkinnyArgs a, const void* W, const void* W2, int ldw, c
     CUtensorMap tmW, tmW2, tmX;
     int rc = tc5::make_map(&tmW, W, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)ldw, 64, 64);
     if (rc) return rc;
-    rc = tc5::make_map(&tmW2, W2 ? W2 : W, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)ldw, 64, 64);
+    if (W2 == nullptr) tmW2 = tmW;                           // unused by the kernel in this case
+    else rc = tc5::make_map(&tmW2, W2, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)ldw, 64, 64);
     if (rc) return rc;
     if (a.x_f32 && a.x_shadow == nullptr) tmX = tmW;         // unused by the kernel in this case
     else rc = tc5::make_map(&tmX, a.x_f32 ? (const void*)a.x_shadow : a.x, (uint64_t)a.K, (uint64_t)a.M * groups, (uint64_t)a.ldx, 64, 64);
