@@ -6,6 +6,7 @@ entry point returns an error, the caller gets an exception; nothing falls back t
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_char_p, c_float, c_int, c_size_t, c_void_p
 from pathlib import Path
 
@@ -80,9 +81,20 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_entry: dict = {}
+
+
 def call(name: str, *args) -> None:
     """Invoke an entry point; raise FvlaError with the library's message on failure."""
-    lib = load()
-    status = getattr(lib, name)(*args)
+    fn = _entry.get(name)
+    if fn is None:
+        fn = _entry[name] = getattr(load(), name)
+    status = fn(*args)
     if status != 0:
-        raise FvlaError(f"{name} failed with status {status}: {lib.fvla_last_error().decode()}")
+        raise FvlaError(f"{name} failed with status {status}: {load().fvla_last_error().decode()}")
+
+
+@functools.lru_cache(maxsize=1024)
+def gemm_workspace_bytes(M: int, N: int, K: int, dual: int = 0) -> int:
+    """`fvla_gemm_workspace_bytes`, remembered: a pure function of the shape that walks every plan on each call."""
+    return load().fvla_gemm_workspace_bytes(M, N, K, dual)

@@ -136,7 +136,8 @@ def _ws(role: str, nbytes: int, device):
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """torch's current stream as a raw handle (without the Stream object that `torch.cuda.current_stream` builds)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _is_f32(name: str, t: torch.Tensor) -> int:
@@ -154,7 +155,7 @@ def _chk(name: str, t: torch.Tensor, shape=None, dtype=torch.bfloat16) -> int:
         raise ValueError(f"{name}: expected {dtype}, got {t.dtype}")
     if not t.is_contiguous():
         raise ValueError(f"{name}: expected a contiguous tensor, got strides {t.stride()}")
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != shape:           # torch.Size compares as a tuple
         raise ValueError(f"{name}: expected shape {tuple(shape)}, got {tuple(t.shape)}")
     return t.data_ptr()
 
@@ -260,7 +261,7 @@ def _linear_bias_residual(role, x, weight, bias, res, out):
     M = x.numel() // K
     if res.numel() != M * N or out.numel() != M * N:
         raise ValueError("linear_bias_residual: res/out have the wrong size")
-    ws, nb = _ws(role, _lib.load().fvla_gemm_workspace_bytes(M, N, K, 0), x.device)
+    ws, nb = _ws(role, _lib.gemm_workspace_bytes(M, N, K, 0), x.device)
     _lib.call("fvla_vision_linear_bias_residual", _chk("x", x), _chk("weight", weight),
               _chk("bias", bias, (N,)), _chk("res", res), _chk("out", out), M, N, K, ws, nb, _stream())
     return out
@@ -356,8 +357,7 @@ def _linear_residual(role, x, weight, out):
         x, out = x.reshape(-1, x.shape[2]), out.reshape(-1, out.shape[2])
     M, K = x.shape
     N = weight.shape[1]
-    lib = _lib.load()
-    ws, nb = _ws(role, lib.fvla_gemm_workspace_bytes(M, N, K, 0), x.device)
+    ws, nb = _ws(role, _lib.gemm_workspace_bytes(M, N, K, 0), x.device)
     _lib.call("fvla_linear_residual", _chk("x", x), _chk("weight", weight, (K, N)),
               _chk("out", out, (M, N), dtype=None), _is_f32("out", out), _shadow_of(out), M, N, K, group_rows, ws, nb,
               _stream())
@@ -388,8 +388,7 @@ def encoder_ffn_down_residual(x, weight, out):
 def _small_proj(role, x, weight, bias, out, act):
     K, N = weight.shape
     M = x.numel() // K
-    lib = _lib.load()
-    ws, nb = _ws(role, lib.fvla_gemm_workspace_bytes(M, N, K, 0) if K > 64 else 0, x.device)
+    ws, nb = _ws(role, _lib.gemm_workspace_bytes(M, N, K, 0) if K > 64 else 0, x.device)
     if out.numel() != M * N:
         raise ValueError(f"{role}: out has the wrong size")
     _lib.call("fvla_decoder_small_proj", _chk("x", x, dtype=None), _is_f32("x", x),
@@ -423,13 +422,12 @@ def decoder_norm_qkv_rope(x, weight_qkv, rope, Q, K, V, norm_factor):
     hd = V.shape[-1]
     heads = Q.shape[0] // M
     N = (heads + 2) * hd
-    lib = _lib.load()
     k_ptr, group, pitch = _kv_destination("K", K, M, hd)
     v_ptr, group_v, pitch_v = _kv_destination("V", V, M, hd)
     if (group, pitch) != (group_v, pitch_v):
         raise ValueError("decoder_norm_qkv_rope: K and V must have the same layout")
     rope_rows = group or M
-    ws, nb = _ws("dec_qkv_ws", lib.fvla_gemm_workspace_bytes(M, N, Kdim, 0), x.device)
+    ws, nb = _ws("dec_qkv_ws", _lib.gemm_workspace_bytes(M, N, Kdim, 0), x.device)
     _lib.call("fvla_decoder_norm_qkv_rope", _chk("x", x, dtype=None), _is_f32("x", x), _shadow_of(x),
               _chk("weight_qkv", weight_qkv, (Kdim, N)),
               _chk("rope", rope[:rope_rows], (rope_rows, hd)), _chk("Q", Q, (M * heads, hd)), k_ptr, v_ptr,
@@ -481,8 +479,7 @@ def decoder_ffn_down_residual(x, weight, out):
 def _gated_ffn(x, gate_w, up_w, out, norm_factor):
     M, K = x.shape
     N = gate_w.shape[1]
-    lib = _lib.load()
-    ws, nb = _ws("dec_gate_ws", lib.fvla_gemm_workspace_bytes(M, N, K, 1), x.device)
+    ws, nb = _ws("dec_gate_ws", _lib.gemm_workspace_bytes(M, N, K, 1), x.device)
     nf = None if norm_factor is None else _chk("norm_factor", norm_factor[:M], (M,))
     _lib.call("fvla_decoder_norm_gated_ffn", _chk("x", x, dtype=None), _is_f32("x", x), _shadow_of(x),
               _chk("gate_w", gate_w, (K, N)),

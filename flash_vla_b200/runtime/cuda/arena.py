@@ -17,13 +17,20 @@ import torch
 class ScratchPool:
     def __init__(self) -> None:
         self._slabs: dict[tuple, torch.Tensor] = {}
+        self._seen: dict[tuple, torch.Tensor] = {}      # the same slabs by the arguments as they were passed
         self._frozen = False
 
     def get(self, role: str, shape, dtype, device) -> torch.Tensor:
         """The buffer registered for (role, shape, dtype, device); created zeroed on first use."""
+        asked = (role, shape, dtype, device) if type(shape) is tuple else None
+        slab = self._seen.get(asked)
+        if slab is not None:
+            return slab
         key = (role, tuple(int(s) for s in shape), dtype, str(device))
         slab = self._slabs.get(key)
         if slab is not None:
+            if asked is not None:
+                self._seen[asked] = slab
             return slab
         if self._frozen:
             raise RuntimeError(
