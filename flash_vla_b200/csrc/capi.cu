@@ -725,6 +725,39 @@ int fvla_convert_copy(const void* src, int src_is_f32, void* dst, int dst_is_f32
     return check_launch("convert_copy_kernel");
 }
 
+int fvla_decoder_steps_run(const struct fvla_decoder_steps* d, void* stream) {
+    FVLA_REQUIRE(d != nullptr && d->first_step >= 0 && d->steps >= d->first_step && d->layers >= 1 && d->chunk >= 1 && d->prefix >= 1 &&
+                 d->cache_rows == d->prefix + d->chunk + 1, "decoder_steps: bad shape");
+    constexpr int W = 1024, HEADS = 8, HD = 256, QD = HEADS * HD, QKV = QD + 2 * HD, FFN = 4096, ACT = 32, TIMES = 10;
+    const int D = d->chunk + 1;
+    const size_t chunk_elems = (size_t)d->chunk * ACT;
+    float* x = static_cast<float*>(d->x);
+    bf16* shadow = Bm(d->x_shadow);
+    int rc = FVLA_OK;
+    if (d->first_step == 0) rc = fvla_convert_copy(d->noise, 0, d->noise_f32, 1, nullptr, chunk_elems, stream);
+    for (int step = d->first_step; step < d->steps && rc == FVLA_OK; ++step) {
+        rc = fvla_convert_copy(d->state, 0, x, 1, shadow, W, stream);
+        if (!rc) rc = fvla_decoder_small_proj(d->noise_f32, 1, d->in_w, B(d->time_bias) + (size_t)(step % TIMES) * W, d->in_buf, 0, nullptr, d->chunk, W, ACT, 2, nullptr, 0, stream);
+        if (!rc) rc = fvla_decoder_small_proj(d->in_buf, 0, d->mlp_w, d->mlp_b, x + W, 1, shadow ? shadow + W : nullptr, d->chunk, W, W, 0, d->ws_mlp, d->ws_mlp_bytes, stream);
+        for (int l = 0; l < d->layers && rc == FVLA_OK; ++l) {
+            bf16* k = Bm(d->k_cache) + (size_t)l * d->cache_rows * HD;
+            bf16* v = Bm(d->v_cache) + (size_t)l * d->cache_rows * HD;
+            const size_t tail = (size_t)d->prefix * HD;
+            rc = fvla_decoder_norm_qkv_rope(x, 1, shadow, B(d->qkv_w) + (size_t)l * W * QKV, d->rope, d->q, k + tail, v + tail, nullptr, D, W, HEADS, HD, 0, 0,
+                                            d->ws_qkv, d->ws_qkv_bytes, stream);
+            if (!rc) rc = fvla_decoder_attention(d->q, k, v, d->q, D * HEADS, d->cache_rows, HD, HEADS, d->prefix, 1, (long long)D * HEADS * HD, 0,
+                                                 d->ws_attn, d->ws_attn_bytes, stream);
+            if (!rc) rc = fvla_linear_residual(d->q, B(d->attn_o_w) + (size_t)l * QD * W, x, 1, shadow, D, W, QD, 0, d->ws_o, d->ws_o_bytes, stream);
+            if (!rc) rc = fvla_decoder_norm_gated_ffn(x, 1, shadow, B(d->gate_w) + (size_t)l * W * FFN, B(d->up_w) + (size_t)l * W * FFN, d->hidden, nullptr, D, FFN, W,
+                                                      d->ws_gate, d->ws_gate_bytes, stream);
+            if (!rc) rc = fvla_linear_residual(d->hidden, B(d->down_w) + (size_t)l * FFN * W, x, 1, shadow, D, W, FFN, 0, d->ws_down, d->ws_down_bytes, stream);
+        }
+        if (!rc) rc = fvla_decoder_action_out_proj(x + W, 1, d->out_w, d->out_b, d->noise_f32, 1, nullptr, nullptr, d->chunk, ACT, W, stream);
+    }
+    if (!rc) rc = fvla_convert_copy(d->noise_f32, 1, d->noise, 0, nullptr, chunk_elems, stream);
+    return rc;
+}
+
 int fvla_embed_rows(const void* table, const long long* ids, void* out, int rows, int dim, long long vocab, void* stream) {
     FVLA_REQUIRE(rows > 0 && dim > 0 && dim % 8 == 0 && vocab > 0, "embed_rows: bad shape rows=%d dim=%d (dim %% 8 == 0)", rows, dim);
     FVLA_REQUIRE(table != nullptr && ids != nullptr && out != nullptr && aligned16(table) && aligned16(out), "embed_rows: null or misaligned pointer");

@@ -3,7 +3,8 @@
 A backend is a module with two dicts of call-site wrappers sharing one signature per name:
 `ALL_WRAPPERS` (every call site) and `FUSED_WRAPPERS` (overlays used when `fused=True`).
 Same contract as the reference's registry (`.../h100/pi0/backends/__init__.py:10-40`); this
-target registers one backend, "cuda".
+target registers one backend, "cuda". A backend may also offer `STAGES`, whole pipeline stages as one call, which
+ride in its fused table.
 """
 from __future__ import annotations
 
@@ -23,4 +24,5 @@ def build_table(backend: str = "cuda", fused: bool = True) -> SimpleNamespace:
     table = dict(module.ALL_WRAPPERS)
     if fused:
         table.update(module.FUSED_WRAPPERS)
+        table.update(module.STAGES)
     return SimpleNamespace(**table)

@@ -14,6 +14,16 @@ LIB_PATH = Path(__file__).resolve().parents[6] / "libfvla_b200.so"
 
 _P, _I, _Z, _F = c_void_p, c_int, c_size_t, c_float
 
+
+class DecoderSteps(ctypes.Structure):
+    """`struct fvla_decoder_steps` of the header."""
+    _fields_ = ([(n, _P) for n in ("in_w", "time_bias", "mlp_w", "mlp_b", "qkv_w", "attn_o_w", "gate_w", "up_w", "down_w",
+                                   "out_w", "out_b", "rope", "state", "noise", "noise_f32", "x", "x_shadow", "in_buf", "q",
+                                   "hidden", "k_cache", "v_cache", "ws_mlp", "ws_qkv", "ws_attn", "ws_o", "ws_gate", "ws_down")] +
+                [(n, _Z) for n in ("ws_mlp_bytes", "ws_qkv_bytes", "ws_attn_bytes", "ws_o_bytes", "ws_gate_bytes", "ws_down_bytes")] +
+                [(n, _I) for n in ("chunk", "prefix", "cache_rows", "first_step", "steps", "layers")])
+
+
 # name -> argument ctypes (every function returns int except the three queries below)
 SIGNATURES: dict[str, list] = {
     "fvla_vision_patch_embed": [_P, _P, _P, _P, _P, _I, _P, _Z, _P],
@@ -35,6 +45,7 @@ SIGNATURES: dict[str, list] = {
     "fvla_decoder_attention": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, ctypes.c_longlong, ctypes.c_longlong, _P, _Z, _P],
     "fvla_decoder_norm_gated_ffn": [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P, _Z, _P],
     "fvla_decoder_action_out_proj": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P],
+    "fvla_decoder_steps_run": [ctypes.POINTER(DecoderSteps), _P],
     "fvla_embed_rows": [_P, _P, _P, _I, _I, ctypes.c_longlong, _P],
     "fvla_convert_copy": [_P, _I, _P, _I, _P, _Z, _P],
     "fvla_selftest_wait_timeout": [_P, _P, _P, _I, _I, _I, ctypes.c_uint, _P],

@@ -28,6 +28,8 @@ def op_table(fused: bool = True, backend: str = "cuda",
             table[name] = module.FUSED_WRAPPERS[name]
         elif name in module.ALL_WRAPPERS:
             table[name] = module.ALL_WRAPPERS[name]
+    if fused and set(plan.values()) <= {backend}:      # a stage stands for ops of one backend only
+        table.update(BACKENDS[backend].STAGES)
     return SimpleNamespace(**table)
 
 

@@ -208,9 +208,16 @@ def decoder_epilogue(buffers, ops=None):
 def transformer_decoder(ops, weights, buffers, encoder_seq_len, steps=DIFFUSION_STEPS,
                         layers=ENCODER_LAYERS, first_step=0):
     """Denoise the action chunk in `diffusion_noise` over `steps` Euler steps. `first_step > 0` resumes
-    after steps that were run separately (prologue included), see `Pi0Inference`."""
+    after steps that were run separately (prologue included), see `Pi0Inference`. A table that offers the loop as one
+    stage issues the same launches by that one call."""
     b = buffers
     master = b.get("diffusion_noise_f32")
+    if hasattr(ops, "decoder_steps"):
+        if first_step == 0:
+            ops.decoder_state_proj(b["observation_state_normalized"], weights["decoder_state_in_proj_w"],
+                                   weights["decoder_state_in_proj_b"], b["decoder_state_buf"])
+        if ops.decoder_steps(weights, b, encoder_seq_len, steps, layers, first_step):
+            return
     if first_step == 0:
         decoder_prologue(ops, weights, b)
     for step in range(first_step, steps):

@@ -214,6 +214,21 @@ int fvla_decoder_action_out_proj(const void* x, int x_is_f32, const void* weight
                                  int out_is_f32, void* mirror, void* norm_factor, int M, int N,
                                  int K, void* stream);
 
+/* Euler steps [first_step, steps) of one episode (pipeline.py:95-135, without the state projection) enqueued by ONE call:
+ * the same launches in the same order as the per-op calls above, issued from native code, so that a caller outside a
+ * CUDA graph is not bound by its own per-op overhead (93 launches per step). Pointers and sizes as in those calls; weights are
+ * the stacked checkpoint tensors. x is the fp32 residual stream (chunk + 1, 1024) with its bf16 copy x_shadow;
+ * noise is the bf16 chunk the loop starts from (first_step 0) and ends in, noise_f32 its fp32 master. ws_*: scratch of
+ * fvla_gemm_workspace_bytes / fvla_decoder_attention_workspace_bytes, one each. */
+struct fvla_decoder_steps {
+    const void *in_w, *time_bias, *mlp_w, *mlp_b, *qkv_w, *attn_o_w, *gate_w, *up_w, *down_w, *out_w, *out_b, *rope, *state;
+    void *noise, *noise_f32, *x, *x_shadow, *in_buf, *q, *hidden, *k_cache, *v_cache;
+    void *ws_mlp, *ws_qkv, *ws_attn, *ws_o, *ws_gate, *ws_down;
+    size_t ws_mlp_bytes, ws_qkv_bytes, ws_attn_bytes, ws_o_bytes, ws_gate_bytes, ws_down_bytes;
+    int chunk, prefix, cache_rows, first_step, steps, layers;
+};
+int fvla_decoder_steps_run(const struct fvla_decoder_steps* args, void* stream);
+
 /* No counterpart in the reference, where these are torch `copy_` calls inside the pipeline (pipeline.py:103,
  * engine.py:60): dst[i] = src[i] for `count` contiguous elements, each side bf16 or fp32; dst_shadow (may be
  * NULL; fp32 dst only) also receives the value as bf16. Keeps the small copies of the decoder step inside the
