@@ -347,8 +347,12 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
     } else if (warp == 1) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (lane == 0) {
+            // The issue loop is kept free of divisions and of descriptor arithmetic: ring position and parity are running
+            // values, a k16 step is an addition to the descriptors of the stage. One thread issues everything, and what it
+            // spends per stage beside the MMAs (46 clk each) adds to them as soon as the sum exceeds their run time.
             constexpr uint32_t idesc = instr_desc(BN);
-            uint32_t it = 0, tcount = 0;
+            const uint64_t adesc0 = smem_desc(smem_base, 16, 1024), bdesc0 = smem_desc(smem_base + Cfg::A_BYTES, Cfg::SLAB, 1024);
+            uint32_t s = 0, ph = 0, tcount = 0;
             for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tcount) {
                 const int acc = tcount & 1;
                 const uint32_t acc_ph = (tcount >> 1) & 1u;
@@ -357,23 +361,21 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                 const uint32_t d_tmem = tmem_base + acc * Cfg::ACC_COLS;
                 const int split = tile % args.splits;
                 const int kt_beg = split * args.k_per_split, kt_end = min(args.k_iters, kt_beg + args.k_per_split);
-                for (int kt = kt_beg; kt < kt_end; ++kt, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                uint32_t accumulate = 0;
+                for (int kt = kt_beg; kt < kt_end; ++kt) {
                     if (!mbar_wait(full_bar(s), ph, abort_flag)) goto mma_done;
                     tc_fence_after();
-                    if (it == 0) FVLA_STAMP_ANY(2);
-                    const uint32_t sA = smem_base + s * Cfg::STAGE_BYTES;
+                    if (tcount == 0 && kt == kt_beg) FVLA_STAMP_ANY(2);
+                    const uint64_t adesc = adesc0 + s * (Cfg::STAGE_BYTES >> 4), bdesc = bdesc0 + s * (Cfg::STAGE_BYTES >> 4);
 #pragma unroll
                     for (int k16 = 0; k16 < BK / 16; ++k16) {
-                        const uint64_t adesc = smem_desc(sA + k16 * 32, 16, 1024);
 #pragma unroll
-                        for (int nb = 0; nb < NB; ++nb) {
-                            const uint64_t bdesc = smem_desc(sA + Cfg::A_BYTES + nb * Cfg::B_BYTES + k16 * 2048, Cfg::SLAB, 1024);
-                            umma_bf16(d_tmem + nb * BN, adesc, bdesc, idesc, (kt > kt_beg || k16 > 0) ? 1u : 0u);
-                        }
+                        for (int nb = 0; nb < NB; ++nb)
+                            umma_bf16(d_tmem + nb * BN, adesc + k16 * 2, bdesc + nb * (Cfg::B_BYTES >> 4) + k16 * 128, idesc, k16 > 0 ? 1u : accumulate);
                     }
+                    accumulate = 1;
                     umma_commit(empty_bar(s));              // slot reusable once these MMAs have read it
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
                 umma_commit(accfull_bar(acc));              // accumulator complete
                 if (tcount == 0) FVLA_STAMP_ANY(3);

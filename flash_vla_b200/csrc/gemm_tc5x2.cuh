@@ -156,7 +156,9 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (lane == 0 && rank == 0) {
             constexpr uint32_t idesc = pair_idesc();
-            uint32_t it = 0, tcount = 0;
+            // (running ring position and descriptors: see the one-SM kernel)
+            const uint64_t adesc0 = smem_desc(smem_base, 16, 1024), bdesc0 = smem_desc(smem_base + 16384, 8192, 1024);
+            uint32_t s = 0, ph = 0, tcount = 0;
             for (int tile = pair; tile < num_tiles; tile += pairs, ++tcount) {
                 const int acc = tcount & 1;
                 const uint32_t acc_ph = (tcount >> 1) & 1u;
@@ -165,19 +167,17 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
                 const uint32_t d_tmem = tmem_base + acc * 256;
                 const int split = tile % args.splits;
                 const int kt_beg = split * args.k_per_split, kt_end = min(args.k_iters, kt_beg + args.k_per_split);
-                for (int kt = kt_beg; kt < kt_end; ++kt, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                uint32_t accumulate = 0;
+                for (int kt = kt_beg; kt < kt_end; ++kt) {
                     if (!mbar_wait(full_bar(s), ph, abort_flag)) goto mma_done;
                     tc_fence_after();
-                    const uint32_t sA = smem_base + s * STAGE_BYTES;
+                    const uint64_t adesc = adesc0 + s * (STAGE_BYTES >> 4), bdesc = bdesc0 + s * (STAGE_BYTES >> 4);
 #pragma unroll
-                    for (int k16 = 0; k16 < BK / 16; ++k16) {
-                        const uint64_t adesc = smem_desc(sA + k16 * 32, 16, 1024);
-                        const uint64_t bdesc = smem_desc(sA + 16384 + k16 * 2048, 8192, 1024);
-                        umma_bf16_pair(d_tmem, adesc, bdesc, idesc, (kt > kt_beg || k16 > 0) ? 1u : 0u);
-                    }
+                    for (int k16 = 0; k16 < BK / 16; ++k16)
+                        umma_bf16_pair(d_tmem, adesc + k16 * 2, bdesc + k16 * 128, idesc, k16 > 0 ? 1u : accumulate);
+                    accumulate = 1;
                     umma_commit_pair(empty_bar(s));
+                    if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
                 umma_commit_pair(accfull_bar(acc));
             }
