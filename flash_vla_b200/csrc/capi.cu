@@ -490,10 +490,11 @@ static int refresh_shadow(const void* src, void* dst, size_t count, cudaStream_t
 int fvla_linear_residual(const void* x, const void* weight, void* out, int out_is_f32, void* out_shadow, int M,
                          int N, int K, int group_rows, void* ws, size_t ws_bytes, void* stream) {
     FVLA_REQUIRE(group_rows >= 0 && (group_rows == 0 || M % group_rows == 0), "linear_residual: M=%d is not a whole number of groups of %d rows", M, group_rows);
-    // rows as several groups of at most 64 (a batch of episodes): the decoder's cluster GEMM once per group in
-    // one launch, each group streaming the weights from L2 after the first has pulled them from HBM
-    const int rows = group_rows > 0 ? group_rows : M, groups = group_rows > 0 ? M / group_rows : 1;
-    if (tc5_enabled() && skinny::plan_skinny(rows, N, K, false).ok && aligned16(x) && aligned16(weight)) {
+    // rows as several groups (a batch of episodes): the decoder's cluster GEMM once per group in one launch, each group
+    // streaming the weights from L2 after the first has pulled them from HBM. Up to 128 rows are one group whatever
+    // they are made of: one pass over the weights instead of several.
+    const int rows = group_rows > 0 && M > 128 ? group_rows : M, groups = M / rows;
+    if (tc5_enabled() && skinny::skinny_supports(rows, N, K, false, true) && aligned16(x) && aligned16(weight)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = 0; sa.ldx = K; sa.M = rows; sa.N = N; sa.K = K; sa.groups = groups;
         sa.out = out; sa.out_f32 = out_is_f32; sa.ldo = N; sa.out_shadow = Bm(out_shadow);
@@ -564,7 +565,7 @@ int fvla_decoder_small_proj(const void* x, int x_is_f32, const void* weight, con
         if (e != cudaSuccess) { set_error("small_k_proj_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
         return check_launch("small_k_proj_kernel");
     }
-    if (tc5_enabled() && skinny::plan_skinny(M, N, K, false).ok && aligned16(x) && aligned16(weight)) {
+    if (tc5_enabled() && skinny::skinny_supports(M, N, K, false, !x_is_f32) && aligned16(x) && aligned16(weight)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.ldx = K; sa.M = M; sa.N = N; sa.K = K;
         sa.out = out; sa.out_f32 = out_is_f32; sa.ldo = N; sa.bias = B(bias); sa.act = act;
@@ -607,11 +608,12 @@ int fvla_decoder_norm_qkv_rope(const void* x, int x_is_f32, const void* x_shadow
     const int N = (heads + 2) * head_dim;
     FVLA_REQUIRE(group_rows >= 0 && (group_rows == 0 || (M % group_rows == 0 && kv_group_pitch >= group_rows)),
                  "decoder_norm_qkv_rope: M=%d is not a whole number of sequences of %d rows (K/V pitch %d rows)", M, group_rows, kv_group_pitch);
-    if (group_rows == 0 && tc5_enabled() && skinny::plan_skinny(M, N, Kdim, false).ok && aligned16(x) && aligned16(weight_qkv) &&
+    if (tc5_enabled() && skinny::skinny_supports(M, N, Kdim, false, !x_is_f32 || x_shadow != nullptr) && aligned16(x) && aligned16(weight_qkv) &&
         head_dim % 2 == 0) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.x_shadow = B(x_shadow); sa.ldx = Kdim; sa.M = M; sa.N = N; sa.K = Kdim; sa.need_factor = 1;
         sa.rope = B(rope); sa.q = Bm(Q); sa.k = Bm(K); sa.v = Bm(V); sa.heads = heads; sa.head_dim = head_dim;
+        if (group_rows > 0) { sa.group_rows = group_rows; sa.kv_skip = kv_group_pitch - group_rows; sa.inv_group = ((1u << 20) + group_rows - 1) / group_rows; }
         sa.factor_out = Bm(norm_factor); sa.status = device_status_ptr(); FVLA_DBG_ATTACH(sa);
         return skinny::launch_skinny<skinny::EPI_QKV_ROPE>(sa, weight_qkv, nullptr, N, S(stream));
     }
@@ -677,7 +679,7 @@ int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* ou
 
 int fvla_decoder_norm_gated_ffn(const void* x, int x_is_f32, const void* x_shadow, const void* gate_w, const void* up_w, void* out,
                                 void* norm_factor, int M, int N, int K, void* ws, size_t ws_bytes, void* stream) {
-    if (tc5_enabled() && skinny::plan_skinny(M, N, K, true).ok && aligned16(x) && aligned16(gate_w) && aligned16(up_w)) {
+    if (tc5_enabled() && skinny::skinny_supports(M, N, K, true, !x_is_f32 || x_shadow != nullptr) && aligned16(x) && aligned16(gate_w) && aligned16(up_w)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.x_shadow = B(x_shadow); sa.ldx = K; sa.M = M; sa.N = N; sa.K = K; sa.need_factor = 1;
         sa.out = out; sa.out_f32 = 0; sa.ldo = N; sa.factor_out = Bm(norm_factor); sa.status = device_status_ptr(); FVLA_DBG_ATTACH(sa);

@@ -96,6 +96,7 @@ def allocate_batched_decoder_buffers(chunk_size: int, episodes: int, encoder_seq
     add("diffusion_noise_f32", E * chunk_size, ACTION_DIM, dtype=torch.float32)
     add("decoder_rope_weights", D, HEAD_DIM)
     add("decoder_x", E * D, DECODER_DIM, dtype=torch.float32)
+    add("decoder_x_bf16", E * D, DECODER_DIM)
     add("decoder_x_buf", E * chunk_size, DECODER_DIM)
     add("decoder_mlp_out", E * chunk_size, DECODER_DIM, dtype=torch.float32)
     add("decoder_x_rows", E * chunk_size, DECODER_DIM, dtype=torch.float32)

@@ -100,6 +100,8 @@ class Pi0Inference:
             self.prefix_pool = ScratchPool()
         if self.batch_decoder:
             self.decoder_buffers = allocate_batched_decoder_buffers(chunk_size, episodes, self.encoder_seq_len, device)
+            if episodes * (chunk_size + 1) <= 128:        # few enough rows for the weight-streaming GEMM, which reads bf16 rows
+                wrappers.register_bf16_shadow(self.decoder_buffers["decoder_x"], self.decoder_buffers["decoder_x_bf16"])
             self.decoder_pool = ScratchPool()
             self.pools = [self.decoder_pool]
             self._batched_observation_state_normalized = self.decoder_buffers["observation_state_normalized"]

@@ -166,6 +166,8 @@ def decoder_step_batched(ops, weights, prefix, dec, encoder_seq_len, step, episo
                                w["decoder_action_fused_time_biases"][step % DIFFUSION_STEPS], dec["decoder_x_buf"])
     ops.decoder_action_mlp(dec["decoder_x_buf"], w["decoder_action_mlp_w"], w["decoder_action_mlp_b"], dec["decoder_mlp_out"])
     x3[:, 1:].copy_(dec["decoder_mlp_out"].view(E, D - 1, x.shape[1]))
+    if hasattr(ops, "sync_shadow"):
+        ops.sync_shadow(x)
     for layer in range(layers):
         k_all, v_all = prefix["encoder_K"][:, layer], prefix["encoder_V"][:, layer]      # (E, S + D, 256) views
         if before_layer is not None:

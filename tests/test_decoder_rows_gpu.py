@@ -1,0 +1,58 @@
+"""The decoder's cluster GEMM beyond 64 rows (128 token slots): the edges of its range, one sequence and several."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from conftest import assert_close
+from oracle import pi0_ref as O
+
+pytestmark = pytest.mark.gpu
+bf16 = torch.bfloat16
+
+
+def rnd(gen, *shape, scale=1.0):
+    return (torch.randn(*shape, generator=gen) * scale).to(bf16)
+
+
+# 64 | 65: the last shape of 64 slots and the first of 128; 102 = two episodes of 51; 128: every slot a row
+@pytest.mark.parametrize("M,group", [(64, 0), (65, 0), (102, 51), (120, 8), (128, 64)])
+def test_decoder_gemms_by_row_count(M, group):
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib, wrappers
+    ops, ref_ops = op_table(False), O.op_table(False)
+    g = torch.Generator().manual_seed(M)
+    x32 = torch.randn(M, 1024, generator=g) * 3.0
+    x = x32.cuda()
+    shadow = torch.zeros(M, 1024, dtype=bf16, device="cuda")
+    wrappers.register_bf16_shadow(x, shadow)
+    xr = x32.to(bf16).float()
+
+    D, E, S = group or M, M // (group or M), 24
+    w, rope = rnd(g, 1024, 2560, scale=0.02), O.rope_table(D, S)
+    cache = torch.zeros(2, E, S + D, 256, dtype=bf16, device="cuda")
+    Q, nf = torch.zeros(M * 8, 256, dtype=bf16, device="cuda"), torch.zeros(M, dtype=bf16, device="cuda")
+    K, V = (c[:, S:] if group else c[0, S:] for c in cache)
+    ops.decoder_norm_qkv_rope(x, w.cuda(), rope.cuda(), Q, K, V, nf)
+    for e in range(E):
+        refs = [torch.zeros(D * 8, 256), torch.zeros(D, 256), torch.zeros(D, 256), torch.zeros(D)]
+        ref_ops.decoder_norm_qkv_rope(xr[e * D:(e + 1) * D], w.float(), rope.float(), *refs)
+        got = (Q.view(E, D * 8, 256)[e], cache[0, e, S:], cache[1, e, S:], nf[e * D:(e + 1) * D])
+        for a, b, what in zip(got, refs, "Q K V factor".split()):
+            assert_close(a, b, what=f"decoder_norm_qkv_rope.{what}, sequence {e}")
+    assert (cache[:, :, :S] == 0).all()
+
+    wg, wu = rnd(g, 1024, 4096, scale=0.02), rnd(g, 1024, 4096, scale=0.02)
+    ref, out = torch.zeros(M, 4096), torch.zeros(M, 4096, dtype=bf16, device="cuda")
+    ref_ops.decoder_norm_gated_ffn(xr, wg.float(), wu.float(), ref, torch.zeros(M))
+    ops.decoder_norm_gated_ffn(x, wg.cuda(), wu.cuda(), out, nf)
+    assert_close(out, ref, what="decoder_norm_gated_ffn")
+
+    for name, Kd in (("decoder_out_proj_residual", 2048), ("decoder_ffn_down_residual", 4096)):
+        a, w2 = rnd(g, M, Kd), rnd(g, Kd, 1024, scale=0.02)
+        ref = x.cpu().clone()
+        getattr(ref_ops, name)(a.float(), w2.float(), ref)
+        getattr(ops, name)(a.cuda().view(E, D, Kd) if group else a.cuda(), w2.cuda(), x.view(E, D, 1024) if group else x)
+        assert_close(x, ref, what=name)
+        assert torch.equal(shadow, x.to(bf16)), name
+    assert _lib.load().fvla_device_status(None) == 0
