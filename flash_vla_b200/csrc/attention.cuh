@@ -273,22 +273,24 @@ inline int launch_attention(const AttnArgs& a, dim3 grid, cudaStream_t st) {
 
 
 // ---------------------------------------------------------------------------------------------
-// Decoder attention in one launch: keys split over the CTAs of a thread-block cluster (8 for up to
-// 1024 keys, one more per further 128 keys, at most 11), partial results merged through distributed
-// shared memory (no partial buffers in global memory, no second kernel). Grid = (ceil(queries / 32),
-// splits), cluster (1, splits), 8 warps per CTA. Warp w works on
-// query rows 16 (w & 1) .. + 16 of the 32-row block, key block (w >> 1) & 1 of the CTA's <= 128 keys
-// and half (w >> 2) of the head dimension: it sums Q K^T over its 128 of the 256 dimensions, swaps
-// that partial 16 x 64 score tile with the warp holding the other half (both then own the full
-// scores and run the same softmax) and multiplies P with its 128 columns of V. The two key blocks are
-// merged in shared memory, the normalised 32 x 256 partial and its log-sum-exp are staged, and rank
-// r < 8 receives rows 4r .. 4r+3 from all ranks by bulk copy, combines them with log-sum-exp weights
-// in rank order and writes bf16.
+// Decoder attention in one launch: a cluster of 4 to 11 CTAs has 32 flat query rows (4 tokens x 8 heads) and shares out
+// the keys: every CTA takes an equal part of the prefix and of the step's own keys. Both products run on tcgen05 with the
+// KEYS (then the head dimensions) as the 128-row operand and the query rows as N = 32:
+//   S^T = K Q^T   one or two key tiles, accumulator lane = key, column = query row;
+//   softmax       thread = one key x 16 rows; row maxima and sums by a halving butterfly (16 shuffles for 16 rows), the
+//                 four 32-key quadrants meet in shared memory; P goes to shared memory as the next operand;
+//   O^T = V^T P^T two 128-dim tiles, accumulator lane = dim, column = query row.
+// A thread's accumulator column then IS what an owner of 4 rows needs from it: it goes straight from registers to the owners'
+// shared memory (st.async, 16 bytes = 4 rows of one dim), over the K tile, which nobody reads any more. Owners
+// weight the parts by log-sum-exp in rank order and write bf16.
+// Measured at 51 rows x 819 keys inside the decoder's chain: 5.9 us per launch, against 7.8 us for the warp-level form that this
+// replaced (mma.sync on 8 warps, 64-key halves merged and staged in shared memory, bulk copies). What bounds it is a chain of
+// latencies: dependency wait 0.9, Q 0.7, S^T 0.6, softmax and O^T 1.6, exchange 1.2 (28 KB per CTA; distributed shared memory
+// moves 16 B/clk per SM when all SMs send), combine 0.7; DRAM and the tensor pipes idle.
 // ---------------------------------------------------------------------------------------------
 struct DecAttnArgs {
     const bf16* q; const bf16* k; const bf16* v; bf16* out;
-    int nq, nk, keys_per_split;
-    int splits;                 // cluster size: CTAs sharing the keys of one 32-row query block (8..11)
+    int nq, nk;
     // a batch of independent episodes (grid.z): element offsets between consecutive episodes' Q / out rows
     // and between their K / V caches; nq and nk are per episode
     long long q_episode_stride, kv_episode_stride;
@@ -296,33 +298,72 @@ struct DecAttnArgs {
     float scale_log2;
     int mask_rows, mask_key_le;
     int prefix_keys;            // keys [0, prefix_keys) were not written by the preceding kernel
+    // plan
+    int splits;                 // cluster size
+    int kp, nd;                 // prefix keys and own keys per CTA
+    int pad;                    // rows of a CTA's K / V tile: kp + nd rounded up to 16
+    int k_region;               // bytes of the K tile, or of the receive area that takes its place if that is larger
     int* status;
     FVLA_DBG_MEMBER
 };
 
 namespace decattn {
-constexpr int HD = 256, BQ = 32, MIN_SPL = 8, MAX_SPL = 11, PITCH = HD * 2 + 16, CH = HD / 8, THREADS = 256;
-constexpr int OP = HD + 8;                          // fp32 row pitch of the merge / staging buffers: rows 8 banks apart
-constexpr int SLICE = 4 * OP * 4;                   // bytes of the 4 staged rows one owner receives from one rank
-// K and V tiles: 128 keys x 256 dims as four 64-dim blocks of [128 rows][128 bytes] in the 128-byte swizzle a tensor
-// load writes (16-byte piece c of row r at piece c ^ (r & 7): eight consecutive keys of one piece sit in eight
-// different bank groups, which is what ldmatrix wants); the tiles lead the buffer so that they are 1 KB aligned.
-// Q keeps the padded row pitch.
-constexpr int Q_BYTES = BQ * PITCH, KV_BYTES = 128 * HD * 2, KV_BLOCK = 128 * 128;
-constexpr int OFF_K = 0, OFF_V = OFF_K + KV_BYTES, OFF_Q = OFF_V + KV_BYTES;
-constexpr int OFF_SX = OFF_Q + Q_BYTES;                                                  // score swap: [warp 8][32][lane 32] fp32
-constexpr int OFF_BAR = OFF_SX + 8 * 32 * 32 * 4;
-constexpr int OFF_RED = OFF_BAR + 64;                                                    // RED: [src spl][4 rows][OP] fp32, then LSE_IN [src spl][4] fp32
-constexpr int smem_bytes(int spl) { return 1024 + OFF_RED + spl * (SLICE + 16); }      // 1 KB of slack to align the tiles
-// shared-memory address of 16-byte piece `piece` (0..31) of row `row` of a K / V tile
-__device__ __forceinline__ uint32_t kv_piece(uint32_t tile, int row, int piece) {
-    return tile + (uint32_t)(piece >> 3) * KV_BLOCK + (uint32_t)row * 128u + (uint32_t)(((piece & 7) ^ (row & 7)) << 4);
+constexpr int HD = 256, BQ = 32, UNIT = 4, MIN_SPL = 4, MAX_SPL = 11, THREADS = 256;
+constexpr int S_COL = 64;                           // TMEM columns: O^T at 0 and 32; S^T at S_COL + 64 tile + 32 (half of the dims)
+constexpr int MAX_PAD = 208;                        // K + V tiles of 208 rows, Q / P and the rest just fit the SM
+constexpr int QP_BYTES = 16384;                     // Q: 4 blocks of 64 dims x 32 rows; later P: up to 4 blocks of 64 keys x 32 rows
+constexpr int UNIT_BYTES = HD * UNIT * 4;           // what one CTA sends for four rows
+constexpr int OFF_PART = 64;                        // behind the barriers: row maxima, then sums, per (row half, quadrant, 16 rows)
+constexpr int OFF_MAX = OFF_PART + 1024, OFF_STATS = OFF_MAX + 128;        // this CTA's row maxima; received (max, sum): [src][slot 2][row 4]
+constexpr int MISC_BYTES = OFF_STATS + MAX_SPL * 64;
+constexpr float NO_KEY = -1e30f;                    // maximum of a row that sees none of a CTA's keys: its weight in the merge is 0
+constexpr int units_per_owner(int spl) { return (BQ / UNIT + spl - 1) / spl; }
+inline int k_region_bytes(int spl, int pad) {
+    const int recv = spl * units_per_owner(spl) * UNIT_BYTES;
+    return pad * 512 > recv ? pad * 512 : recv;
 }
-static_assert(smem_bytes(MAX_SPL) <= 227 * 1024, "the largest cluster's receive buffers must fit in shared memory");
-// staging areas alias K (half-merge buffer) and V (final partial) once the MMAs are done
-constexpr int OFF_HALF = OFF_K;                    // [32 rows][OP] fp32 + m[32] + l[32]
-constexpr int OFF_STAGE = OFF_V;                   // [32 rows][OP] fp32 + lse[32]
-static_assert(BQ * OP * 4 + 256 <= KV_BYTES, "merge buffers must fit in the K / V tiles they alias");
+inline int smem_bytes(int spl, int pad) { return 1024 + k_region_bytes(spl, pad) + pad * 512 + QP_BYTES + MISC_BYTES; }
+
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) { return tc5::mbar_wait(bar, parity, abort_flag); }
+__device__ __forceinline__ uint32_t idesc(bool a_mn) { return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | ((uint32_t)(BQ >> 3) << 17) | (8u << 24); }
+
+// Reduce 16 values per lane over the 32 lanes of a warp: each step sends away the half of the values that the lane will not
+// keep, so 16 rows take 16 shuffles. Afterwards lanes 2 k and 2 k + 1 hold row k.
+template <typename Op>
+__device__ __forceinline__ float butterfly16(float (&v)[16], int lane, Op op) {
+#pragma unroll
+    for (int half = 8; half >= 1; half >>= 1) {
+        const bool up = lane & (2 * half);
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+            v[i] = op(keep, __shfl_xor_sync(0xffffffffu, send, 2 * half));
+        }
+    }
+    return op(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float lds1(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts1(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts4u(uint32_t a, const uint4& v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void sts_bf16(uint32_t a, float v) {
+    asm volatile("st.shared.b16 [%0], %1;" ::"r"(a), "h"(__bfloat16_as_ushort(__float2bfloat16_rn(v))) : "memory");
+}
 }  // namespace decattn
 
 __device__ __forceinline__ uint32_t dsm_map(uint32_t local_addr, uint32_t rank) {
@@ -331,328 +372,334 @@ __device__ __forceinline__ uint32_t dsm_map(uint32_t local_addr, uint32_t rank) 
     return r;
 }
 
+template <int KT>                                         // key tiles of 128 per CTA
 __global__ void __launch_bounds__(decattn::THREADS, 1)
-decoder_attention_cluster_kernel(const DecAttnArgs p, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV) {
+decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV) {
     using namespace decattn;
+    constexpr int S_ISSUERS = 2 * KT, TMEM_COLS = KT == 1 ? 128 : 256;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* smem = smem_raw + (sbase - smem_u32(smem_raw));
-    const uint32_t sQ = sbase + OFF_Q, sK = sbase + OFF_K, sV = sbase + OFF_V;
-    const uint32_t in_bar = sbase + OFF_BAR;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_BAR + 16);
-    const int SPL = p.splits;
-    const int OFF_LSE_IN = OFF_RED + SPL * SLICE;
+    const uint32_t sK = (smem_u32(smem_raw) + 1023u) & ~1023u, sV = sK + p.k_region, sQ = sV + p.pad * 512, misc = sQ + QP_BYTES;
+    uint8_t* gmisc = smem_raw + (misc - smem_u32(smem_raw));
+    const uint32_t pre_bar = misc, in_bar = misc + 8, s_bar = misc + 16, o_bar = misc + 24;
+    const uint32_t part = misc + OFF_PART, row_max = misc + OFF_MAX, stats_in = misc + OFF_STATS;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gmisc + 32);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gmisc + 36);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     FVLA_DBG_CTA(p, (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
     FVLA_STAMP(0);
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    const bf16* gq = p.q + (size_t)blockIdx.z * p.q_episode_stride;
-    const bf16* gk = p.k + (size_t)blockIdx.z * p.kv_episode_stride;
-    const bf16* gv = p.v + (size_t)blockIdx.z * p.kv_episode_stride;
-    bf16* gout = p.out + (size_t)blockIdx.z * p.q_episode_stride;
-    const int q0 = blockIdx.x * BQ;
-    const int key_beg = (int)rank * p.keys_per_split;
-    const int key_end = min(p.nk, key_beg + p.keys_per_split);
-    const int rows_here = min(BQ, p.nq - q0);
-    const int owners = (rows_here + 3) / 4;                  // at most 8: ranks beyond that only send
-    const bool i_own = (int)rank < owners;
+    const int SPL = p.splits, q0 = blockIdx.x * BQ, rows_here = min(BQ, p.nq - q0), units = (rows_here + UNIT - 1) / UNIT;
+    const float scale = p.scale_log2;
+    const int pre_rows = min(p.prefix_keys, p.nk);
+    const int key0 = (int)rank * p.kp, prefix_here = max(0, min(p.kp, pre_rows - key0));        // local keys [0, prefix_here): prefix
+    const int new0 = (int)rank * p.nd, new_here = max(0, min(p.nd, p.nk - pre_rows - new0));    // then new_here of the step's own
+    const int owned = (int)rank < units ? 1 + ((int)rank + SPL < units ? 1 : 0) : 0;            // units rank, rank + SPL
 
-    // Prefix keys were written long before the preceding kernel: fetch them while it finishes. Rows
-    // past the end (keys of the ragged last split, queries of the last block) must read as zero.
-    const int pre_end = min(key_end, p.prefix_keys);
-    const uint32_t pre_bar = sbase + OFF_BAR + 24;
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(in_bar) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pre_bar) : "memory");
+        tc5::mbar_init(pre_bar, 1);
+        tc5::mbar_init(in_bar, 1);
+        tc5::mbar_init(s_bar, S_ISSUERS);
+        tc5::mbar_init(o_bar, 2);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (i_own)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(in_bar), "r"(SPL * (SLICE + 16)) : "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(pre_bar), "r"(2 * KV_BYTES) : "memory");      // whole boxes, zero fill included
-    }
-    // relaxed: the fence above already published the barrier to the cluster
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-
-    // The prefix K and V rows (almost all of the tile) arrive as four tensor loads per tile (64 dims x 128 keys each)
-    // through maps that END at the prefix: the rows behind it, which the preceding kernel is still writing, are
-    // not touched in memory and read as zero. Eight copy requests per CTA, which is what a CTA that could only
-    // start after the previous kernel left its SM waits for.
-    auto bounded_wait = [&](uint32_t bar) {
-        for (uint32_t i = 0; i < (1u << 22); ++i) {
-            uint32_t done;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                         : "=r"(done) : "r"(bar), "r"(0) : "memory");
-            if (done) return;
-            if ((i & 1023u) == 1023u && *abort_flag) return;
-        }
-        *abort_flag = 1;
-    };
-    __syncthreads();                                           // the barriers are initialised
-    if (tid == 0) {
+        if (owned > 0) tc5::mbar_expect_tx(in_bar, (uint32_t)(owned * SPL) * (UNIT_BYTES + UNIT * 8));
+        // The prefix rows of K and V arrive as one box of 64 dims x pad rows per block, through maps that END at the prefix:
+        // the rows behind it, which the preceding kernel may still be writing, are not touched in memory and read as
+        // zero. (Rows past prefix_here hold the next CTA's keys; the own keys overwrite some, the rest is masked.)
+        tc5::mbar_expect_tx(pre_bar, 2u * p.pad * 512u);
 #pragma unroll
-        for (int cb = 0; cb < HD / 64; ++cb) {
-            tc5::tma_load_3d(sK + cb * KV_BLOCK, &tmK, pre_bar, cb * 64, key_beg, blockIdx.z);
-            tc5::tma_load_3d(sV + cb * KV_BLOCK, &tmV, pre_bar, cb * 64, key_beg, blockIdx.z);
-        }
+        for (int cb = 0; cb < HD / 64; ++cb) tc5::tma_load_3d(sK + cb * p.pad * 128, &tmK, pre_bar, cb * 64, key0, blockIdx.z);
+#pragma unroll
+        for (int cb = 0; cb < HD / 64; ++cb) tc5::tma_load_3d(sV + cb * p.pad * 128, &tmV, pre_bar, cb * 64, key0, blockIdx.z);
     }
-    // (Rows of the tile past this split's last key hold the next split's keys, or zeros past the prefix: their
-    // scores are masked below and their probabilities are zero, so they need no clearing.)
-    for (int idx = tid; idx < BQ * CH; idx += THREADS) {
-        int r = idx / CH, c = idx % CH;
-        if (q0 + r >= p.nq) *reinterpret_cast<uint4*>(smem + OFF_Q + r * PITCH + c * 16) = make_uint4(0, 0, 0, 0);
+    if (warp == 1) {
+        tc5::tmem_alloc(misc + 32, TMEM_COLS);
+        tc5::tmem_relinquish();
     }
+    tc5::tc_fence_before();
+    __syncthreads();
+    tc5::tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     FVLA_STAMP(1);
-    // What the preceding kernel wrote (Q, and the new keys in the last split) is small and is what every CTA
-    // waits for next: 16-byte async copies reach shared memory sooner than a bulk copy does (about 1.0 us
-    // against 1.4 us from request to data), so they keep the old path.
+    // What the preceding kernel wrote, Q and the own keys, comes through registers: plain 16-byte loads reach them sooner than
+    // any bulk copy reaches shared memory. Both land in the swizzled operand layout (piece c of row r at c ^ (r & 7)).
     {
-        const int post_lo = max(key_beg, pre_end);
-        for (int idx = tid; idx < BQ * CH; idx += THREADS) {
-            const int r = idx / CH, c = idx % CH;
-            if (q0 + r < p.nq) cp_async16(sQ + r * PITCH + c * 16, gq + (size_t)(q0 + r) * HD + c * 8, 16);
+        const bf16* gq = p.q + (size_t)blockIdx.z * p.q_episode_stride + (size_t)q0 * HD;
+        const size_t kv0 = (size_t)blockIdx.z * p.kv_episode_stride + (size_t)(pre_rows + new0) * HD;
+        constexpr int QV = BQ * 32 / THREADS;
+        uint4 qv[QV];
+#pragma unroll
+        for (int i = 0; i < QV; ++i) {
+            const int idx = tid + i * THREADS;
+            qv[i] = idx < rows_here * 32 ? *reinterpret_cast<const uint4*>(gq + (size_t)idx * 8) : make_uint4(0, 0, 0, 0);
         }
-        cp_async_commit();
-        if (post_lo < key_end) {
-            // the new keys land on rows the tensor loads zero-filled: wait for those loads first
-            bounded_wait(pre_bar);
-            for (int idx = tid; idx < 128 * CH; idx += THREADS) {
-                const int r = idx / CH, c = idx % CH, g = key_beg + r;
-                if (g >= post_lo && g < key_end) {
-                    cp_async16(kv_piece(sK, r, c), gk + (size_t)g * HD + c * 8, 16);
-                    cp_async16(kv_piece(sV, r, c), gv + (size_t)g * HD + c * 8, 16);
-                }
+        uint4 kvv[2];                                        // first batch of own rows: 8 rows of K and V
+        const int total = new_here * 32;
+        if (tid < total) {
+            kvv[0] = *reinterpret_cast<const uint4*>(p.k + kv0 + (size_t)tid * 8);
+            kvv[1] = *reinterpret_cast<const uint4*>(p.v + kv0 + (size_t)tid * 8);
+        }
+#pragma unroll
+        for (int i = 0; i < QV; ++i) {
+            const int idx = tid + i * THREADS, r = idx >> 5, c = idx & 31;
+            sts4u(sQ + (c >> 3) * (BQ * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), qv[i]);
+        }
+        wait(pre_bar, 0, abort_flag);                        // the own rows go over what the boxes brought in
+        for (int idx = tid; idx < total; idx += THREADS) {
+            if (idx != tid) {
+                kvv[0] = *reinterpret_cast<const uint4*>(p.k + kv0 + (size_t)idx * 8);
+                kvv[1] = *reinterpret_cast<const uint4*>(p.v + kv0 + (size_t)idx * 8);
             }
-            cp_async_commit();
-        }
-        cp_async_wait<0>();
-    }
-    bounded_wait(pre_bar);
-    __syncthreads();
-    FVLA_STAMP(2);
-
-    const int rg = warp & 1, kh = (warp >> 1) & 1, dh = warp >> 2;
-    const int row_lo = q0 + rg * 16 + (lane >> 2);
-    float o[HD / 16][4];                               // this warp's 128 output columns
-    float m_run[2], l_run[2];
-    {
-        const int kv_row0 = kh * 64;                       // this warp's half of the tile's keys
-        float s[8][4];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f; }
-#pragma unroll
-        for (int k8 = 0; k8 < HD / 32; ++k8) {
-            const int kk = dh * (HD / 32) + k8;
-            uint32_t a[4];
-            ldmatrix_x4(a, sQ + (rg * 16 + (lane & 15)) * PITCH + (kk * 2 + (lane >> 4)) * 16);
-#pragma unroll
-            for (int nj = 0; nj < 4; ++nj) {
-                uint32_t b[4];
-                int key = nj * 16 + (lane & 7) + (lane >> 4) * 8;
-                ldmatrix_x4(b, kv_piece(sK, kv_row0 + key, kk * 2 + ((lane >> 3) & 1)));
-                mma_bf16_16816(s[2 * nj], a, b[0], b[1]);
-                mma_bf16_16816(s[2 * nj + 1], a, b[2], b[3]);
-            }
-        }
-        // Swap partial scores with the warp that summed the other half of the head dimension (same rows,
-        // same keys, hence the same fragment layout: element j of lane l pairs with element j of lane l).
-        {
-            float* sx = reinterpret_cast<float*>(smem + OFF_SX);
-            float* mine = sx + warp * 1024;
-            const float* theirs = sx + (warp ^ 4) * 1024;
-#pragma unroll
-            for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) mine[(ni * 4 + e) * 32 + lane] = s[ni][e];
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
-#pragma unroll
-            for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[ni][e] += theirs[(ni * 4 + e) * 32 + lane];
-        }
-        const int kbase = key_beg + kh * 64;
-        float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-        for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                int key = kbase + ni * 8 + (lane & 3) * 2 + (e & 1);
-                int row = row_lo + (e >> 1) * 8;
-                bool keep = key < key_end && (row >= p.mask_rows || key <= p.mask_key_le);
-                float v = keep ? s[ni][e] * p.scale_log2 : -INFINITY;
-                s[ni][e] = v;
-                mx[e >> 1] = fmaxf(mx[e >> 1], v);
-            }
-        float psum[2] = {0.f, 0.f}, m_use[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-            m_use[h] = mx[h] == -INFINITY ? 0.f : mx[h];
-            m_run[h] = mx[h];
-        }
-#pragma unroll
-        for (int ni = 0; ni < 8; ++ni)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float pv = exp2f(s[ni][e] - m_use[e >> 1]);
-                s[ni][e] = pv;
-                psum[e >> 1] += pv;
-            }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            psum[h] += __shfl_xor_sync(0xffffffffu, psum[h], 1);
-            psum[h] += __shfl_xor_sync(0xffffffffu, psum[h], 2);
-            l_run[h] = psum[h];
-        }
-#pragma unroll
-        for (int i = 0; i < HD / 16; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            uint32_t a[4];
-            a[0] = pack_bf16x2(s[2 * kk][0], s[2 * kk][1]);
-            a[1] = pack_bf16x2(s[2 * kk][2], s[2 * kk][3]);
-            a[2] = pack_bf16x2(s[2 * kk + 1][0], s[2 * kk + 1][1]);
-            a[3] = pack_bf16x2(s[2 * kk + 1][2], s[2 * kk + 1][3]);
-#pragma unroll
-            for (int dl = 0; dl < HD / 32; ++dl) {
-                const int dj = dh * (HD / 32) + dl;
-                uint32_t b[4];
-                int key = kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-                ldmatrix_x4_trans(b, kv_piece(sV, kv_row0 + key, dj * 2 + (lane >> 4)));
-                mma_bf16_16816(o[2 * dl], a, b[0], b[1]);
-                mma_bf16_16816(o[2 * dl + 1], a, b[2], b[3]);
-            }
-        }
-    }
-    __syncthreads();                                   // K and V are dead from here on
-    FVLA_STAMP(3);
-
-    float* half_o = reinterpret_cast<float*>(smem + OFF_HALF);            // [32][OP]
-    float* half_ml = half_o + BQ * OP;                                      // m[32], l[32]
-    float* stage_o = reinterpret_cast<float*>(smem + OFF_STAGE);          // [32][OP]
-    float* stage_lse = stage_o + BQ * OP;                                   // [32]
-    const int r_in_blk = rg * 16 + (lane >> 2);
-    const int c_base = dh * (HD / 2) + (lane & 3) * 2;                      // column of o[i][0]: c_base + 8 i
-    if (kh == 1) {
-#pragma unroll
-        for (int i = 0; i < HD / 16; ++i)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float2*>(half_o + (r_in_blk + h * 8) * OP + c_base + i * 8) = make_float2(o[i][2 * h], o[i][2 * h + 1]);
-        if (dh == 0 && (lane & 3) == 0) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                half_ml[r_in_blk + h * 8] = m_run[h];
-                half_ml[BQ + r_in_blk + h * 8] = l_run[h];
-            }
-        }
-    }
-    __syncthreads();
-    if (kh == 0) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = r_in_blk + h * 8;
-            const float m1 = half_ml[r], l1 = half_ml[BQ + r];
-            const float mn = fmaxf(m_run[h], m1);
-            const float mu = mn == -INFINITY ? 0.f : mn;
-            const float a0 = exp2f(m_run[h] - mu), a1 = exp2f(m1 - mu);      // exp2(-inf) = 0
-            const float l = l_run[h] * a0 + l1 * a1;
-            const float inv = l > 0.f ? 1.0f / l : 0.f;
-#pragma unroll
-            for (int i = 0; i < HD / 16; ++i) {
-                const int c = c_base + i * 8;
-                const float2 o1 = *reinterpret_cast<const float2*>(half_o + r * OP + c);
-                *reinterpret_cast<float2*>(stage_o + r * OP + c) =
-                    make_float2((o[i][2 * h] * a0 + o1.x * a1) * inv, (o[i][2 * h + 1] * a0 + o1.y * a1) * inv);
-            }
-            if (dh == 0 && (lane & 3) == 0) stage_lse[r] = l > 0.f ? mn + log2f(l) : -INFINITY;
+            const int r = prefix_here + (idx >> 5), c = idx & 31;
+            const uint32_t at = (c >> 3) * p.pad * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+            sts4u(sK + at, kvv[0]);
+            sts4u(sV + at, kvv[1]);
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    FVLA_STAMP(4);
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");     // peers' barriers are initialised
-    if (tid == 0) {
-        for (int r = 0; r < owners; ++r) {
-            const uint32_t bar_r = dsm_map(in_bar, (uint32_t)r);
-            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(dsm_map(sbase + OFF_RED + rank * SLICE, (uint32_t)r)),
-                           "r"(sbase + OFF_STAGE + r * SLICE), "r"(SLICE), "r"(bar_r) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(dsm_map(sbase + OFF_LSE_IN + rank * 16, (uint32_t)r)),
-                           "r"(sbase + OFF_STAGE + BQ * OP * 4 + r * 16), "r"(16), "r"(bar_r) : "memory");
-        }
+    FVLA_STAMP(2);
+    // Issuing threads: for S^T one per key tile and half of the head dimension (accumulators added below), for O^T one per 128
+    // dims. A thread needs 46 clk per MMA and more for the first, the tensor pipe 39.
+    if (lane == 0 && warp < S_ISSUERS) {
+        tc5::tc_fence_after();
+        const int t = warp >> 1, h = warp & 1;
+        const uint64_t a0 = tc5::smem_desc(sK + t * 128 * 128 + h * p.pad * 256, 16, 1024), b0 = tc5::smem_desc(sQ + h * (BQ * 256), 16, 1024);
+#pragma unroll
+        for (int cb = 0; cb < 2; ++cb)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                tc5::umma_bf16(tmem + S_COL + warp * 32, a0 + cb * (p.pad * 8) + k * 2, b0 + cb * (BQ * 8) + k * 2, idesc(false), (cb | k) ? 1u : 0u);
+        tc5::umma_commit(s_bar);
     }
-    if (i_own) {
-        bool ok = false;
-        for (uint32_t i = 0; i < (1u << 24); ++i) {
-            uint32_t done;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                         : "=r"(done) : "r"(in_bar), "r"(0) : "memory");
-            if (done) { ok = true; break; }
-        }
-        if (!ok) *abort_flag = 1;
-        FVLA_STAMP(5);
-        const float* red = reinterpret_cast<const float*>(smem + OFF_RED);
-        const float* lse_in = reinterpret_cast<const float*>(smem + OFF_LSE_IN);
-        const int r4 = tid >> 6, c4 = (tid & 63) * 4;
-        const int row = q0 + (int)rank * 4 + r4;
-        if (ok && row < p.nq) {
-            float mx = -INFINITY;
-            for (int s = 0; s < SPL; ++s) mx = fmaxf(mx, lse_in[s * 4 + r4]);
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            float wsum = 0.f;
-#pragma unroll 4
-            for (int s = 0; s < SPL; ++s) {
-                const float l = lse_in[s * 4 + r4];
-                const float w = l == -INFINITY ? 0.f : exp2f(l - mx);
-                wsum += w;
-                const float4 v0 = *reinterpret_cast<const float4*>(red + (s * 4 + r4) * OP + c4);
-                acc[0] += w * v0.x; acc[1] += w * v0.y; acc[2] += w * v0.z; acc[3] += w * v0.w;
+    __syncwarp();
+    wait(s_bar, 0, abort_flag);
+    __syncwarp();
+    tc5::tc_fence_after();
+    // This CTA's MMAs have read its K tile: the peers may send into it (the matching wait stands before the first send). Relaxed:
+    // no data is handed over, and a releasing arrive waits 0.4 us for the thread's earlier accesses.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    FVLA_STAMP(3);
+    const int quad = warp & 3, half = warp >> 2;             // keys 32 quad .. + 31 of a tile, rows 16 half .. + 15
+    {
+        float v[KT][16], red[16];
+#pragma unroll
+        for (int t = 0; t < KT; ++t) {
+            const uint32_t at = tmem + S_COL + t * 64 + half * 16 + ((uint32_t)(quad * 32) << 16);
+            tc5::tmem_ld16(at, v[t]);
+            tc5::tmem_ld16(at + 32, red);
+            const int key = t * 128 + quad * 32 + lane;
+            const bool see = key < prefix_here + new_here;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[t][i] = see ? (v[t][i] + red[i]) * scale : -INFINITY;
+            // the state token's rows (the first of the sequence) see keys up to mask_key_le only
+            if (q0 + half * 16 < p.mask_rows && key >= prefix_here && pre_rows + new0 + key - prefix_here > p.mask_key_le) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (q0 + half * 16 + i < p.mask_rows) v[t][i] = -INFINITY;
             }
-            const float inv = wsum > 0.f ? 1.0f / wsum : 0.f;
-            *reinterpret_cast<uint2*>(gout + (size_t)row * HD + c4) =
-                make_uint2(pack_bf16x2(acc[0] * inv, acc[1] * inv), pack_bf16x2(acc[2] * inv, acc[3] * inv));
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) red[i] = KT == 1 ? v[0][i] : fmaxf(v[0][i], v[KT - 1][i]);
+        const float m = butterfly16(red, lane, [](float a, float b) { return fmaxf(a, b); });
+        if ((lane & 1) == 0) sts1(part + ((half * 4 + quad) * 16 + (lane >> 1)) * 4, fmaxf(m, NO_KEY));
+        __syncthreads();
+        float mx[16];
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+            float4 a = lds4(part + (half * 64 + i) * 4);
+#pragma unroll
+            for (int qd = 1; qd < 4; ++qd) {
+                const float4 b = lds4(part + (half * 64 + qd * 16 + i) * 4);
+                a.x = fmaxf(a.x, b.x); a.y = fmaxf(a.y, b.y); a.z = fmaxf(a.z, b.z); a.w = fmaxf(a.w, b.w);
+            }
+            mx[i] = a.x; mx[i + 1] = a.y; mx[i + 2] = a.z; mx[i + 3] = a.w;
+        }
+        if (quad == 0 && lane == 0) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) sts1(row_max + (half * 16 + i) * 4, mx[i]);
+        }
+#pragma unroll
+        for (int t = 0; t < KT; ++t) {
+            const int key = t * 128 + quad * 32 + lane;
+            // P over Q, whose readers are done; rows of a 64-key block are 128 bytes, 16-byte piece c of row r at c ^ (r & 7)
+            const uint32_t dst = sQ + (key >> 6) * (BQ * 128) + half * 16 * 128 + (key & 7) * 2, c = ((key & 63) >> 3) << 4;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float e = ex2(v[t][i] - mx[i]);
+                red[i] = t == 0 ? e : red[i] + e;
+                v[t][i] = e;
+            }
+            if (key < p.pad) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sts_bf16(dst + (c ^ ((i & 7) << 4)) + i * 128, v[t][i]);
+            }
+        }
+        tc5::tc_fence_before();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (lane == 0 && warp < 2) {
+            tc5::tc_fence_after();
+            const uint64_t a0 = tc5::smem_desc(sV + warp * 2 * p.pad * 128, p.pad * 128, 1024), b0 = tc5::smem_desc(sQ, 16, 1024);
+            for (int k = 0; k < p.pad / 16; ++k)
+                tc5::umma_bf16(tmem + warp * 32, a0 + k * 128, b0 + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true), k ? 1u : 0u);
+            tc5::umma_commit(o_bar);
+        }
+        __syncwarp();
+        const float l = butterfly16(red, lane, [](float a, float b) { return a + b; });
+        if ((lane & 1) == 0) sts1(part + 512 + ((half * 4 + quad) * 16 + (lane >> 1)) * 4, l);
+    }
+    __syncthreads();                                         // sums and maxima of all rows are in place
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < units * UNIT) {                                // row tid's (max, sum) to its owner
+        const int u = tid >> 2, owner = u % SPL, slot = u / SPL, h = tid >> 4, i = tid & 15;
+        const uint32_t pl = part + 512 + (h * 64 + i) * 4;
+        const float l = lds1(pl) + lds1(pl + 64) + lds1(pl + 128) + lds1(pl + 192);
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
+                     ::"r"(dsm_map(misc + OFF_STATS + rank * 64 + slot * 32 + (tid & 3) * 8, owner)), "f"(lds1(row_max + tid * 4)), "f"(l), "r"(dsm_map(in_bar, owner)) : "memory");
+    }
+    wait(o_bar, 0, abort_flag);
+    __syncwarp();
+    tc5::tc_fence_after();
+    FVLA_STAMP(4);
+    {
+        float o[32];
+        tc5::tmem_ld32(tmem + half * 32 + ((uint32_t)(quad * 32) << 16), o);                   // dim 128 half + 32 quad + lane
+        const uint32_t at = sK + rank * UNIT_BYTES + (half * 128 + quad * 32 + lane) * 16;
+#pragma unroll
+        for (int u = 0; u < BQ / UNIT; ++u) {
+            if (u >= units) break;
+            const int owner = u % SPL, slot = u / SPL;
+            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                         ::"r"(dsm_map(at + slot * SPL * UNIT_BYTES, owner)), "f"(o[4 * u]), "f"(o[4 * u + 1]), "f"(o[4 * u + 2]), "f"(o[4 * u + 3]),
+                           "r"(dsm_map(in_bar, owner)) : "memory");
         }
     }
-    // outgoing copies read this CTA's staging area: stay until every owner has everything
-    // (execution barrier only; nothing read after it was written by a peer)
+    tc5::tc_fence_before();
+    if (owned > 0) wait(in_bar, 0, abort_flag);
+    __syncwarp();
+    FVLA_STAMP(5);
+    // Nobody may leave while a peer can still send to it: after this arrive nothing is outstanding towards this CTA, so
+    // the wait at the end costs nothing unless a peer is late.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    for (int slot = 0; slot < owned; ++slot) {
+        const int row0 = q0 + ((int)rank + slot * SPL) * UNIT;
+        // log-sum-exp weights: lane = (source, row), a second one for sources 8 and up
+        const int s0 = lane >> 2;
+        const uint32_t st = stats_in + s0 * 64 + slot * 32 + (lane & 3) * 8;
+        const float m0 = s0 < SPL ? lds1(st) : NO_KEY, m1 = s0 + 8 < SPL ? lds1(st + 512) : NO_KEY;
+        float mx = fmaxf(m0, m1);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float w0 = s0 < SPL ? ex2(m0 - mx) : 0.f, w1 = s0 + 8 < SPL ? ex2(m1 - mx) : 0.f;
+        float wsum = (s0 < SPL ? w0 * lds1(st + 4) : 0.f) + (s0 + 8 < SPL ? w1 * lds1(st + 516) : 0.f);
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+        const float inv = wsum > 0.f ? 1.0f / wsum : 0.f;
+        w0 *= inv; w1 *= inv;
+        float acc[UNIT] = {0.f, 0.f, 0.f, 0.f};
+        const uint32_t src = sK + slot * SPL * UNIT_BYTES + tid * 16;
+#pragma unroll 4
+        for (int s = 0; s < SPL; ++s) {
+            const float4 a = lds4(src + s * UNIT_BYTES);
+            const float w = s < 8 ? w0 : w1;
+            const int from = (s & 7) * 4;
+            acc[0] = fmaf(__shfl_sync(0xffffffffu, w, from), a.x, acc[0]);
+            acc[1] = fmaf(__shfl_sync(0xffffffffu, w, from + 1), a.y, acc[1]);
+            acc[2] = fmaf(__shfl_sync(0xffffffffu, w, from + 2), a.z, acc[2]);
+            acc[3] = fmaf(__shfl_sync(0xffffffffu, w, from + 3), a.w, acc[3]);
+        }
+        // two adjacent dims of two rows per lane, so that a store is a bf16 pair: even lanes rows 0 and 1, odd lanes 2 and 3
+        const bool odd = lane & 1;
+        const float r0 = __shfl_xor_sync(0xffffffffu, odd ? acc[0] : acc[2], 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? acc[1] : acc[3], 1);
+        const uint32_t v0 = odd ? pack_bf16x2(r0, acc[2]) : pack_bf16x2(acc[0], r0), v1 = odd ? pack_bf16x2(r1, acc[3]) : pack_bf16x2(acc[1], r1);
+        const int row = row0 + (odd ? 2 : 0);
+        bf16* out = p.out + (size_t)blockIdx.z * p.q_episode_stride + (size_t)row * HD + (tid & ~1);
+        if (row < p.nq) *reinterpret_cast<uint32_t*>(out) = v0;
+        if (row + 1 < p.nq) *reinterpret_cast<uint32_t*>(out + HD) = v1;
+    }
     FVLA_STAMP(6);
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        tc5::tc_fence_after();
+        tc5::tmem_dealloc(tmem, TMEM_COLS);
+    }
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     FVLA_STAMP(7);
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 3);
 }
 
+inline bool configure_decoder_attention() {
+    static PerDeviceFlag configured;
+    if (configured.get()) return true;
+    for (auto kern : {decoder_attention_cluster_kernel<1>, decoder_attention_cluster_kernel<2>}) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);      // clusters of 9..11
+        if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return false; }
+    }
+    configured.set();
+    return true;
+}
+
+// Clusters of `spl` CTAs that the device holds at once with one CTA per SM (B200: 33 of 4, 26 of 5, 22 of 6, 15 of 7 to 9, 11 of
+// 10, 7 of 11: SMs of a GPC that do not fill a cluster stay idle). Asked once per device and size.
+inline int resident_attention_clusters(int spl) {
+    static std::atomic<int> cached[kMaxDevices][decattn::MAX_SPL + 1];
+    std::atomic<int>& c = cached[current_device()][spl];
+    int n = c.load(std::memory_order_acquire);
+    if (n == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1, spl); cfg.blockDim = dim3(decattn::THREADS); cfg.dynamicSmemBytes = 160 * 1024;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = spl; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, decoder_attention_cluster_kernel<1>, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 1; }
+        c.store(n, std::memory_order_release);
+    }
+    return n;
+}
+
+// Cluster size, smallest first in every order of preference. Ask that all clusters of the launch are resident together, with
+// one key tile of at most 128 rows and 4 or 8 CTAs, so that the eight owners' shares come out even (819 keys: 8 CTAs 29.7 us per
+// layer-step, 5 or 7 CTAs 30.7); then any size with one key tile; then with two (65 tokens x 882 keys: 40.5 us with 5
+// CTAs, all 17 clusters resident, 44.3 with 8, of which 15 are). Failing that the smallest that fits the SM at all. Returns whether
+// all clusters are resident; 0 splits: the shape does not fit.
+inline bool plan_decoder_attention(DecAttnArgs& a) {
+    using namespace decattn;
+    a.splits = 0;
+    if (a.prefix_keys <= 0 || !configure_decoder_attention()) return false;
+    const int clusters = ((a.nq + BQ - 1) / BQ) * (a.episodes > 1 ? a.episodes : 1), pre = a.prefix_keys < a.nk ? a.prefix_keys : a.nk;
+    for (int pass = 0; pass < 4; ++pass)
+        for (int spl = MIN_SPL; spl <= MAX_SPL; ++spl) {
+            const int kp = (pre + spl - 1) / spl, nd = (a.nk - pre + spl - 1) / spl, pad = (kp + nd + 15) / 16 * 16;
+            if (pass == 0 && spl != 4 && spl != 8) continue;
+            if (pad > (pass < 2 ? 128 : MAX_PAD) || smem_bytes(spl, pad) > 232448) continue;
+            if (pass < 3 && clusters > resident_attention_clusters(spl)) continue;
+            a.splits = spl; a.kp = kp; a.nd = nd; a.pad = pad; a.k_region = k_region_bytes(spl, pad);
+            return pass < 3;
+        }
+    return false;
+}
+
 inline int launch_decoder_attention_cluster(const DecAttnArgs& a, bool pdl, cudaStream_t st) {
-    auto kern = decoder_attention_cluster_kernel;
     // K / V maps that end at the prefix (rows the preceding kernel may still be writing are never fetched by them)
     CUtensorMap tmK, tmV;
     const int seqs = a.episodes > 1 ? a.episodes : 1;
     const int pre_rows = a.prefix_keys < a.nk ? a.prefix_keys : a.nk;
-    if (pre_rows <= 0) { set_error("decoder attention: no prefix keys"); return FVLA_ERR_UNSUPPORTED; }
-    int rc = tc5::make_map3d(&tmK, a.k, decattn::HD, (uint64_t)pre_rows, (uint64_t)seqs, decattn::HD, (uint64_t)a.kv_episode_stride, 64, 128);
+    if (a.splits <= 0 || pre_rows <= 0) { set_error("decoder attention: %d keys (%d of the prefix) do not fit", a.nk, pre_rows); return FVLA_ERR_UNSUPPORTED; }
+    int rc = tc5::make_map3d(&tmK, a.k, decattn::HD, (uint64_t)pre_rows, (uint64_t)seqs, decattn::HD, (uint64_t)a.kv_episode_stride, 64, (uint32_t)a.pad);
     if (rc) return rc;
-    rc = tc5::make_map3d(&tmV, a.v, decattn::HD, (uint64_t)pre_rows, (uint64_t)seqs, decattn::HD, (uint64_t)a.kv_episode_stride, 64, 128);
+    rc = tc5::make_map3d(&tmV, a.v, decattn::HD, (uint64_t)pre_rows, (uint64_t)seqs, decattn::HD, (uint64_t)a.kv_episode_stride, 64, (uint32_t)a.pad);
     if (rc) return rc;
-    static PerDeviceFlag configured;
-    if (!configured.get()) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, decattn::smem_bytes(decattn::MAX_SPL));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);      // clusters of 9..11
-        if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
-        configured.set();
-    }
     cudaLaunchConfig_t cfg = {};
-    if (a.splits < decattn::MIN_SPL || a.splits > decattn::MAX_SPL || a.keys_per_split > 128 || a.keys_per_split * a.splits < a.nk) {
-        set_error("decoder attention: %d keys do not fit %d splits of %d", a.nk, a.splits, a.keys_per_split);
-        return FVLA_ERR_UNSUPPORTED;
-    }
-    cfg.gridDim = dim3((a.nq + decattn::BQ - 1) / decattn::BQ, a.splits, a.episodes > 1 ? a.episodes : 1);
+    cfg.gridDim = dim3((a.nq + decattn::BQ - 1) / decattn::BQ, a.splits, seqs);
     cfg.blockDim = dim3(decattn::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = decattn::smem_bytes(a.splits);
+    cfg.dynamicSmemBytes = decattn::smem_bytes(a.splits, a.pad);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -661,7 +708,7 @@ inline int launch_decoder_attention_cluster(const DecAttnArgs& a, bool pdl, cuda
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, tmK, tmV);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, a.pad > 128 ? decoder_attention_cluster_kernel<2> : decoder_attention_cluster_kernel<1>, a, tmK, tmV);
     if (e != cudaSuccess) { set_error("decoder_attention_cluster_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
     return check_launch("decoder_attention_cluster_kernel");
 }

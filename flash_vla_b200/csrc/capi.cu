@@ -636,28 +636,29 @@ int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* ou
                                    kv_episode_stride >= (long long)keys * head_dim && q_episode_stride % 8 == 0 && kv_episode_stride % 8 == 0),
                  "decoder_attention: a batch of episodes needs the tcgen05 kernels and 16-byte aligned episode strides");
     if (head_dim != 256) { set_error("decoder_attention: head_dim %d not built (256 only)", head_dim); return FVLA_ERR_UNSUPPORTED; }
-    // A batch of episodes goes to the tcgen05 flash kernel (128 flat query rows per CTA, one grid row per episode,
-    // state-token mask): at one episode its 4 query tiles would occupy 8 SMs and the cluster kernel below is faster,
-    // but the cluster kernel's 8-CTA clusters are resident 15 at a time, so E episodes take E / 1.15 rounds of it.
+    // The cluster kernel (32 flat query rows per cluster) is the faster one while all its clusters are resident together: one
+    // episode, or two with up to 1 040 keys. A larger batch goes to the tcgen05 flash kernel (128 rows per CTA, one grid row
+    // per episode), whose CTAs then fill the device.
     static int batched_tc5 = -1;
     if (batched_tc5 < 0) { const char* v = getenv("FVLA_DEC_ATTN"); batched_tc5 = (v != nullptr && strcmp(v, "cluster") == 0) ? 0 : 1; }
-    if (episodes > 1 && batched_tc5 && tc5_enabled() && aligned16(Q) && aligned16(K) && aligned16(V) && aligned16(out))
+    DecAttnArgs d{};
+    d.q = B(Q); d.k = B(K); d.v = B(V); d.out = Bm(out);
+    d.nq = queries; d.nk = keys; d.scale_log2 = kLog2e / sqrtf((float)head_dim);
+    d.mask_rows = heads; d.mask_key_le = encoder_seq_len; d.prefix_keys = encoder_seq_len;
+    d.episodes = episodes; d.q_episode_stride = q_episode_stride; d.kv_episode_stride = kv_episode_stride;
+    d.status = device_status_ptr();
+    const bool aligned = aligned16(Q) && aligned16(K) && aligned16(V) && aligned16(out);
+    const bool resident = tc5_enabled() && aligned && plan_decoder_attention(d);
+    if (episodes > 1 && batched_tc5 && tc5_enabled() && aligned && !resident)
         return attn5::launch_attention_tc5(Q, K, V, out, queries, keys, kLog2e / sqrtf((float)head_dim), device_status_ptr(), S(stream),
                                            episodes, q_episode_stride, kv_episode_stride, heads, encoder_seq_len);
-    FVLA_REQUIRE(episodes == 1 || keys <= decattn::MAX_SPL * 128, "decoder_attention: the cluster kernel takes at most %d keys", decattn::MAX_SPL * 128);
+    FVLA_REQUIRE(episodes == 1 || d.splits > 0, "decoder_attention: %d keys do not fit the cluster kernel", keys);
     if (ws == nullptr || ws_bytes < fvla_decoder_attention_workspace_bytes(queries, keys)) {
         set_error("decoder_attention: workspace of %zu bytes needed", fvla_decoder_attention_workspace_bytes(queries, keys));
         return FVLA_ERR_WORKSPACE;
     }
-    if (tc5_enabled() && keys <= decattn::MAX_SPL * 128 && aligned16(Q) && aligned16(K) && aligned16(V)) {        // cluster kernel: 8..11 key splits of at most 128 keys
-        DecAttnArgs d{};
-        d.q = B(Q); d.k = B(K); d.v = B(V); d.out = Bm(out);
-        d.splits = (keys + 127) / 128 < decattn::MIN_SPL ? decattn::MIN_SPL : (keys + 127) / 128;
-        d.nq = queries; d.nk = keys; d.keys_per_split = ((keys + d.splits - 1) / d.splits + 7) / 8 * 8;
-        d.scale_log2 = kLog2e / sqrtf((float)head_dim);
-        d.mask_rows = heads; d.mask_key_le = encoder_seq_len; d.prefix_keys = encoder_seq_len;
-        d.episodes = episodes; d.q_episode_stride = q_episode_stride; d.kv_episode_stride = kv_episode_stride;
-        d.status = device_status_ptr(); FVLA_DBG_ATTACH(d);
+    if (tc5_enabled() && aligned && d.splits > 0) {
+        FVLA_DBG_ATTACH(d);
         return launch_decoder_attention_cluster(d, pdl_enabled(), S(stream));
     }
     const int splits = (keys + 127) / 128;

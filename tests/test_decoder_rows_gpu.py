@@ -56,3 +56,21 @@ def test_decoder_gemms_by_row_count(M, group):
         assert_close(x, ref, what=name)
         assert torch.equal(shadow, x.to(bf16)), name
     assert _lib.load().fvla_device_status(None) == 0
+
+
+# one key tile of 128 per CTA and two; 4 CTAs per cluster and more; a single token; two episodes that are resident together
+@pytest.mark.parametrize("tokens,S,episodes", [(1, 40, 1), (11, 273, 1), (51, 816, 1), (65, 817, 1), (64, 1280, 1), (51, 768, 2), (5, 1024, 2)])
+def test_decoder_attention_by_shape(tokens, S, episodes):
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
+    g = torch.Generator().manual_seed(tokens * S)
+    keys = S + tokens
+    Q, K, V = rnd(g, episodes, tokens * 8, 256), rnd(g, episodes, keys, 256), rnd(g, episodes, keys, 256)
+    q = Q.cuda().clone().view(-1, 256)
+    k, v = (t.cuda() if episodes > 1 else t[0].cuda() for t in (K, V))
+    op_table(True).decoder_attention(q, k, v, None, q, S)                    # out aliases Q
+    for e in range(episodes):
+        ref = torch.zeros(tokens * 8, 256)
+        O.op_table(True).decoder_attention(Q[e].float(), K[e].float(), V[e].float(), None, ref, S)
+        assert_close(q.view(episodes, -1, 256)[e], ref, what=f"decoder_attention, episode {e}")
+    assert _lib.load().fvla_device_status(None) == 0
