@@ -9,8 +9,8 @@
 //     of it at kernel start (<= 8 boxes of 64 k x 128 n, 128B-swizzled, used in place as an
 //     MN-major operand) and issues KC/16 tcgen05.mma into one TMEM accumulator;
 //   * the S CTAs of a K-split form a thread-block cluster. Each reads its partial accumulator
-//     from TMEM and scatters it over distributed shared memory so that CTA r receives the
-//     partials of its slice of tokens; after one cluster barrier CTA r sums them in rank order
+//     from TMEM and sends it, registers to distributed shared memory, so that CTA r receives the
+//     partials of its slice of tokens; once its barrier has counted them CTA r sums them in rank order
 //     (deterministic) and runs the fused epilogue: RMS-factor + RoPE + scatter to Q/K/V, GeGLU,
 //     bias, or in-place residual add into the fp32 stream.
 // The activation operand arrives by TMA as bf16 rows: either the activation itself (bf16) or the bf16
@@ -41,12 +41,9 @@ constexpr int MAX_KB = 8;        // k-blocks of 64 per CTA
 // 32 KB and the exchange 64 KB, so at most five have one and the rest reuse the first ones' when their MMAs (and the readers of
 // the sums of squares) are done.
 __host__ __device__ constexpr int slots_of(int tok, int kblocks) { return tok == 64 || kblocks < 5 ? kblocks : 5; }
-__host__ __device__ constexpr int w_region_bytes(int tok, int slots) {      // weight slots; the partial tile and 64 / 128 sums are staged over them
-    return slots * 16384 > tok * 512 + 1024 ? slots * 16384 + (tok == 64 ? 1024 : 0) : tok * 512 + 1024;
-}
 constexpr int misc_bytes(int tok) { return tok * 4 + tok * 8 + (2 * MAX_KB + 2) * 8 + 32; }     // received sums, own sums, barriers, TMEM slot, flag
 constexpr size_t smem_bytes(int tok, int kblocks) {
-    return 1024 + (size_t)w_region_bytes(tok, slots_of(tok, kblocks)) + (size_t)slots_of(tok, kblocks) * tok * 128 + tok * 512 + misc_bytes(tok);
+    return 1024 + (size_t)slots_of(tok, kblocks) * (16384 + tok * 128) + tok * 512 + misc_bytes(tok);
 }
 static_assert(smem_bytes(64, MAX_KB) <= 232448 && smem_bytes(128, MAX_KB) <= 232448, "shared memory of one CTA");
 
@@ -98,20 +95,19 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 
 // Shared memory map (offsets from a 1024-byte aligned base):
-//   W      slots x 16 KB     [slot][atom(2)][64 k rows x 128 B]  (atom = 64 of the tile's 128 n);
-//          after the MMAs it is reused as the staging area of this CTA's partial tile
-//          ([token TOK][n 128] fp32 + TOK partial sums of squares)
+//   W      slots x 16 KB     [slot][atom(2)][64 k rows x 128 B]  (atom = 64 of the tile's 128 n)
 //   X      slots x TOK x 128 B  [slot][token][64 k]            (K-major, 128B swizzle)
-//   RED    S x TS x 128 fp32 = TOK x 512 B   partials received from the S ranks, [src][token][n]
+//   RED    S x TS x 128 fp32 = TOK x 512 B   partials of the S ranks (the own one too), [src][4 tokens][n][4]
 //   SSQ    S x TS fp32       partial sums of squares received, [src][token]
 //   ssq_local TOK x 2 fp32, barriers, tmem slot, abort flag
 constexpr int THREADS = 512;
 
-__device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst_cluster_addr, uint32_t src_cta_addr, uint32_t bytes,
-                                                 uint32_t mbar_cluster_addr) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(dst_cluster_addr), "r"(src_cta_addr), "r"(bytes), "r"(mbar_cluster_addr) : "memory");
+__device__ __forceinline__ void st_async4(uint32_t dst, uint32_t bar, float a, float b, float c, float d) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(dst), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_async1(uint32_t dst, uint32_t bar, float a) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(a), "r"(bar) : "memory");
 }
 
 template <int EPI, int TOK>
@@ -124,11 +120,9 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     constexpr uint32_t XB = TOK * 128, RED_BYTES = TOK * 512, ACC_COLS = 2 * TOK;      // one accumulator per issuing thread
     constexpr int SSQ_WARPS = TOK == 64 ? THREADS / 32 : 8;                                  // warps that add up the rows' squares
     const int KB = p.kblocks, S = p.splits, TS = TOK / S, NS = slots_of(TOK, KB);
-    const uint32_t w_bytes = w_region_bytes(TOK, NS);
+    const uint32_t w_bytes = NS * 16384u;
     const uint32_t sW = base, sX = sW + w_bytes;
     const uint32_t off_red = w_bytes + NS * XB;
-    float* stage = reinterpret_cast<float*>(gen);                                // aliases W
-    float* red = reinterpret_cast<float*>(gen + off_red);                        // [S][TS][128]
     float* ssq_in = reinterpret_cast<float*>(gen + off_red + RED_BYTES);                   // [S][TS]
     float* ssq_local = reinterpret_cast<float*>(gen + off_red + RED_BYTES + TOK * 4);      // [TOK][2]
     const uint32_t off_bar = off_red + RED_BYTES + TOK * 12;
@@ -157,7 +151,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         mbar_init(in_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (i_own) mbar_expect_tx(in_bar, (uint32_t)(S - 1) * (uint32_t)TS * (512u + (p.need_factor ? 4u : 0u)) + p.expect_extra_bytes);      // S - 1 peers send
+        if (i_own)                                           // S - 1 peers send
+            mbar_expect_tx(in_bar, (uint32_t)(S - 1) * ((uint32_t)(min(TS, p.M - (int)rank * TS) + 3) / 4 * 2048u + (p.need_factor ? TS * 4u : 0u)) + p.expect_extra_bytes);
     }
     auto request_w = [&](int kb, int slot) {
         mbar_expect_tx(bars + kb * 8, x_by_tma ? 16384 + XB : 16384);
@@ -199,38 +194,39 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
 
     // Epilogue operands that do not depend on the product (RoPE entries, residual values, bias) are
     // fetched now, so that their latency overlaps the weight stream instead of following the MMA.
-    // Owner work items: (token of this rank's slice) x (group of 4 adjacent columns).
-    constexpr int QPT = (EPI == EPI_GEGLU) ? 16 : 32;         // column quads per token
-    constexpr int PRE = 4;                                    // TS * QPT <= 2048 = 4 x THREADS
-    const int items = TS * QPT;
+    // Owner work items: (4 tokens of this rank's slice) x (column); after two lanes have swapped, a lane finishes two tokens
+    // (ta, ta + 1) of two adjacent columns.
+    constexpr int COLS = (EPI == EPI_GEGLU) ? 64 : 128;
+    constexpr int PRE = 4;                                    // TS / 4 * COLS <= 2048 = 4 x THREADS
+    const int items = (TS >> 2) * COLS, odd = lane & 1;
     uint4 pre[PRE];
 #pragma unroll
     for (int j = 0; j < PRE; ++j) {
         pre[j] = make_uint4(0, 0, 0, 0);
-        const int item = tid + j * THREADS;
-        const int tl = item / QPT, c4 = (item % QPT) * 4;
-        const int token = (int)rank * TS + tl;
-        if (item < items && token < p.M) {
-            const int n = tile * TN + c4;
-            if (EPI == EPI_QKV_ROPE) {
-                if (n < (p.heads + 1) * p.head_dim) {
-                    const int pos = token - (int)((uint32_t)token * p.inv_group >> 20) * p.group_rows;
-                    const uint2 cs = __ldg(reinterpret_cast<const uint2*>(p.rope + (size_t)pos * p.head_dim + (n % p.head_dim)));
-                    pre[j].x = cs.x; pre[j].y = cs.y;
-                }
-            } else if (EPI == EPI_RESIDUAL) {
-                if (p.out_f32) {
-                    pre[j] = *reinterpret_cast<const uint4*>(static_cast<const float*>(p.out) + (size_t)(row0 + token) * p.ldo + n);
-                } else {
-                    const uint2 r = *reinterpret_cast<const uint2*>(static_cast<const bf16*>(p.out) + (size_t)(row0 + token) * p.ldo + n);
-                    const float2 r0 = unpack_bf16x2(r.x), r1 = unpack_bf16x2(r.y);
-                    pre[j] = make_uint4(__float_as_uint(r0.x), __float_as_uint(r0.y), __float_as_uint(r1.x), __float_as_uint(r1.y));
-                }
-            } else if (EPI == EPI_BIAS) {
-                const uint2 bv = __ldg(reinterpret_cast<const uint2*>(p.bias + n));
-                const float2 b0 = unpack_bf16x2(bv.x), b1 = unpack_bf16x2(bv.y);
-                pre[j] = make_uint4(__float_as_uint(b0.x), __float_as_uint(b0.y), __float_as_uint(b1.x), __float_as_uint(b1.y));
+        const int item = tid + j * THREADS, n = tile * COLS + (item % COLS & ~1), ta = (int)rank * TS + item / COLS * 4 + odd * 2;
+        if (item >= items || ta >= p.M) continue;
+        const bool second = ta + 1 < p.M;
+        if (EPI == EPI_QKV_ROPE) {
+            if (n < (p.heads + 1) * p.head_dim) {
+                const bf16* rp = p.rope + (n % p.head_dim);
+                const int pos0 = ta - (int)((uint32_t)ta * p.inv_group >> 20) * p.group_rows, pos1 = ta + 1 - (int)((uint32_t)(ta + 1) * p.inv_group >> 20) * p.group_rows;
+                pre[j].x = __ldg(reinterpret_cast<const uint32_t*>(rp + (size_t)pos0 * p.head_dim));
+                if (second) pre[j].z = __ldg(reinterpret_cast<const uint32_t*>(rp + (size_t)pos1 * p.head_dim));
             }
+        } else if (EPI == EPI_RESIDUAL) {
+            const size_t at = (size_t)(row0 + ta) * p.ldo + n;
+            if (p.out_f32) {
+                const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at);
+                const uint2 b = second ? *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at + p.ldo) : make_uint2(0, 0);
+                pre[j] = make_uint4(a.x, a.y, b.x, b.y);
+            } else {
+                const float2 a = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at));
+                const float2 b = unpack_bf16x2(second ? *reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at + p.ldo) : 0u);
+                pre[j] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+            }
+        } else if (EPI == EPI_BIAS) {
+            const float2 b = unpack_bf16x2(__ldg(reinterpret_cast<const uint32_t*>(p.bias + n)));
+            pre[j] = make_uint4(__float_as_uint(b.x), __float_as_uint(b.y), __float_as_uint(b.x), __float_as_uint(b.y));
         }
     }
 
@@ -336,125 +332,137 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         for (int o = 1; o < LPT; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if (sub == 0) { ssq_local[t * 2] = ss; ssq_local[t * 2 + 1] = 0.f; }
     }
-    const bool done = mbar_wait(done_bar, 0, abort_flag);
+    mbar_wait(done_bar, 0, abort_flag);                // (after an expired wait the sums are garbage and the status says so)
+    __syncwarp();
     tc5::tc_fence_after();
     FVLA_STAMP(3);
-    __syncthreads();                                   // sums of squares are complete
-    // Stage this CTA's partial tile as [token][n] fp32 over the (now idle) weight region. All 16 warps
-    // take part: warp w reads TMEM lanes 32 (w & 3) .. + 32 (its n) and token columns 16 (w >> 2) .. + 16 (and + 64).
+    // Hand the partial tile out: warp w reads TMEM lanes 32 (w & 3) .. + 32 (its columns) and tokens 16 (w >> 2) .. + 16 (and
+    // + 64), and what a thread holds of four tokens goes as 16 bytes from registers to their owner's receive buffer
+    // [src][4 tokens][column][4], which counts the bytes on its barrier; the own slice takes an ordinary store. (Staged in
+    // shared memory and sent by bulk copies the exchange took 0.4 us longer.)
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has initialised its barriers
+    const int ts_sh = 31 - __clz(TS);
+    const uint32_t red_mine = base + off_red + rank * (TS * 512u);
 #pragma unroll
     for (int h = 0; h < TOK / 64; ++h) {
         const int q = warp & 3, g = (warp >> 2) + h * 4;
         float part[16];
         tc5::tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + g * 16, part);
         if (KB > 1) {
-            float odd[16];
-            tc5::tmem_ld16(tmem + TOK + ((uint32_t)(q * 32) << 16) + g * 16, odd);
+            float second[16];
+            tc5::tmem_ld16(tmem + TOK + ((uint32_t)(q * 32) << 16) + g * 16, second);
 #pragma unroll
-            for (int t = 0; t < 16; ++t) part[t] += odd[t];
+            for (int t = 0; t < 16; ++t) part[t] += second[t];
         }
 #pragma unroll
-        for (int t = 0; t < 16; ++t) stage[(g * 16 + t) * TN + q * 32 + lane] = done ? part[t] : 0.f;
-    }
-    if (p.need_factor && tid < TOK)
-        stage[TOK * TN + tid] = tid < p.M ? ssq_local[tid * 2] + (KB == 8 ? ssq_local[tid * 2 + 1] : 0.f) : 0.f;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");       // staging writes -> visible to the bulk copies
-    tc5::tc_fence_before();
-    __syncthreads();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has initialised its barriers
-    if (tid < owners && tid != (int)rank) {
-        // one bulk copy per owner, issued by a lane of its own: its slice of tokens goes to slot [src = my rank] of its RED
-        // buffer (an owner reads its own slice where it was staged)
-        const int r = tid;
-        bulk_copy_to_cta(map_to_cta(base + off_red + (uint32_t)(rank * TS) * 512u, (uint32_t)r),
-                         base + (uint32_t)(r * TS) * 512u, (uint32_t)TS * 512u, map_to_cta(in_bar, (uint32_t)r));
-        if (p.need_factor)
-            bulk_copy_to_cta(map_to_cta(base + off_red + RED_BYTES + (uint32_t)(rank * TS) * 4u, (uint32_t)r),
-                             base + (uint32_t)(TOK * TN) * 4u + (uint32_t)(r * TS) * 4u, (uint32_t)TS * 4u,
-                             map_to_cta(in_bar, (uint32_t)r));
-    }
-    __syncwarp();
-
-    FVLA_STAMP(4);
-    // Owner phase: this CTA finishes tokens [rank*TS, rank*TS + TS), summing partials in rank order.
-    if (i_own) {
-        mbar_wait(in_bar, 0, abort_flag, p.spin_limit ? p.spin_limit : tc5::kSpinLimit);
-        FVLA_STAMP(5);
-#pragma unroll
-        for (int j = 0; j < PRE; ++j) {
-            const int item = tid + j * THREADS;
-            const int tl = item / QPT, c4 = (item % QPT) * 4;
-            const int token = (int)rank * TS + tl;
-            if (item >= items || token >= p.M) continue;
-            // partial of source rank s for this token: received in RED, or (own rank) still in the staging area
-            auto part_row = [&](int s) { return s == (int)rank ? stage + ((int)rank * TS + tl) * TN : red + (s * TS + tl) * TN; };
-            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < S; ++s) {
-                const float4 v = *reinterpret_cast<const float4*>(part_row(s) + c4);
-                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-            }
-            float factor = 1.f;
-            if (p.need_factor) {
-                float ss = 0.f;
-                for (int s = 0; s < S; ++s) ss += s == (int)rank ? stage[TOK * TN + (int)rank * TS + tl] : ssq_in[s * TS + tl];
-                factor = rsqrtf(ss * (1.0f / (float)p.K) + 1e-6f);
-                if (p.factor_out && tile == 0 && c4 == 0) p.factor_out[token] = __float2bfloat16_rn(factor);
-            }
-            const int n = tile * TN + c4;
-            if (EPI == EPI_QKV_ROPE) {
-                float v0 = sum.x * factor, v1 = sum.y * factor, v2 = sum.z * factor, v3 = sum.w * factor;
-                const int hd = p.head_dim, qd = p.heads * hd;
-                const int kv_row = token + (int)((uint32_t)token * p.inv_group >> 20) * p.kv_skip;
-                bf16* dst;
-                if (n < qd + hd) {
-                    const float2 c0 = unpack_bf16x2(pre[j].x), c1 = unpack_bf16x2(pre[j].y);
-                    const float r0 = v0 * c0.x - v1 * c0.y, r1 = v1 * c0.x + v0 * c0.y;
-                    const float r2 = v2 * c1.x - v3 * c1.y, r3 = v3 * c1.x + v2 * c1.y;
-                    v0 = r0; v1 = r1; v2 = r2; v3 = r3;
-                    dst = n < qd ? p.q + (size_t)token * qd + n : p.k + (size_t)kv_row * hd + (n - qd);
-                } else {
-                    dst = p.v + (size_t)kv_row * hd + (n - qd - hd);
-                }
-                *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v0, v1), pack_bf16x2(v2, v3));
-            } else if (EPI == EPI_GEGLU) {
-                // columns 0..63 of the tile are gate columns, 64..127 the matching up columns
-                float4 up = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int s = 0; s < S; ++s) {
-                    const float4 v = *reinterpret_cast<const float4*>(part_row(s) + 64 + c4);
-                    up.x += v.x; up.y += v.y; up.z += v.z; up.w += v.w;
-                }
-                const float f2 = factor;
-                *reinterpret_cast<uint2*>(static_cast<bf16*>(p.out) + (size_t)(row0 + token) * p.ldo + tile * 64 + c4) =
-                    make_uint2(pack_bf16x2(gelu_f(sum.x * f2) * (up.x * f2), gelu_f(sum.y * f2) * (up.y * f2)),
-                               pack_bf16x2(gelu_f(sum.z * f2) * (up.z * f2), gelu_f(sum.w * f2) * (up.w * f2)));
-            } else {
-                float v0 = sum.x, v1 = sum.y, v2 = sum.z, v3 = sum.w;
-                // pre = bias (EPI_BIAS) or residual (EPI_RESIDUAL), as four floats
-                v0 += __uint_as_float(pre[j].x); v1 += __uint_as_float(pre[j].y);
-                v2 += __uint_as_float(pre[j].z); v3 += __uint_as_float(pre[j].w);
-                if (EPI == EPI_BIAS && p.act == 2) { v0 = silu_f(v0); v1 = silu_f(v1); v2 = silu_f(v2); v3 = silu_f(v3); }
-                if (p.out_shadow)
-                    *reinterpret_cast<uint2*>(p.out_shadow + (size_t)(row0 + token) * p.ldo + n) =
-                        make_uint2(pack_bf16x2(v0, v1), pack_bf16x2(v2, v3));
-                if (p.out_f32)
-                    *reinterpret_cast<float4*>(static_cast<float*>(p.out) + (size_t)(row0 + token) * p.ldo + n) = make_float4(v0, v1, v2, v3);
-                else
-                    *reinterpret_cast<uint2*>(static_cast<bf16*>(p.out) + (size_t)(row0 + token) * p.ldo + n) =
-                        make_uint2(pack_bf16x2(v0, v1), pack_bf16x2(v2, v3));
-            }
+        for (int t = 0; t < 16; t += 4) {
+            const int token = g * 16 + t, r = token >> ts_sh;
+            if (token >= p.M) break;
+            const uint32_t at = red_mine + (uint32_t)((token & (TS - 1)) >> 2) * 2048u + (q * 32 + lane) * 16u;
+            if (r == (int)rank) *reinterpret_cast<float4*>(gen + (at - base)) = make_float4(part[t], part[t + 1], part[t + 2], part[t + 3]);
+            else st_async4(map_to_cta(at, (uint32_t)r), map_to_cta(in_bar, (uint32_t)r), part[t], part[t + 1], part[t + 2], part[t + 3]);
         }
     }
-
-    // No CTA may leave while a peer can still be reading its staging area: once every owner has
-    // received all of its slices, every outgoing copy of every CTA has completed.
-    FVLA_STAMP(6);
     tc5::tc_fence_before();
-    // (execution barrier only: nothing read after it was written by a peer)
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    __syncthreads();                                   // sums of squares complete, own slice stored, accumulators read
+    if (p.need_factor && tid < TOK && (tid >> ts_sh) < owners) {
+        const float ss = tid < p.M ? ssq_local[tid * 2] + (KB == 8 ? ssq_local[tid * 2 + 1] : 0.f) : 0.f;
+        const int r = tid >> ts_sh;
+        if (r == (int)rank) ssq_in[rank * TS + (tid & (TS - 1))] = ss;
+        else st_async1(map_to_cta(base + off_red + RED_BYTES + (rank * TS + (tid & (TS - 1))) * 4u, (uint32_t)r), map_to_cta(in_bar, (uint32_t)r), ss);
+    }
     if (warp == 0) {
         tc5::tc_fence_after();
         tc5::tmem_dealloc(tmem, ACC_COLS);
     }
+    if (p.need_factor) __syncthreads();                // the own sums of squares are in place
+
+    FVLA_STAMP(4);
+    // Owner phase: this CTA finishes tokens [rank*TS, rank*TS + TS), summing partials in rank order.
+    if (i_own) mbar_wait(in_bar, 0, abort_flag, p.spin_limit ? p.spin_limit : tc5::kSpinLimit);
+    __syncwarp();
+    FVLA_STAMP(5);
+    // Nobody may leave while a peer can still send to it. Past this arrive nothing is outstanding towards this CTA, and the wait
+    // at the end finds the peers here too.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (i_own) {
+        const float* red = reinterpret_cast<const float*>(gen + off_red);
+#pragma unroll
+        for (int j = 0; j < PRE; ++j) {
+            const int item = tid + j * THREADS, group = item / COLS, c = item % COLS;
+            const int tl = group * 4 + odd * 2, ta = (int)rank * TS + tl;
+            if (item >= items || (int)rank * TS + group * 4 >= p.M) continue;            // uniform within a warp
+            auto sum_sources = [&](int col, float2 (&t)[2]) {
+                const float* src = red + (group * 128 + col) * 4;
+                float4 in[8];                              // all sources requested before the first is used
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if (s < S) in[s] = *reinterpret_cast<const float4*>(src + s * TS * 128);
+                float4 a = in[0];
+#pragma unroll
+                for (int s = 1; s < 8; ++s)
+                    if (s < S) { a.x += in[s].x; a.y += in[s].y; a.z += in[s].z; a.w += in[s].w; }
+                // swap with the lane of the neighbouring column: even lanes keep tokens 0, 1, odd lanes 2, 3
+                const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a.x : a.z, 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? a.y : a.w, 1);
+                t[0] = odd ? make_float2(r0, a.z) : make_float2(a.x, r0);
+                t[1] = odd ? make_float2(r1, a.w) : make_float2(a.y, r1);
+            };
+            float factor[2] = {1.f, 1.f};
+            if (p.need_factor) {
+                float2 ss = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if (s < S) {
+                        const float2 q = *reinterpret_cast<const float2*>(ssq_in + s * TS + tl);
+                        ss.x += q.x; ss.y += q.y;
+                    }
+                const float inv_k = 1.0f / (float)p.K;
+                factor[0] = rsqrtf(ss.x * inv_k + 1e-6f);
+                factor[1] = rsqrtf(ss.y * inv_k + 1e-6f);
+            }
+            float2 v[2], up[2];
+            sum_sources(c, v);
+            if (EPI == EPI_GEGLU) sum_sources(64 + c, up);        // columns 0..63 of the tile are gate columns, 64..127 the matching up columns
+            const int n = tile * COLS + (c & ~1);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int token = ta + i;
+                if (token >= p.M) break;
+                if (p.need_factor && p.factor_out && tile == 0 && c < 2) p.factor_out[token] = __float2bfloat16_rn(factor[i]);
+                const uint32_t p0 = i == 0 ? pre[j].x : pre[j].z, p1 = i == 0 ? pre[j].y : pre[j].w;
+                if (EPI == EPI_QKV_ROPE) {
+                    float v0 = v[i].x * factor[i], v1 = v[i].y * factor[i];
+                    const int hd = p.head_dim, qd = p.heads * hd;
+                    const int kv_row = token + (int)((uint32_t)token * p.inv_group >> 20) * p.kv_skip;
+                    bf16* dst;
+                    if (n < qd + hd) {
+                        const float2 cs = unpack_bf16x2(p0);
+                        const float r0 = v0 * cs.x - v1 * cs.y, r1 = v1 * cs.x + v0 * cs.y;
+                        v0 = r0; v1 = r1;
+                        dst = n < qd ? p.q + (size_t)token * qd + n : p.k + (size_t)kv_row * hd + (n - qd);
+                    } else {
+                        dst = p.v + (size_t)kv_row * hd + (n - qd - hd);
+                    }
+                    *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(v0, v1);
+                } else if (EPI == EPI_GEGLU) {
+                    const float f = factor[i];
+                    *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + (size_t)(row0 + token) * p.ldo + n) =
+                        pack_bf16x2(gelu_f(v[i].x * f) * (up[i].x * f), gelu_f(v[i].y * f) * (up[i].y * f));
+                } else {
+                    // p0, p1 = bias (EPI_BIAS) or residual (EPI_RESIDUAL)
+                    float v0 = v[i].x + __uint_as_float(p0), v1 = v[i].y + __uint_as_float(p1);
+                    if (EPI == EPI_BIAS && p.act == 2) { v0 = silu_f(v0); v1 = silu_f(v1); }
+                    const size_t at = (size_t)(row0 + token) * p.ldo + n;
+                    const uint32_t word = pack_bf16x2(v0, v1);
+                    if (p.out_shadow) *reinterpret_cast<uint32_t*>(p.out_shadow + at) = word;
+                    if (p.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(p.out) + at) = make_float2(v0, v1);
+                    else *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + at) = word;
+                }
+            }
+        }
+    }
+    FVLA_STAMP(6);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     FVLA_STAMP(7);
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 2);
 }
