@@ -118,7 +118,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
     constexpr uint32_t XB = TOK * 128, RED_BYTES = TOK * 512, ACC_COLS = 2 * TOK;      // one accumulator per issuing thread
-    constexpr int SSQ_WARPS = TOK == 64 ? THREADS / 32 : 8;                                  // warps that add up the rows' squares
+    // The upper warps add up the rows' squares: the MMA issuers' warps come too late for it (gate/up: 1.6 us after the last MMA)
+    constexpr int SSQ_WARPS = 8;
     const int KB = p.kblocks, S = p.splits, TS = TOK / S, NS = slots_of(TOK, KB);
     const uint32_t w_bytes = NS * 16384u;
     const uint32_t sW = base, sX = sW + w_bytes;
@@ -309,8 +310,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     __syncwarp();
     if (x_by_tma && p.need_factor && warp >= THREADS / 32 - SSQ_WARPS) {
         // Sums of squares over this CTA's K slice, read back from the bf16 operand tile in shared
-        // memory while the MMAs run (8 lanes per token, one 16-byte chunk per k-block each; with 128 slots two lanes of the
-        // upper eight warps).
+        // memory while the MMAs run (4 or 2 lanes per token).
         constexpr int LPT = SSQ_WARPS * 32 / TOK;            // lanes per token
         const int st = tid - (THREADS - SSQ_WARPS * 32), t = st / LPT, sub = st % LPT;
         float ss = 0.f;
