@@ -110,7 +110,7 @@ __device__ __forceinline__ void st_async1(uint32_t dst, uint32_t bar, float a) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(a), "r"(bar) : "memory");
 }
 
-template <int EPI, int TOK>
+template <int EPI, int TOK, int PRE>        // PRE: owner work items per thread
 __global__ void __launch_bounds__(THREADS, 1)
 skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                    const __grid_constant__ CUtensorMap tmX) {
@@ -197,37 +197,51 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     // fetched now, so that their latency overlaps the weight stream instead of following the MMA.
     // Owner work items: (4 tokens of this rank's slice) x (column); after two lanes have swapped, a lane finishes two tokens
     // (ta, ta + 1) of two adjacent columns.
+    // All index arithmetic is done here too: what follows the exchange is on the critical path of 16 warps.
     constexpr int COLS = (EPI == EPI_GEGLU) ? 64 : 128;
-    constexpr int PRE = 4;                                    // TS / 4 * COLS <= 2048 = 4 x THREADS
     const int items = (TS >> 2) * COLS, odd = lane & 1;
+    const float inv_k = 1.0f / (float)p.K;
     uint4 pre[PRE];
+    bf16* dst[PRE];                                           // QKV: Q, K or V
+    uint32_t at[PRE][2];                                      // element offsets of the two tokens in the destination
+    bool live[PRE][2], work[PRE];
 #pragma unroll
     for (int j = 0; j < PRE; ++j) {
         pre[j] = make_uint4(0, 0, 0, 0);
-        const int item = tid + j * THREADS, n = tile * COLS + (item % COLS & ~1), ta = (int)rank * TS + item / COLS * 4 + odd * 2;
-        if (item >= items || ta >= p.M) continue;
-        const bool second = ta + 1 < p.M;
+        dst[j] = nullptr;
+        const int item = tid + j * THREADS, c = item % COLS & ~1, n = tile * COLS + c, t4 = (int)rank * TS + item / COLS * 4, ta = t4 + odd * 2;
+        work[j] = item < items && t4 < p.M;                   // uniform within a warp
+        live[j][0] = work[j] && ta < p.M;
+        live[j][1] = work[j] && ta + 1 < p.M;
         if (EPI == EPI_QKV_ROPE) {
-            if (n < (p.heads + 1) * p.head_dim) {
-                const bf16* rp = p.rope + (n % p.head_dim);
-                const int pos0 = ta - (int)((uint32_t)ta * p.inv_group >> 20) * p.group_rows, pos1 = ta + 1 - (int)((uint32_t)(ta + 1) * p.inv_group >> 20) * p.group_rows;
-                pre[j].x = __ldg(reinterpret_cast<const uint32_t*>(rp + (size_t)pos0 * p.head_dim));
-                if (second) pre[j].z = __ldg(reinterpret_cast<const uint32_t*>(rp + (size_t)pos1 * p.head_dim));
+            const int hd = p.head_dim, qd = p.heads * hd;
+            const int seq0 = (int)((uint32_t)ta * p.inv_group >> 20), seq1 = (int)((uint32_t)(ta + 1) * p.inv_group >> 20);
+            if (n < qd + hd) {
+                const bf16* rp = p.rope + (n % hd);
+                if (live[j][0]) pre[j].x = __ldg(reinterpret_cast<const uint32_t*>(rp + (size_t)(ta - seq0 * p.group_rows) * hd));
+                if (live[j][1]) pre[j].z = __ldg(reinterpret_cast<const uint32_t*>(rp + (size_t)(ta + 1 - seq1 * p.group_rows) * hd));
             }
-        } else if (EPI == EPI_RESIDUAL) {
-            const size_t at = (size_t)(row0 + ta) * p.ldo + n;
-            if (p.out_f32) {
-                const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at);
-                const uint2 b = second ? *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at + p.ldo) : make_uint2(0, 0);
-                pre[j] = make_uint4(a.x, a.y, b.x, b.y);
+            if (n < qd) {
+                dst[j] = p.q;
+                at[j][0] = (uint32_t)(ta * qd + n); at[j][1] = at[j][0] + qd;
             } else {
-                const float2 a = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at));
-                const float2 b = unpack_bf16x2(second ? *reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at + p.ldo) : 0u);
-                pre[j] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+                dst[j] = n < qd + hd ? p.k : p.v;
+                const int col = n - qd - (n < qd + hd ? 0 : hd);
+                at[j][0] = (uint32_t)((ta + seq0 * p.kv_skip) * hd + col); at[j][1] = (uint32_t)((ta + 1 + seq1 * p.kv_skip) * hd + col);
             }
-        } else if (EPI == EPI_BIAS) {
-            const float2 b = unpack_bf16x2(__ldg(reinterpret_cast<const uint32_t*>(p.bias + n)));
-            pre[j] = make_uint4(__float_as_uint(b.x), __float_as_uint(b.y), __float_as_uint(b.x), __float_as_uint(b.y));
+        } else {
+            at[j][0] = (uint32_t)((row0 + ta) * p.ldo + n); at[j][1] = at[j][0] + p.ldo;
+            if (EPI == EPI_RESIDUAL && p.out_f32) {
+                if (live[j][0]) { const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at[j][0]); pre[j].x = a.x; pre[j].y = a.y; }
+                if (live[j][1]) { const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at[j][1]); pre[j].z = a.x; pre[j].w = a.y; }
+            } else if (EPI == EPI_RESIDUAL) {
+                const float2 a = unpack_bf16x2(live[j][0] ? *reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at[j][0]) : 0u);
+                const float2 b = unpack_bf16x2(live[j][1] ? *reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at[j][1]) : 0u);
+                pre[j] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+            } else if (EPI == EPI_BIAS) {
+                const float2 b = unpack_bf16x2(__ldg(reinterpret_cast<const uint32_t*>(p.bias + n)));
+                pre[j] = make_uint4(__float_as_uint(b.x), __float_as_uint(b.y), __float_as_uint(b.x), __float_as_uint(b.y));
+            }
         }
     }
 
@@ -277,6 +291,13 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     __syncthreads();
     tc5::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has initialised its barriers
+    const int ts_sh = 31 - __clz(TS);
+    auto hand_out_ss = [&](int t, float ss) {          // a row's sum of squares over this CTA's K slice, to the row's owner
+        const int r = t >> ts_sh, slot = (int)rank * TS + (t & (TS - 1));
+        if (r == (int)rank) ssq_in[slot] = ss;
+        else if (r < owners) st_async1(map_to_cta(base + off_red + RED_BYTES + slot * 4u, (uint32_t)r), map_to_cta(in_bar, (uint32_t)r), ss);
+    };
     FVLA_STAMP(2);
 
     // Two threads issue the MMAs, k-blocks in turn, each into an accumulator of its own. One thread needs 46 clk per MMA and
@@ -330,8 +351,10 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         }
 #pragma unroll
         for (int o = 1; o < LPT; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (sub == 0) { ssq_local[t * 2] = ss; ssq_local[t * 2 + 1] = 0.f; }
+        if (sub == 0) hand_out_ss(t, ss);
     }
+    if (TOK == 64 && !x_by_tma && p.need_factor && tid < TOK)
+        hand_out_ss(tid, tid < p.M ? ssq_local[tid * 2] + (KB == 8 ? ssq_local[tid * 2 + 1] : 0.f) : 0.f);
     mbar_wait(done_bar, 0, abort_flag);                // (after an expired wait the sums are garbage and the status says so)
     __syncwarp();
     tc5::tc_fence_after();
@@ -340,8 +363,6 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     // + 64), and what a thread holds of four tokens goes as 16 bytes from registers to their owner's receive buffer
     // [src][4 tokens][column][4], which counts the bytes on its barrier; the own slice takes an ordinary store. (Staged in
     // shared memory and sent by bulk copies the exchange took 0.4 us longer.)
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has initialised its barriers
-    const int ts_sh = 31 - __clz(TS);
     const uint32_t red_mine = base + off_red + rank * (TS * 512u);
 #pragma unroll
     for (int h = 0; h < TOK / 64; ++h) {
@@ -364,19 +385,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         }
     }
     tc5::tc_fence_before();
-    __syncthreads();                                   // sums of squares complete, own slice stored, accumulators read
-    if (p.need_factor && tid < TOK && (tid >> ts_sh) < owners) {
-        const float ss = tid < p.M ? ssq_local[tid * 2] + (KB == 8 ? ssq_local[tid * 2 + 1] : 0.f) : 0.f;
-        const int r = tid >> ts_sh;
-        if (r == (int)rank) ssq_in[rank * TS + (tid & (TS - 1))] = ss;
-        else st_async1(map_to_cta(base + off_red + RED_BYTES + (rank * TS + (tid & (TS - 1))) * 4u, (uint32_t)r), map_to_cta(in_bar, (uint32_t)r), ss);
-    }
-    if (warp == 0) {
-        tc5::tc_fence_after();
-        tc5::tmem_dealloc(tmem, ACC_COLS);
-    }
-    if (p.need_factor) __syncthreads();                // the own sums of squares are in place
-
+    __syncthreads();                                   // own slice and sums stored, accumulators read
     FVLA_STAMP(4);
     // Owner phase: this CTA finishes tokens [rank*TS, rank*TS + TS), summing partials in rank order.
     if (i_own) mbar_wait(in_bar, 0, abort_flag, p.spin_limit ? p.spin_limit : tc5::kSpinLimit);
@@ -389,9 +398,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         const float* red = reinterpret_cast<const float*>(gen + off_red);
 #pragma unroll
         for (int j = 0; j < PRE; ++j) {
-            const int item = tid + j * THREADS, group = item / COLS, c = item % COLS;
-            const int tl = group * 4 + odd * 2, ta = (int)rank * TS + tl;
-            if (item >= items || (int)rank * TS + group * 4 >= p.M) continue;            // uniform within a warp
+            if (!work[j]) continue;
+            const int item = tid + j * THREADS, group = item / COLS, c = item % COLS, tl = group * 4 + odd * 2;
             auto sum_sources = [&](int col, float2 (&t)[2]) {
                 const float* src = red + (group * 128 + col) * 4;
                 float4 in[8];                              // all sources requested before the first is used
@@ -416,50 +424,45 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
                         const float2 q = *reinterpret_cast<const float2*>(ssq_in + s * TS + tl);
                         ss.x += q.x; ss.y += q.y;
                     }
-                const float inv_k = 1.0f / (float)p.K;
                 factor[0] = rsqrtf(ss.x * inv_k + 1e-6f);
                 factor[1] = rsqrtf(ss.y * inv_k + 1e-6f);
             }
             float2 v[2], up[2];
             sum_sources(c, v);
             if (EPI == EPI_GEGLU) sum_sources(64 + c, up);        // columns 0..63 of the tile are gate columns, 64..127 the matching up columns
-            const int n = tile * COLS + (c & ~1);
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int token = ta + i;
-                if (token >= p.M) break;
-                if (p.need_factor && p.factor_out && tile == 0 && c < 2) p.factor_out[token] = __float2bfloat16_rn(factor[i]);
+                if (!live[j][i]) break;
+                if (p.need_factor && p.factor_out && tile == 0 && c < 2) p.factor_out[(int)rank * TS + tl + i] = __float2bfloat16_rn(factor[i]);
                 const uint32_t p0 = i == 0 ? pre[j].x : pre[j].z, p1 = i == 0 ? pre[j].y : pre[j].w;
                 if (EPI == EPI_QKV_ROPE) {
                     float v0 = v[i].x * factor[i], v1 = v[i].y * factor[i];
-                    const int hd = p.head_dim, qd = p.heads * hd;
-                    const int kv_row = token + (int)((uint32_t)token * p.inv_group >> 20) * p.kv_skip;
-                    bf16* dst;
-                    if (n < qd + hd) {
+                    if (dst[j] != p.v) {
                         const float2 cs = unpack_bf16x2(p0);
                         const float r0 = v0 * cs.x - v1 * cs.y, r1 = v1 * cs.x + v0 * cs.y;
                         v0 = r0; v1 = r1;
-                        dst = n < qd ? p.q + (size_t)token * qd + n : p.k + (size_t)kv_row * hd + (n - qd);
-                    } else {
-                        dst = p.v + (size_t)kv_row * hd + (n - qd - hd);
                     }
-                    *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(v0, v1);
+                    *reinterpret_cast<uint32_t*>(dst[j] + at[j][i]) = pack_bf16x2(v0, v1);
                 } else if (EPI == EPI_GEGLU) {
                     const float f = factor[i];
-                    *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + (size_t)(row0 + token) * p.ldo + n) =
+                    *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + at[j][i]) =
                         pack_bf16x2(gelu_f(v[i].x * f) * (up[i].x * f), gelu_f(v[i].y * f) * (up[i].y * f));
                 } else {
                     // p0, p1 = bias (EPI_BIAS) or residual (EPI_RESIDUAL)
                     float v0 = v[i].x + __uint_as_float(p0), v1 = v[i].y + __uint_as_float(p1);
                     if (EPI == EPI_BIAS && p.act == 2) { v0 = silu_f(v0); v1 = silu_f(v1); }
-                    const size_t at = (size_t)(row0 + token) * p.ldo + n;
                     const uint32_t word = pack_bf16x2(v0, v1);
-                    if (p.out_shadow) *reinterpret_cast<uint32_t*>(p.out_shadow + at) = word;
-                    if (p.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(p.out) + at) = make_float2(v0, v1);
-                    else *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + at) = word;
+                    if (p.out_shadow) *reinterpret_cast<uint32_t*>(p.out_shadow + at[j][i]) = word;
+                    if (p.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(p.out) + at[j][i]) = make_float2(v0, v1);
+                    else *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + at[j][i]) = word;
                 }
             }
         }
+    }
+    if (warp == 0) {
+        __syncwarp();
+        tc5::tc_fence_after();
+        tc5::tmem_dealloc(tmem, ACC_COLS);
     }
     FVLA_STAMP(6);
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
@@ -524,8 +527,8 @@ inline bool skinny_supports(int M, int N, int K, bool geglu, bool bf16_operand) 
     return pl.ok && (pl.tok == 64 || bf16_operand);
 }
 
-template <int EPI, int TOK>
-inline int launch_skinny_tok(SkinnyArgs a, const SkinnyPlan& pl, const void* W, const void* W2, int ldw, cudaStream_t st) {
+template <int EPI, int TOK, int PRE>
+inline int launch_skinny_cfg(SkinnyArgs a, const SkinnyPlan& pl, const void* W, const void* W2, int ldw, cudaStream_t st) {
     a.splits = pl.splits; a.kblocks = pl.kblocks;
     const int groups = a.groups > 1 ? a.groups : 1;
     if (groups > 1 && (EPI == EPI_QKV_ROPE || a.need_factor || (a.x_f32 && a.x_shadow == nullptr))) {
@@ -533,7 +536,7 @@ inline int launch_skinny_tok(SkinnyArgs a, const SkinnyPlan& pl, const void* W, 
         return FVLA_ERR_UNSUPPORTED;
     }
     if (TOK > 64 && a.x_f32 && a.x_shadow == nullptr) { set_error("skinny gemm: more than 64 rows need a bf16 operand"); return FVLA_ERR_UNSUPPORTED; }
-    auto kern = skinny_gemm_kernel<EPI, TOK>;
+    auto kern = skinny_gemm_kernel<EPI, TOK, PRE>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -573,7 +576,11 @@ template <int EPI>
 inline int launch_skinny(const SkinnyArgs& a, const void* W, const void* W2, int ldw, cudaStream_t st) {
     const SkinnyPlan pl = plan_skinny(a.M, a.N, a.K, EPI == EPI_GEGLU, a.groups > 1 ? a.groups : 1);
     if (!pl.ok) { set_error("skinny gemm: shape %dx%dx%d not supported", a.M, a.N, a.K); return FVLA_ERR_UNSUPPORTED; }
-    return pl.tok == 64 ? launch_skinny_tok<EPI, 64>(a, pl, W, W2, ldw, st) : launch_skinny_tok<EPI, 128>(a, pl, W, W2, ldw, st);
+    const int items = pl.tok / pl.splits / 4 * (EPI == EPI_GEGLU ? 64 : 128);      // of an owner, THREADS at a time
+    if (pl.tok == 64)
+        return items <= THREADS ? launch_skinny_cfg<EPI, 64, 1>(a, pl, W, W2, ldw, st) : launch_skinny_cfg<EPI, 64, 4>(a, pl, W, W2, ldw, st);
+    return items <= THREADS ? launch_skinny_cfg<EPI, 128, 1>(a, pl, W, W2, ldw, st)
+                            : (items <= 2 * THREADS ? launch_skinny_cfg<EPI, 128, 2>(a, pl, W, W2, ldw, st) : launch_skinny_cfg<EPI, 128, 4>(a, pl, W, W2, ldw, st));
 }
 
 }  // namespace skinny
