@@ -372,7 +372,7 @@ __device__ __forceinline__ uint32_t dsm_map(uint32_t local_addr, uint32_t rank) 
     return r;
 }
 
-template <int KT>                                         // key tiles of 128 per CTA
+template <int KT, int SPL>                                // key tiles of 128 per CTA, cluster size
 __global__ void __launch_bounds__(decattn::THREADS, 1)
 decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV) {
     using namespace decattn;
@@ -390,7 +390,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     FVLA_STAMP(0);
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    const int SPL = p.splits, q0 = blockIdx.x * BQ, rows_here = min(BQ, p.nq - q0), units = (rows_here + UNIT - 1) / UNIT;
+    const int q0 = blockIdx.x * BQ, rows_here = min(BQ, p.nq - q0), units = (rows_here + UNIT - 1) / UNIT;
     const float scale = p.scale_log2;
     const int pre_rows = min(p.prefix_keys, p.nk);
     const int key0 = (int)rank * p.kp, prefix_here = max(0, min(p.kp, pre_rows - key0));        // local keys [0, prefix_here): prefix
@@ -484,6 +484,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     // no data is handed over, and a releasing arrive waits 0.4 us for the thread's earlier accesses.
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     FVLA_STAMP(3);
+    const uint64_t vd = tc5::smem_desc(sV + warp * 2 * p.pad * 128, p.pad * 128, 1024), pd = tc5::smem_desc(sQ, 16, 1024);      // warps 0, 1: operands of O^T
     const int quad = warp & 3, half = warp >> 2;             // keys 32 quad .. + 31 of a tile, rows 16 half .. + 15
     {
         float v[KT][16], red[16];
@@ -544,9 +545,9 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         __syncthreads();
         if (lane == 0 && warp < 2) {
             tc5::tc_fence_after();
-            const uint64_t a0 = tc5::smem_desc(sV + warp * 2 * p.pad * 128, p.pad * 128, 1024), b0 = tc5::smem_desc(sQ, 16, 1024);
-            for (int k = 0; k < p.pad / 16; ++k)
-                tc5::umma_bf16(tmem + warp * 32, a0 + k * 128, b0 + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true), k ? 1u : 0u);
+#pragma unroll
+            for (int k = 0; k < (KT == 1 ? 8 : MAX_PAD / 16); ++k)
+                if (k * 16 < p.pad) tc5::umma_bf16(tmem + warp * 32, vd + k * 128, pd + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true), k ? 1u : 0u);
             tc5::umma_commit(o_bar);
         }
         __syncwarp();
@@ -591,21 +592,25 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         // log-sum-exp weights: lane = (source, row), a second one for sources 8 and up
         const int s0 = lane >> 2;
         const uint32_t st = stats_in + s0 * 64 + slot * 32 + (lane & 3) * 8;
-        const float m0 = s0 < SPL ? lds1(st) : NO_KEY, m1 = s0 + 8 < SPL ? lds1(st + 512) : NO_KEY;
+        const bool have0 = SPL >= 8 || s0 < SPL, have1 = SPL > 8 && s0 + 8 < SPL;
+        const float m0 = have0 ? lds1(st) : NO_KEY, m1 = have1 ? lds1(st + 512) : NO_KEY;
         float mx = fmaxf(m0, m1);
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        float w0 = s0 < SPL ? ex2(m0 - mx) : 0.f, w1 = s0 + 8 < SPL ? ex2(m1 - mx) : 0.f;
-        float wsum = (s0 < SPL ? w0 * lds1(st + 4) : 0.f) + (s0 + 8 < SPL ? w1 * lds1(st + 516) : 0.f);
+        float w0 = have0 ? ex2(m0 - mx) : 0.f, w1 = have1 ? ex2(m1 - mx) : 0.f;
+        float wsum = (have0 ? w0 * lds1(st + 4) : 0.f) + (have1 ? w1 * lds1(st + 516) : 0.f);
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
         const float inv = wsum > 0.f ? 1.0f / wsum : 0.f;
         w0 *= inv; w1 *= inv;
         float acc[UNIT] = {0.f, 0.f, 0.f, 0.f};
         const uint32_t src = sK + slot * SPL * UNIT_BYTES + tid * 16;
-#pragma unroll 4
+        float4 in[SPL];                                       // all sources requested before the first is used
+#pragma unroll
+        for (int s = 0; s < SPL; ++s) in[s] = lds4(src + s * UNIT_BYTES);
+#pragma unroll
         for (int s = 0; s < SPL; ++s) {
-            const float4 a = lds4(src + s * UNIT_BYTES);
+            const float4 a = in[s];
             const float w = s < 8 ? w0 : w1;
             const int from = (s & 7) * 4;
             acc[0] = fmaf(__shfl_sync(0xffffffffu, w, from), a.x, acc[0]);
@@ -633,10 +638,20 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 3);
 }
 
+using DecAttnKernel = void (*)(const DecAttnArgs, const CUtensorMap, const CUtensorMap);
+template <int KT>
+inline DecAttnKernel decoder_attention_kernel(int spl) {
+    static const DecAttnKernel table[] = {decoder_attention_cluster_kernel<KT, 4>, decoder_attention_cluster_kernel<KT, 5>, decoder_attention_cluster_kernel<KT, 6>,
+                                          decoder_attention_cluster_kernel<KT, 7>, decoder_attention_cluster_kernel<KT, 8>, decoder_attention_cluster_kernel<KT, 9>,
+                                          decoder_attention_cluster_kernel<KT, 10>, decoder_attention_cluster_kernel<KT, 11>};
+    return table[spl - decattn::MIN_SPL];
+}
 inline bool configure_decoder_attention() {
     static PerDeviceFlag configured;
     if (configured.get()) return true;
-    for (auto kern : {decoder_attention_cluster_kernel<1>, decoder_attention_cluster_kernel<2>}) {
+    for (int i = 0; i < 2 * (decattn::MAX_SPL - decattn::MIN_SPL + 1); ++i) {
+        const int spl = decattn::MIN_SPL + i / 2;
+        const DecAttnKernel kern = i & 1 ? decoder_attention_kernel<2>(spl) : decoder_attention_kernel<1>(spl);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);      // clusters of 9..11
         if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return false; }
@@ -658,7 +673,7 @@ inline int resident_attention_clusters(int spl) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = spl; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&n, decoder_attention_cluster_kernel<1>, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 1; }
+        if (cudaOccupancyMaxActiveClusters(&n, decoder_attention_kernel<1>(spl), &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = 1; }
         c.store(n, std::memory_order_release);
     }
     return n;
@@ -708,7 +723,7 @@ inline int launch_decoder_attention_cluster(const DecAttnArgs& a, bool pdl, cuda
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, a.pad > 128 ? decoder_attention_cluster_kernel<2> : decoder_attention_cluster_kernel<1>, a, tmK, tmV);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, a.pad > 128 ? decoder_attention_kernel<2>(a.splits) : decoder_attention_kernel<1>(a.splits), a, tmK, tmV);
     if (e != cudaSuccess) { set_error("decoder_attention_cluster_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
     return check_launch("decoder_attention_cluster_kernel");
 }

@@ -56,7 +56,6 @@ struct SkinnyArgs {
     int M, N, K;
     int groups;                               // independent row groups of M rows each, laid end to end (grid.z); 0 or 1 = one
     int kblocks;                              // 64-wide k-blocks per CTA (K / 64 / splits)
-    int splits;                               // cluster size along K
     int need_factor;                          // compute rsqrt(mean(x^2)+1e-6) per token
     // epilogue operands
     void* out; int out_f32; int ldo;          // RESIDUAL / BIAS / GEGLU destination
@@ -110,7 +109,7 @@ __device__ __forceinline__ void st_async1(uint32_t dst, uint32_t bar, float a) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(dst), "f"(a), "r"(bar) : "memory");
 }
 
-template <int EPI, int TOK, int PRE>        // PRE: owner work items per thread
+template <int EPI, int TOK, int S>          // S: cluster size along K
 __global__ void __launch_bounds__(THREADS, 1)
 skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                    const __grid_constant__ CUtensorMap tmX) {
@@ -120,7 +119,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     constexpr uint32_t XB = TOK * 128, RED_BYTES = TOK * 512, ACC_COLS = 2 * TOK;      // one accumulator per issuing thread
     // The upper warps add up the rows' squares: the MMA issuers' warps come too late for it (gate/up: 1.6 us after the last MMA)
     constexpr int SSQ_WARPS = 8;
-    const int KB = p.kblocks, S = p.splits, TS = TOK / S, NS = slots_of(TOK, KB);
+    constexpr int TS = TOK / S, COLS = EPI == EPI_GEGLU ? 64 : 128, ITEMS = TS / 4 * COLS, PRE = (ITEMS + THREADS - 1) / THREADS;      // owner: tokens, work items, per thread
+    const int KB = p.kblocks, NS = slots_of(TOK, KB);
     const uint32_t w_bytes = NS * 16384u;
     const uint32_t sW = base, sX = sW + w_bytes;
     const uint32_t off_red = w_bytes + NS * XB;
@@ -198,8 +198,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     // Owner work items: (4 tokens of this rank's slice) x (column); after two lanes have swapped, a lane finishes two tokens
     // (ta, ta + 1) of two adjacent columns.
     // All index arithmetic is done here too: what follows the exchange is on the critical path of 16 warps.
-    constexpr int COLS = (EPI == EPI_GEGLU) ? 64 : 128;
-    const int items = (TS >> 2) * COLS, odd = lane & 1;
+    const int odd = lane & 1;
     const float inv_k = 1.0f / (float)p.K;
     uint4 pre[PRE];
     bf16* dst[PRE];                                           // QKV: Q, K or V
@@ -210,7 +209,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         pre[j] = make_uint4(0, 0, 0, 0);
         dst[j] = nullptr;
         const int item = tid + j * THREADS, c = item % COLS & ~1, n = tile * COLS + c, t4 = (int)rank * TS + item / COLS * 4, ta = t4 + odd * 2;
-        work[j] = item < items && t4 < p.M;                   // uniform within a warp
+        work[j] = item < ITEMS && t4 < p.M;                   // uniform within a warp
         live[j][0] = work[j] && ta < p.M;
         live[j][1] = work[j] && ta + 1 < p.M;
         if (EPI == EPI_QKV_ROPE) {
@@ -292,9 +291,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     tc5::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // every peer has initialised its barriers
-    const int ts_sh = 31 - __clz(TS);
     auto hand_out_ss = [&](int t, float ss) {          // a row's sum of squares over this CTA's K slice, to the row's owner
-        const int r = t >> ts_sh, slot = (int)rank * TS + (t & (TS - 1));
+        const int r = t / TS, slot = (int)rank * TS + t % TS;
         if (r == (int)rank) ssq_in[slot] = ss;
         else if (r < owners) st_async1(map_to_cta(base + off_red + RED_BYTES + slot * 4u, (uint32_t)r), map_to_cta(in_bar, (uint32_t)r), ss);
     };
@@ -377,9 +375,9 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         }
 #pragma unroll
         for (int t = 0; t < 16; t += 4) {
-            const int token = g * 16 + t, r = token >> ts_sh;
+            const int token = g * 16 + t, r = token / TS;
             if (token >= p.M) break;
-            const uint32_t at = red_mine + (uint32_t)((token & (TS - 1)) >> 2) * 2048u + (q * 32 + lane) * 16u;
+            const uint32_t at = red_mine + (uint32_t)((token % TS) >> 2) * 2048u + (q * 32 + lane) * 16u;
             if (r == (int)rank) *reinterpret_cast<float4*>(gen + (at - base)) = make_float4(part[t], part[t + 1], part[t + 2], part[t + 3]);
             else st_async4(map_to_cta(at, (uint32_t)r), map_to_cta(in_bar, (uint32_t)r), part[t], part[t + 1], part[t + 2], part[t + 3]);
         }
@@ -402,14 +400,12 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
             const int item = tid + j * THREADS, group = item / COLS, c = item % COLS, tl = group * 4 + odd * 2;
             auto sum_sources = [&](int col, float2 (&t)[2]) {
                 const float* src = red + (group * 128 + col) * 4;
-                float4 in[8];                              // all sources requested before the first is used
+                float4 in[S];                              // all sources requested before the first is used
 #pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    if (s < S) in[s] = *reinterpret_cast<const float4*>(src + s * TS * 128);
+                for (int s = 0; s < S; ++s) in[s] = *reinterpret_cast<const float4*>(src + s * TS * 128);
                 float4 a = in[0];
 #pragma unroll
-                for (int s = 1; s < 8; ++s)
-                    if (s < S) { a.x += in[s].x; a.y += in[s].y; a.z += in[s].z; a.w += in[s].w; }
+                for (int s = 1; s < S; ++s) { a.x += in[s].x; a.y += in[s].y; a.z += in[s].z; a.w += in[s].w; }
                 // swap with the lane of the neighbouring column: even lanes keep tokens 0, 1, odd lanes 2, 3
                 const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a.x : a.z, 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? a.y : a.w, 1);
                 t[0] = odd ? make_float2(r0, a.z) : make_float2(a.x, r0);
@@ -419,11 +415,10 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
             if (p.need_factor) {
                 float2 ss = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    if (s < S) {
-                        const float2 q = *reinterpret_cast<const float2*>(ssq_in + s * TS + tl);
-                        ss.x += q.x; ss.y += q.y;
-                    }
+                for (int s = 0; s < S; ++s) {
+                    const float2 q = *reinterpret_cast<const float2*>(ssq_in + s * TS + tl);
+                    ss.x += q.x; ss.y += q.y;
+                }
                 factor[0] = rsqrtf(ss.x * inv_k + 1e-6f);
                 factor[1] = rsqrtf(ss.y * inv_k + 1e-6f);
             }
@@ -527,16 +522,16 @@ inline bool skinny_supports(int M, int N, int K, bool geglu, bool bf16_operand) 
     return pl.ok && (pl.tok == 64 || bf16_operand);
 }
 
-template <int EPI, int TOK, int PRE>
+template <int EPI, int TOK, int S>
 inline int launch_skinny_cfg(SkinnyArgs a, const SkinnyPlan& pl, const void* W, const void* W2, int ldw, cudaStream_t st) {
-    a.splits = pl.splits; a.kblocks = pl.kblocks;
+    a.kblocks = pl.kblocks;
     const int groups = a.groups > 1 ? a.groups : 1;
     if (groups > 1 && (EPI == EPI_QKV_ROPE || a.need_factor || (a.x_f32 && a.x_shadow == nullptr))) {
         set_error("skinny gemm: row groups are only built for the bias / residual forms with a bf16 operand");
         return FVLA_ERR_UNSUPPORTED;
     }
     if (TOK > 64 && a.x_f32 && a.x_shadow == nullptr) { set_error("skinny gemm: more than 64 rows need a bf16 operand"); return FVLA_ERR_UNSUPPORTED; }
-    auto kern = skinny_gemm_kernel<EPI, TOK, PRE>;
+    auto kern = skinny_gemm_kernel<EPI, TOK, S>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -576,11 +571,18 @@ template <int EPI>
 inline int launch_skinny(const SkinnyArgs& a, const void* W, const void* W2, int ldw, cudaStream_t st) {
     const SkinnyPlan pl = plan_skinny(a.M, a.N, a.K, EPI == EPI_GEGLU, a.groups > 1 ? a.groups : 1);
     if (!pl.ok) { set_error("skinny gemm: shape %dx%dx%d not supported", a.M, a.N, a.K); return FVLA_ERR_UNSUPPORTED; }
-    const int items = pl.tok / pl.splits / 4 * (EPI == EPI_GEGLU ? 64 : 128);      // of an owner, THREADS at a time
     if (pl.tok == 64)
-        return items <= THREADS ? launch_skinny_cfg<EPI, 64, 1>(a, pl, W, W2, ldw, st) : launch_skinny_cfg<EPI, 64, 4>(a, pl, W, W2, ldw, st);
-    return items <= THREADS ? launch_skinny_cfg<EPI, 128, 1>(a, pl, W, W2, ldw, st)
-                            : (items <= 2 * THREADS ? launch_skinny_cfg<EPI, 128, 2>(a, pl, W, W2, ldw, st) : launch_skinny_cfg<EPI, 128, 4>(a, pl, W, W2, ldw, st));
+        switch (pl.splits) {
+            case 1: return launch_skinny_cfg<EPI, 64, 1>(a, pl, W, W2, ldw, st);
+            case 2: return launch_skinny_cfg<EPI, 64, 2>(a, pl, W, W2, ldw, st);
+            case 4: return launch_skinny_cfg<EPI, 64, 4>(a, pl, W, W2, ldw, st);
+            default: return launch_skinny_cfg<EPI, 64, 8>(a, pl, W, W2, ldw, st);
+        }
+    switch (pl.splits) {
+        case 2: return launch_skinny_cfg<EPI, 128, 2>(a, pl, W, W2, ldw, st);
+        case 4: return launch_skinny_cfg<EPI, 128, 4>(a, pl, W, W2, ldw, st);
+        default: return launch_skinny_cfg<EPI, 128, 8>(a, pl, W, W2, ldw, st);
+    }
 }
 
 }  // namespace skinny
