@@ -251,7 +251,10 @@ struct Tc5Cfg {
 // NORM: the row norm of A is folded in (GemmArgs::norm_mode): the epilogue warps also consume every operand stage,
 // so a stage returns to the producer after the MMAs AND the eight epilogue warps have read it. Meant for one tile
 // per CTA; with more, a tile's statistics wait for the previous tile's epilogue (correct, but the overlap is lost).
-template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, bool NORM = false>
+// EP: what the staged epilogue does, as a set of EP_* bits, so that it carries no run-time choices (they cost as much as
+// the arithmetic); EP_ANY reads it from GemmArgs.
+constexpr int EP_ANY = -1, EP_BIAS = 1, EP_RES = 2, EP_GELU = 4, EP_ROPE = 8;      // EP_ROPE: with rounding first, as the prefix encoder's
+template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, bool NORM = false, int EP = EP_ANY>
 __global__ void __launch_bounds__(320, 1)
 tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                 const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2) {
@@ -396,7 +399,10 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
         uint8_t* stg = smem_gen + STAGES * Cfg::STAGE_BYTES + Cfg::BAR_BYTES + ew * Cfg::EPI_STAGE_BYTES;
         // staged path: bf16 destination(s); the preloaded operand is the bf16 residual or, for the RoPE +
         // scatter epilogue, the cos/sin entries of the chunk (one or the other)
-        const bool plain = !p.c_f32 && (ROPE ? !(p.R != nullptr || p.bias != nullptr || p.act != 0) : p.rope == nullptr);
+        const bool plain = EP != EP_ANY || (!p.c_f32 && (ROPE ? !(p.R != nullptr || p.bias != nullptr || p.act != 0) : p.rope == nullptr));
+        const bool with_rope = ROPE && (EP != EP_ANY || p.rope != nullptr), round_first = EP != EP_ANY || p.round_first;
+        const bool has_res = EP != EP_ANY ? (EP & EP_RES) != 0 : p.R != nullptr;
+        const int act = EP != EP_ANY ? ((EP & EP_GELU) ? 1 : 0) : p.act;
         const int rope_qd = p.heads * p.head_dim;            // RoPE epilogue: columns [0, qd) are Q, then K, then V
         const int sr = lane >> 2, sp = lane & 3;              // staged access: row sr + 8 i, 16-byte piece sp
         uint32_t tcount = 0;
@@ -416,7 +422,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
             // Per-column constants of this tile (bias; column sums for the folded LayerNorm) go to shared memory
             // as fp32, one column per thread; the chunk loop reads them back as broadcast 16-byte loads. Two sets,
             // alternating with the accumulator stage, so a warp that runs ahead never overwrites values in use.
-            const bool has_bias = p.bias != nullptr || p.bias_f32 != nullptr;
+            const bool has_bias = EP != EP_ANY ? (EP & EP_BIAS) != 0 : p.bias != nullptr || p.bias_f32 != nullptr;
             float* colc = reinterpret_cast<float*>(smem_gen + STAGES * Cfg::STAGE_BYTES + Cfg::BAR_BYTES + Cfg::EPI_WARPS * Cfg::EPI_STAGE_BYTES + Cfg::NORM_BYTES) + acc * 2 * BN;
             {
                 const int t = (int)threadIdx.x - 64, col = (t_idx / args.tiles_m) * BN + t;
@@ -424,7 +430,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                     float bv = 0.f, cv = 0.f;
                     if (col < p.N) {
                         bv = p.bias_f32 ? __ldg(p.bias_f32 + col) : (p.bias ? __bfloat162float(__ldg(p.bias + col)) : 0.f);
-                        if (NORM && p.colsum) cv = __ldg(p.colsum + col);
+                        if (NORM && (EP != EP_ANY ? !ROPE : p.colsum != nullptr)) cv = __ldg(p.colsum + col);
                     }
                     colc[t] = bv;
                     if (NORM) colc[BN + t] = cv;
@@ -438,10 +444,10 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                     rco[c][i] = make_uint4(0, 0, 0, 0);
                     if (sym && c != whalf) continue;
                     const int grow = m0 + quad * 32 + sr + 8 * i, gcol = n0 + c * 32 + sp * 8;
-                    if (ROPE && plain && p.rope) {
+                    if (ROPE && plain && with_rope) {
                         if (grow < p.M && gcol < rope_qd + p.head_dim)
                             rco[c][i] = __ldg(reinterpret_cast<const uint4*>(p.rope + (size_t)rope_row(p, grow) * p.head_dim + (gcol % p.head_dim)));
-                    } else if (plain && p.R && grow < p.M && gcol < p.N) {
+                    } else if (plain && has_res && grow < p.M && gcol < p.N) {
                         const int rr = p.res_mod > 0 ? grow % p.res_mod : grow;
                         rco[c][i] = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.R) + (size_t)rr * p.ldr + gcol);
                     }
@@ -478,7 +484,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                 // both threads of a row add the two halves in the same order
                 const float t1 = whalf == 0 ? s1 + other.x : other.x + s1, t2 = whalf == 0 ? s2 + other.y : other.y + s2;
                 const float invk = 1.f / (float)p.K;
-                if (p.norm_mode == 2) {
+                if (EP != EP_ANY ? !ROPE : p.norm_mode == 2) {
                     nrm_mean = t1 * invk;
                     nrm_rstd = rsqrtf(t2 * invk - nrm_mean * nrm_mean + 1e-5f);
                 } else {
@@ -646,7 +652,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                 }
                 if (plain) {
                     float res[32];
-                    if (p.R || (ROPE && p.rope)) {
+                    if (has_res || with_rope) {
                         // residual arrives coalesced (8 rows x 64 B per request); hand each thread its own row
 #pragma unroll
                         for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(stg + (sr + 8 * i) * 80 + sp * 16) = rco[c][i];
@@ -665,7 +671,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                     const float* colc_chunk = colc + chalf * HALF + c * 32;
                     if (NORM) {
                         // the norm of this thread's row, applied to the raw product
-                        if (p.norm_mode == 2) {
+                        if (EP != EP_ANY ? !ROPE : p.norm_mode == 2) {
 #pragma unroll
                             for (int j = 0; j < 32; j += 4) {
                                 const float4 cs = *reinterpret_cast<const float4*>(colc_chunk + BN + j);
@@ -692,20 +698,20 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float v = act(a[j]);
-                            a[j] = p.R ? v + res[j] : v;
+                            a[j] = has_res ? v + res[j] : v;
                         }
                     };
                     const int col0 = n0 + c * 32;                  // first column of this chunk
                     bf16* out_base = static_cast<bf16*>(p.C);
                     int out_ld = p.ldc, out_col = col0;
                     bool kv_dst = false;                           // K / V destination: rows follow the sequence-group mapping
-                    if (ROPE && p.rope) {
+                    if (with_rope) {
                         // res[] holds this row's 16 (cos, sin) pairs for the chunk's 16 column pairs
                         if (col0 < rope_qd + p.head_dim) {
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
                                 float x0 = a[2 * i], x1 = a[2 * i + 1];
-                                if (p.round_first) { x0 = round_bf16(x0); x1 = round_bf16(x1); }
+                                if (round_first) { x0 = round_bf16(x0); x1 = round_bf16(x1); }
                                 a[2 * i] = x0 * res[2 * i] - x1 * res[2 * i + 1];
                                 a[2 * i + 1] = x1 * res[2 * i] + x0 * res[2 * i + 1];
                             }
@@ -713,8 +719,8 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                         if (col0 < rope_qd) { out_base = p.q; out_ld = rope_qd; }
                         else if (col0 < rope_qd + p.head_dim) { out_base = p.k; out_ld = p.head_dim; out_col = col0 - rope_qd; kv_dst = true; }
                         else { out_base = p.v; out_ld = p.head_dim; out_col = col0 - rope_qd - p.head_dim; kv_dst = true; }
-                    } else if (p.act == 1) finish([](float v) { return gelu_f(v); });
-                    else if (p.act == 2) finish([](float v) { return silu_f(v); });
+                    } else if (act == 1) finish([](float v) { return gelu_f(v); });
+                    else if (act == 2) finish([](float v) { return silu_f(v); });
                     else finish([](float v) { return v; });
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
@@ -870,10 +876,10 @@ inline Tc5Plan plan_tc5(int M, int N, int K, bool ws_ok) {
     return best;
 }
 
-template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, bool NORM = false>
-inline int launch_tc5_cfg(const GemmArgs& g, int* status, cudaStream_t st, int splits = 1, void* ws = nullptr) {
+template <int BN, bool DUAL, int STAGES, bool ROPE, bool CLUSTER, bool NORM, int EP>
+inline int launch_tc5_ep(const GemmArgs& g, int* status, cudaStream_t st, int splits, void* ws) {
     using Cfg = Tc5Cfg<BN, DUAL, STAGES>;
-    auto kern = tc5_gemm_kernel<BN, DUAL, STAGES, ROPE, CLUSTER, NORM>;
+    auto kern = tc5_gemm_kernel<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
@@ -922,6 +928,31 @@ inline int launch_tc5_cfg(const GemmArgs& g, int* status, cudaStream_t st, int s
     }
     if (e != cudaSuccess) { set_error("tc5_gemm_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
     return check_launch("tc5_gemm_kernel");
+}
+
+// The epilogues of the model's call sites have kernels of their own, anything else takes the run-time one.
+template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, bool NORM = false>
+inline int launch_tc5_cfg(const GemmArgs& g, int* status, cudaStream_t st, int splits = 1, void* ws = nullptr) {
+    if constexpr (!DUAL && !ROPE) {
+        const bool bias = g.bias != nullptr || g.bias_f32 != nullptr;
+        if (!g.c_f32 && g.rope == nullptr && g.act <= 1) {
+            if constexpr (NORM) {
+                if (g.norm_mode != 2) return FVLA_ERR_UNSUPPORTED;
+                if (bias && g.R == nullptr && g.act == 0) return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_BIAS>(g, status, st, splits, ws);
+                if (bias && g.R == nullptr) return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_BIAS | EP_GELU>(g, status, st, splits, ws);
+            } else {
+                if (bias && g.R == nullptr && g.act == 0) return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_BIAS>(g, status, st, splits, ws);
+                if (bias && g.R == nullptr) return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_BIAS | EP_GELU>(g, status, st, splits, ws);
+                if (bias && g.act == 0) return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_BIAS | EP_RES>(g, status, st, splits, ws);
+                if (!bias && g.act == 0 && g.R != nullptr) return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_RES>(g, status, st, splits, ws);
+            }
+        }
+    }
+    if constexpr (ROPE) {
+        if (g.rope != nullptr && g.round_first && g.R == nullptr && g.bias == nullptr && g.bias_f32 == nullptr && g.act == 0)
+            return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ROPE>(g, status, st, splits, ws);
+    }
+    return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ANY>(g, status, st, splits, ws);
 }
 
 // Shapes this path takes: at least one full 128-row tile of work and 16-byte aligned rows.
