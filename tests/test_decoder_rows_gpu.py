@@ -74,3 +74,22 @@ def test_decoder_attention_by_shape(tokens, S, episodes):
         O.op_table(True).decoder_attention(Q[e].float(), K[e].float(), V[e].float(), None, ref, S)
         assert_close(q.view(episodes, -1, 256)[e], ref, what=f"decoder_attention, episode {e}")
     assert _lib.load().fvla_device_status(None) == 0
+
+
+# prefix QKV with the row norm inside the GEMM by tile width (128, 192, 256 columns; the last with a ragged row tile), and past
+# it, where the norm is a kernel of its own
+@pytest.mark.parametrize("S", [257, 769, 1281, 1793])
+def test_prefix_qkv_by_tile_width(S):
+    from flash_vla_b200 import op_table
+    g = torch.Generator().manual_seed(S)
+    x, w, rope = rnd(g, S, 2048, scale=2.0), rnd(g, 2048, 2560, scale=0.02), O.rope_table(S, 0)
+    outs = []
+    for fused in (True, False):
+        Q, K, V = (torch.zeros(n, 256, dtype=bf16, device="cuda") for n in (S * 8, S, S))
+        op_table(fused).encoder_norm_qkv_rope(x.cuda(), w.cuda(), rope.cuda(), Q, K, V, torch.zeros(S, 2048, dtype=bf16, device="cuda"))
+        outs.append((Q, K, V))
+    refs = [torch.zeros(S * 8, 256), torch.zeros(S, 256), torch.zeros(S, 256)]
+    O.op_table(False).encoder_norm_qkv_rope(x.float(), w.float(), rope.float(), *refs, torch.zeros(S, 2048))
+    for got in outs:
+        for a, b, what in zip(got, refs, "Q K V".split()):
+            assert_close(a, b, rtol=2e-2, atol_rms=4e-2, what=f"encoder_norm_qkv_rope.{what}")
