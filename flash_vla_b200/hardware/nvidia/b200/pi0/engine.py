@@ -11,12 +11,10 @@ episodes that share the weights:
   * SigLIP and the prefix encoder run ONCE over all episodes' tokens (M = E x S rows): every vision and
     prefix weight (4.8 of the 5.4 GB) is streamed once for the whole batch and the GEMMs have E times
     the tiles to fill the GPU with; only the attention kernels, which mix tokens, run per episode;
-  * each episode has its own KV cache; the action-expert decoder also runs ONCE over all episodes' rows
-    (M = E x 51): QKV and the gated FFN as one GEMM over all rows, the two residual projections as the
-    weight-streaming cluster GEMM once per episode inside one launch, attention for all episodes in one
-    launch of the tcgen05 flash kernel (one grid row per episode, each against its own KV cache). At 2
-    episodes (or with `batch_decoder=False`) the decoders run as E single-episode decoders on E streams
-    instead, which fill each other's idle SMs and are the faster form there.
+  * each episode has its own KV cache; the action-expert decoder also runs over several episodes' rows at once: one
+    or two groups of episodes (`decoder_groups`) on streams of their own, where they fill each other's idle SMs. Every
+    projection runs once over a group's rows, attention for all its episodes in one launch. With `batch_decoder=False` the decoders
+    run as E single-episode decoders on E streams instead.
     Decoder layer L starts as soon as the batched encoder has produced layer L's prefix K/V.
 `batch_prefix=False` keeps the older form (E complete single-episode passes on E streams), whose
 per-episode results are bit-identical to the single-episode engine; the batched form runs the same
@@ -33,6 +31,21 @@ from . import pipeline
 from .backends.cuda import wrappers
 from .buffers import allocate_batched_buffers, allocate_batched_decoder_buffers, allocate_static_buffers
 from .ops import op_table
+
+
+MAX_GROUP_ROWS = 128       # rows that the weight-streaming decoder GEMM takes
+
+
+def decoder_groups(episodes: int, rows: int):
+    """Episodes whose decoders run as one batch, as (first, last + 1) pairs: one or two groups that the weight-streaming
+    GEMM takes, else one group on the general kernels. Measured, ms per replay, two groups against one: 17.6 / 19.4 for
+    three episodes of 51 rows, 23.2 / 23.8 for four; more groups lose (four of 65 rows 18.4 / 15.1, eight episodes in four
+    groups 42.3 / 40.4): every group streams the weights for itself."""
+    count = -(-episodes // max(1, MAX_GROUP_ROWS // rows))
+    if count > 2:
+        count = 1
+    cuts = [episodes * i // count for i in range(count + 1)]
+    return list(zip(cuts, cuts[1:]))
 
 
 class Pi0Inference:
@@ -88,27 +101,30 @@ class Pi0Inference:
             self.weights[name] = value.to(device=device, dtype=torch.bfloat16).contiguous()
         self.episode_buffers, self.pools = [], []
         self.batch_prefix = bool(batch_prefix) and episodes > 1
-        # measured on B200: the batched decoder beats concurrent single-episode decoders from 3 episodes on
-        # (E = 3: 11.2 against 13.0 ms, E = 4: 11.7 against 17.4 ms) and loses at 2 (11.5 against 9.1 ms)
         if batch_decoder is None:
-            batch_decoder = episodes >= 3
+            batch_decoder = episodes >= 2
         self.batch_decoder = self.batch_prefix and bool(batch_decoder)
-        self.prefix_buffers, self.prefix_pool, self.decoder_buffers = None, None, None
+        self.prefix_buffers, self.prefix_pool, self.decoder_groups, self.streams = None, None, [], []
         if self.batch_prefix:
             self.prefix_buffers, self.episode_buffers, self.encoder_seq_len = allocate_batched_buffers(
                 num_views, chunk_size, self.prompt_len, episodes, device)
             self.prefix_pool = ScratchPool()
         if self.batch_decoder:
-            self.decoder_buffers = allocate_batched_decoder_buffers(chunk_size, episodes, self.encoder_seq_len, device)
-            if episodes * (chunk_size + 1) <= 128:        # few enough rows for the weight-streaming GEMM, which reads bf16 rows
-                wrappers.register_bf16_shadow(self.decoder_buffers["decoder_x"], self.decoder_buffers["decoder_x_bf16"])
-            self.decoder_pool = ScratchPool()
-            self.pools = [self.decoder_pool]
-            self._batched_observation_state_normalized = self.decoder_buffers["observation_state_normalized"]
-            self._batched_diffusion_noise = self.decoder_buffers["diffusion_noise"]
+            for name in ("observation_state_normalized", "diffusion_noise"):
+                shape = (episodes,) + tuple(self.episode_buffers[0][name].shape)
+                setattr(self, "_batched_" + name, torch.zeros(shape, dtype=torch.bfloat16, device=device))
             self._batched_observation_images_normalized = self.prefix_buffers["observation_images_normalized"].view(
                 episodes, num_views, 224, 224, 3)
-            self.streams = [torch.cuda.Stream(device=device)]
+            for first, last in decoder_groups(episodes, chunk_size + 1):
+                group = allocate_batched_decoder_buffers(chunk_size, last - first, self.encoder_seq_len, device)
+                if (last - first) * (chunk_size + 1) <= MAX_GROUP_ROWS:      # the weight-streaming GEMM reads bf16 rows
+                    wrappers.register_bf16_shadow(group["decoder_x"], group["decoder_x_bf16"])
+                for name in ("observation_state_normalized", "diffusion_noise"):
+                    group[name] = getattr(self, "_batched_" + name)[first:last]
+                caches = {name: self.prefix_buffers[name][first:last] for name in ("encoder_K", "encoder_V")}
+                self.decoder_groups.append((group, caches, last - first))
+                self.pools.append(ScratchPool())
+                self.streams.append(torch.cuda.Stream(device=device))
         elif self.batch_prefix:
             for buffers in self.episode_buffers:
                 wrappers.register_bf16_shadow(buffers["decoder_x"], buffers["decoder_x_bf16"])
@@ -170,28 +186,31 @@ class Pi0Inference:
                                          steps=self.steps, layers=self.layers, first_step=1)
 
     def _run_fully_batched(self):
-        """Throughput plan with the decoder batched as well: prefix pass on the current stream, the one
-        batched decoder on a second stream, its first step one layer behind the encoder."""
-        E, S, p, d = self.episodes, self.encoder_seq_len, self.prefix_buffers, self.decoder_buffers
-        main, side = torch.cuda.current_stream(), self.streams[0]
+        """Throughput plan with the decoder batched as well: prefix pass on the current stream, the decoder
+        groups on streams of their own, their first step one layer behind the encoder."""
+        E, S, p = self.episodes, self.encoder_seq_len, self.prefix_buffers
+        main = torch.cuda.current_stream()
         self._write_prompt_rows()
-        side.wait_stream(main)
-        with torch.cuda.stream(side), wrappers.use_pool(self.decoder_pool):
-            pipeline.decoder_prologue_batched(self.ops, self.weights, d)
+        for (d, _, _), side, pool in zip(self.decoder_groups, self.streams, self.pools):
+            side.wait_stream(main)
+            with torch.cuda.stream(side), wrappers.use_pool(pool):
+                pipeline.decoder_prologue_batched(self.ops, self.weights, d)
         kv_ready = [torch.cuda.Event() for _ in range(pipeline.ENCODER_LAYERS)]
         with wrappers.use_pool(self.prefix_pool):
             pipeline.vision_encoder(self.ops, self.weights, p, self.num_views)
             pipeline.transformer_encoder_batched(self.ops, self.weights, p, S, self.num_views, E,
                                                  after_qkv=lambda layer: kv_ready[layer].record(main),
                                                  per_episode=self._attention_fork())
-        with torch.cuda.stream(side), wrappers.use_pool(self.decoder_pool):
-            if self.steps == 0:
-                side.wait_event(kv_ready[-1])
-            for step in range(self.steps):
-                gate = (lambda layer: side.wait_event(kv_ready[layer])) if step == 0 else None
-                pipeline.decoder_step_batched(self.ops, self.weights, p, d, S, step, E, self.layers, before_layer=gate)
-            pipeline.decoder_epilogue_batched(d)
-        main.wait_stream(side)
+        for (d, caches, n), side, pool in zip(self.decoder_groups, self.streams, self.pools):
+            with torch.cuda.stream(side), wrappers.use_pool(pool):
+                if self.steps == 0:
+                    side.wait_event(kv_ready[-1])
+                for step in range(self.steps):
+                    gate = (lambda layer, st=side: st.wait_event(kv_ready[layer])) if step == 0 else None
+                    pipeline.decoder_step_batched(self.ops, self.weights, caches, d, S, step, n, self.layers, before_layer=gate)
+                pipeline.decoder_epilogue_batched(d)
+        for side in self.streams:
+            main.wait_stream(side)
 
     def _attention_fork(self):
         """`per_episode` hook of the batched prefix encoder: episode e's attention goes to a stream of its own,

@@ -333,3 +333,10 @@ def test_pinned_plan_table_validates_on_the_host():
     lib.fvla_gemm_plan_clear()
     assert autotune.grid(bn=[128, 256], splits=[1, 2]) == [{"bn": 128, "splits": 1}, {"bn": 128, "splits": 2},
                                                             {"bn": 256, "splits": 1}, {"bn": 256, "splits": 2}]
+
+
+@pytest.mark.parametrize("episodes,rows,want", [(2, 51, [(0, 2)]), (3, 51, [(0, 1), (1, 3)]), (4, 51, [(0, 2), (2, 4)]), (5, 51, [(0, 5)]),
+                                                (8, 11, [(0, 8)]), (2, 65, [(0, 1), (1, 2)]), (3, 65, [(0, 3)]), (2, 200, [(0, 1), (1, 2)])])
+def test_decoder_groups(episodes, rows, want):
+    from flash_vla_b200.hardware.nvidia.b200.pi0.engine import decoder_groups
+    assert decoder_groups(episodes, rows) == want
