@@ -490,37 +490,42 @@ static int refresh_shadow(const void* src, void* dst, size_t count, cudaStream_t
 int fvla_linear_residual(const void* x, const void* weight, void* out, int out_is_f32, void* out_shadow, int M,
                          int N, int K, int group_rows, void* ws, size_t ws_bytes, void* stream) {
     FVLA_REQUIRE(group_rows >= 0 && (group_rows == 0 || M % group_rows == 0), "linear_residual: M=%d is not a whole number of groups of %d rows", M, group_rows);
-    // rows as several groups (a batch of episodes): the decoder's cluster GEMM once per group in one launch, each group
+    // Rows as several groups (a batch of episodes): the decoder's cluster GEMM once per group in one launch, each group
     // streaming the weights from L2 after the first has pulled them from HBM. Up to 128 rows are one group whatever
-    // they are made of: one pass over the weights instead of several.
-    const int rows = group_rows > 0 && M > 128 ? group_rows : M, groups = M / rows;
-    if (tc5_enabled() && skinny::skinny_supports(rows, N, K, false, true) && aligned16(x) && aligned16(weight)) {
+    // they are made of. The clusters of one launch may not all be resident at once (about 15 clusters of 8, 33 of 4, 74
+    // of 2), and a second round of clusters costs as much as the first, so K is cut into parts, one launch each, with the
+    // widest split whose clusters of all groups ARE resident together; every launch after the first accumulates onto
+    // the result of the one before (the residual form does that anyway). Groups of up to 128 rows instead of one per
+    // episode are taken when they need fewer launches (8 episodes of 51 rows, down projection: 2 instead of 4, o: 1 of 2).
+    auto resident = [](int splits) { return splits >= 8 ? 15 * 8 : (splits == 4 ? 33 * 4 : 148); };
+    auto parts_for = [&](int rows, int groups) {         // launches needed, 0: no plan keeps all clusters resident
+        for (int parts = 1; parts <= 8; parts *= 2) {
+            if (K % parts || (K / parts) % 64) break;
+            const skinny::SkinnyPlan part = skinny::plan_skinny(rows, N, K / parts, false, groups);
+            if (part.ok && (groups == 1 || part.tiles * part.splits * groups <= resident(part.splits))) return parts;
+        }
+        return 0;
+    };
+    int rows = group_rows > 0 && M > 128 ? group_rows : M, groups = M / rows, parts = 1;
+    if (groups > 1) {
+        parts = parts_for(rows, groups);
+        int wide = (M + 127) / 128;                      // the fewest equal groups of at most 128 rows
+        while (wide < groups && M % wide) ++wide;
+        const int wide_parts = wide < groups ? parts_for(M / wide, wide) : 0;
+        if (wide_parts > 0 && (parts == 0 || wide_parts < parts)) { rows = M / wide; groups = wide; parts = wide_parts; }
+        if (parts == 0) parts = 1;
+    }
+    if (tc5_enabled() && skinny::skinny_supports(rows, N, K / parts, false, true) && aligned16(x) && aligned16(weight)) {
         skinny::SkinnyArgs sa{};
-        sa.x = x; sa.x_f32 = 0; sa.ldx = K; sa.M = rows; sa.N = N; sa.K = K; sa.groups = groups;
+        sa.x = x; sa.x_f32 = 0; sa.ldx = K; sa.M = rows; sa.N = N; sa.K = K / parts; sa.groups = groups;
         sa.out = out; sa.out_f32 = out_is_f32; sa.ldo = N; sa.out_shadow = Bm(out_shadow);
         sa.status = device_status_ptr(); FVLA_DBG_ATTACH(sa);
-        // With several row groups the clusters of one launch may not all be resident at once (about 15 clusters of
-        // 8, 33 of 4, 74 of 2), and a second round of clusters costs as much as the first. K is then cut into 2, 4 or
-        // 8 parts, one launch each, with the widest split whose clusters of all groups ARE resident together; every
-        // launch after the first accumulates onto the result of the one before (the residual form does that anyway).
-        auto resident = [](int splits) { return splits >= 8 ? 15 * 8 : (splits == 4 ? 33 * 4 : 148); };
-        const skinny::SkinnyPlan whole = skinny::plan_skinny(rows, N, K, false, groups);
-        if (groups > 1 && whole.tiles * whole.splits * groups > resident(whole.splits)) {
-            for (int parts = 2; parts <= 8; parts *= 2) {
-                if (K % parts || (K / parts) % 64) break;
-                const skinny::SkinnyPlan part = skinny::plan_skinny(rows, N, K / parts, false, groups);
-                if (!part.ok || part.tiles * part.splits * groups > resident(part.splits)) continue;
-                sa.K = K / parts;
-                for (int i = 0; i < parts; ++i) {
-                    sa.x = B(x) + (size_t)i * (K / parts);
-                    int rc = skinny::launch_skinny<skinny::EPI_RESIDUAL>(sa, B(weight) + (size_t)i * (K / parts) * N, nullptr, N, S(stream));
-                    if (rc) return rc;
-                }
-                return FVLA_OK;
-            }
-            sa.K = K; sa.x = x;
+        for (int i = 0; i < parts; ++i) {
+            sa.x = B(x) + (size_t)i * sa.K;
+            int rc = skinny::launch_skinny<skinny::EPI_RESIDUAL>(sa, B(weight) + (size_t)i * sa.K * N, nullptr, N, S(stream));
+            if (rc) return rc;
         }
-        return skinny::launch_skinny<skinny::EPI_RESIDUAL>(sa, weight, nullptr, N, S(stream));
+        return FVLA_OK;
     }
     FVLA_REQUIRE(out_shadow == nullptr || out_is_f32, "linear_residual: a bf16 shadow only makes sense for an fp32 `out`");
     GemmArgs a;

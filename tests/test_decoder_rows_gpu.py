@@ -93,3 +93,15 @@ def test_prefix_qkv_by_tile_width(S):
     for got in outs:
         for a, b, what in zip(got, refs, "Q K V".split()):
             assert_close(a, b, rtol=2e-2, atol_rms=4e-2, what=f"encoder_norm_qkv_rope.{what}")
+
+
+# a batch's residual projection: groups per episode in one launch or several, and regrouped into up to 128 rows
+@pytest.mark.parametrize("episodes,rows,K", [(3, 51, 2048), (4, 51, 4096), (5, 51, 4096), (8, 51, 2048), (8, 51, 4096), (7, 23, 4096), (3, 127, 2048)])
+def test_batched_residual_projection(episodes, rows, K):
+    from flash_vla_b200 import op_table
+    g = torch.Generator().manual_seed(episodes * rows)
+    x, w, out = rnd(g, episodes, rows, K), rnd(g, K, 1024, scale=0.02), torch.randn(episodes, rows, 1024, generator=g)
+    ref, got = out.view(-1, 1024).clone(), out.cuda()
+    O.op_table(False).decoder_ffn_down_residual(x.float().view(-1, K), w.float(), ref)
+    op_table(True).decoder_ffn_down_residual(x.cuda(), w.cuda(), got)
+    assert_close(got.view(-1, 1024), ref, what="decoder_ffn_down_residual")
