@@ -1041,13 +1041,12 @@ inline int launch_gemm_tc5(GemmArgs g, int* status, cudaStream_t st, void* ws = 
 inline int normed_tile_width(int M, int N, int K, bool rope) {
     if (M <= 64 || N % 8 != 0 || K % BK != 0) return 0;
     const int tiles_m = (M + BM - 1) / BM, sms = num_sms();
-    if (rope) {                                // the narrowest tile of which every CTA gets one at most: up to 768, 1 280 and 1 792 rows at N = 2560
-        for (int bn = 128; bn <= 256; bn += 64)
+    if (rope) {                                // the narrowest tile of which every CTA gets one at most: up to 384, 896, 1 280 and 1 792 rows at N = 2560
+        for (int bn = 64; bn <= 256; bn += 64)
             if (tiles_m * ((N + bn - 1) / bn) <= sms) return bn;
         return 0;
     }
     int bn = plan_tc5(M, N, K, false).bn;      // the widest tile that still gives every CTA exactly one, starting from the plain kernel's plan
-    if (bn < 128) bn = 128;                    // the fused-norm variants start at 128 columns
     while (bn < 256 && tiles_m * ((N + bn - 1) / bn) > sms) bn += 64;
     return tiles_m * ((N + bn - 1) / bn) <= sms ? bn : 0;
 }
@@ -1064,12 +1063,14 @@ inline int launch_gemm_tc5_normed(GemmArgs g, int* status, cudaStream_t st) {
         switch (bn) {
             case 256: return launch_tc5_cfg<256, false, 4, true, false, true>(g, status, st);
             case 192: return launch_tc5_cfg<192, false, 5, true, false, true>(g, status, st);
+            case 64: return launch_tc5_cfg<64, false, 8, true, false, true>(g, status, st);
             default: return launch_tc5_cfg<128, false, 6, true, false, true>(g, status, st);
         }
     }
     switch (bn) {
         case 256: return launch_tc5_cfg<256, false, 4, false, false, true>(g, status, st);
         case 192: return launch_tc5_cfg<192, false, 5, false, false, true>(g, status, st);
+        case 64: return launch_tc5_cfg<64, false, 8, false, false, true>(g, status, st);
         default: return launch_tc5_cfg<128, false, 6, false, false, true>(g, status, st);
     }
 }

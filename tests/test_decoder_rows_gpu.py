@@ -76,7 +76,7 @@ def test_decoder_attention_by_shape(tokens, S, episodes):
     assert _lib.load().fvla_device_status(None) == 0
 
 
-# prefix QKV with the row norm inside the GEMM by tile width (128, 192, 256 columns; the last with a ragged row tile), and past
+# prefix QKV with the row norm inside the GEMM by tile width (64, 128, 192, 256 columns; the last with a ragged row tile), and past
 # it, where the norm is a kernel of its own
 @pytest.mark.parametrize("S", [257, 769, 1281, 1793])
 def test_prefix_qkv_by_tile_width(S):
