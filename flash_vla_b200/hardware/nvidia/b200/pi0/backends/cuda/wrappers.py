@@ -347,8 +347,8 @@ def encoder_attention(Q, K, V, scale, out):
 
 def _linear_residual(role, x, weight, out):
     """out += x @ weight. Extension for batches of episodes: 3-D `x` (episodes, rows, K) and `out` (episodes,
-    rows, N), contiguous, mean that many independent row groups; with at most 64 rows per group the
-    decoder's weight-streaming kernel serves every group inside one launch."""
+    rows, N), contiguous, mean that many independent row groups; with at most 128 rows per group the
+    decoder's weight-streaming kernel serves them in as few launches as it can."""
     group_rows = 0
     if x.ndim == 3:
         if out.ndim != 3 or out.shape[:2] != x.shape[:2]:

@@ -175,8 +175,8 @@ def decoder_step_batched(ops, weights, prefix, dec, encoder_seq_len, step, episo
         ops.decoder_norm_qkv_rope(x, w["decoder_attn_qkv_w"][layer], dec["decoder_rope_weights"], q,
                                   k_all[:, S:], v_all[:, S:], nf)
         ops.decoder_attention(q, k_all, v_all, None, q, S)
-        # the two residual projections see the rows as E groups of D (3-D operands): with D <= 64 the backend
-        # runs its weight-streaming decoder kernel once per episode inside one launch
+        # the two residual projections see the rows as E groups of D (3-D operands): with D <= 128 the backend
+        # runs its weight-streaming decoder kernel over row groups inside as few launches as it can
         ops.decoder_out_proj_residual(q.view(E, D, DECODER_HEADS * HEAD_DIM), w["decoder_attn_o_w"][layer], x3)
         ops.decoder_norm_gated_ffn(x, w["decoder_ffn_gate_w"][layer], w["decoder_ffn_up_w"][layer], dec["decoder_hidden"], nf)
         ops.decoder_ffn_down_residual(dec["decoder_hidden"].view(E, D, -1), w["decoder_ffn_down_w"][layer], x3)

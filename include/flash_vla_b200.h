@@ -47,7 +47,7 @@ unsigned long long fvla_launch_count(void);
 int fvla_device_status(void* stream);
 /* No counterpart in the reference (which has no device-side error reporting, only Python exceptions).
  * Failure-detection self-test: runs the decoder's cluster GEMM (out += x(M,K) @ W(K,N), all bf16, a
- * shape fvla_linear_residual serves with M <= 64) with the CTAs that finish the tiles told to wait for
+ * shape fvla_linear_residual serves with M <= 128) with the CTAs that finish the tiles told to wait for
  * 16 bytes that no CTA ever sends, and with that wait limited to `spin_limit` polls (1..65536). The
  * kernel must give up, release its tensor memory and return within milliseconds; fvla_device_status
  * then reports 2 and `out` is unspecified. Nothing faults and the context stays usable. */
@@ -58,7 +58,7 @@ int fvla_selftest_wait_timeout(const void* x, const void* weight, void* out, int
  * Counterpart of the reference's per-kernel configuration sweep (benchmarks/autotune.py), whose winners the
  * reference writes into its TileLang kernel definitions. Here a measured-best launch plan can be pinned
  * per GEMM shape at run time; unpinned shapes use the library's cost models. `kind`: 0 plain (bias /
- * activation / residual epilogues), 1 QKV + RoPE, 2 gated FFN, 3 decoder cluster GEMM (M <= 64), 4 its
+ * activation / residual epilogues), 1 QKV + RoPE, 2 gated FFN, 3 decoder cluster GEMM (M <= 128), 4 its
  * gated form. `engine`: 1 one-SM tcgen05 kernel with tile width bn (64, 128, 192, 256) and K split `splits`
  * (1..4) through caller scratch; 2 the same kernel, 128-wide tiles, K split (2..4) inside a thread-block
  * cluster; 3 the two-SM kernel, K split 1..6 through scratch (gated FFN: 1); 4 the decoder cluster GEMM
@@ -160,9 +160,10 @@ int fvla_encoder_attention(const void* Q, const void* K, const void* V, void* ou
 /* wrappers.py:366-371, :383-392 (encoder) and :176-189 (decoder): out += x(M,K) @ W(K,N). out is
  * bf16, or an fp32 residual stream when out_is_f32 != 0. out_shadow (may be NULL; fp32 out only) is a
  * bf16 tensor of out's shape that receives the rounded new value, for a later GEMM to read: written by
- * the GEMM's own epilogue for M <= 64, by a small conversion kernel after it otherwise.
+ * the GEMM's own epilogue where the decoder's cluster GEMM runs (up to 128 rows, and groups), by a small conversion kernel after it otherwise.
  * group_rows > 0 (an extension for batches of episodes): the M rows are M / group_rows groups of at most
- * 64 rows; the decoder's weight-streaming kernel then runs once per group inside one launch. 0: one group. */
+ * 128 rows, which the decoder's weight-streaming kernel takes as row groups of as few launches as it can (it may cut
+ * the rows into other groups where that reads the weight fewer times). 0: one group. */
 int fvla_linear_residual(const void* x, const void* weight, void* out, int out_is_f32, void* out_shadow,
                          int M, int N, int K, int group_rows, void* ws, size_t ws_bytes, void* stream);
 /* wrappers.py:374-380: x_norm = rms(x); out = gelu(x_norm @ Wg) * (x_norm @ Wu). */
@@ -197,8 +198,9 @@ int fvla_decoder_norm_qkv_rope(const void* x, int x_is_f32, const void* x_shadow
  * the stream writes the prefix rows must put an event or another kernel between the two.
  * episodes > 1 (an extension): that many independent episodes in one launch; `queries` and `keys` are
  * per episode, episode e reads Q + e * q_episode_stride and K / V + e * kv_episode_stride (strides in
- * elements, multiples of 8) and writes out + e * q_episode_stride. A batch runs on the tcgen05 flash
- * kernel (one grid row per episode), which waits for its predecessor before any read. */
+ * elements, multiples of 8) and writes out + e * q_episode_stride. A batch whose clusters are all resident at
+ * once runs on the same kernel as one episode, a larger one on the tcgen05 flash kernel (one grid row per
+ * episode), which waits for its predecessor before any read. */
 int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* out, int queries,
                            int keys, int head_dim, int heads, int encoder_seq_len, int episodes,
                            long long q_episode_stride, long long kv_episode_stride, void* ws,
