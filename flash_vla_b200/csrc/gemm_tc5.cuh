@@ -847,14 +847,22 @@ inline int make_map3d(CUtensorMap* map, const void* base, uint64_t inner, uint64
 
 struct Tc5Plan { int bn, splits; size_t ws_bytes; float est_us; };
 
-// Per-step times (us) of one 64-wide k step at tile width 64 / 128 / 192 / 256, as measured on B200: the
-// shared-memory traffic of a step (every operand byte written once by TMA and read once by the tensor core, at
-// 128 B/clk), not the MMA, sets them.
-inline float k_step_us(int bn) { return bn == 64 ? 0.26f : (bn == 128 ? 0.30f : (bn == 192 ? 0.37f : 0.43f)); }
+// Times (us) of one 64-wide k step and of a launch's two ends (first fill, last epilogue) at tile width 64 / 128 / 192 / 256,
+// fitted on B200 to 256 to 6 144 rows of the four residual projections (K 1 152 to 16 384, N 1 152 and 2 048): the shared-memory
+// traffic of a step (every operand byte written once by TMA and read once by the tensor core), not the MMA, sets
+// them, and from about 108 busy SMs on what these pull through L2 together.
+inline float k_step_us(int bn, int busy = 0) {
+    const float base = bn == 64 ? 0.275f : (bn == 128 ? 0.28f : (bn == 192 ? 0.292f : 0.37f));
+    return base + (busy > 108 ? (busy - 108) * (bn <= 128 ? 0.0005f : 0.0014f) : 0.f);
+}
+inline float ends_us(int bn) { return bn == 64 ? 3.9f : (bn == 128 ? 4.5f : (bn == 192 ? 5.6f : 6.0f)); }
 
 // Tile width and K split for a plain (non-gated) GEMM: minimise the estimated time of the slowest SM,
-// (waves of work items) x (k steps per item) x (time per step), plus, for a split, the cost of writing
-// and re-reading the fp32 partials. A split needs caller scratch and is only offered when `ws_ok`.
+// (waves of work items) x (k steps per item) x (time per step) plus the two ends (between them an item's epilogue runs
+// beside the next item's k steps), plus, for a split, the cost of writing and re-reading the fp32 partials. A split
+// needs caller scratch and is only offered when `ws_ok`. (The ends used to be charged once per wave and the steps were those of
+// a slower issue loop, which kept the prefix encoder's output projection at 1 280 to 3 264 rows on 256-wide pair tiles: 33.5 us
+// against 26.9 at 1 280 rows, 37.9 against 32.8 at 3 072.)
 inline Tc5Plan plan_tc5(int M, int N, int K, bool ws_ok) {
     const int tiles_m = (M + BM - 1) / BM, sms = num_sms(), k_iters = (K + BK - 1) / BK;
     Tc5Plan best{128, 1, 0, 1e30f};
@@ -865,7 +873,7 @@ inline Tc5Plan plan_tc5(int M, int N, int K, bool ws_ok) {
             if (s > 1 && k_iters / s < 16) break;
             const int per = (k_iters + s - 1) / s;
             const int waves = (tiles * s + sms - 1) / sms;
-            float t = waves * (per * k_step_us(bn) + 4.0f);
+            float t = waves * per * k_step_us(bn, (tiles * s + waves - 1) / waves) + ends_us(bn);
             if (s > 1) t += 3.0f + (float)s * M * N * 8.0f / 4.0e6f;      // partial traffic at about 4 TB/s
             if (t < best_t) { best_t = t; best = Tc5Plan{bn, s, 0, t}; }
         }
@@ -1019,8 +1027,8 @@ inline int launch_gemm_tc5(GemmArgs g, int* status, cudaStream_t st, void* ws = 
         float best_t = pl.est_us;
         for (int sp = 2; sp <= 4; ++sp) {
             if (tiles * sp > num_sms() || k_iters / sp < 8) break;
-            // two mates reduce-scatter their halves (about 1.5 us); more splits gather one 64 KB tile each into the split-0 CTA
-            const float t = ((k_iters + sp - 1) / sp) * k_step_us(128) + 4.0f + (sp == 2 ? 1.5f : 2.5f + (sp - 1) * 2.1f);
+            // two mates reduce-scatter their halves (about 2.5 us); more splits gather one 64 KB tile each into the split-0 CTA
+            const float t = ((k_iters + sp - 1) / sp) * k_step_us(128) + ends_us(128) + (sp == 2 ? 2.5f : 2.5f + (sp - 1) * 2.1f);
             if (t < best_t) { best_t = t; best_s = sp; }
         }
         if (best_s) return launch_tc5_cfg<128, false, 6, false, true>(g, status, st, best_s, nullptr);

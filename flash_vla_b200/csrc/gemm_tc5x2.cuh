@@ -394,7 +394,10 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
 
 struct PairPlan { bool ok; int splits; size_t ws_bytes; float est_us; };
 
-// Plain residual GEMM on CTA pairs: 256 x 256 tiles; K is split so that the work items fill the 74 pairs.
+// Plain residual GEMM on CTA pairs: 256 x 256 tiles; K is split so that the work items fill the 74 pairs in whole rounds. A k
+// step takes 0.30 us on up to 46 pairs and 0.39 on 72 (L2), the ends of a launch 7.5 us, a split item 5.5 us more (its
+// exchange, only partly beside the next item). Fitted to 256 to 6 144 rows at K = 16 384, N = 2 048; with a price per
+// byte of partial sums instead, 1 280 rows had no split (83 us; 74 with three), 1 536 neither (87; 82.6).
 inline PairPlan plan_pair_plain(int M, int N, int K, bool ws_ok) {
     PairPlan pl{false, 1, 0, 1e30f};
     if (M <= 128 || N % 8 || K % 8) return pl;
@@ -403,8 +406,9 @@ inline PairPlan plan_pair_plain(int M, int N, int K, bool ws_ok) {
         if (s > 1 && k_iters / s < 8) break;
         const int per = (k_iters + s - 1) / s;
         const int waves = (tiles * s + pairs - 1) / pairs;
-        float t = waves * (per * 0.28f + 5.0f);
-        if (s > 1) t += 3.0f + (float)s * M * N * 8.0f / 4.0e6f;
+        const int busy = (tiles * s + waves - 1) / waves;      // pairs of the balanced grid
+        const float step = 0.30f + (busy > 46 ? (busy - 46) * 0.0034f : 0.f);
+        const float t = 7.5f + waves * (per * step + (s > 1 ? 5.5f : 0.5f));
         if (t < pl.est_us) { pl.est_us = t; pl.splits = s; pl.ok = true; }
     }
     if (pl.splits > 1) pl.ws_bytes = (((size_t)tiles * 4 * sizeof(int) + 255) / 256) * 256 + (size_t)tiles * pl.splits * 2 * 128 * 256 * sizeof(float);

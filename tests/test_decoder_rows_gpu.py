@@ -105,3 +105,15 @@ def test_batched_residual_projection(episodes, rows, K):
     O.op_table(False).decoder_ffn_down_residual(x.float().view(-1, K), w.float(), ref)
     op_table(True).decoder_ffn_down_residual(x.cuda(), w.cuda(), got)
     assert_close(got.view(-1, 1024), ref, what="decoder_ffn_down_residual")
+
+
+# prefix projections beyond one round of tiles: pair tiles with K split over two rounds of items, 192-wide tiles in one and two rounds
+@pytest.mark.parametrize("op,S,K", [("encoder_ffn_down_residual", 1281, 16384), ("encoder_out_proj_residual", 1281, 2048), ("encoder_out_proj_residual", 2449, 2048)])
+def test_prefix_projection_by_row_count(op, S, K):
+    from flash_vla_b200 import op_table
+    g = torch.Generator().manual_seed(S)
+    x, w, out = rnd(g, S, K), rnd(g, K, 2048, scale=0.02), rnd(g, S, 2048)
+    ref, got = out.float(), out.cuda()
+    getattr(O.op_table(False), op)(x.float(), w.float(), ref)
+    getattr(op_table(True), op)(x.cuda(), w.cuda(), got)
+    assert_close(got, ref, what=op)
