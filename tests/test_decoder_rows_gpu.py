@@ -117,3 +117,15 @@ def test_prefix_projection_by_row_count(op, S, K):
     getattr(O.op_table(False), op)(x.float(), w.float(), ref)
     getattr(op_table(True), op)(x.cuda(), w.cuda(), got)
     assert_close(got, ref, what=op)
+
+
+# gated FFN on single SMs (three row tiles) and on pairs (two)
+@pytest.mark.parametrize("S", [256, 257, 384])
+def test_prefix_gated_ffn_by_row_count(S):
+    from flash_vla_b200 import op_table
+    g = torch.Generator().manual_seed(S)
+    x, wg, wu = rnd(g, S, 2048), rnd(g, 2048, 16384, scale=0.02), rnd(g, 2048, 16384, scale=0.02)
+    ref, got, norm = torch.zeros(S, 16384), torch.zeros(S, 16384, dtype=torch.bfloat16, device="cuda"), torch.zeros(S, 2048)
+    O.op_table(False).encoder_norm_gated_ffn(x.float(), wg.float(), wu.float(), ref, norm)
+    op_table(True).encoder_norm_gated_ffn(x.cuda(), wg.cuda(), wu.cuda(), got, norm.bfloat16().cuda())
+    assert_close(got, ref, rtol=2e-2, atol_rms=4e-2, what="encoder_norm_gated_ffn")
