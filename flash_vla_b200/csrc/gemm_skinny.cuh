@@ -16,8 +16,7 @@
 // The activation operand arrives by TMA as bf16 rows: either the activation itself (bf16) or the bf16
 // shadow that the kernels writing the fp32 residual stream keep beside it; the per-token sum of
 // squares for the RMS factor is read back from that operand tile in shared memory while the MMAs run
-// and is reduced with the partials. Two lanes issue the MMAs of alternate k-blocks into accumulators of their own, since one
-// thread spends 46 clk per instruction and the pipe 39 to 64. What remains is a chain of latencies (dependency 0.9 us after the
+// and is reduced with the partials. What remains is a chain of latencies (dependency 0.9 us after the
 // last CTA of the kernel before, X tile 0.5, MMAs 0.6 to 1.5, exchange 0.5, epilogue 0.6), in which every instruction behind the
 // exchange counts, hence the cluster size and the token slots as template parameters. Per launch inside the chain at 51 rows:
 // QKV 4.3 us (5.7 with one issuer, an exchange through bulk copies and run-time sizes), attention output 3.9 (5.0),
@@ -121,7 +120,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-    constexpr uint32_t XB = TOK * 128, RED_BYTES = TOK * 512, ACC_COLS = 2 * TOK;      // one accumulator per issuing thread
+    constexpr int ISSUERS = TOK == 64 ? 1 : 2;                // MMA-issuing threads, an accumulator each
+    constexpr uint32_t XB = TOK * 128, RED_BYTES = TOK * 512, ACC_COLS = ISSUERS * TOK;
     // The upper warps add up the rows' squares: the MMA issuers' warps come too late for it (gate/up: 1.6 us after the last MMA)
     constexpr int SSQ_WARPS = 8;
     constexpr int TS = TOK / S, COLS = EPI == EPI_GEGLU ? 64 : 128, ITEMS = TS / 4 * COLS, PRE = (ITEMS + THREADS - 1) / THREADS;      // owner: tokens, work items, per thread
@@ -153,7 +153,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     if (tid == 32) { tc5::prefetch_tensormap(&tmW); if (EPI == EPI_GEGLU) tc5::prefetch_tensormap(&tmW2); }
     if (tid == 64 && x_by_tma) tc5::prefetch_tensormap(&tmX);
     if (tid == 0) {
-        mbar_init(done_bar, 2);                              // one commit from each issuing thread
+        mbar_init(done_bar, ISSUERS);                        // one commit from each issuing thread
         mbar_init(in_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -303,23 +303,36 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     };
     FVLA_STAMP(2);
 
-    // Two threads issue the MMAs, k-blocks in turn, each into an accumulator of its own. One thread needs 46 clk per MMA and
-    // another 110 - 290 per k-block for its wait, the descriptors and the next address, so that 8 k-blocks took 2 400 clk
-    // against 1 540 of tensor pipe (N = 64: 48 clk per MMA); two hide that from one another.
-    if (warp < 2 && lane == 0) {
-        constexpr uint32_t idesc = skinny_idesc(TOK);
-        const uint64_t ad = smem_desc(sW, 8192, 1024), bd = smem_desc(sX, 16, 1024);
-        bool ok = true;
-        for (int kb = warp; kb < KB && ok; kb += 2) {
-            ok = mbar_wait(bars + kb * 8, 0, abort_flag);
-            tc5::tc_fence_after();
-            if (!ok) break;
-            const int slot = TOK > 64 && kb >= NS ? kb - NS : kb;
+    // 64 slots: one thread adds up all k-blocks in order in one accumulator, so that a product is a single fp32 sum over the CTA's
+    // K slice from front to back, whatever issues it (decodes of several steps amplify a changed order of summation). Its warp
+    // waits for all k-blocks at once, a lane each: they land within 0.1 us of one another, and waits in between take longer. MMAs
+    // done after the X tile, at 51 rows: QKV 0.87 us, o 0.87, gate / up 1.9, down 1.3 (two threads with an accumulator each 0.92, 0.87, 2.4, 1.7).
+    // 128 slots: two threads issue the k-blocks in turn, each into an accumulator of its own.
+    constexpr uint32_t idesc = skinny_idesc(TOK);
+    const uint64_t ad = smem_desc(sW, 8192, 1024), bd = smem_desc(sX, 16, 1024);
+    auto issue_block = [&](int kb, uint32_t acc, bool first) {
+        const int slot = TOK > 64 && kb >= NS ? kb - NS : kb;
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16)
-                tc5::umma_bf16(tmem + warp * TOK, ad + slot * (16384 >> 4) + k16 * (2048 >> 4), bd + slot * (XB >> 4) + k16 * (32 >> 4), idesc,
-                               (kb > 1 || k16 > 0) ? 1u : 0u);
-            if (TOK > 64 && kb + NS < KB) tc5::umma_commit(free_bars + kb * 8);
+        for (int k16 = 0; k16 < 4; ++k16)
+            tc5::umma_bf16(acc, ad + slot * (16384 >> 4) + k16 * (2048 >> 4), bd + slot * (XB >> 4) + k16 * (32 >> 4), idesc, !first || k16 > 0 ? 1u : 0u);
+    };
+    if (ISSUERS == 1 && __shfl_sync(0xffffffffu, warp, 0) == 0) {
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + min(lane, KB - 1) * 8, 0, abort_flag));
+        __syncwarp();                                        // what the lanes saw is in order before the elected lane's MMAs
+        tc5::tc_fence_after();
+        if (tc5::elect_one()) {
+#pragma unroll
+            for (int kb = 0; kb < MAX_KB; ++kb)
+                if (kb < KB && ok) issue_block(kb, tmem, kb == 0);
+            tc5::umma_commit(done_bar);
+        }
+    }
+    if (ISSUERS == 2 && warp < 2 && lane == 0) {
+        for (int kb = warp; kb < KB; kb += 2) {
+            if (!mbar_wait(bars + kb * 8, 0, abort_flag)) break;
+            tc5::tc_fence_after();
+            issue_block(kb, tmem + warp * TOK, kb < 2);
+            if (kb + NS < KB) tc5::umma_commit(free_bars + kb * 8);
         }
         tc5::umma_commit(done_bar);
     }
@@ -337,7 +350,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         // memory while the MMAs run (4 or 2 lanes per token).
         constexpr int LPT = SSQ_WARPS * 32 / TOK;            // lanes per token
         const int st = tid - (THREADS - SSQ_WARPS * 32), t = st / LPT, sub = st % LPT;
-        float ss = 0.f;
+        float part[8 / LPT] = {};                            // one sum per 16-byte piece of the rows, added up pairwise below
         for (int kb = 0; kb < KB; ++kb) {
             mbar_wait(bars + kb * 8, 0, abort_flag);
             const int slot = TOK > 64 && kb >= NS ? kb - NS : kb;
@@ -345,7 +358,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
             for (int h = 0; h < 8 / LPT; ++h) {
                 const uint4 a = *reinterpret_cast<const uint4*>(gen + w_bytes + slot * XB + t * 128 + (sub + h * LPT) * 16);
                 const float2 f0 = unpack_bf16x2(a.x), f1 = unpack_bf16x2(a.y), f2 = unpack_bf16x2(a.z), f3 = unpack_bf16x2(a.w);
-                ss += f0.x * f0.x + f0.y * f0.y + f1.x * f1.x + f1.y * f1.y + f2.x * f2.x + f2.y * f2.y + f3.x * f3.x + f3.y * f3.y;
+                part[h] += f0.x * f0.x + f0.y * f0.y + f1.x * f1.x + f1.y * f1.y + f2.x * f2.x + f2.y * f2.y + f3.x * f3.x + f3.y * f3.y;
             }
             if (TOK > 64 && kb + NS < KB) {
                 __syncwarp();
@@ -353,8 +366,14 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
             }
         }
 #pragma unroll
-        for (int o = 1; o < LPT; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (sub == 0) hand_out_ss(t, ss);
+        for (int o = 1; o < LPT; o <<= 1)
+#pragma unroll
+            for (int h = 0; h < 8 / LPT; ++h) part[h] += __shfl_xor_sync(0xffffffffu, part[h], o);
+#pragma unroll
+        for (int n = 8 / LPT; n > 1; n /= 2)
+#pragma unroll
+            for (int h = 0; h < n / 2; ++h) part[h] = part[2 * h] + part[2 * h + 1];
+        if (sub == 0) hand_out_ss(t, part[0]);
     }
     if (TOK == 64 && !x_by_tma && p.need_factor && tid < TOK)
         hand_out_ss(tid, tid < p.M ? ssq_local[tid * 2] + (KB == 8 ? ssq_local[tid * 2 + 1] : 0.f) : 0.f);
@@ -372,7 +391,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         const int q = warp & 3, g = (warp >> 2) + h * 4;
         float part[16];
         tc5::tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + g * 16, part);
-        if (KB > 1) {
+        if (ISSUERS == 2 && KB > 1) {
             float second[16];
             tc5::tmem_ld16(tmem + TOK + ((uint32_t)(q * 32) << 16) + g * 16, second);
 #pragma unroll

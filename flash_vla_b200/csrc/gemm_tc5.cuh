@@ -48,6 +48,13 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
+// True in one lane of a converged warp. The compiler keeps a block behind it free of the moves to uniform registers that it puts
+// before every tcgen05 instruction behind `lane == 0`: 50 clk less per MMA in the decoder's cluster GEMM.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : : "memory");
+    return ok != 0;
+}
 // Bounded wait; false when the limit ran out (the caller then abandons its loop). `limit` is the number
 // of polls; the default is far beyond any legitimate wait of these kernels (tens of microseconds).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
