@@ -274,19 +274,26 @@ inline int launch_attention(const AttnArgs& a, dim3 grid, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------------------------
 // Decoder attention in one launch: a cluster of 4 to 11 CTAs has 32 flat query rows (4 tokens x 8 heads) and shares out
-// the keys: every CTA takes an equal part of the prefix and of the step's own keys. Both products run on tcgen05 with the
-// KEYS (then the head dimensions) as the 128-row operand and the query rows as N = 32:
+// the keys. Both products run on tcgen05 with the KEYS (then the head dimensions) as the 128-row operand and the query
+// rows as N = 32:
 //   S^T = K Q^T   one or two key tiles, accumulator lane = key, column = query row;
-//   softmax       thread = one key x 16 rows; row maxima and sums by a halving butterfly (16 shuffles for 16 rows), the
-//                 four 32-key quadrants meet in shared memory; P goes to shared memory as the next operand;
+//   softmax       thread = one key x 16 rows; row maxima by a halving butterfly (16 shuffles for 16 rows), the
+//                 32-key quadrants meet in shared memory; P goes to shared memory as the next operand;
 //   O^T = V^T P^T two 128-dim tiles, accumulator lane = dim, column = query row.
-// A thread's accumulator column then IS what an owner of 4 rows needs from it: it goes straight from registers to the owners'
-// shared memory (st.async, 16 bytes = 4 rows of one dim), over the K tile, which nobody reads any more. Owners
+// A thread's accumulator column then IS what an owner of 4 rows needs from it: normalised, it goes straight from registers to the
+// owners' shared memory (st.async, 16 bytes = 4 rows of one dim), over the K tile, which nobody reads any more. Owners
 // weight the parts by log-sum-exp in rank order and write bf16.
-// Measured at 51 rows x 819 keys inside the decoder's chain: 5.9 us per launch, against 7.8 us for the warp-level form that this
-// replaced (mma.sync on 8 warps, 64-key halves merged and staged in shared memory, bulk copies). What bounds it is a chain of
-// latencies: dependency wait 0.9, Q 0.7, S^T 0.6, softmax and O^T 1.6, exchange 1.2 (28 KB per CTA; distributed shared memory
-// moves 16 B/clk per SM when all SMs send), combine 0.7; DRAM and the tensor pipes idle.
+// One key tile (KT = 1): a CTA has a contiguous range of at most 128 keys, in two groups of 64 with a maximum, a sum and an accumulator
+// of their own, merged before the exchange. Ranges, groups and the order of every sum are those of the warp-level kernel
+// that this one replaced (two groups of warps, mma.sync), and mma.sync and tcgen05.mma add up the same bits, so the results are the
+// same bits too: P is rounded to bf16 against its group's maximum, and ten Euler steps multiply any other rounding.
+// Two key tiles (KT = 2), where that keeps more clusters resident: equal parts of the prefix and of the step's own keys, four groups.
+// (With one maximum per CTA instead of per group fewer probabilities are exactly 1: 2.17e-3 from the 64-bit result at 65 tokens x 882
+// unit-variance keys, 2.08e-3 with groups of 64.)
+// Measured at 51 rows x 819 keys inside the decoder's chain: 6.4 us per launch, against 7.8 us for the warp-level form
+// (mma.sync on 8 warps, halves staged in shared memory, bulk copies). What bounds it is a chain of
+// latencies: dependency wait 0.9, Q 0.7, S^T 0.6, softmax and O^T 1.8, exchange 1.1 (28 KB per CTA; distributed shared memory
+// moves 16 B/clk per SM when all SMs send), combine 0.5; DRAM and the tensor pipes idle.
 // ---------------------------------------------------------------------------------------------
 struct DecAttnArgs {
     const bf16* q; const bf16* k; const bf16* v; bf16* out;
@@ -300,7 +307,7 @@ struct DecAttnArgs {
     int prefix_keys;            // keys [0, prefix_keys) were not written by the preceding kernel
     // plan
     int splits;                 // cluster size
-    int kp, nd;                 // prefix keys and own keys per CTA
+    int kp, nd;                 // KT = 1: keys per CTA, 0; KT = 2: prefix keys and own keys per CTA
     int pad;                    // rows of a CTA's K / V tile: kp + nd rounded up to 16
     int k_region;               // bytes of the K tile, or of the receive area that takes its place if that is larger
     int* status;
@@ -309,20 +316,21 @@ struct DecAttnArgs {
 
 namespace decattn {
 constexpr int HD = 256, BQ = 32, UNIT = 4, MIN_SPL = 4, MAX_SPL = 11, THREADS = 256;
-constexpr int S_COL = 64;                           // TMEM columns: O^T at 0 and 32; S^T at S_COL + 64 tile + 32 (half of the dims)
+// TMEM columns: O^T at 64 group + 32 (tile of 128 dims), behind them S^T at 64 tile + 32 (half of the dims)
 constexpr int MAX_PAD = 208;                        // K + V tiles of 208 rows, Q / P and the rest just fit the SM
 constexpr int QP_BYTES = 16384;                     // Q: 4 blocks of 64 dims x 32 rows; later P: up to 4 blocks of 64 keys x 32 rows
 constexpr int UNIT_BYTES = HD * UNIT * 4;           // what one CTA sends for four rows
-constexpr int OFF_PART = 64;                        // behind the barriers: row maxima, then sums, per (row half, quadrant, 16 rows)
-constexpr int OFF_MAX = OFF_PART + 1024, OFF_STATS = OFF_MAX + 128;        // this CTA's row maxima; received (max, sum): [src][slot 2][row 4]
-constexpr int MISC_BYTES = OFF_STATS + MAX_SPL * 64;
-constexpr float NO_KEY = -1e30f;                    // maximum of a row that sees none of a CTA's keys: its weight in the merge is 0
-constexpr int units_per_owner(int spl) { return (BQ / UNIT + spl - 1) / spl; }
+constexpr int OFF_PART = 64;                        // behind the barriers: row maxima and sums of one key tile
+constexpr int OFF_STATS = OFF_PART + 1024;          // received log-sum-exps: [src][slot 2][row 4]
+constexpr int MISC_BYTES = OFF_STATS + MAX_SPL * 32;
+// KT = 1 only, behind the rest: per warp the weights of the two groups and 1 / sum, 32 rows each; fp32 probabilities, [row][key]
+constexpr int FAC_BYTES = 8 * 384, E_PITCH = 136, E_BYTES = BQ * E_PITCH * 4;
+__host__ __device__ constexpr int units_per_owner(int spl) { return (BQ / UNIT + spl - 1) / spl; }
 inline int k_region_bytes(int spl, int pad) {
     const int recv = spl * units_per_owner(spl) * UNIT_BYTES;
     return pad * 512 > recv ? pad * 512 : recv;
 }
-inline int smem_bytes(int spl, int pad) { return 1024 + k_region_bytes(spl, pad) + pad * 512 + QP_BYTES + MISC_BYTES; }
+inline int smem_bytes(int spl, int pad) { return 1024 + k_region_bytes(spl, pad) + pad * 512 + QP_BYTES + MISC_BYTES + (pad <= 128 ? FAC_BYTES + E_BYTES : 0); }
 
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) { return tc5::mbar_wait(bar, parity, abort_flag); }
 __device__ __forceinline__ uint32_t idesc(bool a_mn) { return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | ((uint32_t)(BQ >> 3) << 17) | (8u << 24); }
@@ -342,14 +350,14 @@ __device__ __forceinline__ float butterfly16(float (&v)[16], int lane, Op op) {
     }
     return op(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1));
 }
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float4 lds4(uint32_t a) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 lds2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ float lds1(uint32_t a) {
@@ -376,12 +384,17 @@ template <int KT, int SPL>                                // key tiles of 128 pe
 __global__ void __launch_bounds__(decattn::THREADS, 1)
 decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV) {
     using namespace decattn;
-    constexpr int S_ISSUERS = 2 * KT, TMEM_COLS = KT == 1 ? 128 : 256;
+    constexpr int S_ISSUERS = 2 * KT, GROUPS = 2 * KT, S_COL = 64 * GROUPS, TMEM_COLS = 256 * KT;
+    constexpr int RECV = SPL * units_per_owner(SPL) * UNIT_BYTES;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     const uint32_t sK = (smem_u32(smem_raw) + 1023u) & ~1023u, sV = sK + p.k_region, sQ = sV + p.pad * 512, misc = sQ + QP_BYTES;
     uint8_t* gmisc = smem_raw + (misc - smem_u32(smem_raw));
     const uint32_t pre_bar = misc, in_bar = misc + 8, s_bar = misc + 16, o_bar = misc + 24;
-    const uint32_t part = misc + OFF_PART, row_max = misc + OFF_MAX, stats_in = misc + OFF_STATS;
+    const uint32_t stats_in = misc + OFF_STATS, esum = misc + MISC_BYTES + FAC_BYTES;
+    // Row maxima, then sums: [tile][row half][quadrant][16 rows] (sums of one tile: [group][row]); weights and 1 / sum per warp. Two tiles
+    // leave no room for them; they lie in the K tile then, behind what the peers send, once the MMAs have read it.
+    const uint32_t maxima = KT == 1 ? misc + OFF_PART : sK + RECV, sums = maxima + KT * 512;
+    const uint32_t fac = (KT == 1 ? misc + MISC_BYTES : sums + KT * 512) + (threadIdx.x >> 5) * (GROUPS + 1) * BQ * 4;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gmisc + 32);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gmisc + 36);
 
@@ -394,7 +407,8 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     const float scale = p.scale_log2;
     const int pre_rows = min(p.prefix_keys, p.nk);
     const int key0 = (int)rank * p.kp, prefix_here = max(0, min(p.kp, pre_rows - key0));        // local keys [0, prefix_here): prefix
-    const int new0 = (int)rank * p.nd, new_here = max(0, min(p.nd, p.nk - pre_rows - new0));    // then new_here of the step's own
+    const int new0 = KT == 1 ? max(0, key0 - pre_rows) : (int)rank * p.nd;                      // then new_here of the step's own
+    const int new_here = max(0, min(KT == 1 ? p.kp - prefix_here : p.nd, p.nk - pre_rows - new0));
     const int owned = (int)rank < units ? 1 + ((int)rank + SPL < units ? 1 : 0) : 0;            // units rank, rank + SPL
 
     if (tid == 0) {
@@ -404,7 +418,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         tc5::mbar_init(o_bar, 2);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (owned > 0) tc5::mbar_expect_tx(in_bar, (uint32_t)(owned * SPL) * (UNIT_BYTES + UNIT * 8));
+        if (owned > 0) tc5::mbar_expect_tx(in_bar, (uint32_t)(owned * SPL) * (UNIT_BYTES + UNIT * 4));
         // The prefix rows of K and V arrive as one box of 64 dims x pad rows per block, through maps that END at the prefix:
         // the rows behind it, which the preceding kernel may still be writing, are not touched in memory and read as
         // zero. (Rows past prefix_here hold the next CTA's keys; the own keys overwrite some, the rest is masked.)
@@ -437,27 +451,34 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
             const int idx = tid + i * THREADS;
             qv[i] = idx < rows_here * 32 ? *reinterpret_cast<const uint4*>(gq + (size_t)idx * 8) : make_uint4(0, 0, 0, 0);
         }
-        uint4 kvv[2];                                        // first batch of own rows: 8 rows of K and V
+        constexpr int OWN = KT == 1 ? 8 : 4;                 // own keys, 8 rows per piece index; with KT = 1 one or two CTAs have them all
+        uint4 kv[OWN], vv[OWN];
         const int total = new_here * 32;
-        if (tid < total) {
-            kvv[0] = *reinterpret_cast<const uint4*>(p.k + kv0 + (size_t)tid * 8);
-            kvv[1] = *reinterpret_cast<const uint4*>(p.v + kv0 + (size_t)tid * 8);
-        }
+        auto fetch_own = [&](int base) {
+#pragma unroll
+            for (int i = 0; i < OWN; ++i) {
+                const int idx = base + tid + i * THREADS;
+                if (idx < total) {
+                    kv[i] = *reinterpret_cast<const uint4*>(p.k + kv0 + (size_t)idx * 8);
+                    vv[i] = *reinterpret_cast<const uint4*>(p.v + kv0 + (size_t)idx * 8);
+                }
+            }
+        };
+        fetch_own(0);
 #pragma unroll
         for (int i = 0; i < QV; ++i) {
             const int idx = tid + i * THREADS, r = idx >> 5, c = idx & 31;
             sts4u(sQ + (c >> 3) * (BQ * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), qv[i]);
         }
         wait(pre_bar, 0, abort_flag);                        // the own rows go over what the boxes brought in
-        for (int idx = tid; idx < total; idx += THREADS) {
-            if (idx != tid) {
-                kvv[0] = *reinterpret_cast<const uint4*>(p.k + kv0 + (size_t)idx * 8);
-                kvv[1] = *reinterpret_cast<const uint4*>(p.v + kv0 + (size_t)idx * 8);
+        for (int base = 0; base < total; base += OWN * THREADS) {
+            if (base > 0) fetch_own(base);
+#pragma unroll
+            for (int i = 0; i < OWN; ++i) {
+                const int idx = base + tid + i * THREADS, r = prefix_here + (idx >> 5), c = idx & 31;
+                const uint32_t at = (c >> 3) * p.pad * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                if (idx < total) { sts4u(sK + at, kv[i]); sts4u(sV + at, vv[i]); }
             }
-            const int r = prefix_here + (idx >> 5), c = idx & 31;
-            const uint32_t at = (c >> 3) * p.pad * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4);
-            sts4u(sK + at, kvv[0]);
-            sts4u(sV + at, kvv[1]);
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -465,15 +486,16 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     FVLA_STAMP(2);
     // Issuing threads: for S^T one per key tile and half of the head dimension (accumulators added below), for O^T one per 128
     // dims. A thread needs 46 clk per MMA and more for the first, the tensor pipe 39.
-    if (lane == 0 && warp < S_ISSUERS) {
+    const int uniform_warp = __shfl_sync(0xffffffffu, warp, 0);
+    if (uniform_warp < S_ISSUERS && tc5::elect_one()) {
         tc5::tc_fence_after();
-        const int t = warp >> 1, h = warp & 1;
+        const int t = uniform_warp >> 1, h = uniform_warp & 1;
         const uint64_t a0 = tc5::smem_desc(sK + t * 128 * 128 + h * p.pad * 256, 16, 1024), b0 = tc5::smem_desc(sQ + h * (BQ * 256), 16, 1024);
 #pragma unroll
         for (int cb = 0; cb < 2; ++cb)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                tc5::umma_bf16(tmem + S_COL + warp * 32, a0 + cb * (p.pad * 8) + k * 2, b0 + cb * (BQ * 8) + k * 2, idesc(false), (cb | k) ? 1u : 0u);
+                tc5::umma_bf16(tmem + S_COL + uniform_warp * 32, a0 + cb * (p.pad * 8) + k * 2, b0 + cb * (BQ * 8) + k * 2, idesc(false), (cb | k) ? 1u : 0u);
         tc5::umma_commit(s_bar);
     }
     __syncwarp();
@@ -484,7 +506,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     // no data is handed over, and a releasing arrive waits 0.4 us for the thread's earlier accesses.
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     FVLA_STAMP(3);
-    const uint64_t vd = tc5::smem_desc(sV + warp * 2 * p.pad * 128, p.pad * 128, 1024), pd = tc5::smem_desc(sQ, 16, 1024);      // warps 0, 1: operands of O^T
+    const uint64_t vd = tc5::smem_desc(sV + uniform_warp * 2 * p.pad * 128, p.pad * 128, 1024), pd = tc5::smem_desc(sQ, 16, 1024);      // warps 0, 1: operands of O^T
     const int quad = warp & 3, half = warp >> 2;             // keys 32 quad .. + 31 of a tile, rows 16 half .. + 15
     {
         float v[KT][16], red[16];
@@ -505,35 +527,29 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
             }
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) red[i] = KT == 1 ? v[0][i] : fmaxf(v[0][i], v[KT - 1][i]);
-        const float m = butterfly16(red, lane, [](float a, float b) { return fmaxf(a, b); });
-        if ((lane & 1) == 0) sts1(part + ((half * 4 + quad) * 16 + (lane >> 1)) * 4, fmaxf(m, NO_KEY));
+        for (int t = 0; t < KT; ++t) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) red[i] = v[t][i];
+            const float m = butterfly16(red, lane, [](float a, float b) { return fmaxf(a, b); });
+            if ((lane & 1) == 0) sts1(maxima + (((t * 2 + half) * 4 + quad) * 16 + (lane >> 1)) * 4, m);
+        }
         __syncthreads();
-        float mx[16];
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-            float4 a = lds4(part + (half * 64 + i) * 4);
-#pragma unroll
-            for (int qd = 1; qd < 4; ++qd) {
-                const float4 b = lds4(part + (half * 64 + qd * 16 + i) * 4);
-                a.x = fmaxf(a.x, b.x); a.y = fmaxf(a.y, b.y); a.z = fmaxf(a.z, b.z); a.w = fmaxf(a.w, b.w);
-            }
-            mx[i] = a.x; mx[i + 1] = a.y; mx[i + 2] = a.z; mx[i + 3] = a.w;
-        }
-        if (quad == 0 && lane == 0) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) sts1(row_max + (half * 16 + i) * 4, mx[i]);
-        }
 #pragma unroll
         for (int t = 0; t < KT; ++t) {
             const int key = t * 128 + quad * 32 + lane;
             // P over Q, whose readers are done; rows of a 64-key block are 128 bytes, 16-byte piece c of row r at c ^ (r & 7)
+            const uint32_t at = maxima + ((t * 2 + half) * 64 + (quad >> 1) * 32) * 4;      // of the key's group, 0 where a row sees none of its keys
             const uint32_t dst = sQ + (key >> 6) * (BQ * 128) + half * 16 * 128 + (key & 7) * 2, c = ((key & 63) >> 3) << 4;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float e = ex2(v[t][i] - mx[i]);
-                red[i] = t == 0 ? e : red[i] + e;
-                v[t][i] = e;
+            for (int i = 0; i < 16; i += 4) {
+                const float4 a = lds4(at + i * 4), b = lds4(at + i * 4 + 64);
+                const float mx[4] = {fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w)};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float e = exp2f(v[t][i + r] - (mx[r] == -INFINITY ? 0.f : mx[r]));
+                    if (KT == 1) sts1(esum + ((half * 16 + i + r) * E_PITCH + key) * 4, e);
+                    v[t][i + r] = e;
+                }
             }
             if (key < p.pad) {
 #pragma unroll
@@ -543,25 +559,76 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         tc5::tc_fence_before();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (lane == 0 && warp < 2) {
+        if (uniform_warp < 2 && tc5::elect_one()) {
             tc5::tc_fence_after();
 #pragma unroll
             for (int k = 0; k < (KT == 1 ? 8 : MAX_PAD / 16); ++k)
-                if (k * 16 < p.pad) tc5::umma_bf16(tmem + warp * 32, vd + k * 128, pd + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true), k ? 1u : 0u);
+                if (k * 16 < p.pad)
+                    tc5::umma_bf16(tmem + (k >> 2) * 64 + uniform_warp * 32, vd + k * 128, pd + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true),
+                                   k & 3 ? 1u : 0u);
             tc5::umma_commit(o_bar);
         }
         __syncwarp();
-        const float l = butterfly16(red, lane, [](float a, float b) { return a + b; });
-        if ((lane & 1) == 0) sts1(part + 512 + ((half * 4 + quad) * 16 + (lane >> 1)) * 4, l);
+        if (KT == 1) {
+            // Sum of a row over a group of 64 keys, four threads: each takes a pair of keys out of every eight, front to back.
+            const int row = (warp >> 1) * 8 + (lane >> 2), group = warp & 1;
+            const uint32_t at = esum + (row * E_PITCH + group * 64 + (lane & 3) * 2) * 4;
+            float2 e[8];
+#pragma unroll
+            for (int n = 0; n < 8; ++n) e[n] = lds2(at + n * 32);
+            float l = 0.f;
+#pragma unroll
+            for (int n = 0; n < 8; ++n) { l += e[n].x; l += e[n].y; }
+            l += __shfl_xor_sync(0xffffffffu, l, 1);
+            l += __shfl_xor_sync(0xffffffffu, l, 2);
+            if ((lane & 3) == 0) sts1(sums + (group * BQ + row) * 4, l);
+        } else {
+#pragma unroll
+            for (int t = 0; t < KT; ++t) {
+                const float l = butterfly16(v[t], lane, [](float a, float b) { return a + b; });
+                if ((lane & 1) == 0) sts1(sums + (((t * 2 + half) * 4 + quad) * 16 + (lane >> 1)) * 4, l);
+            }
+        }
     }
     __syncthreads();                                         // sums and maxima of all rows are in place
+    // Every warp works out what its accumulator columns are multiplied with, lane = row: [group][row], then 1 / sum
+    float f[2][BQ], fi[BQ], lse;                              // (the first two groups' in registers before the accumulators are there)
+    auto factors = [&](int g, float (&out)[BQ]) {
+#pragma unroll
+        for (int i = 0; i < BQ; i += 4) {
+            const float4 a = lds4(fac + (g * BQ + i) * 4);
+            out[i] = a.x; out[i + 1] = a.y; out[i + 2] = a.z; out[i + 3] = a.w;
+        }
+    };
+    {
+        const int row = lane >> 4, i = lane & 15;
+        float m[GROUPS], mn = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            const uint32_t at = maxima + (((g >> 1) * 2 + row) * 64 + (g & 1) * 32 + i) * 4;
+            m[g] = fmaxf(lds1(at), lds1(at + 64));
+            mn = fmaxf(mn, m[g]);
+        }
+        const float mu = mn == -INFINITY ? 0.f : mn;
+#pragma unroll
+        for (int g = 0; g < GROUPS; ++g) {
+            const uint32_t at = sums + (((g >> 1) * 2 + row) * 64 + (g & 1) * 32 + i) * 4;
+            const float a = exp2f(m[g] - mu), lg = KT == 1 ? lds1(sums + (g * BQ + lane) * 4) : lds1(at) + lds1(at + 64);      // exp2(-inf) = 0
+            l = g == 0 ? __fmul_rn(lg, a) : __fmaf_rn(lg, a, l);
+            sts1(fac + (g * BQ + lane) * 4, a);
+        }
+        sts1(fac + (GROUPS * BQ + lane) * 4, l > 0.f ? 1.0f / l : 0.f);
+        lse = l > 0.f ? mn + log2f(l) : -INFINITY;
+        __syncwarp();
+        factors(0, f[0]);
+        factors(1, f[1]);
+        factors(GROUPS, fi);
+    }
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (tid < units * UNIT) {                                // row tid's (max, sum) to its owner
-        const int u = tid >> 2, owner = u % SPL, slot = u / SPL, h = tid >> 4, i = tid & 15;
-        const uint32_t pl = part + 512 + (h * 64 + i) * 4;
-        const float l = lds1(pl) + lds1(pl + 64) + lds1(pl + 128) + lds1(pl + 192);
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
-                     ::"r"(dsm_map(misc + OFF_STATS + rank * 64 + slot * 32 + (tid & 3) * 8, owner)), "f"(lds1(row_max + tid * 4)), "f"(l), "r"(dsm_map(in_bar, owner)) : "memory");
+    if (warp == 0 && lane < units * UNIT) {                  // row lane's log-sum-exp to its owner
+        const int u = lane >> 2, owner = u % SPL, slot = u / SPL;
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];"
+                     ::"r"(dsm_map(stats_in + rank * 32 + slot * 16 + (lane & 3) * 4, owner)), "f"(lse), "r"(dsm_map(in_bar, owner)) : "memory");
     }
     wait(o_bar, 0, abort_flag);
     __syncwarp();
@@ -570,6 +637,19 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     {
         float o[32];
         tc5::tmem_ld32(tmem + half * 32 + ((uint32_t)(quad * 32) << 16), o);                   // dim 128 half + 32 quad + lane
+#pragma unroll
+        for (int i = 0; i < BQ; ++i) o[i] = __fmul_rn(o[i], f[0][i]);      // (the rounding of each step is part of the result: no other contraction)
+#pragma unroll
+        for (int g = 1; g < GROUPS; ++g) {
+            if (g * 64 >= p.pad) break;                      // a group without keys has no accumulator
+            float og[32];
+            tc5::tmem_ld32(tmem + g * 64 + half * 32 + ((uint32_t)(quad * 32) << 16), og);
+            if (g > 1) factors(g, f[1]);
+#pragma unroll
+            for (int i = 0; i < BQ; ++i) o[i] = __fmaf_rn(og[i], f[1][i], o[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < BQ; ++i) o[i] *= fi[i];
         const uint32_t at = sK + rank * UNIT_BYTES + (half * 128 + quad * 32 + lane) * 16;
 #pragma unroll
         for (int u = 0; u < BQ / UNIT; ++u) {
@@ -591,33 +671,32 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         const int row0 = q0 + ((int)rank + slot * SPL) * UNIT;
         // log-sum-exp weights: lane = (source, row), a second one for sources 8 and up
         const int s0 = lane >> 2;
-        const uint32_t st = stats_in + s0 * 64 + slot * 32 + (lane & 3) * 8;
+        const uint32_t st = stats_in + s0 * 32 + slot * 16 + (lane & 3) * 4;
         const bool have0 = SPL >= 8 || s0 < SPL, have1 = SPL > 8 && s0 + 8 < SPL;
-        const float m0 = have0 ? lds1(st) : NO_KEY, m1 = have1 ? lds1(st + 512) : NO_KEY;
-        float mx = fmaxf(m0, m1);
+        const float l0 = have0 ? lds1(st) : -INFINITY, l1 = have1 ? lds1(st + 256) : -INFINITY;
+        float mx = fmaxf(l0, l1);
 #pragma unroll
         for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        float w0 = have0 ? ex2(m0 - mx) : 0.f, w1 = have1 ? ex2(m1 - mx) : 0.f;
-        float wsum = (have0 ? w0 * lds1(st + 4) : 0.f) + (have1 ? w1 * lds1(st + 516) : 0.f);
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
-        const float inv = wsum > 0.f ? 1.0f / wsum : 0.f;
-        w0 *= inv; w1 *= inv;
-        float acc[UNIT] = {0.f, 0.f, 0.f, 0.f};
+        const float w0 = l0 == -INFINITY ? 0.f : exp2f(l0 - mx), w1 = l1 == -INFINITY ? 0.f : exp2f(l1 - mx);
+        float acc[UNIT] = {0.f, 0.f, 0.f, 0.f}, wsum[UNIT] = {0.f, 0.f, 0.f, 0.f};
         const uint32_t src = sK + slot * SPL * UNIT_BYTES + tid * 16;
         float4 in[SPL];                                       // all sources requested before the first is used
 #pragma unroll
         for (int s = 0; s < SPL; ++s) in[s] = lds4(src + s * UNIT_BYTES);
 #pragma unroll
         for (int s = 0; s < SPL; ++s) {
-            const float4 a = in[s];
-            const float w = s < 8 ? w0 : w1;
-            const int from = (s & 7) * 4;
-            acc[0] = fmaf(__shfl_sync(0xffffffffu, w, from), a.x, acc[0]);
-            acc[1] = fmaf(__shfl_sync(0xffffffffu, w, from + 1), a.y, acc[1]);
-            acc[2] = fmaf(__shfl_sync(0xffffffffu, w, from + 2), a.z, acc[2]);
-            acc[3] = fmaf(__shfl_sync(0xffffffffu, w, from + 3), a.w, acc[3]);
+            const float a[UNIT] = {in[s].x, in[s].y, in[s].z, in[s].w};
+#pragma unroll
+            for (int r = 0; r < UNIT; ++r) {
+                const float w = __shfl_sync(0xffffffffu, s < 8 ? w0 : w1, (s & 7) * 4 + r);
+                wsum[r] += w;
+                acc[r] = __fmaf_rn(w, a[r], acc[r]);
+            }
         }
+        const float ws = lane & 2 ? (lane & 1 ? wsum[3] : wsum[2]) : (lane & 1 ? wsum[1] : wsum[0]);
+        const float inv = ws > 0.f ? 1.0f / ws : 0.f;
+#pragma unroll
+        for (int r = 0; r < UNIT; ++r) acc[r] *= __shfl_sync(0xffffffffu, inv, r);
         // two adjacent dims of two rows per lane, so that a store is a bf16 pair: even lanes rows 0 and 1, odd lanes 2 and 3
         const bool odd = lane & 1;
         const float r0 = __shfl_xor_sync(0xffffffffu, odd ? acc[0] : acc[2], 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? acc[1] : acc[3], 1);
@@ -668,7 +747,7 @@ inline int resident_attention_clusters(int spl) {
     int n = c.load(std::memory_order_acquire);
     if (n == 0) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1, spl); cfg.blockDim = dim3(decattn::THREADS); cfg.dynamicSmemBytes = 160 * 1024;
+        cfg.gridDim = dim3(1, spl); cfg.blockDim = dim3(decattn::THREADS); cfg.dynamicSmemBytes = 168 * 1024;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = spl; attr[0].val.clusterDim.z = 1;
@@ -679,23 +758,37 @@ inline int resident_attention_clusters(int spl) {
     return n;
 }
 
-// Cluster size, smallest first in every order of preference. Ask that all clusters of the launch are resident together, with
-// one key tile of at most 128 rows and 4 or 8 CTAs, so that the eight owners' shares come out even (819 keys: 8 CTAs 29.7 us per
-// layer-step, 5 or 7 CTAs 30.7); then any size with one key tile; then with two (65 tokens x 882 keys: 40.5 us with 5
-// CTAs, all 17 clusters resident, 44.3 with 8, of which 15 are). Failing that the smallest that fits the SM at all. Returns whether
-// all clusters are resident; 0 splits: the shape does not fit.
+// How the keys are shared out. One sequence of up to 64 tokens and 1 408 keys: ranges of 8 clusters' CTAs up to 1 024 keys and one
+// CTA more per further 128, whatever is resident, so that the results of such a decode depend on nothing but its shape (and are the
+// bits of the kernel before, see above). Else the cluster size, smallest first in every order of preference: all clusters of the
+// launch resident together, with one key tile of at most 128 rows and 4 or 8 CTAs, so that the eight owners' shares come out even; then
+// any size with one key tile; then with two (65 tokens x 882 keys: 40.5 us per layer-step with 5 CTAs, all 17 clusters resident, 44.3
+// with 8, of which 15 are). Failing that the smallest that fits the SM at all. Returns whether all clusters are resident; 0 splits: the
+// shape does not fit.
 inline bool plan_decoder_attention(DecAttnArgs& a) {
     using namespace decattn;
     a.splits = 0;
     if (a.prefix_keys <= 0 || !configure_decoder_attention()) return false;
     const int clusters = ((a.nq + BQ - 1) / BQ) * (a.episodes > 1 ? a.episodes : 1), pre = a.prefix_keys < a.nk ? a.prefix_keys : a.nk;
+    auto take = [&](int spl) {                               // false: more rows than the SM holds
+        const int range = ((a.nk + spl - 1) / spl + 7) / 8 * 8;
+        a.kp = range <= 128 ? range : (pre + spl - 1) / spl;
+        a.nd = range <= 128 ? 0 : (a.nk - pre + spl - 1) / spl;
+        a.pad = (a.kp + a.nd + 15) / 16 * 16;
+        a.k_region = k_region_bytes(spl, a.pad);
+        return a.pad <= MAX_PAD && smem_bytes(spl, a.pad) <= 232448;
+    };
+    const int ranges = (a.nk + 127) / 128 < 8 ? 8 : (a.nk + 127) / 128;
+    if (a.episodes <= 1 && a.nq <= 512 && ranges <= MAX_SPL && take(ranges)) {
+        a.splits = ranges;
+        return clusters <= resident_attention_clusters(ranges);
+    }
     for (int pass = 0; pass < 4; ++pass)
         for (int spl = MIN_SPL; spl <= MAX_SPL; ++spl) {
-            const int kp = (pre + spl - 1) / spl, nd = (a.nk - pre + spl - 1) / spl, pad = (kp + nd + 15) / 16 * 16;
             if (pass == 0 && spl != 4 && spl != 8) continue;
-            if (pad > (pass < 2 ? 128 : MAX_PAD) || smem_bytes(spl, pad) > 232448) continue;
+            if (!take(spl) || (pass < 2 && a.pad > 128)) continue;
             if (pass < 3 && clusters > resident_attention_clusters(spl)) continue;
-            a.splits = spl; a.kp = kp; a.nd = nd; a.pad = pad; a.k_region = k_region_bytes(spl, pad);
+            a.splits = spl;
             return pass < 3;
         }
     return false;

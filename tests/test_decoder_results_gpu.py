@@ -63,5 +63,53 @@ def test_projections_keep_their_bits(rows):
     assert projections(rows) == json.loads(GOLDEN.read_text())[f"projections {rows}"]
 
 
+# one group of 64 keys per CTA and two; ranks without keys; 8 ranges of keys and 11; the last rows of a cluster missing
+ATTENTION = [(1, 40), (11, 273), (51, 768), (33, 1000), (64, 1280), (20, 1357)]
+
+
+def attention(tokens, S):
+    from flash_vla_b200 import op_table
+    g = torch.Generator().manual_seed(tokens * S)
+    q, k, v = rnd(g, tokens * 8, 256), rnd(g, S + tokens, 256), rnd(g, S + tokens, 256)
+    op_table(True).decoder_attention(q, k, v, None, q, S)
+    return digest(q)
+
+
+@pytest.mark.parametrize("tokens,S", ATTENTION)
+def test_attention_keeps_its_bits(tokens, S):
+    assert attention(tokens, S) == json.loads(GOLDEN.read_text())[f"attention {tokens} {S}"]
+
+
+def decode(chunk, views, prompt, steps=10, layers=3):
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0 import pipeline
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import wrappers
+    from flash_vla_b200.hardware.nvidia.b200.pi0.buffers import allocate_static_buffers
+    from flash_vla_b200.models.pi0.spec import weight_shapes
+    from flash_vla_b200.runtime.cuda import ScratchPool
+    g = torch.Generator().manual_seed(chunk)
+    w = {n: rnd(g, *((layers, *s[1:]) if s[0] == 18 else s), scale=0.02) for n, s in weight_shapes(0).items() if n.startswith("decoder_")}
+    b, S = allocate_static_buffers(views, chunk, prompt, "cuda")
+    wrappers.register_bf16_shadow(b["decoder_x"], b["decoder_x_bf16"])
+    for cache in ("encoder_K", "encoder_V"):
+        b[cache][:layers, :S].copy_(rnd(g, layers, S, 256))
+    b["observation_state_normalized"].copy_(rnd(g, 32))
+    b["diffusion_noise"].copy_(rnd(g, chunk, 32))
+    with wrappers.use_pool(ScratchPool()):
+        pipeline.transformer_decoder(op_table(True), w, b, S, steps=steps, layers=layers)
+    return digest(b["diffusion_noise"], b["diffusion_noise_f32"], b["encoder_K"], b["encoder_V"])
+
+
+DECODES = [(50, 3, 0), (10, 1, 17), (63, 3, 48)]
+
+
+@pytest.mark.parametrize("chunk,views,prompt", DECODES)
+def test_ten_euler_steps_keep_their_bits(chunk, views, prompt):
+    assert decode(chunk, views, prompt) == json.loads(GOLDEN.read_text())[f"decode {chunk} {views} {prompt}"]
+
+
 if __name__ == "__main__":
-    print(json.dumps({f"projections {M}": projections(M) for M in (1, 33, 51, 64)}, indent=1))
+    got = {f"projections {M}": projections(M) for M in (1, 33, 51, 64)}
+    got.update({f"attention {t} {S}": attention(t, S) for t, S in ATTENTION})
+    got.update({f"decode {c} {v} {p}": decode(c, v, p) for c, v, p in DECODES})
+    print(json.dumps(got, indent=1))
