@@ -237,7 +237,7 @@ using namespace fvla;
 extern "C" {
 
 const char* fvla_last_error(void) { return g_error; }
-int fvla_abi_version(void) { return 4; }
+int fvla_abi_version(void) { return 5; }
 unsigned long long fvla_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 int fvla_device_status(void* stream) {
@@ -760,7 +760,7 @@ int fvla_decoder_steps_run(const struct fvla_decoder_steps* d, void* stream) {
             bf16* k = Bm(d->k_cache) + (size_t)l * d->cache_rows * HD;
             bf16* v = Bm(d->v_cache) + (size_t)l * d->cache_rows * HD;
             const size_t tail = (size_t)d->prefix * HD;
-            rc = fvla_decoder_norm_qkv_rope(x, 1, shadow, B(d->qkv_w) + (size_t)l * W * QKV, d->rope, d->q, k + tail, v + tail, nullptr, D, W, HEADS, HD, 0, 0,
+            rc = fvla_decoder_norm_qkv_rope(x, 1, shadow, B(d->qkv_w) + (size_t)l * W * QKV, d->rope, d->q, k + tail, v + tail, d->norm_factor, D, W, HEADS, HD, 0, 0,
                                             d->ws_qkv, d->ws_qkv_bytes, stream);
             if (!rc) rc = fvla_decoder_attention(d->q, k, v, d->q, D * HEADS, d->cache_rows, HD, HEADS, d->prefix, 1, (long long)D * HEADS * HD, 0,
                                                  d->ws_attn, d->ws_attn_bytes, stream);

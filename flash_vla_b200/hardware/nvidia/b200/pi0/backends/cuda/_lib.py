@@ -21,7 +21,8 @@ class DecoderSteps(ctypes.Structure):
                                    "out_w", "out_b", "rope", "state", "noise", "noise_f32", "x", "x_shadow", "in_buf", "q",
                                    "hidden", "k_cache", "v_cache", "ws_mlp", "ws_qkv", "ws_attn", "ws_o", "ws_gate", "ws_down")] +
                 [(n, _Z) for n in ("ws_mlp_bytes", "ws_qkv_bytes", "ws_attn_bytes", "ws_o_bytes", "ws_gate_bytes", "ws_down_bytes")] +
-                [(n, _I) for n in ("chunk", "prefix", "cache_rows", "first_step", "steps", "layers")])
+                [(n, _I) for n in ("chunk", "prefix", "cache_rows", "first_step", "steps", "layers")] +
+                [("norm_factor", _P)])
 
 
 # name -> argument ctypes (every function returns int except the three queries below)

@@ -192,12 +192,15 @@ def decoder_epilogue_batched(dec):
 def decoder_prologue(ops, weights, buffers):
     """What the decoder needs before its first step and that does not depend on the encoder: the state
     token's projection and the fp32 master copy of the noise."""
-    b = buffers
-    ops.decoder_state_proj(b["observation_state_normalized"], weights["decoder_state_in_proj_w"],
-                           weights["decoder_state_in_proj_b"], b["decoder_state_buf"])
-    master = b.get("diffusion_noise_f32")
+    _project_state(ops, weights, buffers)
+    master = buffers.get("diffusion_noise_f32")
     if master is not None:
-        _copy(ops, master, b["diffusion_noise"])
+        _copy(ops, master, buffers["diffusion_noise"])
+
+
+def _project_state(ops, weights, buffers):
+    ops.decoder_state_proj(buffers["observation_state_normalized"], weights["decoder_state_in_proj_w"],
+                           weights["decoder_state_in_proj_b"], buffers["decoder_state_buf"])
 
 
 def decoder_epilogue(buffers, ops=None):
@@ -211,17 +214,18 @@ def transformer_decoder(ops, weights, buffers, encoder_seq_len, steps=DIFFUSION_
                         layers=ENCODER_LAYERS, first_step=0):
     """Denoise the action chunk in `diffusion_noise` over `steps` Euler steps. `first_step > 0` resumes
     after steps that were run separately (prologue included), see `Pi0Inference`. A table that offers the loop as one
-    stage issues the same launches by that one call."""
+    stage issues the same launches by that one call, as long as it still has the ops that the stage stands for."""
     b = buffers
     master = b.get("diffusion_noise_f32")
-    if hasattr(ops, "decoder_steps"):
-        if first_step == 0:
-            ops.decoder_state_proj(b["observation_state_normalized"], weights["decoder_state_in_proj_w"],
-                                   weights["decoder_state_in_proj_b"], b["decoder_state_buf"])
-        if ops.decoder_steps(weights, b, encoder_seq_len, steps, layers, first_step):
-            return
     if first_step == 0:
-        decoder_prologue(ops, weights, b)
+        _project_state(ops, weights, b)
+    stage = getattr(ops, "decoder_steps", None)
+    stands_for = getattr(stage, "stands_for", None)
+    if stands_for and all(getattr(ops, name, None) is op for name, op in stands_for.items()):
+        if stage(weights, b, encoder_seq_len, steps, layers, first_step):
+            return
+    if first_step == 0 and master is not None:
+        _copy(ops, master, b["diffusion_noise"])
     for step in range(first_step, steps):
         decoder_step(ops, weights, b, encoder_seq_len, step, layers, noise=master)
     decoder_epilogue(b, ops)

@@ -228,6 +228,7 @@ struct fvla_decoder_steps {
     void *ws_mlp, *ws_qkv, *ws_attn, *ws_o, *ws_gate, *ws_down;
     size_t ws_mlp_bytes, ws_qkv_bytes, ws_attn_bytes, ws_o_bytes, ws_gate_bytes, ws_down_bytes;
     int chunk, prefix, cache_rows, first_step, steps, layers;
+    void* norm_factor;      /* chunk + 1 bf16: the factor of the last QKV projection, as fvla_decoder_norm_qkv_rope stores it (may be NULL) */
 };
 int fvla_decoder_steps_run(const struct fvla_decoder_steps* args, void* stream);
 

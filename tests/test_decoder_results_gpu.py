@@ -80,13 +80,10 @@ def test_attention_keeps_its_bits(tokens, S):
     assert attention(tokens, S) == json.loads(GOLDEN.read_text())[f"attention {tokens} {S}"]
 
 
-def decode(chunk, views, prompt, steps=10, layers=3):
-    from flash_vla_b200 import op_table
-    from flash_vla_b200.hardware.nvidia.b200.pi0 import pipeline
+def decoder_state(chunk, views=3, prompt=0, layers=3):
     from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import wrappers
     from flash_vla_b200.hardware.nvidia.b200.pi0.buffers import allocate_static_buffers
     from flash_vla_b200.models.pi0.spec import weight_shapes
-    from flash_vla_b200.runtime.cuda import ScratchPool
     g = torch.Generator().manual_seed(chunk)
     w = {n: rnd(g, *((layers, *s[1:]) if s[0] == 18 else s), scale=0.02) for n, s in weight_shapes(0).items() if n.startswith("decoder_")}
     b, S = allocate_static_buffers(views, chunk, prompt, "cuda")
@@ -95,6 +92,15 @@ def decode(chunk, views, prompt, steps=10, layers=3):
         b[cache][:layers, :S].copy_(rnd(g, layers, S, 256))
     b["observation_state_normalized"].copy_(rnd(g, 32))
     b["diffusion_noise"].copy_(rnd(g, chunk, 32))
+    return w, b, S
+
+
+def decode(chunk, views, prompt, steps=10, layers=3):
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0 import pipeline
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import wrappers
+    from flash_vla_b200.runtime.cuda import ScratchPool
+    w, b, S = decoder_state(chunk, views, prompt, layers)
     with wrappers.use_pool(ScratchPool()):
         pipeline.transformer_decoder(op_table(True), w, b, S, steps=steps, layers=layers)
     return digest(b["diffusion_noise"], b["diffusion_noise_f32"], b["encoder_K"], b["encoder_V"])
@@ -106,6 +112,35 @@ DECODES = [(50, 3, 0), (10, 1, 17), (63, 3, 48)]
 @pytest.mark.parametrize("chunk,views,prompt", DECODES)
 def test_ten_euler_steps_keep_their_bits(chunk, views, prompt):
     assert decode(chunk, views, prompt) == json.loads(GOLDEN.read_text())[f"decode {chunk} {views} {prompt}"]
+
+
+# the loop in native code, the ops one by one, the same with an op replaced, and buffers that the native loop does not take
+@pytest.mark.parametrize("first_step", [0, 1])
+@pytest.mark.parametrize("chunk", [50, 64])
+def test_the_native_loop_gives_the_bits_of_its_ops(chunk, first_step):
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0 import pipeline
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import wrappers
+    from flash_vla_b200.runtime.cuda import ScratchPool
+    native, by_op, replaced, calls = op_table(True), op_table(True), op_table(True), []
+    del by_op.decoder_steps
+    replaced.decoder_attention = lambda *args: (calls.append(1), by_op.decoder_attention(*args))
+    results = []
+    for table, longer_rope in ((native, False), (by_op, False), (replaced, False), (native, True)):
+        w, b, S = decoder_state(chunk)
+        if longer_rope:
+            b["decoder_rope_weights"] = torch.cat([b["decoder_rope_weights"]] * 2)
+        with wrappers.use_pool(ScratchPool()):
+            if first_step:
+                pipeline.decoder_prologue(table, w, b)
+                pipeline.decoder_step(table, w, b, S, 0, 3, noise=b["diffusion_noise_f32"])
+            pipeline.transformer_decoder(table, w, b, S, steps=4, layers=3, first_step=first_step)
+        results.append({n: b[n].clone() for n in ("diffusion_noise", "diffusion_noise_f32", "encoder_K", "encoder_V", "decoder_x",
+                                                  "decoder_x_bf16", "decoder_norm_factor_buf")})
+    assert len(calls) == 4 * 3
+    for other in results[1:]:
+        for name, t in results[0].items():
+            assert torch.equal(t, other[name]), name
 
 
 if __name__ == "__main__":

@@ -340,3 +340,29 @@ def test_pinned_plan_table_validates_on_the_host():
 def test_decoder_groups(episodes, rows, want):
     from flash_vla_b200.hardware.nvidia.b200.pi0.engine import decoder_groups
     assert decoder_groups(episodes, rows) == want
+
+
+def test_a_replaced_decoder_op_is_served():
+    """A table is a lookup per call site: an op that a program put in place of the backend's is called by the whole loop, not
+    bypassed by the stage that stands for the backend's own ops."""
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0 import pipeline
+    from oracle import pi0_ref as O
+
+    table, calls = op_table(True), []
+    for name in [n for n in vars(table) if n.startswith("decoder_") and n != "decoder_steps"]:
+        setattr(table, name, lambda *a, _n=name: calls.append(_n))
+    table.copy_rows = lambda dst, src: dst.copy_(src.view_as(dst))
+    shapes = {"decoder_attn_qkv_w": (2, 1024, 2560), "decoder_attn_o_w": (2, 2048, 1024), "decoder_ffn_gate_w": (2, 1024, 4096),
+              "decoder_ffn_up_w": (2, 1024, 4096), "decoder_ffn_down_w": (2, 4096, 1024), "decoder_action_fused_time_biases": (10, 1024)}
+    w = {n: torch.empty(1).expand(shapes.get(n, (1,))) for n in weight_names("decoder_")}
+    b, S = O.allocate_buffers(1, 7, 0)
+    b["diffusion_noise_f32"] = torch.zeros(7, 32)
+    pipeline.transformer_decoder(table, w, b, S, steps=3, layers=2)
+    assert calls.count("decoder_attention") == 6 and calls.count("decoder_norm_qkv_rope") == 6
+    assert calls.count("decoder_state_proj") == 1 and calls.count("decoder_action_out_proj") == 3
+
+
+def weight_names(prefix):
+    from flash_vla_b200.models.pi0.spec import weight_shapes
+    return [n for n in weight_shapes(0) if n.startswith(prefix)]
