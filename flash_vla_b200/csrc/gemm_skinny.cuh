@@ -175,8 +175,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     if (lane == 0 && warp < KB) {
         const int kb = warp;
         mbar_init(bars + kb * 8, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (TOK > 64) mbar_init(free_bars + kb * 8, 1 + (p.need_factor ? SSQ_WARPS : 0));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");      // both are signalled by the async proxy
         if (kb < NS) request_w(kb, kb);
     }
     __syncwarp();
