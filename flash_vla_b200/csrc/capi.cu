@@ -168,6 +168,7 @@ static bool geglu_on_pairs(int M, int N, int K) {
 }
 
 static int launch_gemm(const GemmArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
+    FVLA_REQUIRE(a.M > 0 && a.N > 0 && a.K > 0, "gemm: empty shape %dx%dx%d", a.M, a.N, a.K);      // the planners divide by tile counts
     PlanChoice pinned;
     if (tc5_enabled() && tc5::tc5_supports(a) &&
         plan_lookup(a.M, a.N, a.K, a.B2 != nullptr ? PLAN_DUAL : (a.rope != nullptr ? PLAN_ROPE : PLAN_PLAIN), &pinned)) {
@@ -498,6 +499,7 @@ static int refresh_shadow(const void* src, void* dst, size_t count, cudaStream_t
 
 int fvla_linear_residual(const void* x, const void* weight, void* out, int out_is_f32, void* out_shadow, int M,
                          int N, int K, int group_rows, void* ws, size_t ws_bytes, void* stream) {
+    FVLA_REQUIRE(M > 0 && N > 0 && K > 0, "linear_residual: empty shape %dx%dx%d", M, N, K);
     FVLA_REQUIRE(group_rows >= 0 && (group_rows == 0 || M % group_rows == 0), "linear_residual: M=%d is not a whole number of groups of %d rows", M, group_rows);
     // Rows as several groups (a batch of episodes): the decoder's cluster GEMM once per group in one launch, each group
     // streaming the weights from L2 after the first has pulled them from HBM. Up to 128 rows are one group whatever
@@ -620,6 +622,7 @@ int fvla_decoder_norm_qkv_rope(const void* x, int x_is_f32, const void* x_shadow
                                void* K, void* V, void* norm_factor, int M, int Kdim, int heads, int head_dim,
                                int group_rows, int kv_group_pitch, void* ws, size_t ws_bytes, void* stream) {
     const int N = (heads + 2) * head_dim;
+    FVLA_REQUIRE(M > 0 && heads > 0 && head_dim > 0 && Kdim > 0, "decoder_norm_qkv_rope: empty shape %dx%dx%d", M, N, Kdim);
     FVLA_REQUIRE(group_rows >= 0 && (group_rows == 0 || (M % group_rows == 0 && kv_group_pitch >= group_rows)),
                  "decoder_norm_qkv_rope: M=%d is not a whole number of sequences of %d rows (K/V pitch %d rows)", M, group_rows, kv_group_pitch);
     if (tc5_enabled() && skinny::skinny_supports(M, N, Kdim, false, !x_is_f32 || x_shadow != nullptr) && aligned16(x) && aligned16(weight_qkv) &&
@@ -694,6 +697,7 @@ int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* ou
 
 int fvla_decoder_norm_gated_ffn(const void* x, int x_is_f32, const void* x_shadow, const void* gate_w, const void* up_w, void* out,
                                 void* norm_factor, int M, int N, int K, void* ws, size_t ws_bytes, void* stream) {
+    FVLA_REQUIRE(M > 0 && N > 0 && K > 0, "decoder_norm_gated_ffn: empty shape %dx%dx%d", M, N, K);
     if (tc5_enabled() && skinny::skinny_supports(M, N, K, true, !x_is_f32 || x_shadow != nullptr) && aligned16(x) && aligned16(gate_w) && aligned16(up_w)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.x_shadow = B(x_shadow); sa.ldx = K; sa.M = M; sa.N = N; sa.K = K; sa.need_factor = 1;

@@ -1054,7 +1054,7 @@ inline int launch_gemm_tc5(GemmArgs g, int* status, cudaStream_t st, void* ws = 
 // normalises A with a kernel of its own and calls the plain GEMM.
 // Tile width at which the fused-norm GEMM takes an M x N x K problem (0: it does not): every CTA gets one tile.
 inline int normed_tile_width(int M, int N, int K, bool rope) {
-    if (M <= 64 || N % 8 != 0 || K % BK != 0) return 0;
+    if (M <= 64 || N <= 0 || N % 8 != 0 || K <= 0 || K % BK != 0) return 0;
     const int tiles_m = (M + BM - 1) / BM, sms = num_sms();
     if (rope) {                                // the narrowest tile of which every CTA gets one at most: up to 384, 896, 1 280 and 1 792 rows at N = 2560
         for (int bn = 64; bn <= 256; bn += 64)

@@ -366,3 +366,29 @@ def test_a_replaced_decoder_op_is_served():
 def weight_names(prefix):
     from flash_vla_b200.models.pi0.spec import weight_shapes
     return [n for n in weight_shapes(0) if n.startswith(prefix)]
+
+
+EMPTY_SHAPES = """
+import itertools, sys
+from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
+lib, P, W = _lib.load(), 1 << 20, 1 << 28
+for M, N, K in itertools.product((-1, 0, 51, 65, 768), (0, 1024, 2560), (0, 1024)):
+    if min(M, N, K) > 0:
+        continue
+    for group in (0, 51):
+        assert lib.fvla_linear_residual(P, P, P, 0, None, M, N, K, group, P, W, None) < 0
+    assert lib.fvla_decoder_norm_gated_ffn(P, 0, None, P, P, P, None, M, N, K, P, W, None) < 0
+    assert lib.fvla_decoder_small_proj(P, 0, P, P, P, 0, None, M, N, K, 0, P, W, None) < 0
+    assert lib.fvla_encoder_norm_gated_ffn(P, P, P, P, P, M, N, K, None) < 0
+    assert lib.fvla_vision_linear_bias_residual(P, P, P, P, P, M, N, K, P, W, None) < 0
+    assert min(M, K) > 0 or lib.fvla_decoder_norm_qkv_rope(P, 0, None, P, P, P, P, P, None, M, K, 8, 256, 0, 0, P, W, None) < 0
+    assert lib.fvla_fused_norm_supported(M, N, K, 0) == 0 and lib.fvla_fused_norm_supported(M, N, K, 1) == 0
+"""
+
+
+def test_empty_shapes_are_errors_at_the_c_entries():
+    """No division by a tile count of zero: every entry returns a status. (In a process of its own: what this guards against ends it.)"""
+    import subprocess
+    import sys
+    proc = subprocess.run([sys.executable, "-c", EMPTY_SHAPES], cwd=ROOT, capture_output=True, text=True)
+    assert proc.returncode == 0, proc.stderr[-500:]
