@@ -664,17 +664,22 @@ int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* ou
     d.mask_rows = heads; d.mask_key_le = encoder_seq_len; d.prefix_keys = encoder_seq_len;
     d.episodes = episodes; d.q_episode_stride = q_episode_stride; d.kv_episode_stride = kv_episode_stride;
     d.status = device_status_ptr();
-    const bool aligned = aligned16(Q) && aligned16(K) && aligned16(V) && aligned16(out);
-    const bool resident = tc5_enabled() && aligned && plan_decoder_attention(d);
-    if (episodes > 1 && batched_tc5 && tc5_enabled() && aligned && !resident)
+    const bool cluster = tc5_enabled() && aligned16(Q) && aligned16(K) && aligned16(V);
+    const bool resident = cluster && plan_decoder_attention(d);
+    if (episodes > 1 && batched_tc5 && cluster && aligned16(out) && !resident)
         return attn5::launch_attention_tc5(Q, K, V, out, queries, keys, kLog2e / sqrtf((float)head_dim), device_status_ptr(), S(stream),
                                            episodes, q_episode_stride, kv_episode_stride, heads, encoder_seq_len);
     FVLA_REQUIRE(episodes == 1 || d.splits > 0, "decoder_attention: %d keys do not fit the cluster kernel", keys);
-    if (ws == nullptr || ws_bytes < fvla_decoder_attention_workspace_bytes(queries, keys)) {
+    const bool batch = episodes > 1 && batched_tc5;          // neither of a batch's kernels takes scratch
+    if (!batch && (ws == nullptr || ws_bytes < fvla_decoder_attention_workspace_bytes(queries, keys))) {
         set_error("decoder_attention: workspace of %zu bytes needed", fvla_decoder_attention_workspace_bytes(queries, keys));
         return FVLA_ERR_WORKSPACE;
     }
-    if (tc5_enabled() && aligned && d.splits > 0) {
+    if (cluster && encoder_seq_len <= 0 && keys <= decattn::MAX_SPL * 128) {
+        set_error("decoder attention: no prefix keys");      // the cluster kernel's tensor maps end at the prefix
+        return FVLA_ERR_UNSUPPORTED;
+    }
+    if (cluster && d.splits > 0) {
         FVLA_DBG_ATTACH(d);
         return launch_decoder_attention_cluster(d, pdl_enabled(), S(stream));
     }

@@ -129,3 +129,17 @@ def test_prefix_gated_ffn_by_row_count(S):
     O.op_table(False).encoder_norm_gated_ffn(x.float(), wg.float(), wu.float(), ref, norm)
     op_table(True).encoder_norm_gated_ffn(x.cuda(), wg.cuda(), wu.cuda(), got, norm.bfloat16().cuda())
     assert_close(got, ref, rtol=2e-2, atol_rms=4e-2, what="encoder_norm_gated_ffn")
+
+
+# a batch of episodes takes no scratch, whichever kernel serves it
+@pytest.mark.parametrize("episodes", [2, 5])
+def test_batched_decoder_attention_without_scratch(episodes):
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
+    g, tokens, S = torch.Generator().manual_seed(episodes), 51, 768
+    q, k, v = (rnd(g, episodes, n, 256).cuda() for n in (tokens * 8, S + tokens, S + tokens))
+    want, got = q.view(-1, 256).clone(), torch.zeros_like(q)
+    op_table(True).decoder_attention(want, k, v, None, want, S)
+    _lib.call("fvla_decoder_attention", q.data_ptr(), k.data_ptr(), v.data_ptr(), got.data_ptr(), tokens * 8, S + tokens, 256, 8, S, episodes,
+              tokens * 8 * 256, (S + tokens) * 256, None, 0, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(got.view(-1, 256), want)

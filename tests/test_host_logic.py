@@ -392,3 +392,12 @@ def test_empty_shapes_are_errors_at_the_c_entries():
     import sys
     proc = subprocess.run([sys.executable, "-c", EMPTY_SHAPES], cwd=ROOT, capture_output=True, text=True)
     assert proc.returncode == 0, proc.stderr[-500:]
+
+
+def test_decoder_attention_without_prefix_keys_is_refused():
+    """The cluster kernel's tensor maps end at the prefix; one episode, and a batch that cannot take the other kernel, have none then."""
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
+    lib, P = _lib.load(), 1 << 20
+    for seq in (0, -1):
+        assert lib.fvla_decoder_attention(P, P, P, P, 408, 51, 256, 8, seq, 1, 0, 0, P, 1 << 28, None) == -4
+        assert b"no prefix keys" in lib.fvla_last_error()
