@@ -411,6 +411,12 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     const int new_here = max(0, min(KT == 1 ? p.kp - prefix_here : p.nd, p.nk - pre_rows - new0));
     const int owned = (int)rank < units ? 1 + ((int)rank + SPL < units ? 1 : 0) : 0;            // units rank, rank + SPL
 
+    auto request_prefix = [&]() {
+#pragma unroll
+        for (int cb = 0; cb < HD / 64; ++cb) tc5::tma_load_3d(sK + cb * p.pad * 128, &tmK, pre_bar, cb * 64, key0, blockIdx.z);
+#pragma unroll
+        for (int cb = 0; cb < HD / 64; ++cb) tc5::tma_load_3d(sV + cb * p.pad * 128, &tmV, pre_bar, cb * 64, key0, blockIdx.z);
+    };
     if (tid == 0) {
         tc5::mbar_init(pre_bar, 1);
         tc5::mbar_init(in_bar, 1);
@@ -421,12 +427,14 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         if (owned > 0) tc5::mbar_expect_tx(in_bar, (uint32_t)(owned * SPL) * (UNIT_BYTES + UNIT * 4));
         // The prefix rows of K and V arrive as one box of 64 dims x pad rows per block, through maps that END at the prefix:
         // the rows behind it, which the preceding kernel may still be writing, are not touched in memory and read as
-        // zero. (Rows past prefix_here hold the next CTA's keys; the own keys overwrite some, the rest is masked.)
+        // zero. A batch, whose prefix rows the
+        // preceding kernel may have written, only has them brought to L2 here and asks for them behind the dependency wait. (Rows past prefix_here hold the next CTA's keys; the own keys overwrite some, the rest is masked.)
         tc5::mbar_expect_tx(pre_bar, 2u * p.pad * 512u);
+        if (p.episodes <= 1) request_prefix();
+        else {
 #pragma unroll
-        for (int cb = 0; cb < HD / 64; ++cb) tc5::tma_load_3d(sK + cb * p.pad * 128, &tmK, pre_bar, cb * 64, key0, blockIdx.z);
-#pragma unroll
-        for (int cb = 0; cb < HD / 64; ++cb) tc5::tma_load_3d(sV + cb * p.pad * 128, &tmV, pre_bar, cb * 64, key0, blockIdx.z);
+            for (int cb = 0; cb < HD / 64; ++cb) { tc5::tma_prefetch_3d(&tmK, cb * 64, key0, blockIdx.z); tc5::tma_prefetch_3d(&tmV, cb * 64, key0, blockIdx.z); }
+        }
     }
     if (warp == 1) {
         tc5::tmem_alloc(misc + 32, TMEM_COLS);
@@ -438,6 +446,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     const uint32_t tmem = *tmem_slot;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid == 0 && p.episodes > 1) request_prefix();
     FVLA_STAMP(1);
     // What the preceding kernel wrote, Q and the own keys, comes through registers: plain 16-byte loads reach them sooner than
     // any bulk copy reaches shared memory. Both land in the swizzled operand layout (piece c of row r at c ^ (r & 7)).

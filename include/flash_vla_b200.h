@@ -200,7 +200,7 @@ int fvla_decoder_norm_qkv_rope(const void* x, int x_is_f32, const void* x_shadow
  * per episode, episode e reads Q + e * q_episode_stride and K / V + e * kv_episode_stride (strides in
  * elements, multiples of 8) and writes out + e * q_episode_stride. A batch whose clusters are all resident at
  * once runs on the same kernel as one episode, a larger one on the tcgen05 flash kernel (one grid row per
- * episode), which waits for its predecessor before any read. */
+ * episode). Either waits for its predecessor before any read of a batch, and takes no scratch (ws may be NULL). */
 int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* out, int queries,
                            int keys, int head_dim, int heads, int encoder_seq_len, int episodes,
                            long long q_episode_stride, long long kv_episode_stride, void* ws,

@@ -143,3 +143,23 @@ def test_batched_decoder_attention_without_scratch(episodes):
     _lib.call("fvla_decoder_attention", q.data_ptr(), k.data_ptr(), v.data_ptr(), got.data_ptr(), tokens * 8, S + tokens, 256, 8, S, episodes,
               tokens * 8 * 256, (S + tokens) * 256, None, 0, torch.cuda.current_stream().cuda_stream)
     assert torch.equal(got.view(-1, 256), want)
+
+
+# a batch reads nothing that the kernel before it in the stream writes, the prefix rows among it, before that kernel has ended
+@pytest.mark.parametrize("episodes", [2, 5])
+def test_batched_decoder_attention_behind_the_kernel_that_writes_its_prefix(episodes):
+    from flash_vla_b200 import op_table
+    g, ops, tokens, S = torch.Generator().manual_seed(episodes), op_table(True), 51, 256
+    x, w, rope = rnd(g, episodes * S, 2048).cuda(), rnd(g, 2048, 2560, scale=0.02).cuda(), O.rope_table(S, 0).to(bf16).cuda()
+    q, scratch = rnd(g, episodes * tokens * 8, 256).cuda(), torch.zeros(episodes * S * 8, 256, dtype=bf16, device="cuda")
+    norm, caches = torch.zeros(episodes * S, 2048, dtype=bf16, device="cuda"), [rnd(g, episodes, S + tokens, 256).cuda() for _ in range(2)]
+    results = [torch.zeros_like(q), torch.zeros_like(q)]
+    for wait, out in zip((True, False), results):
+        for cache in caches:
+            cache[:, :S] = 0
+        torch.cuda.synchronize()
+        ops.encoder_norm_qkv_rope(x, w, rope, scratch, caches[0][:, :S], caches[1][:, :S], norm)
+        if wait:
+            torch.cuda.synchronize()
+        ops.decoder_attention(q, *caches, None, out, S)
+    assert torch.equal(*results)
