@@ -517,16 +517,20 @@ int fvla_linear_residual(const void* x, const void* weight, void* out, int out_i
         }
         return 0;
     };
-    int rows = group_rows > 0 && M > 128 ? group_rows : M, groups = M / rows, parts = 1;
+    // Pinned plans: one for the group leaves the group as it is, one of the general kernels for groups of more than 64 rows is theirs.
+    PlanChoice pinned;
+    const bool keep = group_rows > 0 && plan_lookup(group_rows, N, K, PLAN_SKINNY, &pinned);
+    const bool general = (group_rows > 0 ? group_rows : M) > 64 && plan_lookup(M, N, K, PLAN_PLAIN, &pinned);
+    int rows = group_rows > 0 && (M > 128 || keep) ? group_rows : M, groups = M / rows, parts = 1;
     if (groups > 1) {
         parts = parts_for(rows, groups);
         int wide = (M + 127) / 128;                      // the fewest equal groups of at most 128 rows
         while (wide < groups && M % wide) ++wide;
-        const int wide_parts = wide < groups ? parts_for(M / wide, wide) : 0;
+        const int wide_parts = wide < groups && !keep ? parts_for(M / wide, wide) : 0;
         if (wide_parts > 0 && (parts == 0 || wide_parts < parts)) { rows = M / wide; groups = wide; parts = wide_parts; }
         if (parts == 0) parts = 1;
     }
-    if (tc5_enabled() && skinny::skinny_supports(rows, N, K / parts, false, true) && aligned16(x) && aligned16(weight)) {
+    if (tc5_enabled() && !general && skinny::skinny_supports(rows, N, K / parts, false, true, -1) && aligned16(x) && aligned16(weight)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = 0; sa.ldx = K; sa.M = rows; sa.N = N; sa.K = K / parts; sa.groups = groups;
         sa.out = out; sa.out_f32 = out_is_f32; sa.ldo = N; sa.out_shadow = Bm(out_shadow);
@@ -581,7 +585,7 @@ int fvla_decoder_small_proj(const void* x, int x_is_f32, const void* weight, con
         if (e != cudaSuccess) { set_error("small_k_proj_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
         return check_launch("small_k_proj_kernel");
     }
-    if (tc5_enabled() && skinny::skinny_supports(M, N, K, false, !x_is_f32) && aligned16(x) && aligned16(weight)) {
+    if (tc5_enabled() && skinny::skinny_supports(M, N, K, false, !x_is_f32, PLAN_PLAIN) && aligned16(x) && aligned16(weight)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.ldx = K; sa.M = M; sa.N = N; sa.K = K;
         sa.out = out; sa.out_f32 = out_is_f32; sa.ldo = N; sa.bias = B(bias); sa.act = act;
@@ -625,7 +629,7 @@ int fvla_decoder_norm_qkv_rope(const void* x, int x_is_f32, const void* x_shadow
     FVLA_REQUIRE(M > 0 && heads > 0 && head_dim > 0 && Kdim > 0, "decoder_norm_qkv_rope: empty shape %dx%dx%d", M, N, Kdim);
     FVLA_REQUIRE(group_rows >= 0 && (group_rows == 0 || (M % group_rows == 0 && kv_group_pitch >= group_rows)),
                  "decoder_norm_qkv_rope: M=%d is not a whole number of sequences of %d rows (K/V pitch %d rows)", M, group_rows, kv_group_pitch);
-    if (tc5_enabled() && skinny::skinny_supports(M, N, Kdim, false, !x_is_f32 || x_shadow != nullptr) && aligned16(x) && aligned16(weight_qkv) &&
+    if (tc5_enabled() && skinny::skinny_supports(M, N, Kdim, false, !x_is_f32 || x_shadow != nullptr, PLAN_ROPE) && aligned16(x) && aligned16(weight_qkv) &&
         head_dim % 2 == 0) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.x_shadow = B(x_shadow); sa.ldx = Kdim; sa.M = M; sa.N = N; sa.K = Kdim; sa.need_factor = 1;
@@ -703,7 +707,7 @@ int fvla_decoder_attention(const void* Q, const void* K, const void* V, void* ou
 int fvla_decoder_norm_gated_ffn(const void* x, int x_is_f32, const void* x_shadow, const void* gate_w, const void* up_w, void* out,
                                 void* norm_factor, int M, int N, int K, void* ws, size_t ws_bytes, void* stream) {
     FVLA_REQUIRE(M > 0 && N > 0 && K > 0, "decoder_norm_gated_ffn: empty shape %dx%dx%d", M, N, K);
-    if (tc5_enabled() && skinny::skinny_supports(M, N, K, true, !x_is_f32 || x_shadow != nullptr) && aligned16(x) && aligned16(gate_w) && aligned16(up_w)) {
+    if (tc5_enabled() && skinny::skinny_supports(M, N, K, true, !x_is_f32 || x_shadow != nullptr, PLAN_DUAL) && aligned16(x) && aligned16(gate_w) && aligned16(up_w)) {
         skinny::SkinnyArgs sa{};
         sa.x = x; sa.x_f32 = x_is_f32; sa.x_shadow = B(x_shadow); sa.ldx = K; sa.M = M; sa.N = N; sa.K = K; sa.need_factor = 1;
         sa.out = out; sa.out_f32 = 0; sa.ldo = N; sa.factor_out = Bm(norm_factor); sa.status = device_status_ptr(); FVLA_DBG_ATTACH(sa);

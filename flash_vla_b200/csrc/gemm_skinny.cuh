@@ -541,9 +541,11 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, int groups = 1) {
 
 // Whether the kernel takes a shape. More than 64 rows need the operand as bf16 rows (the activation itself or its shadow):
 // the in-kernel conversion of fp32 rows exists for 64 token slots only.
-inline bool skinny_supports(int M, int N, int K, bool geglu, bool bf16_operand) {
+// A shape of more than 64 rows with a plan of the general kernels (`general_kind`) pinned for it is theirs; -1: no such plan.
+inline bool skinny_supports(int M, int N, int K, bool geglu, bool bf16_operand, int general_kind) {
     const SkinnyPlan pl = plan_skinny(M, N, K, geglu);
-    return pl.ok && (pl.tok == 64 || bf16_operand);
+    PlanChoice pinned;
+    return pl.ok && (pl.tok == 64 || (bf16_operand && !plan_lookup(M, N, K, general_kind, &pinned)));
 }
 
 template <int EPI, int TOK, int S>

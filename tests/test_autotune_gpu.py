@@ -56,3 +56,33 @@ def test_sweep_ranks_the_plans_of_a_call_site(clean_plans):
     assert set(table) == {"device", "plans", "report"} and "dec_o" in table["report"]
     for p in table["plans"]:                                           # a kept winner beats the default by the margin
         assert p["us"] < 0.97 * p["auto_us"]
+
+
+def test_pinned_plans_of_65_to_128_rows(clean_plans):
+    """Rows that the decoder's cluster GEMM takes since it has 128 slots: a plan pinned for the general kernels still is theirs (and an
+    error when it cannot be honoured), a plan pinned for one episode's rows still serves each episode of a batch."""
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib, wrappers
+    from flash_vla_b200.runtime.cuda import ScratchPool
+    autotune, ops, g = clean_plans, op_table(), torch.Generator().manual_seed(4)
+    x, w = torch.randn(102, 2048, generator=g).to(bf16).cuda(), (torch.randn(2048, 1024, generator=g) * 0.02).to(bf16).cuda()
+
+    def pin(**plan):
+        autotune.apply_plans({"plans": [{"N": 1024, "K": 2048, "bn": 128, **plan}]})
+
+    def run(a, *shape):
+        out = torch.zeros(*shape, 1024, device="cuda")
+        with wrappers.use_pool(ScratchPool()):
+            ops.decoder_out_proj_residual(a, w, out)
+        return out
+
+    want = x.float() @ w.float()
+    pin(M=102, kind="plain", engine="tc5_scratch", splits=2)            # an fp32 result cannot take the split through scratch
+    with pytest.raises(_lib.FvlaError, match="pinned plan"):
+        run(x, 102)
+    pin(M=102, kind="plain", engine="tc5_cluster", splits=2)
+    assert_close(run(x, 102), want, what="out_proj under a cluster plan of the general kernels")
+    pin(M=51, kind="skinny", engine="skinny", splits=4)                 # another split than the default's 8, so another sum
+    both, alone = run(x.view(2, 51, 2048), 2, 51), [run(x[:51], 51), run(x[51:], 51)]
+    assert torch.equal(both[0], alone[0]) and torch.equal(both[1], alone[1])
+    assert_close(both.view(102, 1024), want, what="out_proj of two episodes under a plan for one")
