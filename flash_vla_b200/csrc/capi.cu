@@ -159,12 +159,14 @@ static bool pair_enabled() {
 }
 
 // Gated FFN: 256 x 128 tiles on SM pairs or 128 x 128 tiles on single SMs. A round of pair tiles is the shorter one (0.41 against
-// 0.44 us per k step, and 7 us less at the ends), but an odd number of 128-row tiles leaves half of the last pair tile empty:
-// 273 to 384 rows are 3 rounds instead of 4, 51.5 against 55.2 us at K = 2 048, N = 16 384; 5 tiles come out even, 7 do not pay.
+// 0.44 us per k step, and 9 us less at the ends), but an odd number of 128-row tiles leaves half of the last pair tile empty. At
+// K = 2 048, N = 16 384, row norm included, pairs against single SMs: 3 row tiles (257 to 384 rows) 53.4 / 50.3 to 56.3 / 52.7 us, 3 rounds instead
+// of 4; 5 row tiles 76.1 / 76.0 to 81.6 / 83.0, which stay on pairs; 2, 4, 6 and 7 row tiles 4 to 15 us in favour of pairs. (One
+// row tile is the single-SM kernel's whatever this says: the pair kernel takes more than 128 rows.)
 static bool geglu_on_pairs(int M, int N, int K) {
     const int sms = tc5::num_sms(), tiles_n = (N + 127) / 128, k_iters = (K + 63) / 64;
     const int pair_rounds = ((M + 255) / 256 * tiles_n + sms / 2 - 1) / (sms / 2), rounds = ((M + 127) / 128 * tiles_n + sms - 1) / sms;
-    return 3.0f + pair_rounds * k_iters * 0.41f <= 10.0f + rounds * k_iters * 0.44f;
+    return 3.0f + pair_rounds * k_iters * 0.41f <= 12.0f + rounds * k_iters * 0.44f;
 }
 
 static int launch_gemm(const GemmArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {

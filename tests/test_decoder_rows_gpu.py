@@ -76,9 +76,9 @@ def test_decoder_attention_by_shape(tokens, S, episodes):
     assert _lib.load().fvla_device_status(None) == 0
 
 
-# prefix QKV with the row norm inside the GEMM by tile width (64, 128, 192, 256 columns; the last with a ragged row tile), and past
-# it, where the norm is a kernel of its own
-@pytest.mark.parametrize("S", [257, 769, 1281, 1793])
+# prefix QKV with the row norm inside the GEMM by tile width: 64 columns up to 384 rows, 128 up to 896, 192 (the only width whose last
+# column tile is ragged) up to 1 280, 256 up to 1 792, and past it, where the norm is a kernel of its own
+@pytest.mark.parametrize("S", [257, 384, 385, 769, 896, 897, 1000, 1280, 1281, 1792, 1793])
 def test_prefix_qkv_by_tile_width(S):
     from flash_vla_b200 import op_table
     g = torch.Generator().manual_seed(S)
@@ -119,8 +119,8 @@ def test_prefix_projection_by_row_count(op, S, K):
     assert_close(got, ref, what=op)
 
 
-# gated FFN on single SMs (three row tiles) and on pairs (two)
-@pytest.mark.parametrize("S", [256, 257, 384])
+# gated FFN on single SMs (one row tile, three) and on pairs (two, five), at the edges of the row tiles
+@pytest.mark.parametrize("S", [65, 128, 256, 257, 384, 513, 640])
 def test_prefix_gated_ffn_by_row_count(S):
     from flash_vla_b200 import op_table
     g = torch.Generator().manual_seed(S)
