@@ -872,8 +872,8 @@ inline float ends_us(int bn) { return bn == 64 ? 3.9f : (bn == 128 ? 4.5f : (bn 
 // (waves of work items) x (k steps per item) x (time per step) plus the two ends (between them an item's epilogue runs
 // beside the next item's k steps), plus, for a split, the cost of writing and re-reading the fp32 partials. A split
 // needs caller scratch and is only offered when `ws_ok`. (The ends used to be charged once per wave and the steps were those of
-// a slower issue loop, which kept the prefix encoder's output projection at 1 280 to 3 264 rows on 256-wide pair tiles: 33.5 us
-// against 26.9 at 1 280 rows, 37.9 against 32.8 at 3 072.)
+// a slower issue loop, which kept the prefix encoder's output projection at 1 280 to 3 264 rows on 256-wide pair tiles: 19.5 us
+// against 15.8 at 1 280 rows, 29.3 against 25.4 at 3 072; the model says 15.0 and 26.4 for the tiles it takes.)
 inline Tc5Plan plan_tc5(int M, int N, int K, bool ws_ok) {
     const int tiles_m = (M + BM - 1) / BM, sms = num_sms(), k_iters = (K + BK - 1) / BK;
     Tc5Plan best{128, 1, 0, 1e30f};
@@ -1022,7 +1022,9 @@ inline int launch_gemm_tc5(GemmArgs g, int* status, cudaStream_t st, void* ws = 
     if (g.Kb == 0) g.Kb = g.K;
     if (g.B2 != nullptr) return launch_tc5_cfg<128, true, 4>(g, status, st);
     if (g.rope != nullptr) {
-        // several tiles per CTA: 256 columns take 0.43 us per k step against 2 x 0.30 us for two tiles of 128
+        // Several tiles per CTA. Measured at K = 2 048, N = 2 560 behind the row norm, 256 / 192 / 128 columns: 1 793 to 2 304 rows 36.4 / 30.9 /
+        // 37.9 us, 3 072 rows 39.5 / 43.1 / 49.5, 6 144 rows 75.1 / 72.5 / 86.0. 256 beats 128 everywhere; 192, where its two rounds do
+        // with fewer columns, is not in the rule yet.
         if (((g.M + BM - 1) / BM) * ((g.N + 127) / 128) > num_sms()) return launch_tc5_cfg<256, false, 4, true>(g, status, st);
         return launch_tc5_cfg<128, false, 6, true>(g, status, st);
     }

@@ -38,9 +38,9 @@ MAX_GROUP_ROWS = 128       # rows that the weight-streaming decoder GEMM takes
 
 def decoder_groups(episodes: int, rows: int):
     """Episodes whose decoders run as one batch, as (first, last + 1) pairs: one or two groups that the weight-streaming
-    GEMM takes, else one group on the general kernels. Measured, ms per replay, two groups against one: 17.6 / 19.4 for
-    three episodes of 51 rows, 23.2 / 23.8 for four; more groups lose (four of 65 rows 18.4 / 15.1, eight episodes in four
-    groups 42.3 / 40.4): every group streams the weights for itself."""
+    GEMM takes, else one group on the general kernels. Measured, ms per replay of three views and ten steps: three episodes of 51
+    rows 19.2 / 17.8 / 18.7 in one, two and three groups, four 22.7 / 21.9, two of 65 rows 17.3 / 15.4; four of 65 rows 23.6 / 27.6 in
+    one and four, eight of 51 rows 37.8 / 43.1 in one and four: every group streams the weights for itself."""
     count = -(-episodes // max(1, MAX_GROUP_ROWS // rows))
     if count > 2:
         count = 1

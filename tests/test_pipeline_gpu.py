@@ -232,9 +232,9 @@ def test_concurrent_episodes_match_the_single_episode_engine(full_checkpoint, ba
     batch_prefix=False runs E complete single-episode passes on E streams, the same kernels per episode as
     the single-episode engine: results must be bit-identical to it. batch_prefix=True runs SigLIP and the
     prefix encoder once over all episodes' rows (differently shaped launches of the same kernels, so the
-    results agree to rounding, not bit for bit); batch_decoder=True also runs the action expert once over
-    all episodes' rows (M = 153 here), on the general GEMM kernels with per-episode attention inside one
-    launch. Either way every episode is checked against the oracle's result for its own inputs."""
+    results agree to rounding, not bit for bit); batch_decoder=True also runs the action expert over
+    several episodes' rows at once (here one group of 51 rows and one of 102, both on the cluster GEMM, with
+    per-episode attention inside one launch). Either way every episode is checked against the oracle's result for its own inputs."""
     from flash_vla_b200 import Pi0Inference
 
     E = 3
@@ -272,10 +272,9 @@ def test_concurrent_episodes_match_the_single_episode_engine(full_checkpoint, ba
 
 
 def test_engine_with_a_chunk_beyond_the_cluster_gemm(full_checkpoint):
-    """chunk_size 64 gives M = 65 decoder rows, one more than the cluster GEMM's 64 token slots: the
-    decoder GEMMs then run on the general kernels, which cannot refresh the bf16 shadow of the fp32
-    residual stream in their epilogue (a conversion kernel follows them instead). The engine must still
-    build and agree with the oracle (one step, two layers, as the reference's own bisection runs do)."""
+    """chunk_size 64 gives M = 65 decoder rows, one more than 64 token slots: the decoder GEMMs run on the cluster
+    GEMM's 128-slot form. The engine must build and agree with the oracle (one step, two layers, as the
+    reference's own bisection runs do)."""
     from flash_vla_b200 import Pi0Inference
     from oracle import pi0_ref as O
 
@@ -288,6 +287,50 @@ def test_engine_with_a_chunk_beyond_the_cluster_gemm(full_checkpoint):
     print(f"\n[chunk 64] one step, two layers: max-abs {err:.4g}")
     assert err <= STEP_MAX_ABS
     del engine
+    torch.cuda.empty_cache()
+
+
+def test_engine_with_a_chunk_beyond_128_slots(full_checkpoint):
+    """chunk_size 128 gives M = 129 decoder rows, one more than the cluster GEMM's 128 token slots: the decoder GEMMs
+    run on the general kernels, which cannot refresh the bf16 shadow of the fp32 residual stream in their epilogue (a conversion
+    kernel follows them instead)."""
+    from flash_vla_b200 import Pi0Inference
+    from oracle import pi0_ref as O
+
+    images, state, noise = bench_inputs(chunk_size=128)
+    engine = Pi0Inference(full_checkpoint, num_views=3, chunk_size=128, steps=1, layers=2)
+    out = engine.forward(images, state, noise).float().cpu()
+    w32 = {k: v.float() for k, v in full_checkpoint.items()}
+    ref, _ = O.forward(w32, images, state, noise, chunk_size=128, steps=1, layers=2)
+    err = (out - ref).abs().max().item()
+    print(f"\n[chunk 128] one step, two layers: max-abs {err:.4g}")
+    assert err <= STEP_MAX_ABS
+    buffers = engine.buffers
+    assert torch.equal(buffers["decoder_x_bf16"], buffers["decoder_x"].to(torch.bfloat16))
+    del engine
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("episodes", [2, 5, 8])
+def test_episodes_in_one_decoder_group(full_checkpoint, episodes):
+    """All episodes' decoder rows in one group: 102 rows on the cluster GEMM with one cluster attention for both episodes, 255 and 408
+    rows on the general QKV and gated FFN without a shadow, the flash attention and regrouped residual projections. Each
+    episode against the single-episode engine (two steps, two layers: what differs is roundings)."""
+    from flash_vla_b200 import Pi0Inference
+
+    sets = [bench_inputs(seed=e) for e in range(episodes)]
+    single = Pi0Inference(full_checkpoint, num_views=3, chunk_size=50, steps=2, layers=2)
+    want = [single.forward(*s).float().cpu() for s in sets]
+    del single
+    multi = Pi0Inference(full_checkpoint, num_views=3, chunk_size=50, steps=2, layers=2, episodes=episodes)
+    assert multi.batch_decoder and len(multi.decoder_groups) == 1
+    got = multi.forward(*[torch.stack([s[i] for s in sets]) for i in range(3)]).float().cpu()
+    for e in range(episodes):
+        err = (got[e] - want[e]).abs().max().item()
+        print(f"\n[episode {e} of {episodes}] max-abs {err:.4g}, cosine {cosine(got[e], want[e]):.6f}")
+        # each side is within one step's bound of the oracle (`STEP_MAX_ABS`), and both results are rounded to bf16
+        assert err <= 2 * STEP_MAX_ABS + 2.0 ** -8 * want[e].abs().max().item() and cosine(got[e], want[e]) >= 0.9999
+    del multi
     torch.cuda.empty_cache()
 
 
