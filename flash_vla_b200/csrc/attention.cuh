@@ -288,8 +288,8 @@ inline int launch_attention(const AttnArgs& a, dim3 grid, cudaStream_t st) {
 // that this one replaced (two groups of warps, mma.sync), and mma.sync and tcgen05.mma add up the same bits, so the results are the
 // same bits too: P is rounded to bf16 against its group's maximum, and ten Euler steps multiply any other rounding.
 // Two key tiles (KT = 2), where that keeps more clusters resident: equal parts of the prefix and of the step's own keys, four groups.
-// (With one maximum per CTA instead of per group fewer probabilities are exactly 1: 2.17e-3 from the 64-bit result at 65 tokens x 882
-// unit-variance keys, 2.08e-3 with groups of 64.)
+// (With one maximum per CTA instead of per group fewer probabilities are exactly 1: 2.176e-3 from the 64-bit result at 65 tokens x 882
+// unit-variance keys, 2.087e-3 with groups of 64, 2.080e-3 on 8 CTAs with one tile each.)
 // Measured at 51 rows x 819 keys inside the decoder's chain: 6.4 us per launch, against 7.8 us for the warp-level form
 // (mma.sync on 8 warps, halves staged in shared memory, bulk copies). What bounds it is a chain of
 // latencies: dependency wait 0.9, Q 0.7, S^T 0.6, softmax and O^T 1.8, exchange 1.1 (28 KB per CTA; distributed shared memory
@@ -771,7 +771,7 @@ inline int resident_attention_clusters(int spl) {
 // CTA more per further 128, whatever is resident, so that the results of such a decode depend on nothing but its shape (and are the
 // bits of the kernel before, see above). Else the cluster size, smallest first in every order of preference: all clusters of the
 // launch resident together, with one key tile of at most 128 rows and 4 or 8 CTAs, so that the eight owners' shares come out even; then
-// any size with one key tile; then with two (65 tokens x 882 keys: 40.5 us per layer-step with 5 CTAs, all 17 clusters resident, 44.3
+// any size with one key tile; then with two (65 tokens x 882 keys: 33.2 us per layer-step with 5 CTAs, all 17 clusters resident, 37.8
 // with 8, of which 15 are). Failing that the smallest that fits the SM at all. Returns whether all clusters are resident; 0 splits: the
 // shape does not fit.
 inline bool plan_decoder_attention(DecAttnArgs& a) {

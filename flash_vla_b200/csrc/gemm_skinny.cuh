@@ -19,8 +19,8 @@
 // and is reduced with the partials. What remains is a chain of latencies (dependency 0.9 us after the
 // last CTA of the kernel before, X tile 0.5, MMAs 0.6 to 1.5, exchange 0.5, epilogue 0.6), in which every instruction behind the
 // exchange counts, hence the cluster size and the token slots as template parameters. Per launch inside the chain at 51 rows:
-// QKV 4.3 us (5.7 with one issuer, an exchange through bulk copies and run-time sizes), attention output 3.9 (5.0),
-// gate / up 6.3 (8.2), down 4.8 (6.2); 65 rows, which the general GEMM took before, 77.7 -> 32.7 us per layer-step. (An fp32 activation without a shadow is still accepted: the CTA
+// QKV 4.3 us (5.7 with an exchange through bulk copies, run-time sizes and a lane test before the MMAs), attention output 3.9 (5.0),
+// gate / up 6.3 (8.2), down 4.6 (6.2); 65 rows, which the general GEMM took before, 77.7 -> 33 us per layer-step. (An fp32 activation without a shadow is still accepted: the CTA
 // then converts its slice in registers.) No separate norm kernel, no global-memory scratch, no
 // semaphores.
 #pragma once
