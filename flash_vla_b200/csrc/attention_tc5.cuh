@@ -182,7 +182,7 @@ attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tmQ, cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             constexpr uint32_t id_qk = idesc_qk();
             constexpr uint32_t id_pv = tc5::instr_desc(256);
             bool ok = mbar_wait(q_full, 0, abort_flag);
@@ -539,7 +539,7 @@ vision_attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tm
                     tma_load_2d(sV + kb * 16384 + a * 8192, &tmV, v_full, 2 * width + head * HDIM + a * 64, view * TOK + kb * 64);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             bool ok = mbar_wait(qk_full, 0, abort_flag) && mbar_wait(q_fixed, 0, abort_flag);
             if (ok) {
                 tc5::tc_fence_after();

@@ -154,7 +154,7 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
         if (p.trigger_early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // every thread of the CTA signals at the end of its role
     } else if (warp == 1) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t idesc = pair_idesc();
             // (running ring position and descriptors: see the one-SM kernel)
             const uint64_t adesc0 = smem_desc(smem_base, 16, 1024), bdesc0 = smem_desc(smem_base + 16384, 8192, 1024);
