@@ -133,6 +133,13 @@ static bool tc5_enabled() {
     return enabled == 1;
 }
 
+// FVLA_ATTN=mma keeps SigLIP and prefix attention on the warp-level kernels (diagnostic switch).
+static bool attention_on_tc5() {
+    static int on = -1;
+    if (on < 0) { const char* v = getenv("FVLA_ATTN"); on = (v != nullptr && strcmp(v, "mma") == 0) ? 0 : 1; }
+    return on == 1 && tc5_enabled();
+}
+
 #ifdef FVLA_DEBUG
 // Development builds only: the timestamp buffer the instrumented kernels write to. It is registered
 // through fvla_debug_set_timestamps (below), which checks that it is device memory of sufficient size;
@@ -270,9 +277,8 @@ size_t fvla_patch_embed_workspace_bytes(int views) {
     return views > 0 ? (size_t)views * 256 * 592 * sizeof(bf16) : 0;
 }
 
-int fvla_vision_patch_embed(const void* images, const void* patch_w, const void* patch_b,
-                            const void* pos_emb, void* out, int views, void* ws, size_t ws_bytes,
-                            void* stream) {
+static int patch_embed(const void* images, const void* patch_w, const void* patch_b, const void* pos_emb, void* out, float* row_sums,
+                       int views, void* ws, size_t ws_bytes, void* stream) {
     FVLA_REQUIRE(views > 0, "patch_embed: views=%d", views);
     FVLA_REQUIRE(images != nullptr && patch_w != nullptr && patch_b != nullptr && pos_emb != nullptr && out != nullptr,
                  "patch_embed: null pointer");
@@ -289,8 +295,14 @@ int fvla_vision_patch_embed(const void* images, const void* patch_w, const void*
     GemmArgs a;
     a.A = B(ws); a.lda = 592; a.B = B(patch_w); a.ldb = 1152; a.C = out; a.ldc = 1152;
     a.bias = B(patch_b); a.R = pos_emb; a.ldr = 1152; a.res_mod = 256;
-    a.M = M; a.N = 1152; a.K = 592; a.Kb = 588;
+    a.M = M; a.N = 1152; a.K = 592; a.Kb = 588; a.row_sums = row_sums;
     return launch_gemm(a, nullptr, 0, S(stream));
+}
+
+int fvla_vision_patch_embed(const void* images, const void* patch_w, const void* patch_b,
+                            const void* pos_emb, void* out, int views, void* ws, size_t ws_bytes,
+                            void* stream) {
+    return patch_embed(images, patch_w, patch_b, pos_emb, out, nullptr, views, ws, ws_bytes, stream);
 }
 
 // ---- patch embedding without caller-provided scratch -------------------------------------------
@@ -381,15 +393,31 @@ int fvla_fused_norm_supported(int M, int N, int K, int rope) {
     return tc5_enabled() && tc5::normed_tile_width(M, N, K, rope != 0) != 0 ? 1 : 0;
 }
 
+// act(LayerNorm(x) W + b) with the norm folded in; in_sums: the rows' sums, where the kernel that wrote x left them.
+static int folded_norm_linear(const void* x, const float* in_sums, const void* weight_folded, const float* colsum, const float* bias_folded,
+                              void* out, int M, int N, int K, int act, void* stream) {
+    GemmArgs a;
+    a.A = B(x); a.lda = K; a.B = B(weight_folded); a.ldb = N; a.C = out; a.ldc = N;
+    a.act = act; a.M = M; a.N = N; a.K = K; a.trigger_early = act;      // after the up projection the down GEMM follows
+    a.norm_mode = 2; a.colsum = colsum; a.bias_f32 = bias_folded; a.in_sums = in_sums;
+    return tc5_enabled() ? tc5::launch_gemm_tc5_normed(a, device_status_ptr(), S(stream)) : FVLA_ERR_UNSUPPORTED;
+}
+
+// x += a W (+ b), bf16, with the sums of the new rows.
+static int linear_with_sums(const void* in, const bf16* weight, const bf16* bias, void* x, float* row_sums, int squares, int M, int N, int K, void* ws, size_t ws_bytes, void* stream) {
+    GemmArgs a;
+    a.A = B(in); a.lda = K; a.B = weight; a.ldb = N; a.C = x; a.ldc = N; a.bias = bias;
+    a.R = x; a.ldr = N; a.M = M; a.N = N; a.K = K; a.row_sums = row_sums; a.sums_squares = squares;
+    void* gws; size_t gn;
+    gemm_ws(ws, ws_bytes, M, K, &gws, &gn);
+    return launch_gemm(a, gws, gn, S(stream));
+}
+
 int fvla_vision_folded_norm_linear(const void* x, const void* weight_folded, const float* colsum, const float* bias_folded,
                                    void* out, int M, int N, int K, int act, void* stream) {
     FVLA_REQUIRE(x && weight_folded && colsum && bias_folded && out && M > 0 && N > 0 && K > 0 && (act == 0 || act == 1),
                  "vision_folded_norm_linear: bad arguments");
-    GemmArgs a;
-    a.A = B(x); a.lda = K; a.B = B(weight_folded); a.ldb = N; a.C = out; a.ldc = N;
-    a.act = act; a.M = M; a.N = N; a.K = K; a.trigger_early = act;      // after the up projection the down GEMM follows
-    a.norm_mode = 2; a.colsum = colsum; a.bias_f32 = bias_folded;
-    const int rc = tc5_enabled() ? tc5::launch_gemm_tc5_normed(a, device_status_ptr(), S(stream)) : FVLA_ERR_UNSUPPORTED;
+    const int rc = folded_norm_linear(x, nullptr, weight_folded, colsum, bias_folded, out, M, N, K, act, stream);
     if (rc == FVLA_ERR_UNSUPPORTED)
         set_error("vision_folded_norm_linear: M=%d N=%d K=%d is outside the fused form (see fvla_fused_norm_supported)", M, N, K);
     return rc;
@@ -406,9 +434,7 @@ int fvla_vision_attention(const void* qkv, void* out, int views, int tokens, int
     if (head_dim != 72) { set_error("vision_attention: head_dim %d not built (72 only)", head_dim); return FVLA_ERR_UNSUPPORTED; }
     const int width = heads * head_dim;
     // tcgen05 kernel for the model's shape (FVLA_ATTN=mma / FVLA_GEMM=mma keep the warp-level kernel)
-    static int attn_tc5 = -1;
-    if (attn_tc5 < 0) { const char* v = getenv("FVLA_ATTN"); attn_tc5 = (v != nullptr && strcmp(v, "mma") == 0) ? 0 : 1; }
-    if (attn_tc5 && tc5_enabled() && tokens == attn5::vis::TOK && aligned16(qkv) && aligned16(out))
+    if (attention_on_tc5() && tokens == attn5::vis::TOK && aligned16(qkv) && aligned16(out))
         return attn5::vis::launch_vision_attention_tc5(qkv, out, views, heads, device_status_ptr(), S(stream));
     AttnArgs a{};
     a.q = B(qkv); a.k = B(qkv) + width; a.v = B(qkv) + 2 * width; a.out = Bm(out);
@@ -465,9 +491,7 @@ int fvla_encoder_attention(const void* Q, const void* K, const void* V, void* ou
     a.batch_inner = 1; a.nq = queries; a.nk = keys; a.hd = head_dim; a.nq_pad = queries;
     a.scale_log2 = scale * kLog2e; a.splits = 1; a.keys_per_split = keys;
     // tcgen05 kernel (FVLA_ATTN=mma keeps the warp-level kernels: diagnostic switch)
-    static int attn_tc5 = -1;
-    if (attn_tc5 < 0) { const char* v = getenv("FVLA_ATTN"); attn_tc5 = (v != nullptr && strcmp(v, "mma") == 0) ? 0 : 1; }
-    if (attn_tc5 && tc5_enabled() && aligned16(Q) && aligned16(K) && aligned16(V))
+    if (attention_on_tc5() && aligned16(Q) && aligned16(K) && aligned16(V))
         return attn5::launch_attention_tc5(Q, K, V, out, queries, keys, scale * kLog2e, device_status_ptr(), S(stream));
     const int q_tiles = (queries + 63) / 64;
     // With scratch, the keys are split in two: twice the CTAs, each with a one-tile K/V buffer so that two
@@ -787,6 +811,78 @@ int fvla_decoder_steps_run(const struct fvla_decoder_steps* d, void* stream) {
         if (!rc) rc = fvla_decoder_action_out_proj(x + W, 1, d->out_w, d->out_b, d->noise_f32, 1, nullptr, nullptr, d->chunk, ACT, W, stream);
     }
     if (!rc) rc = fvla_convert_copy(d->noise_f32, 1, d->noise, 0, nullptr, chunk_elems, stream);
+    return rc;
+}
+
+// ---- whole prefix stages, with row norms taken from sums that the kernels before left behind ----
+// Without the sums every projection behind a norm either re-reads its operand stages for them (16 KB more shared-memory traffic per
+// k step: SigLIP QKV 12.2 us at 768 rows against 10.9) or, where a CTA has several tiles and in the gated FFN, stands behind a row-norm kernel of its own
+// (4 to 13 us at 768 to 6 144 rows). The residual projections hold every value of a row in registers anyway; what they leave is
+// 8 or 4 bytes per 32 columns, which the next epilogue warps fetch while their MMAs run. Prefix pass, same kernels otherwise: one view 2.77 -> 2.57 ms,
+// three 4.35 -> 4.24, prompt 48 4.92 -> 4.81; two, four, eight episodes' forward 0.4, 0.5, 1.0 ms shorter (a batch's attention in one launch
+// among it). Error of the SigLIP QKV projection against 64 bits: 2.28e-3 with the sums, 2.35e-3 behind a row-norm kernel.
+int fvla_row_sums_supported(int M) { return tc5_enabled() && M > 64 && g_plan_count.load(std::memory_order_acquire) == 0 ? 1 : 0; }
+
+int fvla_vision_tower_run(const struct fvla_vision_tower* t, void* stream) {
+    constexpr int D = 1152, F = 4304, HEADS = 16, HD = 72, TOK = 256;
+    FVLA_REQUIRE(t != nullptr && t->views >= 1 && t->views <= (1 << 16) && t->layers >= 0, "vision_tower: bad shape");
+    const int M = t->views * TOK;
+    bool fits = fvla_row_sums_supported(M) && aligned16(t->x) && aligned16(t->qkv) && aligned16(t->attn) && aligned16(t->hidden) && aligned16(t->row_sums) &&
+                aligned16(t->ws_patch) && aligned16(t->patch_w) && aligned16(t->patch_b) && aligned16(t->pos_emb) && aligned16(t->o_w) && aligned16(t->o_b) &&
+                aligned16(t->down_w) && aligned16(t->down_b);
+    for (int l = 0; l < t->layers && fits; ++l) fits = aligned16(t->qkv_folded[l]) && aligned16(t->up_folded[l]);
+    if (!fits) { set_error("vision_tower: not with these kernels, plans or addresses"); return FVLA_ERR_UNSUPPORTED; }
+    float* sums = static_cast<float*>(t->row_sums);
+    int rc = patch_embed(t->images, t->patch_w, t->patch_b, t->pos_emb, t->x, sums, t->views, t->ws_patch, t->ws_patch_bytes, stream);
+    for (int l = 0; l < t->layers && rc == FVLA_OK; ++l) {
+        rc = folded_norm_linear(t->x, sums, t->qkv_folded[l], t->qkv_colsum[l], t->qkv_bias[l], t->qkv, M, 3 * D, D, 0, stream);
+        if (!rc) rc = fvla_vision_attention(t->qkv, t->attn, t->views, TOK, HEADS, HD, stream);
+        if (!rc) rc = linear_with_sums(t->attn, B(t->o_w) + (size_t)l * D * D, B(t->o_b) + (size_t)l * D, t->x, sums, 0, M, D, D, t->ws_o, t->ws_o_bytes, stream);
+        if (!rc) rc = folded_norm_linear(t->x, sums, t->up_folded[l], t->up_colsum[l], t->up_bias[l], t->hidden, M, F, D, 1, stream);
+        if (!rc) rc = linear_with_sums(t->hidden, B(t->down_w) + (size_t)l * F * D, B(t->down_b) + (size_t)l * D, t->x, sums, 0, M, D, F, t->ws_down, t->ws_down_bytes, stream);
+    }
+    return rc;
+}
+
+int fvla_encoder_layers_run(const struct fvla_encoder_layers* e, void* stream) {
+    constexpr int D = 2048, F = 16384, HEADS = 8, HD = 256, QKV = (HEADS + 2) * HD;
+    FVLA_REQUIRE(e != nullptr && e->sequences >= 1 && e->rows >= 1 && (long long)e->sequences * e->rows <= (1 << 24) && e->first >= 0 && e->last >= e->first &&
+                 e->last <= e->final_layer && e->layer_stride >= (long long)e->rows * HD &&
+                 (e->sequences == 1 || (e->sequence_stride >= (long long)e->rows * HD && e->sequence_stride % HD == 0)), "encoder_layers: bad shape");
+    const int M = e->sequences * e->rows;
+    const void* used[] = {e->qkv_w, e->o_w, e->gate_w, e->up_w, e->down_w, e->rope, e->x, e->x_norm, e->q, e->attn, e->hidden, e->k_cache, e->v_cache, e->row_sums};
+    bool fits = fvla_row_sums_supported(M) && e->layer_stride % 8 == 0 && (e->sequences == 1 || attention_on_tc5());
+    for (const void* p : used) fits = fits && p != nullptr && aligned16(p);
+    if (!fits) { set_error("encoder_layers: not with these kernels, plans or addresses"); return FVLA_ERR_UNSUPPORTED; }
+    float* sums = static_cast<float*>(e->row_sums);
+    const int group = e->sequences > 1 ? e->rows : 0, pitch = e->sequences > 1 ? (int)(e->sequence_stride / HD) : 0;
+    int rc = FVLA_OK;
+    for (int l = e->first; l < e->last && rc == FVLA_OK; ++l) {
+        const bf16 *k = B(e->k_cache) + l * e->layer_stride, *v = B(e->v_cache) + l * e->layer_stride;
+        if (e->sequences == 1) rc = fvla_encoder_attention(e->q, k, v, e->attn, e->rows * HEADS, e->rows, HD, 0.0625f, e->ws_attn, e->ws_attn_bytes, stream);
+        else rc = attn5::launch_attention_tc5(e->q, k, v, e->attn, e->rows * HEADS, e->rows, 0.0625f * kLog2e, device_status_ptr(), S(stream), e->sequences,
+                                              (long long)e->rows * HEADS * HD, e->sequence_stride);
+        if (!rc) rc = linear_with_sums(e->attn, B(e->o_w) + (size_t)l * D * D, nullptr, e->x, sums, 1, M, D, D, e->ws_o, e->ws_o_bytes, stream);
+        const bool final = l + 1 == e->final_layer;
+        const bf16 *gate = B(e->gate_w) + (size_t)l * D * F, *up = B(e->up_w) + (size_t)l * D * F, *qkv = B(e->qkv_w) + (size_t)(l + 1) * D * QKV;
+        bf16 *k1 = Bm(e->k_cache) + (l + 1) * e->layer_stride, *v1 = Bm(e->v_cache) + (l + 1) * e->layer_stride;
+        if (!rc && final) rc = fvla_encoder_norm_gated_ffn(e->x, gate, up, e->hidden, e->x_norm, M, F, D, stream);
+        else if (!rc) {
+            GemmArgs a;
+            a.A = B(e->x); a.lda = D; a.B = gate; a.B2 = up; a.ldb = F; a.C = e->hidden; a.ldc = F; a.M = M; a.N = F; a.K = D;
+            a.norm_mode = 1; a.in_sums = sums; a.trigger_early = 1;
+            rc = launch_gemm(a, nullptr, 0, S(stream));
+        }
+        if (!rc) rc = linear_with_sums(e->hidden, B(e->down_w) + (size_t)l * F * D, nullptr, e->x, sums, 1, M, D, F, e->ws_down, e->ws_down_bytes, stream);
+        if (!rc && final) rc = fvla_encoder_qkv_rope_fused_norm(e->x, qkv, e->rope, e->q, k1, v1, e->x_norm, M, D, HEADS, HD, group, pitch, stream);
+        else if (!rc) {
+            GemmArgs a;
+            a.A = B(e->x); a.lda = D; a.B = qkv; a.ldb = QKV; a.M = M; a.N = QKV; a.K = D;
+            a.rope = B(e->rope); a.q = Bm(e->q); a.k = k1; a.v = v1; a.heads = HEADS; a.head_dim = HD; a.round_first = 1;
+            a.group_rows = group; a.kv_group_pitch = pitch; a.norm_mode = 1; a.in_sums = sums; a.trigger_early = 1;
+            rc = tc5::launch_gemm_tc5_normed(a, device_status_ptr(), S(stream));
+        }
+    }
     return rc;
 }
 

@@ -46,6 +46,13 @@ struct GemmArgs {
     int norm_mode = 0;
     const float* colsum = nullptr;
     const float* bias_f32 = nullptr;
+    // Row sums handed from kernel to kernel: the bf16 residual forms write those of their result's rows to row_sums; with in_sums,
+    // those of A, the row norm takes them instead of adding up the operand stages, and a CTA may have several tiles. One partial sum per
+    // 32 columns, in 16-byte entries [entry][M]: sum and sum of squares of two of them (LayerNorm), or with sums_squares the
+    // sums of squares of four (RMS norm).
+    float* row_sums = nullptr;
+    const float* in_sums = nullptr;
+    int sums_squares = 0;
 };
 
 __device__ __forceinline__ int rope_row(const GemmArgs& p, int row) { return p.group_rows > 0 ? row % p.group_rows : row; }

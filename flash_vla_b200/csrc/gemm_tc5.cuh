@@ -232,6 +232,33 @@ __device__ __forceinline__ void epilogue8(const GemmArgs& p, int row, int col, f
                                                 pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
 }
 
+// Sums of 32 columns of a row, from the words that are stored (the last tile may reach past N: N % 32 == 0).
+__device__ __forceinline__ void store_row_sums(const GemmArgs& p, int row, int col0, const uint32_t (&words)[16]) {
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const float2 f = unpack_bf16x2(words[j]);
+        s1 += f.x + f.y;
+        s2 += f.x * f.x + f.y * f.y;
+    }
+    const int part = col0 >> 5;
+    if (col0 >= p.N) return;
+    if (p.sums_squares) p.row_sums[((size_t)(part >> 2) * p.M + row) * 4 + (part & 3)] = s2;
+    else *reinterpret_cast<float2*>(p.row_sums + ((size_t)(part >> 1) * p.M + row) * 4 + (part & 1) * 2) = make_float2(s1, s2);
+}
+// Entries [first, last) of a row, added up in order.
+template <bool SQUARES>
+__device__ __forceinline__ void add_row_sums(const GemmArgs& p, int row, int first, int last, float& s1, float& s2) {
+    if (row >= p.M) return;
+    const float4* src = reinterpret_cast<const float4*>(p.in_sums) + row;
+#pragma unroll 8
+    for (int i = first; i < last; ++i) {
+        const float4 v = src[(size_t)i * p.M];
+        if (SQUARES) s2 += (v.x + v.y) + (v.z + v.w);
+        else { s1 += v.x + v.z; s2 += v.y + v.w; }
+    }
+}
+
 template <int BN, bool DUAL, int STAGES>
 struct Tc5Cfg {
     static constexpr int NB = DUAL ? 2 : 1;
@@ -259,13 +286,14 @@ struct Tc5Cfg {
 // with split > 0 stage their fp32 partial tile in their own (by then idle) pipeline shared memory and push
 // it with one bulk copy into the idle pipeline memory of the split-0 CTA, which adds the partials in
 // split order and runs the epilogue. No global scratch, no semaphore; needs one work item per CTA.
-// NORM: the row norm of A is folded in (GemmArgs::norm_mode): the epilogue warps also consume every operand stage,
+// NORM: the row norm of A is folded in (GemmArgs::norm_mode). 1: the epilogue warps also consume every operand stage,
 // so a stage returns to the producer after the MMAs AND the eight epilogue warps have read it. Meant for one tile
 // per CTA; with more, a tile's statistics wait for the previous tile's epilogue (correct, but the overlap is lost).
+// 2: the kernel that wrote A left its rows' sums in GemmArgs::in_sums.
 // EP: what the staged epilogue does, as a set of EP_* bits, so that it carries no run-time choices (they cost as much as
 // the arithmetic); EP_ANY reads it from GemmArgs.
 constexpr int EP_ANY = -1, EP_BIAS = 1, EP_RES = 2, EP_GELU = 4, EP_ROPE = 8;      // EP_ROPE: with rounding first, as the prefix encoder's
-template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, bool NORM = false, int EP = EP_ANY>
+template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, int NORM = 0, int EP = EP_ANY>
 __global__ void __launch_bounds__(320, 1)
 tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                 const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmB2) {
@@ -290,7 +318,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
     if (threadIdx.x == 0) FVLA_STAMP_ANY(0);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), NORM ? 1 + Cfg::EPI_WARPS : 1); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), NORM == 1 ? 1 + Cfg::EPI_WARPS : 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(accfull_bar(a), 1); mbar_init(accempty_bar(a), Cfg::EPI_WARPS); }
         mbar_init(bars + (2 * STAGES + 4) * 8 + 16, 1);          // cluster split-K: "the leader's pipeline memory is free"
         mbar_init(bars + (2 * STAGES + 4) * 8 + 24, 1);          // cluster split-K: "the peers' partial tiles have arrived"
@@ -450,32 +478,40 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                     if (NORM) colc[BN + t] = cv;
                 }
             }
-            uint4 rco[CHUNKS][4];
-#pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) {
+            // (of the first two chunks; with more, chunk c + 1's while chunk c is finished: all of them at once spill)
+            constexpr int HELD = CHUNKS < 2 ? CHUNKS : 2;
+            uint4 rco[HELD][4];
+            auto fetch = [&](int c) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    rco[c][i] = make_uint4(0, 0, 0, 0);
+                    rco[c % HELD][i] = make_uint4(0, 0, 0, 0);
                     if (sym && c != whalf) continue;
                     const int grow = m0 + quad * 32 + sr + 8 * i, gcol = n0 + c * 32 + sp * 8;
                     if (ROPE && plain && with_rope) {
                         if (grow < p.M && gcol < rope_qd + p.head_dim)
-                            rco[c][i] = __ldg(reinterpret_cast<const uint4*>(p.rope + (size_t)rope_row(p, grow) * p.head_dim + (gcol % p.head_dim)));
+                            rco[c % HELD][i] = __ldg(reinterpret_cast<const uint4*>(p.rope + (size_t)rope_row(p, grow) * p.head_dim + (gcol % p.head_dim)));
                     } else if (plain && has_res && grow < p.M && gcol < p.N) {
                         const int rr = p.res_mod > 0 ? grow % p.res_mod : grow;
-                        rco[c][i] = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.R) + (size_t)rr * p.ldr + gcol);
+                        rco[c % HELD][i] = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.R) + (size_t)rr * p.ldr + gcol);
                     }
                 }
-            }
+            };
+            fetch(0);
+            if (CHUNKS == 2) fetch(1);
             float nrm_mean = 0.f, nrm_rstd = 1.f;
             if (NORM) {
+                float s1 = 0.f, s2 = 0.f;
+                if (NORM == 2) {                             // half of the row's entries; K is a multiple of 256 (RMS) or 128
+                    constexpr bool SQUARES = ROPE || DUAL;
+                    const int half = SQUARES ? p.K >> 8 : p.K >> 7;
+                    add_row_sums<SQUARES>(p, row, whalf * half, (whalf + 1) * half, s1, s2);
+                }
                 // This thread adds up half of its row: four of the eight 16-byte pieces of each 128-byte operand
                 // row. Sums do not depend on the order of the pieces, so the 128-byte swizzle needs no undoing;
                 // the piece index rotates with the lane so that a quarter warp touches eight different bank groups.
-                float s1 = 0.f, s2 = 0.f;
                 const int kt_beg = split * args.k_per_split, kt_end = min(args.k_iters, kt_beg + args.k_per_split);
                 bool alive = true;
-                for (int kt = kt_beg; kt < kt_end; ++kt, ++nit) {
+                for (int kt = kt_beg; NORM == 1 && kt < kt_end; ++kt, ++nit) {
                     const int s = nit % STAGES;
                     const uint32_t ph = (nit / STAGES) & 1u;
                     if (!mbar_wait(full_bar(s), ph, abort_flag)) { alive = false; break; }
@@ -628,6 +664,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
             for (int c = 0; c < CHUNKS; ++c) {
                 float a[32], u[32];
                 if (sym && c != whalf) continue;
+                if (CHUNKS > 2 && c + 1 < CHUNKS) fetch(c + 1);
                 if (from_partials) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) a[j] = 0.f;
@@ -669,7 +706,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                     if (has_res || with_rope) {
                         // residual arrives coalesced (8 rows x 64 B per request); hand each thread its own row
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(stg + (sr + 8 * i) * 80 + sp * 16) = rco[c][i];
+                        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(stg + (sr + 8 * i) * 80 + sp * 16) = rco[c % HELD][i];
                         __syncwarp();
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
@@ -694,7 +731,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                             }
                         } else {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) a[j] *= nrm_rstd;
+                            for (int j = 0; j < 32; ++j) { a[j] *= nrm_rstd; if (DUAL) u[j] *= nrm_rstd; }
                         }
                     }
                     auto finish = [&](auto act) {
@@ -736,11 +773,13 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                     } else if (act == 1) finish([](float v) { return gelu_f(v); });
                     else if (act == 2) finish([](float v) { return silu_f(v); });
                     else finish([](float v) { return v; });
+                    uint32_t words[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) words[j] = pack_bf16x2(a[2 * j], a[2 * j + 1]);
+                    if (EP != EP_ANY && (EP & EP_RES) && p.row_sums != nullptr && row < p.M) store_row_sums(p, row, col0, words);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        *reinterpret_cast<uint4*>(stg + lane * 80 + j * 16) =
-                            make_uint4(pack_bf16x2(a[8 * j], a[8 * j + 1]), pack_bf16x2(a[8 * j + 2], a[8 * j + 3]),
-                                       pack_bf16x2(a[8 * j + 4], a[8 * j + 5]), pack_bf16x2(a[8 * j + 6], a[8 * j + 7]));
+                        *reinterpret_cast<uint4*>(stg + lane * 80 + j * 16) = make_uint4(words[4 * j], words[4 * j + 1], words[4 * j + 2], words[4 * j + 3]);
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
@@ -898,7 +937,7 @@ inline Tc5Plan plan_tc5(int M, int N, int K, bool ws_ok) {
     return best;
 }
 
-template <int BN, bool DUAL, int STAGES, bool ROPE, bool CLUSTER, bool NORM, int EP>
+template <int BN, bool DUAL, int STAGES, bool ROPE, bool CLUSTER, int NORM, int EP>
 inline int launch_tc5_ep(const GemmArgs& g, int* status, cudaStream_t st, int splits, void* ws) {
     using Cfg = Tc5Cfg<BN, DUAL, STAGES>;
     auto kern = tc5_gemm_kernel<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP>;
@@ -953,7 +992,7 @@ inline int launch_tc5_ep(const GemmArgs& g, int* status, cudaStream_t st, int sp
 }
 
 // The epilogues of the model's call sites have kernels of their own, anything else takes the run-time one.
-template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, bool NORM = false>
+template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, int NORM = 0>
 inline int launch_tc5_cfg(const GemmArgs& g, int* status, cudaStream_t st, int splits = 1, void* ws = nullptr) {
     if constexpr (!DUAL && !ROPE) {
         const bool bias = g.bias != nullptr || g.bias_f32 != nullptr;
@@ -974,7 +1013,8 @@ inline int launch_tc5_cfg(const GemmArgs& g, int* status, cudaStream_t st, int s
         if (g.rope != nullptr && g.round_first && g.R == nullptr && g.bias == nullptr && g.bias_f32 == nullptr && g.act == 0)
             return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ROPE>(g, status, st, splits, ws);
     }
-    return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ANY>(g, status, st, splits, ws);
+    if constexpr (NORM == 2 && !DUAL) return FVLA_ERR_UNSUPPORTED;      // only the epilogues above
+    else return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ANY>(g, status, st, splits, ws);
 }
 
 // Shapes this path takes: at least one full 128-row tile of work and 16-byte aligned rows.
@@ -1023,7 +1063,7 @@ inline int launch_gemm_tc5_pinned(GemmArgs g, const PlanChoice& pc, int* status,
 
 inline int launch_gemm_tc5(GemmArgs g, int* status, cudaStream_t st, void* ws = nullptr, size_t ws_bytes = 0) {
     if (g.Kb == 0) g.Kb = g.K;
-    if (g.B2 != nullptr) return launch_tc5_cfg<128, true, 4>(g, status, st);
+    if (g.B2 != nullptr) return g.in_sums != nullptr ? launch_tc5_cfg<128, true, 4, false, false, 2>(g, status, st) : launch_tc5_cfg<128, true, 4>(g, status, st);
     if (g.rope != nullptr) {
         // Several tiles per CTA. Measured at K = 2 048, N = 2 560 behind the row norm, 256 / 192 / 128 columns: 1 793 to 2 304 rows 36.4 / 30.9 /
         // 37.9 us, 3 072 rows 39.5 / 43.1 / 49.5, 6 144 rows 75.1 / 72.5 / 86.0. 256 beats 128 everywhere; 192, where its two rounds do
@@ -1075,27 +1115,27 @@ inline int normed_tile_width(int M, int N, int K, bool rope) {
     return tiles_m * ((N + bn - 1) / bn) <= sms ? bn : 0;
 }
 
+template <int BN, int STAGES>
+inline int launch_tc5_normed_width(const GemmArgs& g, int* status, cudaStream_t st) {
+    if (g.in_sums != nullptr && g.K % (g.rope != nullptr ? 256 : 128)) return FVLA_ERR_UNSUPPORTED;
+    if (g.in_sums != nullptr)
+        return g.rope != nullptr ? launch_tc5_cfg<BN, false, STAGES, true, false, 2>(g, status, st) : launch_tc5_cfg<BN, false, STAGES, false, false, 2>(g, status, st);
+    return g.rope != nullptr ? launch_tc5_cfg<BN, false, STAGES, true, false, 1>(g, status, st) : launch_tc5_cfg<BN, false, STAGES, false, false, 1>(g, status, st);
+}
+
 inline int launch_gemm_tc5_normed(GemmArgs g, int* status, cudaStream_t st) {
     if (g.Kb == 0) g.Kb = g.K;
     if (!tc5_supports(g) || g.B2 != nullptr || g.c_f32 || g.norm_mode < 1 || g.norm_mode > 2 || g.K % BK != 0 ||
         (g.norm_mode == 2 && g.colsum == nullptr))
         return FVLA_ERR_UNSUPPORTED;
-    const int bn = normed_tile_width(g.M, g.N, g.K, g.rope != nullptr);
+    const int bn = g.in_sums != nullptr ? plan_tc5(g.M, g.N, g.K, false).bn : normed_tile_width(g.M, g.N, g.K, g.rope != nullptr);
     if (bn == 0) return FVLA_ERR_UNSUPPORTED;
-    if (g.rope != nullptr) {
-        if (g.R != nullptr || g.bias != nullptr || g.bias_f32 != nullptr || g.act != 0) return FVLA_ERR_UNSUPPORTED;
-        switch (bn) {
-            case 256: return launch_tc5_cfg<256, false, 4, true, false, true>(g, status, st);
-            case 192: return launch_tc5_cfg<192, false, 5, true, false, true>(g, status, st);
-            case 64: return launch_tc5_cfg<64, false, 8, true, false, true>(g, status, st);
-            default: return launch_tc5_cfg<128, false, 6, true, false, true>(g, status, st);
-        }
-    }
+    if (g.rope != nullptr && (g.R != nullptr || g.bias != nullptr || g.bias_f32 != nullptr || g.act != 0)) return FVLA_ERR_UNSUPPORTED;
     switch (bn) {
-        case 256: return launch_tc5_cfg<256, false, 4, false, false, true>(g, status, st);
-        case 192: return launch_tc5_cfg<192, false, 5, false, false, true>(g, status, st);
-        case 64: return launch_tc5_cfg<64, false, 8, false, false, true>(g, status, st);
-        default: return launch_tc5_cfg<128, false, 6, false, false, true>(g, status, st);
+        case 256: return launch_tc5_normed_width<256, 4>(g, status, st);
+        case 192: return launch_tc5_normed_width<192, 5>(g, status, st);
+        case 64: return launch_tc5_normed_width<64, 8>(g, status, st);
+        default: return launch_tc5_normed_width<128, 6>(g, status, st);
     }
 }
 

@@ -61,7 +61,8 @@ __host__ __device__ constexpr uint32_t pair_idesc() {
     return (1u << 4) | (1u << 7) | (1u << 10) | (0u << 15) | (1u << 16) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 
-template <bool DUAL>
+// NORM (gated form): RMS norm of A from the row sums that the kernel before left in GemmArgs::in_sums; A holds the raw rows.
+template <bool DUAL, bool NORM>
 __global__ void __launch_bounds__(320, 1)
 tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmG,
                    const __grid_constant__ CUtensorMap tmU) {
@@ -221,6 +222,12 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
                             rco[DUAL ? 0 : c][i] = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.R) + (size_t)grow * p.ldr + gcol);
                     }
             }
+            float rstd = 1.f;
+            if (NORM) {
+                float s1 = 0.f, s2 = 0.f;
+                add_row_sums<true>(p, m0 + quad * 32 + lane, 0, p.K >> 7, s1, s2);
+                rstd = rsqrtf(s2 / (float)p.K + 1e-6f);
+            }
             if (!mbar_wait(accfull_bar(acc), acc_ph, abort_flag)) break;
             if (tile + (int)pairs >= num_tiles) { if (p.trigger_early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }      // last accumulator complete
             tc_fence_after();
@@ -331,7 +338,7 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
                     float u[32];
                     tmem_ld32(t_row + 128 + c * 32, u);      // matching up columns
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) a[j] = gelu_f(a[j]) * u[j];
+                    for (int j = 0; j < 32; ++j) a[j] = NORM ? gelu_f(a[j] * rstd) * (u[j] * rstd) : gelu_f(a[j]) * u[j];
                 } else if (p.R) {
                     // hand each thread the residual of its own row (arrived as 8 rows x 64 B per request)
                     uint4 mine[4];
@@ -353,11 +360,13 @@ tc5x2_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA, c
                     }
                     __syncwarp();
                 }
+                uint32_t words[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) words[j] = pack_bf16x2(a[2 * j], a[2 * j + 1]);
+                if (!DUAL && p.row_sums != nullptr && m0 + quad * 32 + lane < p.M) store_row_sums(p, m0 + quad * 32 + lane, n0 + c * 32, words);
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    *reinterpret_cast<uint4*>(stg + lane * 80 + j * 16) =
-                        make_uint4(pack_bf16x2(a[8 * j], a[8 * j + 1]), pack_bf16x2(a[8 * j + 2], a[8 * j + 3]),
-                                   pack_bf16x2(a[8 * j + 4], a[8 * j + 5]), pack_bf16x2(a[8 * j + 6], a[8 * j + 7]));
+                    *reinterpret_cast<uint4*>(stg + lane * 80 + j * 16) = make_uint4(words[4 * j], words[4 * j + 1], words[4 * j + 2], words[4 * j + 3]);
                 __syncwarp();
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -415,9 +424,9 @@ inline PairPlan plan_pair_plain(int M, int N, int K, bool ws_ok) {
     return pl;
 }
 
-template <bool DUAL>
+template <bool DUAL, bool NORM = false>
 inline int launch_pair(const GemmArgs& g, int splits, void* ws, int* status, cudaStream_t st) {
-    auto kern = tc5x2_gemm_kernel<DUAL>;
+    auto kern = tc5x2_gemm_kernel<DUAL, NORM>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
@@ -486,7 +495,7 @@ inline int launch_geglu_pair(const GemmArgs& g, int* status, cudaStream_t st) {
     if (g.B2 == nullptr || g.N % 128 != 0 || g.M <= 128 || g.rope != nullptr || g.c_f32 || g.bias != nullptr || g.R != nullptr ||
         g.act != 0)
         return FVLA_ERR_UNSUPPORTED;
-    return launch_pair<true>(g, 1, nullptr, status, st);
+    return g.in_sums != nullptr ? launch_pair<true, true>(g, 1, nullptr, status, st) : launch_pair<true>(g, 1, nullptr, status, st);
 }
 
 // What the plain form of the pair kernel can take: out = act(A @ W + bias) + residual, destination and residual

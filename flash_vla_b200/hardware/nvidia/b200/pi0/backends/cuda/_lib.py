@@ -25,6 +25,23 @@ class DecoderSteps(ctypes.Structure):
                 [("norm_factor", _P)])
 
 
+class VisionTower(ctypes.Structure):
+    """`struct fvla_vision_tower` of the header."""
+    _fields_ = ([(n, _P) for n in ("images", "patch_w", "patch_b", "pos_emb", "o_w", "o_b", "down_w", "down_b", "qkv_folded", "qkv_colsum",
+                                   "qkv_bias", "up_folded", "up_colsum", "up_bias", "x", "qkv", "attn", "hidden", "row_sums",
+                                   "ws_patch", "ws_o", "ws_down")] +
+                [(n, _Z) for n in ("ws_patch_bytes", "ws_o_bytes", "ws_down_bytes")] + [(n, _I) for n in ("views", "layers")])
+
+
+class EncoderLayers(ctypes.Structure):
+    """`struct fvla_encoder_layers` of the header."""
+    _fields_ = ([(n, _P) for n in ("qkv_w", "o_w", "gate_w", "up_w", "down_w", "rope", "x", "x_norm", "q", "attn", "hidden", "k_cache",
+                                   "v_cache", "row_sums", "ws_attn", "ws_o", "ws_down")] +
+                [(n, _Z) for n in ("ws_attn_bytes", "ws_o_bytes", "ws_down_bytes")] +
+                [(n, ctypes.c_longlong) for n in ("layer_stride", "sequence_stride")] +
+                [(n, _I) for n in ("sequences", "rows", "first", "last", "final_layer")])
+
+
 # name -> argument ctypes (every function returns int except the three queries below)
 SIGNATURES: dict[str, list] = {
     "fvla_vision_patch_embed": [_P, _P, _P, _P, _P, _I, _P, _Z, _P],
@@ -47,6 +64,8 @@ SIGNATURES: dict[str, list] = {
     "fvla_decoder_norm_gated_ffn": [_P, _I, _P, _P, _P, _P, _P, _I, _I, _I, _P, _Z, _P],
     "fvla_decoder_action_out_proj": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P],
     "fvla_decoder_steps_run": [ctypes.POINTER(DecoderSteps), _P],
+    "fvla_vision_tower_run": [ctypes.POINTER(VisionTower), _P],
+    "fvla_encoder_layers_run": [ctypes.POINTER(EncoderLayers), _P],
     "fvla_embed_rows": [_P, _P, _P, _I, _I, ctypes.c_longlong, _P],
     "fvla_convert_copy": [_P, _I, _P, _I, _P, _Z, _P],
     "fvla_selftest_wait_timeout": [_P, _P, _P, _I, _I, _I, ctypes.c_uint, _P],
@@ -57,6 +76,7 @@ QUERIES: dict[str, tuple] = {
     "fvla_last_error": ([], c_char_p),
     "fvla_abi_version": ([], c_int),
     "fvla_fused_norm_supported": ([_I, _I, _I, _I], c_int),
+    "fvla_row_sums_supported": ([_I], c_int),
     "fvla_gemm_plan_count": ([], c_int),
     "fvla_launch_count": ([], ctypes.c_ulonglong),
     "fvla_device_status": ([_P], c_int),

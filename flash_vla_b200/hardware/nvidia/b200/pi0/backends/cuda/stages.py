@@ -9,6 +9,8 @@ import ctypes
 
 import torch
 
+from flash_vla_b200.models.pi0.spec import ENCODER_LAYERS, VISION_LAYERS
+
 from . import _lib, fused_wrappers
 from . import wrappers as _w
 
@@ -60,9 +62,99 @@ def decoder_steps(weights, buffers, encoder_seq_len, steps, layers, first_step=0
     return True
 
 
-# the fused table's entries that the native loop issues
-decoder_steps.stands_for = {n: fused_wrappers.FUSED_WRAPPERS.get(n, _w.ALL_WRAPPERS[n]) for n in (
-    "decoder_action_in_proj", "decoder_action_mlp", "decoder_norm_qkv_rope", "decoder_attention", "decoder_out_proj_residual",
-    "decoder_norm_gated_ffn", "decoder_ffn_down_residual", "decoder_action_out_proj", "copy_rows")}
+_VIS, _VIS_FFN, _ENC, _ENC_FFN = _w.VISION_DIM, 4304, 2048, 16384
 
-STAGES = {"decoder_steps": decoder_steps}
+
+def vision_tower(weights, buffers, num_views) -> bool:
+    """`pipeline.vision_encoder` as one call: the kernels that write the residual stream leave their rows' sums behind and the
+    projections take the LayerNorm from those, so that no launch reads the stream for its statistics alone. Returns False,
+    having done nothing, for whatever is not the plan's contiguous buffers and stacked weights, for launch plans
+    pinned by a program, and where folding a weight or a new scratch buffer would allocate while a graph is captured."""
+    b, w = buffers, weights
+    images, x = b["observation_images_normalized"], b["vision_x"]
+    stacks = {n: w[f"vision_{n}"] for n in ("attn_qkv_w", "attn_qkv_b", "attn_o_w", "attn_o_b", "ffn_up_w", "ffn_up_b", "ffn_down_w", "ffn_down_b",
+                                            "pre_attn_norm_w", "pre_attn_norm_b", "pre_ffn_norm_w", "pre_ffn_norm_b")}
+    if not all(isinstance(t, torch.Tensor) for t in (images, x, *stacks.values())) or x.ndim != 3 or stacks["attn_o_w"].ndim != 3:
+        return False
+    V, L, D, F = x.shape[0], stacks["attn_o_w"].shape[0], _VIS, _VIS_FFN
+    shapes = {"attn_qkv_w": (L, D, 3 * D), "attn_qkv_b": (L, 3 * D), "attn_o_w": (L, D, D), "attn_o_b": (L, D), "ffn_up_w": (L, D, F),
+              "ffn_up_b": (L, F), "ffn_down_w": (L, F, D), "ffn_down_b": (L, D)}
+    plain = {"images": (images, (V, 224, 224, 3)), "patch_w": (w["vision_patch_embedding_w"], (14, 14, 3, D)),
+             "patch_b": (w["vision_patch_embedding_b"], (D,)), "pos_emb": (w["vision_position_embedding"], (_w.VISION_TOKENS, D)),
+             "x": (x, (V, _w.VISION_TOKENS, D)), "qkv": (b["vision_QKV"], (V, _w.VISION_TOKENS, 3 * D)),
+             "attn": (b["vision_attn"], (V, _w.VISION_TOKENS, D)), "hidden": (b["vision_hidden"], (V, _w.VISION_TOKENS, F))}
+    M, dev, lib = V * _w.VISION_TOKENS, x.device, _lib.load()
+    if L != VISION_LAYERS or not all(_fits(t, s) for t, s in plain.values()) or not all(_fits(t, shapes.get(n, (L, D))) for n, t in stacks.items()):
+        return False
+    if not lib.fvla_row_sums_supported(M):
+        return False
+    roles = {"sums": ("vis_row_sums", (M * (D // 32) * 2,), torch.float32), "patch": ("patches", (lib.fvla_patch_embed_workspace_bytes(V),), torch.uint8),
+             "o": ("vis_o_ws", (_lib.gemm_workspace_bytes(M, D, D, 0),), torch.uint8), "down": ("vis_down_ws", (_lib.gemm_workspace_bytes(M, D, F, 0),), torch.uint8)}
+    if not all(_w.scratch_covers(role, shape, dtype, dev) for role, shape, dtype in roles.values()):
+        return False
+    folded = [[_w._folded_layernorm(stacks[f"{lin}_w"][l], stacks[f"{norm}_w"][l], stacks[f"{norm}_b"][l], stacks[f"{lin}_b"][l]) for l in range(L)]
+              for lin, norm in (("attn_qkv", "pre_attn_norm"), ("ffn_up", "pre_ffn_norm"))]
+    if any(f is None for side in folded for f in side):
+        return False
+    bufs = {n: _w.scratch(role, shape, dtype, dev) for n, (role, shape, dtype) in roles.items()}
+    arrays = [(ctypes.c_void_p * L)(*(f[i].data_ptr() for f in side)) for side in folded for i in range(3)]
+    names = ("qkv_folded", "qkv_colsum", "qkv_bias", "up_folded", "up_colsum", "up_bias")
+    args = _lib.VisionTower(
+        views=V, layers=L, o_w=stacks["attn_o_w"].data_ptr(), o_b=stacks["attn_o_b"].data_ptr(), down_w=stacks["ffn_down_w"].data_ptr(),
+        down_b=stacks["ffn_down_b"].data_ptr(), row_sums=bufs["sums"].data_ptr(), **{n: t.data_ptr() for n, (t, _) in plain.items()},
+        **{n: ctypes.addressof(a) for n, a in zip(names, arrays)},
+        **{f"ws_{n}": bufs[n].data_ptr() for n in ("patch", "o", "down")}, **{f"ws_{n}_bytes": bufs[n].numel() for n in ("patch", "o", "down")})
+    _lib.call("fvla_vision_tower_run", ctypes.byref(args), _w._stream())
+    return True
+
+
+def encoder_layers(weights, buffers, rows, sequences=1):
+    """The prefix encoder behind its first QKV projection: a function that enqueues layers [first, last) up to layer `last`'s QKV
+    projection, or None where the ops have to be called one by one (see `vision_tower`). Row norms come from sums that the
+    residual projections leave behind; a batch's attention is one launch over its sequences."""
+    b, w = buffers, weights
+    x, K, V = b["encoder_x"], b["encoder_K"], b["encoder_V"]
+    stacks = {n: w[f"encoder_{n}"] for n in ("attn_qkv_w", "attn_o_w", "ffn_gate_w", "ffn_up_w", "ffn_down_w")}
+    L, M, D, F, hd = ENCODER_LAYERS, rows * sequences, _ENC, _ENC_FFN, 256
+    if not all(isinstance(t, torch.Tensor) for t in (x, K, V, *stacks.values())) or x.ndim != 2 or K.ndim != (3 if sequences == 1 else 4):
+        return None
+    shapes = {"attn_qkv_w": (L, D, _QKV), "attn_o_w": (L, D, D), "ffn_gate_w": (L, D, F), "ffn_up_w": (L, D, F), "ffn_down_w": (L, F, D)}
+    cache = (L, K.shape[-2], hd) if sequences == 1 else (sequences, L, K.shape[-2], hd)
+    plain = {"x": (x, (M, D)), "x_norm": (b["encoder_x_norm"], (M, D)), "q": (b["encoder_Q"], (M * _w.DECODER_HEADS, hd)),
+             "attn": (b["encoder_attn"], (M, D)), "hidden": (b["encoder_hidden"], (M, F)), "rope": (b["encoder_rope_weights"], (rows, hd))}
+    if K.shape[-2] < rows or not all(_fits(t, s) for t, s in plain.values()) or not all(_fits(stacks[n], s) for n, s in shapes.items()):
+        return None
+    if not _fits(K, cache) or not _fits(V, cache) or not _lib.load().fvla_row_sums_supported(M):
+        return None
+    u8, dev = torch.uint8, x.device
+    roles = {"sums": ("enc_row_sums", (M * (D // 32),), torch.float32),
+             "attn": ("enc_attn_ws", (_lib.load().fvla_encoder_attention_workspace_bytes(rows * _w.DECODER_HEADS, rows),), u8),
+             "o": ("enc_o_ws", (_lib.gemm_workspace_bytes(M, D, D, 0),), u8), "down": ("enc_down_ws", (_lib.gemm_workspace_bytes(M, D, F, 0),), u8)}
+    if not all(_w.scratch_covers(role, shape, dtype, dev) for role, shape, dtype in roles.values()):
+        return None
+    bufs = {n: _w.scratch(role, shape, dtype, dev) for n, (role, shape, dtype) in roles.items()}
+    args = _lib.EncoderLayers(
+        sequences=sequences, rows=rows, final_layer=L - 1, layer_stride=K.shape[-2] * hd, sequence_stride=L * K.shape[-2] * hd if sequences > 1 else 0,
+        k_cache=K.data_ptr(), v_cache=V.data_ptr(), row_sums=bufs["sums"].data_ptr(), **{n: t.data_ptr() for n, (t, _) in plain.items()},
+        **{n: stacks[s].data_ptr() for n, s in (("qkv_w", "attn_qkv_w"), ("o_w", "attn_o_w"), ("gate_w", "ffn_gate_w"), ("up_w", "ffn_up_w"), ("down_w", "ffn_down_w"))},
+        **{f"ws_{n}": bufs[n].data_ptr() for n in ("attn", "o", "down")}, **{f"ws_{n}_bytes": bufs[n].numel() for n in ("attn", "o", "down")})
+
+    def run(first, last):
+        args.first, args.last = first, last
+        _lib.call("fvla_encoder_layers_run", ctypes.byref(args), _w._stream())
+    return run
+
+
+def _own(*names):
+    return {n: fused_wrappers.FUSED_WRAPPERS.get(n, _w.ALL_WRAPPERS[n]) for n in names}
+
+
+# the fused table's entries that the native loops issue
+decoder_steps.stands_for = _own("decoder_action_in_proj", "decoder_action_mlp", "decoder_norm_qkv_rope", "decoder_attention", "decoder_out_proj_residual",
+                                "decoder_norm_gated_ffn", "decoder_ffn_down_residual", "decoder_action_out_proj", "copy_rows")
+vision_tower.stands_for = _own("vision_patch_embed", "vision_norm_qkv", "vision_attention", "vision_out_proj_residual", "vision_norm_ffn_up",
+                               "vision_ffn_down_residual")
+encoder_layers.stands_for = _own("encoder_norm_qkv_rope", "encoder_attention", "encoder_out_proj_residual", "encoder_norm_gated_ffn",
+                                 "encoder_ffn_down_residual")
+
+STAGES = {"decoder_steps": decoder_steps, "vision_tower": vision_tower, "encoder_layers": encoder_layers}

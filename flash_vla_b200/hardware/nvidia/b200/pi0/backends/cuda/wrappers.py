@@ -127,6 +127,11 @@ def scratch(role: str, shape, dtype, device) -> torch.Tensor:
     return _POOL.get(role, shape, dtype, device)
 
 
+def scratch_covers(role: str, shape, dtype, device) -> bool:
+    """Whether `scratch` can serve this request: the pool has the buffer, or may still make it."""
+    return not _POOL.frozen or _POOL.has(role, shape, dtype, device)
+
+
 def _ws(role: str, nbytes: int, device):
     """(pointer, size) of a zero-initialised byte scratch, or (None, 0)."""
     if nbytes == 0:

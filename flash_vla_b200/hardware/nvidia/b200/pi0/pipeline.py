@@ -15,6 +15,13 @@ from flash_vla_b200.models.pi0.spec import (DECODER_HEADS, DIFFUSION_STEPS, ENCO
                                            VISION_LAYERS, VISION_TOKENS)
 
 
+def _stage(ops, name):
+    """The table's stage of that name, while the table still has exactly the ops that the stage stands for."""
+    stage = getattr(ops, name, None)
+    stands_for = getattr(stage, "stands_for", None)
+    return stage if stands_for and all(getattr(ops, n, None) is op for n, op in stands_for.items()) else None
+
+
 def vision_encoder(ops, weights, buffers, num_views):
     """Patch-embed the views and run the 27 SigLIP layers in place on `vision_x`. The buffers may hold the
     views of several episodes back to back (`num_views` is the count per episode): every op of the tower
@@ -23,6 +30,9 @@ def vision_encoder(ops, weights, buffers, num_views):
         raise NotImplementedError("num_views == 2 is not supported (as in the reference, pipeline.py:23)")
     w, b = weights, buffers
     x, xn = b["vision_x"], b["vision_x_norm"]
+    stage = _stage(ops, "vision_tower")
+    if stage is not None and stage(w, b, num_views):
+        return
     ops.vision_patch_embed(b["observation_images_normalized"], w["vision_patch_embedding_w"],
                            w["vision_patch_embedding_b"], w["vision_position_embedding"], x)
     for layer in range(VISION_LAYERS):
@@ -51,7 +61,14 @@ def transformer_encoder(ops, weights, buffers, encoder_seq_len, after_qkv=None):
     ops.encoder_projector(b["vision_x"], w["vision_final_norm_w"], w["vision_final_norm_b"],
                           w["encoder_multi_modal_projector_w"], w["encoder_multi_modal_projector_b"],
                           x, b["vision_x_norm"])
+    stage = _stage(ops, "encoder_layers")
+    behind = stage(w, b, S) if stage is not None else None
     for layer in range(ENCODER_LAYERS):
+        if behind is not None and layer > 0:
+            behind(layer - 1, layer)
+            if after_qkv is not None:
+                after_qkv(layer)
+            continue
         k_prefix, v_prefix = b["encoder_K"][layer, :S], b["encoder_V"][layer, :S]
         ops.encoder_norm_qkv_rope(x, w["encoder_attn_qkv_w"][layer], b["encoder_rope_weights"],
                                   b["encoder_Q"], k_prefix, v_prefix, b["encoder_x_norm"])
@@ -59,6 +76,8 @@ def transformer_encoder(ops, weights, buffers, encoder_seq_len, after_qkv=None):
             after_qkv(layer)
         if layer == ENCODER_LAYERS - 1:
             return
+        if behind is not None:
+            continue
         ops.encoder_attention(b["encoder_Q"], k_prefix, v_prefix, HEAD_DIM ** -0.5, b["encoder_attn"])
         ops.encoder_out_proj_residual(b["encoder_attn"], w["encoder_attn_o_w"][layer], x)
         ops.encoder_norm_gated_ffn(x, w["encoder_ffn_gate_w"][layer], w["encoder_ffn_up_w"][layer],
@@ -83,7 +102,14 @@ def transformer_encoder_batched(ops, weights, buffers, encoder_seq_len, num_view
         ops.encoder_projector(b["vision_x"][views], w["vision_final_norm_w"], w["vision_final_norm_b"],
                               w["encoder_multi_modal_projector_w"], w["encoder_multi_modal_projector_b"],
                               x[e * S:(e + 1) * S], b["vision_x_norm"][views])
+    stage = _stage(ops, "encoder_layers")
+    behind = stage(w, b, S, E) if stage is not None and E > 1 else None
     for layer in range(ENCODER_LAYERS):
+        if behind is not None and layer > 0:
+            behind(layer - 1, layer)
+            if after_qkv is not None:
+                after_qkv(layer)
+            continue
         k_prefix, v_prefix = b["encoder_K"][:, layer, :S], b["encoder_V"][:, layer, :S]      # (E, S, 256) views
         ops.encoder_norm_qkv_rope(x, w["encoder_attn_qkv_w"][layer], b["encoder_rope_weights"],
                                   b["encoder_Q"], k_prefix, v_prefix, b["encoder_x_norm"])
@@ -91,6 +117,8 @@ def transformer_encoder_batched(ops, weights, buffers, encoder_seq_len, num_view
             after_qkv(layer)
         if layer == ENCODER_LAYERS - 1:
             return
+        if behind is not None:
+            continue
         for e in range(E):
             rows = slice(e * S, (e + 1) * S)
             with (per_episode(e) if per_episode is not None else contextlib.nullcontext()):
@@ -219,11 +247,9 @@ def transformer_decoder(ops, weights, buffers, encoder_seq_len, steps=DIFFUSION_
     master = b.get("diffusion_noise_f32")
     if first_step == 0:
         _project_state(ops, weights, b)
-    stage = getattr(ops, "decoder_steps", None)
-    stands_for = getattr(stage, "stands_for", None)
-    if stands_for and all(getattr(ops, name, None) is op for name, op in stands_for.items()):
-        if stage(weights, b, encoder_seq_len, steps, layers, first_step):
-            return
+    stage = _stage(ops, "decoder_steps")
+    if stage is not None and stage(weights, b, encoder_seq_len, steps, layers, first_step):
+        return
     if first_step == 0 and master is not None:
         _copy(ops, master, b["diffusion_noise"])
     for step in range(first_step, steps):

@@ -40,6 +40,10 @@ class ScratchPool:
         self._slabs[key] = slab
         return slab
 
+    def has(self, role: str, shape, dtype, device) -> bool:
+        """Whether the buffer for these arguments exists."""
+        return (role, tuple(int(s) for s in shape), dtype, str(device)) in self._slabs
+
     def freeze(self) -> None:
         """Disallow new buffers from here on (call after warm-up, before capture)."""
         self._frozen = True

@@ -232,6 +232,44 @@ struct fvla_decoder_steps {
 };
 int fvla_decoder_steps_run(const struct fvla_decoder_steps* args, void* stream);
 
+/* The SigLIP tower (pipeline.py:21-45) over `views` images in ONE call: patch embedding and `layers` layers of LayerNorm + QKV,
+ * attention, output projection + residual, LayerNorm + FFN up, FFN down + residual, in place on x (views * 256, 1152). The kernels
+ * that write x leave their rows' sums and sums of squares in row_sums (views * 256 * 72 floats), from which the projections
+ * behind them take the LayerNorm, folded into weights as by fvla_fold_layernorm: arrays of `layers` pointers each. Stacked
+ * weights otherwise. FVLA_ERR_UNSUPPORTED, with nothing launched, where fvla_row_sums_supported(views * 256) is 0. */
+struct fvla_vision_tower {
+    const void *images, *patch_w, *patch_b, *pos_emb, *o_w, *o_b, *down_w, *down_b;
+    const void* const* qkv_folded;
+    const float* const* qkv_colsum;
+    const float* const* qkv_bias;
+    const void* const* up_folded;
+    const float* const* up_colsum;
+    const float* const* up_bias;
+    void *x, *qkv, *attn, *hidden, *row_sums;
+    void *ws_patch, *ws_o, *ws_down;
+    size_t ws_patch_bytes, ws_o_bytes, ws_down_bytes;
+    int views, layers;
+};
+int fvla_vision_tower_run(const struct fvla_vision_tower* args, void* stream);
+
+/* Layers [first, last) of the prefix encoder (pipeline.py:48-92) behind layer `first`'s QKV projection, up to and including layer `last`'s:
+ * attention, output projection + residual, RMS norm + gated FFN, FFN down + residual, RMS norm + QKV projection + RoPE, for
+ * `sequences` sequences of `rows` tokens laid end to end in x (sequences * rows, 2048). K / V rows of layer l and sequence s go to
+ * k_cache / v_cache + l * layer_stride + s * sequence_stride elements. row_sums: sequences * rows * 64 floats, as above. The FFN of
+ * layer final_layer - 1 and the QKV projection of layer final_layer run as fvla_encoder_norm_gated_ffn and
+ * fvla_encoder_qkv_rope_fused_norm, which leaves x_norm as they do. Same refusal as above. */
+struct fvla_encoder_layers {
+    const void *qkv_w, *o_w, *gate_w, *up_w, *down_w, *rope;
+    void *x, *x_norm, *q, *attn, *hidden, *k_cache, *v_cache, *row_sums;
+    void *ws_attn, *ws_o, *ws_down;
+    size_t ws_attn_bytes, ws_o_bytes, ws_down_bytes;
+    long long layer_stride, sequence_stride;
+    int sequences, rows, first, last, final_layer;
+};
+int fvla_encoder_layers_run(const struct fvla_encoder_layers* args, void* stream);
+/* 1 where the two calls above take that many rows: tcgen05 kernels in use, more than 64 rows, no pinned launch plans. */
+int fvla_row_sums_supported(int M);
+
 /* No counterpart in the reference, where these are torch `copy_` calls inside the pipeline (pipeline.py:103,
  * engine.py:60): dst[i] = src[i] for `count` contiguous elements, each side bf16 or fp32; dst_shadow (may be
  * NULL; fp32 dst only) also receives the value as bf16. Keeps the small copies of the decoder step inside the
