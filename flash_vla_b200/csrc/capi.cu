@@ -538,7 +538,7 @@ int fvla_linear_residual(const void* x, const void* weight, void* out, int out_i
     auto parts_for = [&](int rows, int groups) {         // launches needed, 0: no plan keeps all clusters resident
         for (int parts = 1; parts <= 8; parts *= 2) {
             if (K % parts || (K / parts) % 64) break;
-            const skinny::SkinnyPlan part = skinny::plan_skinny(rows, N, K / parts, false, groups);
+            const skinny::SkinnyPlan part = skinny::plan_skinny(rows, N, K / parts, false, true, groups);
             if (part.ok && (groups == 1 || part.tiles * part.splits * groups <= resident(part.splits))) return parts;
         }
         return 0;
@@ -932,7 +932,7 @@ int fvla_selftest_wait_timeout(const void* x, const void* weight, void* out, int
     FVLA_REQUIRE(spin_limit > 0 && spin_limit <= (1u << 16), "selftest: spin_limit must be in 1..65536");
     FVLA_REQUIRE(x != nullptr && weight != nullptr && out != nullptr && aligned16(x) && aligned16(weight) && aligned16(out),
                  "selftest: null or misaligned pointer");
-    if (!skinny::plan_skinny(M, N, K, false).ok) { set_error("selftest: shape %dx%dx%d is not a cluster-GEMM shape", M, N, K); return FVLA_ERR_UNSUPPORTED; }
+    if (!skinny::plan_skinny(M, N, K, false, true).ok) { set_error("selftest: shape %dx%dx%d is not a cluster-GEMM shape", M, N, K); return FVLA_ERR_UNSUPPORTED; }
     skinny::SkinnyArgs sa{};
     sa.x = x; sa.x_f32 = 0; sa.ldx = K; sa.M = M; sa.N = N; sa.K = K;
     sa.out = out; sa.out_f32 = 0; sa.ldo = N;

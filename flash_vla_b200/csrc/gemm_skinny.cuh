@@ -3,8 +3,8 @@
 // These GEMMs are bound by the HBM read of W (5-17 MB per call, read once, always cold), so the
 // kernel is built around getting every byte of W in flight at once:
 //   * the problem is transposed: the 128-wide slice of N is the MMA's M (TMEM lanes), the tokens
-//     are its N (TMEM columns): 64 slots, or 128 for 65 to 128 rows (a chunk of 64 actions and its state token, two
-//     episodes of 51 rows), so no tensor-core or shared-memory work is spent on padding 51 rows to 128;
+//     are its N (TMEM columns): 32, 64, 96 or 128 slots, whichever hold the rows, so no tensor-core or shared-memory work is
+//     spent on padding 51 rows to 128, and of the activations only the rows there are (in eights) are fetched;
 //   * grid = (N / 128 tiles) x (S K-splits); each CTA owns a W[KC, 128] block, asks TMA for all
 //     of it at kernel start (<= 8 boxes of 64 k x 128 n, 128B-swizzled, used in place as an
 //     MN-major operand) and issues KC/16 tcgen05.mma into one TMEM accumulator;
@@ -20,7 +20,10 @@
 // last CTA of the kernel before, X tile 0.5, MMAs 0.6 to 1.5, exchange 0.5, epilogue 0.6), in which every instruction behind the
 // exchange counts, hence the cluster size and the token slots as template parameters. Per launch inside the chain at 51 rows:
 // QKV 4.3 us (5.7 with an exchange through bulk copies, run-time sizes and a lane test before the MMAs), attention output 3.9 (5.0),
-// gate / up 6.3 (8.2), down 4.6 (6.2); 65 rows, which the general GEMM took before, 77.7 -> 33 us per layer-step. (An fp32 activation without a shadow is still accepted: the CTA
+// gate / up 6.3 (8.2), down 4.6 (6.2); 65 rows, which the general GEMM took before, 77.7 -> 33 us per layer-step. A layer-step by
+// token slots: 11 rows 24.1 us on 64 slots and 512 threads, 21.6 on 32 and 256; 32 rows 24.2 -> 22.8; 65 rows 33.3 us on 128 slots with whole
+// tiles of 128 activation rows (five k-blocks at a time), 31.1 on 96 with tiles of 72 (seven); 51 rows 25.03 -> 24.96. (256 threads on 64 slots:
+// 26.1 at 51 rows; 33 to 64 rows as two parts of 32 slots: no difference.) (An fp32 activation without a shadow is still accepted: the CTA
 // then converts its slice in registers.) No separate norm kernel, no global-memory scratch, no
 // semaphores.
 #pragma once
@@ -41,15 +44,20 @@ using tc5::smem_desc;
 
 constexpr int TN = 128;          // N columns per CTA (MMA M)
 constexpr int MAX_KB = 8;        // k-blocks of 64 per CTA
-// TOK: token slots (MMA N), 64 or 128. With 64 every k-block of a CTA has a place in shared memory. With 128 a k-block takes
-// 32 KB and the exchange 64 KB, so at most five have one and the rest reuse the first ones' when their MMAs (and the readers of
-// the sums of squares) are done.
-__host__ __device__ constexpr int slots_of(int tok, int kblocks) { return tok == 64 || kblocks < 5 ? kblocks : 5; }
+// TOK: token slots (MMA N): 32, 64, 96 or 128, of which the activation tile fills the rows there are, in eights (the MMAs read on into what
+// lies behind; those columns are nobody's). Up to 64 slots every k-block of a CTA has a place in shared memory. With more, a k-block
+// takes up to 32 KB and the exchange 48 or 64 KB, so only five to eight have one and the rest reuse the first ones' when their MMAs (and
+// the readers of the sums of squares) are done.
 constexpr int misc_bytes(int tok) { return tok * 4 + tok * 8 + (2 * MAX_KB + 2) * 8 + 32; }     // received sums, own sums, barriers, TMEM slot, flag
-constexpr size_t smem_bytes(int tok, int kblocks) {
-    return 1024 + (size_t)slots_of(tok, kblocks) * (16384 + tok * 128) + tok * 512 + misc_bytes(tok);
+constexpr size_t smem_bytes(int tok, int x_rows, int slots) {
+    return 1024 + (size_t)slots * (16384 + x_rows * 128) + tok * 512 + misc_bytes(tok);
 }
-static_assert(smem_bytes(64, MAX_KB) <= 232448 && smem_bytes(128, MAX_KB) <= 232448, "shared memory of one CTA");
+constexpr int slots_of(int tok, int x_rows, int kblocks) {
+    int n = kblocks;
+    while (n > 1 && smem_bytes(tok, x_rows, n) > 232448) --n;
+    return n;
+}
+static_assert(slots_of(64, 64, MAX_KB) == MAX_KB && slots_of(128, 128, MAX_KB) == 5 && slots_of(96, 72, MAX_KB) == 7, "shared memory of one CTA");
 
 enum Epi { EPI_QKV_ROPE = 0, EPI_RESIDUAL = 1, EPI_GEGLU = 2, EPI_BIAS = 3 };
 
@@ -60,6 +68,7 @@ struct SkinnyArgs {
     int M, N, K;
     int groups;                               // independent row groups of M rows each, laid end to end (grid.z); 0 or 1 = one
     int kblocks;                              // 64-wide k-blocks per CTA (K / 64 / splits)
+    int slots, x_rows;                        // of them in shared memory at a time; rows of an activation tile (a multiple of 8)
     int need_factor;                          // compute rsqrt(mean(x^2)+1e-6) per token
     // epilogue operands
     void* out; int out_f32; int ldo;          // RESIDUAL / BIAS / GEGLU destination
@@ -99,11 +108,11 @@ __device__ __forceinline__ void cluster_sync_all() {
 
 // Shared memory map (offsets from a 1024-byte aligned base):
 //   W      slots x 16 KB     [slot][atom(2)][64 k rows x 128 B]  (atom = 64 of the tile's 128 n)
-//   X      slots x TOK x 128 B  [slot][token][64 k]            (K-major, 128B swizzle)
+//   X      slots x rows x 128 B  [slot][token][64 k]           (K-major, 128B swizzle)
 //   RED    S x TS x 128 fp32 = TOK x 512 B   partials of the S ranks (the own one too), [src][4 tokens][n][4]
 //   SSQ    S x TS fp32       partial sums of squares received, [src][token]
 //   ssq_local TOK x 2 fp32, barriers, tmem slot, abort flag
-constexpr int THREADS = 512;
+__host__ __device__ constexpr int threads_of(int tok) { return tok == 32 ? 256 : 512; }
 
 __device__ __forceinline__ void st_async4(uint32_t dst, uint32_t bar, float a, float b, float c, float d) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
@@ -114,18 +123,19 @@ __device__ __forceinline__ void st_async1(uint32_t dst, uint32_t bar, float a) {
 }
 
 template <int EPI, int TOK, int S>          // S: cluster size along K
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(threads_of(TOK), 1)
 skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                    const __grid_constant__ CUtensorMap tmX) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-    constexpr int ISSUERS = TOK == 64 ? 1 : 2;                // MMA-issuing threads, an accumulator each
-    constexpr uint32_t XB = TOK * 128, RED_BYTES = TOK * 512, ACC_COLS = ISSUERS * TOK;
+    constexpr int THREADS = threads_of(TOK), ISSUERS = TOK <= 64 ? 1 : 2;      // MMA-issuing threads, an accumulator each
+    constexpr uint32_t RED_BYTES = TOK * 512, ACC_COLS = TOK == 96 ? 256 : ISSUERS * TOK;
     // The upper warps add up the rows' squares: the MMA issuers' warps come too late for it (gate/up: 1.6 us after the last MMA)
-    constexpr int SSQ_WARPS = 8;
+    constexpr int SSQ_WARPS = TOK == 96 ? 6 : THREADS / 64;
     constexpr int TS = TOK / S, COLS = EPI == EPI_GEGLU ? 64 : 128, ITEMS = TS / 4 * COLS, PRE = (ITEMS + THREADS - 1) / THREADS;      // owner: tokens, work items, per thread
-    const int KB = p.kblocks, NS = slots_of(TOK, KB);
+    const int KB = p.kblocks, NS = p.slots;
+    const uint32_t XB = p.x_rows * 128;
     const uint32_t w_bytes = NS * 16384u;
     const uint32_t sW = base, sX = sW + w_bytes;
     const uint32_t off_red = w_bytes + NS * XB;
@@ -387,8 +397,9 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     // shared memory and sent by bulk copies the exchange took 0.4 us longer.)
     const uint32_t red_mine = base + off_red + rank * (TS * 512u);
 #pragma unroll
-    for (int h = 0; h < TOK / 64; ++h) {
-        const int q = warp & 3, g = (warp >> 2) + h * 4;
+    for (int h = 0; h < (TOK * 8 + THREADS - 1) / THREADS; ++h) {
+        const int q = warp & 3, g = (warp >> 2) + h * (THREADS / 128);
+        if (TOK == 96 && g >= TOK / 16) break;
         float part[16];
         tc5::tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + g * 16, part);
         if (ISSUERS == 2 && KB > 1) {
@@ -490,30 +501,38 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-struct SkinnyPlan { int tok, splits, kblocks, tiles; size_t smem; bool ok; };
+struct SkinnyPlan { int tok, splits, kblocks, tiles, slots, x_rows; size_t smem; bool ok; };
 
-inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, int groups = 1) {
+inline void place_skinny(SkinnyPlan& pl, int M, bool bf16_operand) {
+    pl.x_rows = bf16_operand ? (M + 7) / 8 * 8 : pl.tok;      // (the in-kernel conversion of fp32 rows fills the whole tile)
+    pl.slots = slots_of(pl.tok, pl.x_rows, pl.kblocks);
+    pl.smem = smem_bytes(pl.tok, pl.x_rows, pl.slots);
+    pl.ok = true;
+}
+
+// bf16_operand: rows as bf16 (the activation itself or its shadow).
+inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, bool bf16_operand, int groups = 1) {
     SkinnyPlan pl{};
     pl.ok = false;
     const int tile_n = geglu ? 64 : TN;
     if (M <= 0 || M > 128 || N % tile_n || K % 64) return pl;
-    pl.tok = M <= 64 ? 64 : 128;
+    // The fewest token slots that hold the rows: measured per layer-step above. (The in-kernel conversion of fp32 rows exists for 64.)
+    pl.tok = M <= 32 && bf16_operand ? 32 : (M <= 64 ? 64 : (M <= 96 ? 96 : 128));
     pl.tiles = N / tile_n;
     const int kb_total = K / 64;
     PlanChoice pinned;
     if (plan_lookup(M, N, K, geglu ? PLAN_SKINNY_DUAL : PLAN_SKINNY, &pinned)) {
         // a pinned cluster size: 1, 2, 4 or 8 CTAs along K, at most 8 k-blocks each
         const int s = pinned.splits;
-        if (s < (pl.tok == 64 ? 1 : 2) || s > 8 || (s & (s - 1)) || kb_total % s || kb_total / s > MAX_KB || ((kb_total / s) & (kb_total / s - 1))) return pl;
+        if (s < (pl.tok <= 64 ? 1 : 2) || s > 8 || (s & (s - 1)) || kb_total % s || kb_total / s > MAX_KB || ((kb_total / s) & (kb_total / s - 1))) return pl;
         pl.splits = s;
         pl.kblocks = kb_total / s;
-        pl.smem = smem_bytes(pl.tok, pl.kblocks);
-        pl.ok = true;
+        place_skinny(pl, M, bf16_operand);
         return pl;
     }
     // largest cluster (<= 8) that divides the k-blocks, keeps <= 8 k-blocks per CTA and stays near one wave
     int best = 0;
-    for (int s = pl.tok == 64 ? 1 : 2; s <= 8; s *= 2) {       // 8 = largest portable cluster; larger ones schedule in waves
+    for (int s = pl.tok <= 64 ? 1 : 2; s <= 8; s *= 2) {       // 8 = largest portable cluster; larger ones schedule in waves
         if (kb_total % s) continue;
         const int kb = kb_total / s;
         if (kb > MAX_KB || kb < 1 || (kb & (kb - 1))) continue;
@@ -525,7 +544,7 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, int groups = 1) {
         // Several row groups in one launch multiply the CTA count. Clusters are placed GPC by GPC: about 33
         // clusters of 4 or 15 of 8 are resident at once, so prefer the largest split whose clusters of all
         // groups are resident together (one wave) over the single-group choice.
-        for (int s = best; s >= (pl.tok == 64 ? 1 : 2); s /= 2) {
+        for (int s = best; s >= (pl.tok <= 64 ? 1 : 2); s /= 2) {
             const int kb = kb_total / s;
             if (kb_total % s || kb > MAX_KB) break;
             const int resident = s >= 8 ? 15 * 8 : (s == 4 ? 33 * 4 : 148);
@@ -534,8 +553,7 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, int groups = 1) {
     }
     pl.splits = best;
     pl.kblocks = kb_total / best;
-    pl.smem = smem_bytes(pl.tok, pl.kblocks);
-    pl.ok = true;
+    place_skinny(pl, M, bf16_operand);
     return pl;
 }
 
@@ -543,20 +561,20 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, int groups = 1) {
 // the in-kernel conversion of fp32 rows exists for 64 token slots only.
 // A shape of more than 64 rows with a plan of the general kernels (`general_kind`) pinned for it is theirs; -1: no such plan.
 inline bool skinny_supports(int M, int N, int K, bool geglu, bool bf16_operand, int general_kind) {
-    const SkinnyPlan pl = plan_skinny(M, N, K, geglu);
+    const SkinnyPlan pl = plan_skinny(M, N, K, geglu, bf16_operand);
     PlanChoice pinned;
-    return pl.ok && (pl.tok == 64 || (bf16_operand && !plan_lookup(M, N, K, general_kind, &pinned)));
+    return pl.ok && (pl.tok <= 64 || (bf16_operand && !plan_lookup(M, N, K, general_kind, &pinned)));
 }
 
 template <int EPI, int TOK, int S>
 inline int launch_skinny_cfg(SkinnyArgs a, const SkinnyPlan& pl, const void* W, const void* W2, int ldw, cudaStream_t st) {
-    a.kblocks = pl.kblocks;
+    a.kblocks = pl.kblocks; a.slots = pl.slots; a.x_rows = pl.x_rows;
     const int groups = a.groups > 1 ? a.groups : 1;
     if (groups > 1 && (EPI == EPI_QKV_ROPE || a.need_factor || (a.x_f32 && a.x_shadow == nullptr))) {
         set_error("skinny gemm: row groups are only built for the bias / residual forms with a bf16 operand");
         return FVLA_ERR_UNSUPPORTED;
     }
-    if (TOK > 64 && a.x_f32 && a.x_shadow == nullptr) { set_error("skinny gemm: more than 64 rows need a bf16 operand"); return FVLA_ERR_UNSUPPORTED; }
+    if (TOK != 64 && a.x_f32 && a.x_shadow == nullptr) { set_error("skinny gemm: more than 64 rows need a bf16 operand"); return FVLA_ERR_UNSUPPORTED; }
     auto kern = skinny_gemm_kernel<EPI, TOK, S>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
@@ -572,11 +590,11 @@ inline int launch_skinny_cfg(SkinnyArgs a, const SkinnyPlan& pl, const void* W, 
     else rc = tc5::make_map(&tmW2, W2, (uint64_t)a.N, (uint64_t)a.K, (uint64_t)ldw, 64, 64);
     if (rc) return rc;
     if (a.x_f32 && a.x_shadow == nullptr) tmX = tmW;         // unused by the kernel in this case
-    else rc = tc5::make_map(&tmX, a.x_f32 ? (const void*)a.x_shadow : a.x, (uint64_t)a.K, (uint64_t)a.M * groups, (uint64_t)a.ldx, 64, TOK);
+    else rc = tc5::make_map(&tmX, a.x_f32 ? (const void*)a.x_shadow : a.x, (uint64_t)a.K, (uint64_t)a.M * groups, (uint64_t)a.ldx, 64, (uint32_t)pl.x_rows);
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.tiles, pl.splits, groups);
-    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.blockDim = dim3(threads_of(TOK), 1, 1);
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -593,21 +611,27 @@ inline int launch_skinny_cfg(SkinnyArgs a, const SkinnyPlan& pl, const void* W, 
     return check_launch("skinny_gemm_kernel");
 }
 
+template <int EPI, int TOK>
+inline int launch_skinny_tok(const SkinnyArgs& a, const SkinnyPlan& pl, const void* W, const void* W2, int ldw, cudaStream_t st) {
+    switch (pl.splits) {
+        case 1:
+            if constexpr (TOK <= 64) return launch_skinny_cfg<EPI, TOK, 1>(a, pl, W, W2, ldw, st);
+            else { set_error("skinny gemm: no cluster of one for %d rows", a.M); return FVLA_ERR_UNSUPPORTED; }
+        case 2: return launch_skinny_cfg<EPI, TOK, 2>(a, pl, W, W2, ldw, st);
+        case 4: return launch_skinny_cfg<EPI, TOK, 4>(a, pl, W, W2, ldw, st);
+        default: return launch_skinny_cfg<EPI, TOK, 8>(a, pl, W, W2, ldw, st);
+    }
+}
+
 template <int EPI>
 inline int launch_skinny(const SkinnyArgs& a, const void* W, const void* W2, int ldw, cudaStream_t st) {
-    const SkinnyPlan pl = plan_skinny(a.M, a.N, a.K, EPI == EPI_GEGLU, a.groups > 1 ? a.groups : 1);
+    const SkinnyPlan pl = plan_skinny(a.M, a.N, a.K, EPI == EPI_GEGLU, !a.x_f32 || a.x_shadow != nullptr, a.groups > 1 ? a.groups : 1);
     if (!pl.ok) { set_error("skinny gemm: shape %dx%dx%d not supported", a.M, a.N, a.K); return FVLA_ERR_UNSUPPORTED; }
-    if (pl.tok == 64)
-        switch (pl.splits) {
-            case 1: return launch_skinny_cfg<EPI, 64, 1>(a, pl, W, W2, ldw, st);
-            case 2: return launch_skinny_cfg<EPI, 64, 2>(a, pl, W, W2, ldw, st);
-            case 4: return launch_skinny_cfg<EPI, 64, 4>(a, pl, W, W2, ldw, st);
-            default: return launch_skinny_cfg<EPI, 64, 8>(a, pl, W, W2, ldw, st);
-        }
-    switch (pl.splits) {
-        case 2: return launch_skinny_cfg<EPI, 128, 2>(a, pl, W, W2, ldw, st);
-        case 4: return launch_skinny_cfg<EPI, 128, 4>(a, pl, W, W2, ldw, st);
-        default: return launch_skinny_cfg<EPI, 128, 8>(a, pl, W, W2, ldw, st);
+    switch (pl.tok) {
+        case 32: return launch_skinny_tok<EPI, 32>(a, pl, W, W2, ldw, st);
+        case 64: return launch_skinny_tok<EPI, 64>(a, pl, W, W2, ldw, st);
+        case 96: return launch_skinny_tok<EPI, 96>(a, pl, W, W2, ldw, st);
+        default: return launch_skinny_tok<EPI, 128>(a, pl, W, W2, ldw, st);
     }
 }
 

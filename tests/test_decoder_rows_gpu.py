@@ -58,6 +58,13 @@ def test_decoder_gemms_by_row_count(M, group):
     assert _lib.load().fvla_device_status(None) == 0
 
 
+# token slots: 32 up to 32 rows, 64 to 64, 96 to 96, then 128; activation tiles of 8, 16, 32, 40, 72, 80, 96 and 104 rows, seven k-blocks of the
+# largest cluster in shared memory at a time, six (96 rows) and five
+@pytest.mark.parametrize("M,group", [(1, 0), (11, 0), (32, 0), (33, 0), (72, 0), (73, 0), (96, 0), (96, 32), (97, 0)])
+def test_decoder_gemms_by_token_slots(M, group):
+    test_decoder_gemms_by_row_count(M, group)
+
+
 # one key tile of 128 per CTA and two; 4 CTAs per cluster and more; a single token; two episodes that are resident together
 @pytest.mark.parametrize("tokens,S,episodes", [(1, 40, 1), (11, 273, 1), (51, 816, 1), (65, 817, 1), (64, 1280, 1), (51, 768, 2), (5, 1024, 2)])
 def test_decoder_attention_by_shape(tokens, S, episodes):
