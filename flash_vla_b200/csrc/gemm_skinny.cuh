@@ -59,7 +59,7 @@ constexpr int slots_of(int tok, int x_rows, int kblocks) {
 }
 static_assert(slots_of(64, 64, MAX_KB) == MAX_KB && slots_of(128, 128, MAX_KB) == 5 && slots_of(96, 72, MAX_KB) == 7, "shared memory of one CTA");
 
-enum Epi { EPI_QKV_ROPE = 0, EPI_RESIDUAL = 1, EPI_GEGLU = 2, EPI_BIAS = 3 };
+enum Epi { EPI_QKV_ROPE = 0, EPI_RESIDUAL = 1, EPI_GEGLU = 2, EPI_BIAS = 3, EPI_RESIDUAL_SUMS = 4 };
 
 struct SkinnyArgs {
     const void* x; int x_f32; int ldx;        // activations [M, K]
@@ -77,6 +77,7 @@ struct SkinnyArgs {
     int group_rows, kv_skip;                  // rows per sequence, and rows of a sequence's cache that are not written (0, 0: one sequence)
     uint32_t inv_group;                       // sequence of a row = row * inv_group >> 20 (rows < 128); 0 for one sequence
     bf16* factor_out;                         // optional bf16 copy of the factors
+    float* row_sums; int sum_rows;            // RESIDUAL_SUMS: sums of squares of the rows as bf16, per 32 columns, [columns / 128][sum_rows][4]
     int* status;
     uint32_t spin_limit;                       // polls before a wait gives up (0 = the default limit)
     uint32_t expect_extra_bytes;               // self-test only: bytes the owners wait for that no peer sends
@@ -129,6 +130,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+    constexpr bool RESIDUAL = EPI == EPI_RESIDUAL || EPI == EPI_RESIDUAL_SUMS;
     constexpr int THREADS = threads_of(TOK), ISSUERS = TOK <= 64 ? 1 : 2;      // MMA-issuing threads, an accumulator each
     constexpr uint32_t RED_BYTES = TOK * 512, ACC_COLS = TOK == 96 ? 256 : ISSUERS * TOK;
     // The upper warps add up the rows' squares: the MMA issuers' warps come too late for it (gate/up: 1.6 us after the last MMA)
@@ -245,10 +247,10 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
             }
         } else {
             at[j][0] = (uint32_t)((row0 + ta) * p.ldo + n); at[j][1] = at[j][0] + p.ldo;
-            if (EPI == EPI_RESIDUAL && p.out_f32) {
+            if (RESIDUAL && p.out_f32) {
                 if (live[j][0]) { const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at[j][0]); pre[j].x = a.x; pre[j].y = a.y; }
                 if (live[j][1]) { const uint2 a = *reinterpret_cast<const uint2*>(static_cast<const float*>(p.out) + at[j][1]); pre[j].z = a.x; pre[j].w = a.y; }
-            } else if (EPI == EPI_RESIDUAL) {
+            } else if (RESIDUAL) {
                 const float2 a = unpack_bf16x2(live[j][0] ? *reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at[j][0]) : 0u);
                 const float2 b = unpack_bf16x2(live[j][1] ? *reinterpret_cast<const uint32_t*>(static_cast<const bf16*>(p.out) + at[j][1]) : 0u);
                 pre[j] = make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
@@ -458,6 +460,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
                 factor[1] = rsqrtf(ss.y * inv_k + 1e-6f);
             }
             float2 v[2], up[2];
+            float squares[2] = {0.f, 0.f};
             sum_sources(c, v);
             if (EPI == EPI_GEGLU) sum_sources(64 + c, up);        // columns 0..63 of the tile are gate columns, 64..127 the matching up columns
 #pragma unroll
@@ -485,7 +488,19 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
                     if (p.out_shadow) *reinterpret_cast<uint32_t*>(p.out_shadow + at[j][i]) = word;
                     if (p.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(p.out) + at[j][i]) = make_float2(v0, v1);
                     else *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + at[j][i]) = word;
+                    if (EPI == EPI_RESIDUAL_SUMS) { const float2 w = unpack_bf16x2(word); squares[i] = w.x * w.x + w.y * w.y; }
                 }
+            }
+            if (EPI == EPI_RESIDUAL_SUMS) {      // a warp has 32 columns of four tokens, even lanes the first two
+#pragma unroll
+                for (int o = 2; o < 32; o <<= 1) {
+                    squares[0] += __shfl_xor_sync(0xffffffffu, squares[0], o);
+                    squares[1] += __shfl_xor_sync(0xffffffffu, squares[1], o);
+                }
+                const int part = (tile * TN + c) >> 5, row = row0 + (int)rank * TS + tl;
+                float* to = p.row_sums + ((size_t)(part >> 2) * p.sum_rows + row) * 4 + (part & 3);
+                if (lane < 2 && live[j][0]) to[0] = squares[0];
+                if (lane < 2 && live[j][1]) to[4] = squares[1];
             }
         }
     }

@@ -292,7 +292,7 @@ struct Tc5Cfg {
 // 2: the kernel that wrote A left its rows' sums in GemmArgs::in_sums.
 // EP: what the staged epilogue does, as a set of EP_* bits, so that it carries no run-time choices (they cost as much as
 // the arithmetic); EP_ANY reads it from GemmArgs.
-constexpr int EP_ANY = -1, EP_BIAS = 1, EP_RES = 2, EP_GELU = 4, EP_ROPE = 8;      // EP_ROPE: with rounding first, as the prefix encoder's
+constexpr int EP_ANY = -1, EP_BIAS = 1, EP_RES = 2, EP_GELU = 4, EP_ROPE = 8, EP_RAW = 16;      // EP_ROPE: with rounding first, as the prefix encoder's; EP_RAW: without
 template <int BN, bool DUAL, int STAGES, bool ROPE = false, bool CLUSTER = false, int NORM = 0, int EP = EP_ANY>
 __global__ void __launch_bounds__(320, 1)
 tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
@@ -442,7 +442,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
         // staged path: bf16 destination(s); the preloaded operand is the bf16 residual or, for the RoPE +
         // scatter epilogue, the cos/sin entries of the chunk (one or the other)
         const bool plain = EP != EP_ANY || (!p.c_f32 && (ROPE ? !(p.R != nullptr || p.bias != nullptr || p.act != 0) : p.rope == nullptr));
-        const bool with_rope = ROPE && (EP != EP_ANY || p.rope != nullptr), round_first = EP != EP_ANY || p.round_first;
+        const bool with_rope = ROPE && (EP != EP_ANY || p.rope != nullptr), round_first = EP != EP_ANY ? (EP & EP_RAW) == 0 : p.round_first != 0;
         const bool has_res = EP != EP_ANY ? (EP & EP_RES) != 0 : p.R != nullptr;
         const int act = EP != EP_ANY ? ((EP & EP_GELU) ? 1 : 0) : p.act;
         const int rope_qd = p.heads * p.head_dim;            // RoPE epilogue: columns [0, qd) are Q, then K, then V
@@ -1012,6 +1012,10 @@ inline int launch_tc5_cfg(const GemmArgs& g, int* status, cudaStream_t st, int s
     if constexpr (ROPE) {
         if (g.rope != nullptr && g.round_first && g.R == nullptr && g.bias == nullptr && g.bias_f32 == nullptr && g.act == 0)
             return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ROPE>(g, status, st, splits, ws);
+        if constexpr (NORM == 2) {
+            if (g.rope != nullptr && !g.round_first && g.R == nullptr && g.bias == nullptr && g.bias_f32 == nullptr && g.act == 0)
+                return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ROPE | EP_RAW>(g, status, st, splits, ws);
+        }
     }
     if constexpr (NORM == 2 && !DUAL) return FVLA_ERR_UNSUPPORTED;      // only the epilogues above
     else return launch_tc5_ep<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP_ANY>(g, status, st, splits, ws);

@@ -42,6 +42,14 @@ class EncoderLayers(ctypes.Structure):
                 [(n, _I) for n in ("sequences", "rows", "first", "last", "final_layer")])
 
 
+class DecoderBatchLayers(ctypes.Structure):
+    """`struct fvla_decoder_batch_layers` of the header."""
+    _fields_ = ([(n, _P) for n in ("qkv_w", "o_w", "gate_w", "up_w", "down_w", "rope", "x", "x_shadow", "q", "hidden", "k_cache", "v_cache",
+                                   "norm_factor", "row_sums", "ws_qkv", "ws_attn")] + [(n, _Z) for n in ("ws_qkv_bytes", "ws_attn_bytes")] +
+                [(n, ctypes.c_longlong) for n in ("layer_stride", "episode_stride")] +
+                [(n, _I) for n in ("episodes", "tokens", "prefix", "first", "last", "layers")])
+
+
 # name -> argument ctypes (every function returns int except the three queries below)
 SIGNATURES: dict[str, list] = {
     "fvla_vision_patch_embed": [_P, _P, _P, _P, _P, _I, _P, _Z, _P],
@@ -65,6 +73,7 @@ SIGNATURES: dict[str, list] = {
     "fvla_decoder_action_out_proj": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P],
     "fvla_decoder_steps_run": [ctypes.POINTER(DecoderSteps), _P],
     "fvla_vision_tower_run": [ctypes.POINTER(VisionTower), _P],
+    "fvla_decoder_batch_layers_run": [ctypes.POINTER(DecoderBatchLayers), _P],
     "fvla_encoder_layers_run": [ctypes.POINTER(EncoderLayers), _P],
     "fvla_embed_rows": [_P, _P, _P, _I, _I, ctypes.c_longlong, _P],
     "fvla_convert_copy": [_P, _I, _P, _I, _P, _Z, _P],
@@ -77,6 +86,7 @@ QUERIES: dict[str, tuple] = {
     "fvla_abi_version": ([], c_int),
     "fvla_fused_norm_supported": ([_I, _I, _I, _I], c_int),
     "fvla_row_sums_supported": ([_I], c_int),
+    "fvla_decoder_batch_supported": ([_I, _I], c_int),
     "fvla_gemm_plan_count": ([], c_int),
     "fvla_launch_count": ([], ctypes.c_ulonglong),
     "fvla_device_status": ([_P], c_int),

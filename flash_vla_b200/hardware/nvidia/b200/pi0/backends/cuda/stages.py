@@ -145,6 +145,43 @@ def encoder_layers(weights, buffers, rows, sequences=1):
     return run
 
 
+def decoder_batch_layers(weights, caches, buffers, encoder_seq_len, episodes, layers):
+    """The layers of one Euler step of a batch of more than 128 rows: a function that enqueues layers [first, last), or None where
+    the ops have to be called one by one (fewer rows have cluster kernels of their own; see `vision_tower`)."""
+    w, b, K, V = weights, buffers, caches["encoder_K"], caches["encoder_V"]
+    x, shadow = b["decoder_x"], b.get("decoder_x_bf16")
+    stacks = {n: w[f"decoder_{n}"] for n in ("attn_qkv_w", "attn_o_w", "ffn_gate_w", "ffn_up_w", "ffn_down_w")}
+    if not all(isinstance(t, torch.Tensor) for t in (x, shadow, K, V, *stacks.values())) or x.ndim != 2 or K.ndim != 4 or episodes < 2:
+        return None
+    M, L, S = x.shape[0], stacks["attn_qkv_w"].shape[0], encoder_seq_len
+    D, hd = M // episodes, 256
+    shapes = {"attn_qkv_w": (L, _WIDTH, _QKV), "attn_o_w": (L, _Q, _WIDTH), "ffn_gate_w": (L, _WIDTH, _FFN), "ffn_up_w": (L, _WIDTH, _FFN), "ffn_down_w": (L, _FFN, _WIDTH)}
+    plain = {"q": (b["decoder_q_buf"], (M * _w.DECODER_HEADS, hd)), "hidden": (b["decoder_hidden"], (M, _FFN)), "rope": (b["decoder_rope_weights"], (D, hd)),
+             "norm_factor": (b["decoder_norm_factor_buf"], (M,))}
+    if M != D * episodes or S < 1 or not 1 <= layers <= L or not _fits(x, (M, _WIDTH), torch.float32) or not _fits(shadow, (M, _WIDTH)):
+        return None
+    if not all(_fits(t, s) for t, s in plain.values()) or not all(_fits(stacks[n], s) for n, s in shapes.items()):
+        return None
+    if K.shape[1] < layers or not _fits(K, (episodes, K.shape[1], S + D, hd)) or not _fits(V, K.shape) or not _lib.load().fvla_decoder_batch_supported(episodes, D):
+        return None
+    ws_bytes = _lib.gemm_workspace_bytes(M, _QKV, _WIDTH, 0)
+    attn_bytes = _lib.load().fvla_decoder_attention_workspace_bytes(D * _w.DECODER_HEADS, S + D)
+    roles = (("dec_row_sums", (M * (_WIDTH // 32),), torch.float32), ("dec_qkv_ws", (ws_bytes,), torch.uint8), ("dec_attn_ws", (attn_bytes,), torch.uint8))
+    if not all(_w.scratch_covers(*r, x.device) for r in roles):
+        return None
+    sums, ws, ws_attn = (_w.scratch(*r, x.device) for r in roles)
+    args = _lib.DecoderBatchLayers(
+        x=x.data_ptr(), x_shadow=_w._shadow_of(x) or shadow.data_ptr(), k_cache=K.data_ptr(), v_cache=V.data_ptr(), row_sums=sums.data_ptr(),
+        ws_qkv=ws.data_ptr(), ws_qkv_bytes=ws_bytes, ws_attn=ws_attn.data_ptr(), ws_attn_bytes=attn_bytes, layer_stride=(S + D) * hd, episode_stride=K.shape[1] * (S + D) * hd, episodes=episodes, tokens=D,
+        prefix=S, layers=layers, **{n: t.data_ptr() for n, (t, _) in plain.items()},
+        **{n: stacks[s].data_ptr() for n, s in (("qkv_w", "attn_qkv_w"), ("o_w", "attn_o_w"), ("gate_w", "ffn_gate_w"), ("up_w", "ffn_up_w"), ("down_w", "ffn_down_w"))})
+
+    def run(first, last):
+        args.first, args.last = first, last
+        _lib.call("fvla_decoder_batch_layers_run", ctypes.byref(args), _w._stream())
+    return run
+
+
 def _own(*names):
     return {n: fused_wrappers.FUSED_WRAPPERS.get(n, _w.ALL_WRAPPERS[n]) for n in names}
 
@@ -152,9 +189,12 @@ def _own(*names):
 # the fused table's entries that the native loops issue
 decoder_steps.stands_for = _own("decoder_action_in_proj", "decoder_action_mlp", "decoder_norm_qkv_rope", "decoder_attention", "decoder_out_proj_residual",
                                 "decoder_norm_gated_ffn", "decoder_ffn_down_residual", "decoder_action_out_proj", "copy_rows")
+decoder_batch_layers.stands_for = _own("decoder_norm_qkv_rope", "decoder_attention", "decoder_out_proj_residual", "decoder_norm_gated_ffn",
+                                       "decoder_ffn_down_residual")
 vision_tower.stands_for = _own("vision_patch_embed", "vision_norm_qkv", "vision_attention", "vision_out_proj_residual", "vision_norm_ffn_up",
                                "vision_ffn_down_residual")
 encoder_layers.stands_for = _own("encoder_norm_qkv_rope", "encoder_attention", "encoder_out_proj_residual", "encoder_norm_gated_ffn",
                                  "encoder_ffn_down_residual")
 
-STAGES = {"decoder_steps": decoder_steps, "vision_tower": vision_tower, "encoder_layers": encoder_layers}
+STAGES = {"decoder_steps": decoder_steps, "vision_tower": vision_tower, "encoder_layers": encoder_layers,
+          "decoder_batch_layers": decoder_batch_layers}

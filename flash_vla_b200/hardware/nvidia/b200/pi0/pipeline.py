@@ -196,7 +196,15 @@ def decoder_step_batched(ops, weights, prefix, dec, encoder_seq_len, step, episo
     x3[:, 1:].copy_(dec["decoder_mlp_out"].view(E, D - 1, x.shape[1]))
     if hasattr(ops, "sync_shadow"):
         ops.sync_shadow(x)
-    for layer in range(layers):
+    stage = _stage(ops, "decoder_batch_layers")
+    run = stage(w, prefix, dec, S, E, layers) if stage is not None else None
+    if run is not None and before_layer is None:
+        run(0, layers)
+    for layer in range(layers if run is None or before_layer is not None else 0):
+        if run is not None:
+            before_layer(layer)
+            run(layer, layer + 1)
+            continue
         k_all, v_all = prefix["encoder_K"][:, layer], prefix["encoder_V"][:, layer]      # (E, S + D, 256) views
         if before_layer is not None:
             before_layer(layer)

@@ -267,7 +267,22 @@ struct fvla_encoder_layers {
     int sequences, rows, first, last, final_layer;
 };
 int fvla_encoder_layers_run(const struct fvla_encoder_layers* args, void* stream);
-/* 1 where the two calls above take that many rows: tcgen05 kernels in use, more than 64 rows, no pinned launch plans. */
+/* Layers [first, last) of `layers` of one Euler step of a batch of episodes of more than 128 rows together (pipeline.py:95-135 per layer): x
+ * (episodes * tokens, 1024) is the fp32 residual stream, x_shadow its bf16 copy, which the residual projections write with the rows' sums of
+ * squares (row_sums, episodes * tokens * 32 floats) and the projections behind them read. Layer 0's and the last layer's QKV projections
+ * run as fvla_decoder_norm_qkv_rope (the first needs no shadow, the last leaves norm_factor). K / V of layer l and episode e: k_cache / v_cache +
+ * l * layer_stride + e * episode_stride elements, prefix + tokens rows. FVLA_ERR_UNSUPPORTED, with nothing launched, where
+ * fvla_decoder_batch_supported(episodes, tokens) is 0. */
+struct fvla_decoder_batch_layers {
+    const void *qkv_w, *o_w, *gate_w, *up_w, *down_w, *rope;
+    void *x, *x_shadow, *q, *hidden, *k_cache, *v_cache, *norm_factor, *row_sums, *ws_qkv, *ws_attn;
+    size_t ws_qkv_bytes, ws_attn_bytes;
+    long long layer_stride, episode_stride;
+    int episodes, tokens, prefix, first, last, layers;
+};
+int fvla_decoder_batch_layers_run(const struct fvla_decoder_batch_layers* args, void* stream);
+int fvla_decoder_batch_supported(int episodes, int tokens);
+/* 1 where the two prefix calls above take that many rows: tcgen05 kernels in use, more than 64 rows, no pinned launch plans. */
 int fvla_row_sums_supported(int M);
 
 /* No counterpart in the reference, where these are torch `copy_` calls inside the pipeline (pipeline.py:103,
