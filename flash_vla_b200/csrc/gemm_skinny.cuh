@@ -44,11 +44,14 @@ using tc5::smem_desc;
 
 constexpr int TN = 128;          // N columns per CTA (MMA M)
 constexpr int MAX_KB = 8;        // k-blocks of 64 per CTA
+// Beyond 64 slots they go through a ring, and row groups may have twice as many: the down projection of a batch is one launch then instead of two of
+// half of K each (eight episodes of 51 rows, 7.3 + 8.8 us end to end; forward 36.2 -> 35.5 ms, of one camera each 18.2 -> 17.5, five episodes 24.9 -> 24.35).
+__host__ __device__ constexpr int max_kb(int tok) { return tok > 64 ? 2 * MAX_KB : MAX_KB; }
 // TOK: token slots (MMA N): 32, 64, 96 or 128, of which the activation tile fills the rows there are, in eights (the MMAs read on into what
 // lies behind; those columns are nobody's). Up to 64 slots every k-block of a CTA has a place in shared memory. With more, a k-block
 // takes up to 32 KB and the exchange 48 or 64 KB, so only five to eight have one and the rest reuse the first ones' when their MMAs (and
 // the readers of the sums of squares) are done.
-constexpr int misc_bytes(int tok) { return tok * 4 + tok * 8 + (2 * MAX_KB + 2) * 8 + 32; }     // received sums, own sums, barriers, TMEM slot, flag
+constexpr int misc_bytes(int tok) { return tok * 4 + tok * 8 + (2 * max_kb(tok) + 2) * 8 + 32; }     // received sums, own sums, barriers, TMEM slot, flag
 constexpr size_t smem_bytes(int tok, int x_rows, int slots) {
     return 1024 + (size_t)slots * (16384 + x_rows * 128) + tok * 512 + misc_bytes(tok);
 }
@@ -57,7 +60,7 @@ constexpr int slots_of(int tok, int x_rows, int kblocks) {
     while (n > 1 && smem_bytes(tok, x_rows, n) > 232448) --n;
     return n;
 }
-static_assert(slots_of(64, 64, MAX_KB) == MAX_KB && slots_of(128, 128, MAX_KB) == 5 && slots_of(96, 72, MAX_KB) == 7, "shared memory of one CTA");
+static_assert(slots_of(64, 64, MAX_KB) == MAX_KB && slots_of(128, 128, MAX_KB) == 5 && slots_of(96, 72, MAX_KB) == 7 && slots_of(128, 128, 2) == 2, "shared memory of one CTA");
 
 enum Epi { EPI_QKV_ROPE = 0, EPI_RESIDUAL = 1, EPI_GEGLU = 2, EPI_BIAS = 3, EPI_RESIDUAL_SUMS = 4 };
 
@@ -145,9 +148,10 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     float* ssq_local = reinterpret_cast<float*>(gen + off_red + RED_BYTES + TOK * 4);      // [TOK][2]
     const uint32_t off_bar = off_red + RED_BYTES + TOK * 12;
     const uint32_t bars = base + off_bar;                                        // a full barrier per k-block, done, incoming, a free barrier per slot
-    const uint32_t done_bar = bars + MAX_KB * 8, in_bar = bars + (MAX_KB + 1) * 8, free_bars = bars + (MAX_KB + 2) * 8;
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + off_bar + (2 * MAX_KB + 2) * 8);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + off_bar + (2 * MAX_KB + 2) * 8 + 8);
+    constexpr int BARS = max_kb(TOK);
+    const uint32_t done_bar = bars + BARS * 8, in_bar = bars + (BARS + 1) * 8, free_bars = bars + (BARS + 2) * 8;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + off_bar + (2 * BARS + 2) * 8);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + off_bar + (2 * BARS + 2) * 8 + 8);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     FVLA_DBG_CTA(p, (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
@@ -193,7 +197,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     }
     __syncwarp();
     if (warp == 0) {
-        tc5::tmem_alloc(base + off_bar + (2 * MAX_KB + 2) * 8, ACC_COLS);
+        tc5::tmem_alloc(base + off_bar + (2 * BARS + 2) * 8, ACC_COLS);
         tc5::tmem_relinquish();
     }
     // Programmatic dependent launch: everything above touched only weights and this CTA's own
@@ -322,8 +326,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     // 128 slots: two threads issue the k-blocks in turn, each into an accumulator of its own.
     constexpr uint32_t idesc = skinny_idesc(TOK);
     const uint64_t ad = smem_desc(sW, 8192, 1024), bd = smem_desc(sX, 16, 1024);
-    auto issue_block = [&](int kb, uint32_t acc, bool first) {
-        const int slot = TOK > 64 && kb >= NS ? kb - NS : kb;
+    auto issue_block = [&](int slot, uint32_t acc, bool first) {
 #pragma unroll
         for (int k16 = 0; k16 < 4; ++k16)
             tc5::umma_bf16(acc, ad + slot * (16384 >> 4) + k16 * (2048 >> 4), bd + slot * (XB >> 4) + k16 * (32 >> 4), idesc, !first || k16 > 0 ? 1u : 0u);
@@ -340,21 +343,24 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         }
     }
     if (ISSUERS == 2 && warp < 2 && lane == 0) {
-        for (int kb = warp; kb < KB; kb += 2) {
+        for (int kb = warp, slot = warp; kb < KB; kb += 2) {
             if (!mbar_wait(bars + kb * 8, 0, abort_flag)) break;
             tc5::tc_fence_after();
-            issue_block(kb, tmem + warp * TOK, kb < 2);
+            issue_block(slot, tmem + warp * TOK, kb < 2);
             if (kb + NS < KB) tc5::umma_commit(free_bars + kb * 8);
+            slot += 2;
+            if (slot >= NS) slot -= NS;
         }
         tc5::umma_commit(done_bar);
     }
     // The k-blocks that had no slot of their own: one lane asks for block kb + NS once block kb's slot is free, that is read
     // by its MMAs and by the warps below (neither this lane's nor the issuers': those would wait for themselves).
     if (TOK > 64 && warp == 2 && lane == 0)
-        for (int kb = 0; kb + NS < KB; ++kb) {
+        for (int kb = 0, slot = 0; kb + NS < KB; ++kb) {
             if (!mbar_wait(free_bars + kb * 8, 0, abort_flag)) break;
-            request_w(kb + NS, kb);
-            tma_load_2d(sX + kb * XB, &tmX, bars + (kb + NS) * 8, k0 + (kb + NS) * 64, row0);
+            request_w(kb + NS, slot);
+            tma_load_2d(sX + slot * XB, &tmX, bars + (kb + NS) * 8, k0 + (kb + NS) * 64, row0);
+            if (++slot == NS) slot = 0;
         }
     __syncwarp();
     if (x_by_tma && p.need_factor && warp >= THREADS / 32 - SSQ_WARPS) {
@@ -363,9 +369,8 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
         constexpr int LPT = SSQ_WARPS * 32 / TOK;            // lanes per token
         const int st = tid - (THREADS - SSQ_WARPS * 32), t = st / LPT, sub = st % LPT;
         float part[8 / LPT] = {};                            // one sum per 16-byte piece of the rows, added up pairwise below
-        for (int kb = 0; kb < KB; ++kb) {
+        for (int kb = 0, slot = 0; kb < KB; ++kb) {
             mbar_wait(bars + kb * 8, 0, abort_flag);
-            const int slot = TOK > 64 && kb >= NS ? kb - NS : kb;
 #pragma unroll
             for (int h = 0; h < 8 / LPT; ++h) {
                 const uint4 a = *reinterpret_cast<const uint4*>(gen + w_bytes + slot * XB + t * 128 + (sub + h * LPT) * 16);
@@ -376,6 +381,7 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
                 __syncwarp();
                 if (lane == 0) tc5::mbar_arrive(free_bars + kb * 8);
             }
+            if (++slot == NS) slot = 0;
         }
 #pragma unroll
         for (int o = 1; o < LPT; o <<= 1)
@@ -561,7 +567,7 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, bool bf16_operand
         // groups are resident together (one wave) over the single-group choice.
         for (int s = best; s >= (pl.tok <= 64 ? 1 : 2); s /= 2) {
             const int kb = kb_total / s;
-            if (kb_total % s || kb > MAX_KB) break;
+            if (kb_total % s || kb > max_kb(pl.tok)) break;
             const int resident = s >= 8 ? 15 * 8 : (s == 4 ? 33 * 4 : 148);
             if (pl.tiles * s * groups <= resident) { best = s; break; }
         }

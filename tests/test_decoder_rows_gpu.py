@@ -114,6 +114,12 @@ def test_batched_residual_projection(episodes, rows, K):
     assert_close(got.view(-1, 1024), ref, what="decoder_ffn_down_residual")
 
 
+# groups of 65 rows and more, K = 4 096 in one launch: sixteen k-blocks per CTA through a ring of seven, six and five places
+@pytest.mark.parametrize("episodes,rows", [(2, 72), (3, 96), (4, 97), (3, 127), (4, 128)])
+def test_batched_down_projection_in_one_launch(episodes, rows):
+    test_batched_residual_projection(episodes, rows, 4096)
+
+
 # prefix projections beyond one round of tiles: pair tiles with K split over two rounds of items, 192-wide tiles in one and two rounds
 @pytest.mark.parametrize("op,S,K", [("encoder_ffn_down_residual", 1281, 16384), ("encoder_out_proj_residual", 1281, 2048), ("encoder_out_proj_residual", 2449, 2048)])
 def test_prefix_projection_by_row_count(op, S, K):
