@@ -332,6 +332,9 @@ inline int k_region_bytes(int spl, int pad) {
 }
 inline int smem_bytes(int spl, int pad) { return 1024 + k_region_bytes(spl, pad) + pad * 512 + QP_BYTES + MISC_BYTES + (pad <= 128 ? FAC_BYTES + E_BYTES : 0); }
 
+__host__ __device__ constexpr int block_threads(int kt) { return THREADS + 64 * kt; }      // and the warps that issue the MMAs
+template <int KT> __device__ __forceinline__ void all_sync() { asm volatile("bar.sync 2, %0;" ::"n"(block_threads(KT)) : "memory"); }
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) { return tc5::mbar_wait(bar, parity, abort_flag); }
 __device__ __forceinline__ uint32_t idesc(bool a_mn) { return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | ((uint32_t)(BQ >> 3) << 17) | (8u << 24); }
 
@@ -381,7 +384,7 @@ __device__ __forceinline__ uint32_t dsm_map(uint32_t local_addr, uint32_t rank) 
 }
 
 template <int KT, int SPL>                                // key tiles of 128 per CTA, cluster size
-__global__ void __launch_bounds__(decattn::THREADS, 1)
+__global__ void __launch_bounds__(decattn::block_threads(KT), 1)
 decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV) {
     using namespace decattn;
     constexpr int S_ISSUERS = 2 * KT, GROUPS = 2 * KT, S_COL = 64 * GROUPS, TMEM_COLS = 256 * KT;
@@ -458,7 +461,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
 #pragma unroll
         for (int i = 0; i < QV; ++i) {
             const int idx = tid + i * THREADS;
-            qv[i] = idx < rows_here * 32 ? *reinterpret_cast<const uint4*>(gq + (size_t)idx * 8) : make_uint4(0, 0, 0, 0);
+            qv[i] = tid < THREADS && idx < rows_here * 32 ? *reinterpret_cast<const uint4*>(gq + (size_t)idx * 8) : make_uint4(0, 0, 0, 0);
         }
         constexpr int OWN = KT == 1 ? 8 : 4;                 // own keys, 8 rows per piece index; with KT = 1 one or two CTAs have them all
         uint4 kv[OWN], vv[OWN];
@@ -467,7 +470,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
 #pragma unroll
             for (int i = 0; i < OWN; ++i) {
                 const int idx = base + tid + i * THREADS;
-                if (idx < total) {
+                if (tid < THREADS && idx < total) {
                     kv[i] = *reinterpret_cast<const uint4*>(p.k + kv0 + (size_t)idx * 8);
                     vv[i] = *reinterpret_cast<const uint4*>(p.v + kv0 + (size_t)idx * 8);
                 }
@@ -477,7 +480,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
 #pragma unroll
         for (int i = 0; i < QV; ++i) {
             const int idx = tid + i * THREADS, r = idx >> 5, c = idx & 31;
-            sts4u(sQ + (c >> 3) * (BQ * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), qv[i]);
+            if (tid < THREADS) sts4u(sQ + (c >> 3) * (BQ * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), qv[i]);
         }
         wait(pre_bar, 0, abort_flag);                        // the own rows go over what the boxes brought in
         for (int base = 0; base < total; base += OWN * THREADS) {
@@ -486,28 +489,50 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
             for (int i = 0; i < OWN; ++i) {
                 const int idx = base + tid + i * THREADS, r = prefix_here + (idx >> 5), c = idx & 31;
                 const uint32_t at = (c >> 3) * p.pad * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4);
-                if (idx < total) { sts4u(sK + at, kv[i]); sts4u(sV + at, vv[i]); }
+                if (tid < THREADS && idx < total) { sts4u(sK + at, kv[i]); sts4u(sV + at, vv[i]); }
             }
         }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     FVLA_STAMP(2);
-    // Issuing threads: for S^T one per key tile and half of the head dimension (accumulators added below), for O^T one per 128
-    // dims. A thread needs 46 clk per MMA and more for the first, the tensor pipe 39.
-    const int uniform_warp = __shfl_sync(0xffffffffu, warp, 0);
-    if (uniform_warp < S_ISSUERS && tc5::elect_one()) {
+    // Issuing threads, in warps of their own behind the others: for S^T one per key tile and half of the head dimension (accumulators
+    // added below), for O^T one per 128 dims. A thread needs 46 clk per MMA and more for the first, the tensor pipe 39; while two of the
+    // softmax warps issued, their rows' sums came 500 clk after the others'. Per layer-step 24.94 -> 24.81 us at 51 rows, 22.94 -> 22.65 at 32,
+    // 30.9 -> 30.5 at 65.
+    const int issuer = __shfl_sync(0xffffffffu, warp, 0) - THREADS / 32;
+    if (issuer >= 0) {
+      if (tc5::elect_one()) {
         tc5::tc_fence_after();
-        const int t = uniform_warp >> 1, h = uniform_warp & 1;
+        const int t = issuer >> 1, h = issuer & 1;
         const uint64_t a0 = tc5::smem_desc(sK + t * 128 * 128 + h * p.pad * 256, 16, 1024), b0 = tc5::smem_desc(sQ + h * (BQ * 256), 16, 1024);
 #pragma unroll
         for (int cb = 0; cb < 2; ++cb)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                tc5::umma_bf16(tmem + S_COL + uniform_warp * 32, a0 + cb * (p.pad * 8) + k * 2, b0 + cb * (BQ * 8) + k * 2, idesc(false), (cb | k) ? 1u : 0u);
+                tc5::umma_bf16(tmem + S_COL + issuer * 32, a0 + cb * (p.pad * 8) + k * 2, b0 + cb * (BQ * 8) + k * 2, idesc(false), (cb | k) ? 1u : 0u);
         tc5::umma_commit(s_bar);
+      }
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+      all_sync<KT>();                                        // P is in place
+      const uint64_t vd = tc5::smem_desc(sV + issuer * 2 * p.pad * 128, p.pad * 128, 1024), pd = tc5::smem_desc(sQ, 16, 1024);
+      if (issuer < 2 && tc5::elect_one()) {
+        tc5::tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < (KT == 1 ? 8 : MAX_PAD / 16); ++k)
+            if (k * 16 < p.pad)
+                tc5::umma_bf16(tmem + (k >> 2) * 64 + issuer * 32, vd + k * 128, pd + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true),
+                               k & 3 ? 1u : 0u);
+        tc5::umma_commit(o_bar);
+      }
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+      all_sync<KT>();                                        // accumulators read
+      asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+      return;
     }
-    __syncwarp();
     wait(s_bar, 0, abort_flag);
     __syncwarp();
     tc5::tc_fence_after();
@@ -515,7 +540,6 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
     // no data is handed over, and a releasing arrive waits 0.4 us for the thread's earlier accesses.
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     FVLA_STAMP(3);
-    const uint64_t vd = tc5::smem_desc(sV + uniform_warp * 2 * p.pad * 128, p.pad * 128, 1024), pd = tc5::smem_desc(sQ, 16, 1024);      // warps 0, 1: operands of O^T
     const int quad = warp & 3, half = warp >> 2;             // keys 32 quad .. + 31 of a tile, rows 16 half .. + 15
     {
         float v[KT][16], red[16];
@@ -542,7 +566,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
             const float m = butterfly16(red, lane, [](float a, float b) { return fmaxf(a, b); });
             if ((lane & 1) == 0) sts1(maxima + (((t * 2 + half) * 4 + quad) * 16 + (lane >> 1)) * 4, m);
         }
-        __syncthreads();
+        compute_sync();
 #pragma unroll
         for (int t = 0; t < KT; ++t) {
             const int key = t * 128 + quad * 32 + lane;
@@ -567,17 +591,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         }
         tc5::tc_fence_before();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (uniform_warp < 2 && tc5::elect_one()) {
-            tc5::tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < (KT == 1 ? 8 : MAX_PAD / 16); ++k)
-                if (k * 16 < p.pad)
-                    tc5::umma_bf16(tmem + (k >> 2) * 64 + uniform_warp * 32, vd + k * 128, pd + (k >> 2) * (BQ * 8) + (k & 3) * 2, idesc(true),
-                                   k & 3 ? 1u : 0u);
-            tc5::umma_commit(o_bar);
-        }
-        __syncwarp();
+        all_sync<KT>();                                      // the issuing warps go on with O^T
         if (KT == 1) {
             // Sum of a row over a group of 64 keys, four threads: each takes a pair of keys out of every eight, front to back.
             const int row = (warp >> 1) * 8 + (lane >> 2), group = warp & 1;
@@ -599,7 +613,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
             }
         }
     }
-    __syncthreads();                                         // sums and maxima of all rows are in place
+    compute_sync();                                          // sums and maxima of all rows are in place
     // Every warp works out what its accumulator columns are multiplied with, lane = row: [group][row], then 1 / sum
     float f[2][BQ], fi[BQ], lse;                              // (the first two groups' in registers before the accumulators are there)
     auto factors = [&](int g, float (&out)[BQ]) {
@@ -716,7 +730,7 @@ decoder_attention_cluster_kernel(const __grid_constant__ DecAttnArgs p, const __
         if (row + 1 < p.nq) *reinterpret_cast<uint32_t*>(out + HD) = v1;
     }
     FVLA_STAMP(6);
-    __syncthreads();
+    all_sync<KT>();
     if (warp == 1) {
         tc5::tc_fence_after();
         tc5::tmem_dealloc(tmem, TMEM_COLS);
@@ -756,7 +770,7 @@ inline int resident_attention_clusters(int spl) {
     int n = c.load(std::memory_order_acquire);
     if (n == 0) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(1, spl); cfg.blockDim = dim3(decattn::THREADS); cfg.dynamicSmemBytes = 168 * 1024;
+        cfg.gridDim = dim3(1, spl); cfg.blockDim = dim3(decattn::block_threads(1)); cfg.dynamicSmemBytes = 168 * 1024;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = spl; attr[0].val.clusterDim.z = 1;
@@ -815,7 +829,7 @@ inline int launch_decoder_attention_cluster(const DecAttnArgs& a, bool pdl, cuda
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.nq + decattn::BQ - 1) / decattn::BQ, a.splits, seqs);
-    cfg.blockDim = dim3(decattn::THREADS, 1, 1);
+    cfg.blockDim = dim3(decattn::block_threads(a.pad > 128 ? 2 : 1), 1, 1);
     cfg.dynamicSmemBytes = decattn::smem_bytes(a.splits, a.pad);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
