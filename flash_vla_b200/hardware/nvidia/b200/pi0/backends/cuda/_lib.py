@@ -136,6 +136,17 @@ def call(name: str, *args) -> None:
         raise FvlaError(f"{name} failed with status {status}: {load().fvla_last_error().decode()}")
 
 
+ERR_UNSUPPORTED = -4
+
+
+def offered(name: str, *args) -> bool:
+    """`call`, for an entry that refuses what it does not take before it launches anything: False then."""
+    status = getattr(load(), name)(*args)
+    if status not in (0, ERR_UNSUPPORTED):
+        raise FvlaError(f"{name} failed with status {status}: {load().fvla_last_error().decode()}")
+    return status == 0
+
+
 @functools.lru_cache(maxsize=1024)
 def gemm_workspace_bytes(M: int, N: int, K: int, dual: int = 0) -> int:
     """`fvla_gemm_workspace_bytes`, remembered: a pure function of the shape that walks every plan on each call."""

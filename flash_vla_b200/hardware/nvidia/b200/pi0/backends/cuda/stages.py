@@ -104,8 +104,7 @@ def vision_tower(weights, buffers, num_views) -> bool:
         down_b=stacks["ffn_down_b"].data_ptr(), row_sums=bufs["sums"].data_ptr(), **{n: t.data_ptr() for n, (t, _) in plain.items()},
         **{n: ctypes.addressof(a) for n, a in zip(names, arrays)},
         **{f"ws_{n}": bufs[n].data_ptr() for n in ("patch", "o", "down")}, **{f"ws_{n}_bytes": bufs[n].numel() for n in ("patch", "o", "down")})
-    _lib.call("fvla_vision_tower_run", ctypes.byref(args), _w._stream())
-    return True
+    return _lib.offered("fvla_vision_tower_run", ctypes.byref(args), _w._stream())
 
 
 def encoder_layers(weights, buffers, rows, sequences=1):
@@ -138,6 +137,8 @@ def encoder_layers(weights, buffers, rows, sequences=1):
         k_cache=K.data_ptr(), v_cache=V.data_ptr(), row_sums=bufs["sums"].data_ptr(), **{n: t.data_ptr() for n, (t, _) in plain.items()},
         **{n: stacks[s].data_ptr() for n, s in (("qkv_w", "attn_qkv_w"), ("o_w", "attn_o_w"), ("gate_w", "ffn_gate_w"), ("up_w", "ffn_up_w"), ("down_w", "ffn_down_w"))},
         **{f"ws_{n}": bufs[n].data_ptr() for n in ("attn", "o", "down")}, **{f"ws_{n}_bytes": bufs[n].numel() for n in ("attn", "o", "down")})
+    if not _lib.offered("fvla_encoder_layers_run", ctypes.byref(args), _w._stream()):      # no layers yet: only whether it takes them
+        return None
 
     def run(first, last):
         args.first, args.last = first, last
@@ -175,6 +176,8 @@ def decoder_batch_layers(weights, caches, buffers, encoder_seq_len, episodes, la
         ws_qkv=ws.data_ptr(), ws_qkv_bytes=ws_bytes, ws_attn=ws_attn.data_ptr(), ws_attn_bytes=attn_bytes, layer_stride=(S + D) * hd, episode_stride=K.shape[1] * (S + D) * hd, episodes=episodes, tokens=D,
         prefix=S, layers=layers, **{n: t.data_ptr() for n, (t, _) in plain.items()},
         **{n: stacks[s].data_ptr() for n, s in (("qkv_w", "attn_qkv_w"), ("o_w", "attn_o_w"), ("gate_w", "ffn_gate_w"), ("up_w", "ffn_up_w"), ("down_w", "ffn_down_w"))})
+    if not _lib.offered("fvla_decoder_batch_layers_run", ctypes.byref(args), _w._stream()):      # no layers yet: only whether it takes them
+        return None
 
     def run(first, last):
         args.first, args.last = first, last
