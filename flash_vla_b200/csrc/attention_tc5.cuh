@@ -452,24 +452,34 @@ inline int launch_attention_tc5(const void* Q, const void* K, const void* V, voi
 }
 
 // ---------------------------------------------------------------------------------------------
-// SigLIP attention on tcgen05: one CTA per (view, head, half of the 256 query tokens). The whole key
-// range (256 tokens) is one S tile, so there is no loop and no rescale: S = Q K^T (5 x m128 n256 k16:
+// SigLIP attention on tcgen05: one CTA per (view, head) and HALVES of the 256 query tokens. The whole key
+// range (256 tokens) is one S tile per half, so there is no loop and no rescale: S = Q K^T (5 x m128 n256 k16:
 // head dim 72 padded to 80), softmax by two threads per row (128 keys each, maxima and sums swapped
 // through shared memory), O = P V (16 x m128 n80 k16). Q, K and V are read by TMA straight from the
 // packed QKV activation ([views * tokens, 3 * heads * 72], head slices of 144 bytes); the 64-wide boxes
 // that cover dims 64..127 of a slice pick up 56 columns that belong to the next slice: dims 72..79 of
 // the Q tile are zeroed in shared memory before the MMA (so the matching K columns do not matter), and
 // output columns 72..79 are simply not stored.
+// A CTA is a chain of latencies (7.5 us, tensor pipe and memory idle through most of it) and fills an SM. With one half per CTA, twice
+// the CTAs, a launch is over sooner while all of them are resident; beyond that a CTA takes both halves: K and V come once, both S tiles
+// are issued together, P of one half lies where Q was and of the other where K was, and PV of the first runs under the second's
+// softmax. One half / both: 3 views 7.6 us / -, 6 views 13.3 / 11.3, 9 views 15.4 / 12.6, 12 views 21.5 / 21.9 (two rounds against three), 24 views 40.3 / 32.7.
 // ---------------------------------------------------------------------------------------------
 namespace vis {
 constexpr int TOK = 256, HDIM = 72, THREADS = 320;
-constexpr int OFF_Q = 0;                       // 2 atoms x [128 rows x 128 B]
-constexpr int OFF_K = 32768;                   // 2 atoms x [256 rows x 128 B]
-constexpr int OFF_V = 98304;                   // [key block 4][dim atom 2][64 rows x 128 B]
-constexpr int OFF_P = 163840;                  // 4 atoms x [128 rows x 128 B]
-constexpr int OFF_BAR = 229376;
-constexpr int SMEM = 1024 + OFF_BAR + 128;
-constexpr uint32_t O_COL = 256;                // TMEM: S at columns 0..255, O at 256..335
+template <int HALVES>
+struct Cfg {
+    static constexpr int OFF_Q = 0;                                  // per half 2 atoms x [128 rows x 128 B]
+    static constexpr int OFF_K = HALVES * 32768;                     // 2 atoms x [256 rows x 128 B]
+    static constexpr int OFF_V = OFF_K + 65536;                      // [key block 4][dim atom 2][64 rows x 128 B]
+    static constexpr int OFF_BEHIND = OFF_V + 65536;                 // P of a single half, else maxima and sums
+    __host__ __device__ static constexpr int off_p(int h) { return HALVES == 1 ? OFF_BEHIND : (h == 0 ? OFF_Q : OFF_K); }      // 4 atoms x [128 rows x 128 B]
+    __host__ __device__ static constexpr int off_x(int h) { return HALVES == 1 ? OFF_Q : OFF_BEHIND + h * 2048; }               // [maxima, sums][2 groups][128 rows]
+    __host__ __device__ static constexpr uint32_t s_col(int h) { return h * 256; }       // TMEM: S of a half at 256 columns, O over it, or behind it with a single half
+    __host__ __device__ static constexpr uint32_t o_col(int h) { return HALVES == 1 ? 256 : h * 256; }
+    static constexpr int OFF_BAR = OFF_BEHIND + (HALVES == 1 ? 65536 : HALVES * 2048);
+    static constexpr int SMEM = 1024 + OFF_BAR + 128;
+};
 
 __host__ __device__ constexpr uint32_t idesc_qk() {      // m128 n256, both operands K-major
     return (1u << 4) | (1u << 7) | (1u << 10) | (0u << 15) | (0u << 16) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -485,27 +495,31 @@ struct Args {
     int* status;
 };
 
+template <int HALVES>
 __global__ void __launch_bounds__(THREADS, 1)
 vision_attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                             const __grid_constant__ CUtensorMap tmV) {
+    using C = Cfg<HALVES>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-    const uint32_t sQ = base + OFF_Q, sK = base + OFF_K, sV = base + OFF_V, sP = base + OFF_P;
-    const uint32_t bars = base + OFF_BAR;
-    const uint32_t qk_full = bars, v_full = bars + 8, q_fixed = bars + 16, s_full = bars + 24, p_full = bars + 32, o_full = bars + 40;
-    const uint32_t tmem_slot = bars + 48;
-    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen + OFF_BAR + 48);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + OFF_BAR + 56);
-    float* xch = reinterpret_cast<float*>(gen + OFF_Q);      // [2 groups][128 rows] maxima, then sums: Q is dead by then
+    const uint32_t sQ = base + C::OFF_Q, sK = base + C::OFF_K, sV = base + C::OFF_V;
+    const uint32_t bars = base + C::OFF_BAR;
+    const uint32_t qk_full = bars, v_full = bars + 8, q_fixed = bars + 16;
+    auto s_full = [&](int h) { return bars + 24 + h * 8; };
+    auto p_full = [&](int h) { return bars + 40 + h * 8; };
+    auto o_full = [&](int h) { return bars + 56 + h * 8; };
+    const uint32_t tmem_slot = bars + 72;
+    volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen + C::OFF_BAR + 72);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + C::OFF_BAR + 80);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int qh = blockIdx.x, head = blockIdx.y, view = blockIdx.z;
+    const int qh = HALVES == 1 ? blockIdx.x : 0, head = blockIdx.y, view = blockIdx.z;
     const int width = p.heads * HDIM;
 
     if (tid == 0) {
         mbar_init(qk_full, 1); mbar_init(v_full, 1); mbar_init(q_fixed, 128);
-        mbar_init(s_full, 1); mbar_init(p_full, 1); mbar_init(o_full, 1);
+        for (int h = 0; h < HALVES; ++h) { mbar_init(s_full(h), 1); mbar_init(p_full(h), 1); mbar_init(o_full(h), 1); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -525,10 +539,12 @@ vision_attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tm
             tc5::prefetch_tensormap(&tmQ);
             tc5::prefetch_tensormap(&tmK);
             tc5::prefetch_tensormap(&tmV);
-            mbar_expect_tx(qk_full, 32768 + 65536);
+            mbar_expect_tx(qk_full, HALVES * 32768 + 65536);
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
-                tma_load_2d(sQ + a * 16384, &tmQ, qk_full, head * HDIM + a * 64, view * TOK + qh * 128);
+#pragma unroll
+                for (int h = 0; h < HALVES; ++h)
+                    tma_load_2d(sQ + h * 32768 + a * 16384, &tmQ, qk_full, head * HDIM + a * 64, view * TOK + (qh + h) * 128);
                 tma_load_2d(sK + a * 32768, &tmK, qk_full, width + head * HDIM + a * 64, view * TOK);
             }
             mbar_expect_tx(v_full, 65536);
@@ -544,23 +560,29 @@ vision_attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tm
             if (ok) {
                 tc5::tc_fence_after();
 #pragma unroll
-                for (int kk = 0; kk < 5; ++kk) {
-                    const uint64_t adesc = smem_desc(sQ + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-                    const uint64_t bdesc = smem_desc(sK + (kk >> 2) * 32768 + (kk & 3) * 32, 16, 1024);
-                    tc5::umma_bf16(tmem, adesc, bdesc, idesc_qk(), kk > 0 ? 1u : 0u);
+                for (int h = 0; h < HALVES; ++h) {
+#pragma unroll
+                    for (int kk = 0; kk < 5; ++kk) {
+                        const uint64_t adesc = smem_desc(sQ + h * 32768 + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
+                        const uint64_t bdesc = smem_desc(sK + (kk >> 2) * 32768 + (kk & 3) * 32, 16, 1024);
+                        tc5::umma_bf16(tmem + C::s_col(h), adesc, bdesc, idesc_qk(), kk > 0 ? 1u : 0u);
+                    }
+                    tc5::umma_commit(s_full(h));
                 }
-                tc5::umma_commit(s_full);
-                ok = mbar_wait(p_full, 0, abort_flag) && mbar_wait(v_full, 0, abort_flag);
+                ok = mbar_wait(v_full, 0, abort_flag);
             }
-            if (ok) {
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h) {
+                ok = ok && mbar_wait(p_full(h), 0, abort_flag);
+                if (!ok) break;
                 tc5::tc_fence_after();
 #pragma unroll
                 for (int k16 = 0; k16 < TOK / 16; ++k16) {
-                    const uint64_t adesc = smem_desc(sP + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024);
+                    const uint64_t adesc = smem_desc(base + C::off_p(h) + (k16 >> 2) * 16384 + (k16 & 3) * 32, 16, 1024);
                     const uint64_t bdesc = smem_desc(sV + (k16 >> 2) * 16384 + (k16 & 3) * 2048, 8192, 1024);
-                    tc5::umma_bf16(tmem + O_COL, adesc, bdesc, idesc_pv(), k16 > 0 ? 1u : 0u);
+                    tc5::umma_bf16(tmem + C::o_col(h), adesc, bdesc, idesc_pv(), k16 > 0 ? 1u : 0u);
                 }
-                tc5::umma_commit(o_full);
+                tc5::umma_commit(o_full(h));
             }
         }
     } else {
@@ -572,61 +594,75 @@ vision_attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tm
         if (g == 0) {
             // dims 72..79 of the Q tile hold the next slice's data: zero them (16-byte piece 1 of atom 1)
             ok = mbar_wait(qk_full, 0, abort_flag);
-            *reinterpret_cast<uint4*>(gen + OFF_Q + 16384 + row * 128 + ((1 ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h)
+                *reinterpret_cast<uint4*>(gen + C::OFF_Q + h * 32768 + 16384 + row * 128 + ((1 ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive_local(q_fixed);
         }
-        ok = mbar_wait(s_full, 0, abort_flag) && ok;
-        __syncwarp();
-        tc5::tc_fence_after();
-        float v[128];
-        ld_row128(tmem + t_lane + g * 128, v);
-        float mx = -INFINITY;
+        float inv[HALVES];
 #pragma unroll
-        for (int i = 0; i < 128; ++i) mx = fmaxf(mx, v[i]);
-        xch[g * 128 + row] = mx;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        const float m = fmaxf(xch[row], xch[128 + row]) * p.scale_log2;      // the scale is positive
-        asm volatile("bar.sync 1, 256;" ::: "memory");                           // maxima read before the sums overwrite them
-        float psum = 0.f;
+        for (int h = 0; h < HALVES; ++h) {
+            float* xch = reinterpret_cast<float*>(gen + C::off_x(h));      // (a single half: over Q, dead once S is complete)
+            ok = mbar_wait(s_full(h), 0, abort_flag) && ok;
+            __syncwarp();
+            tc5::tc_fence_after();
+            float v[128];
+            ld_row128(tmem + C::s_col(h) + t_lane + g * 128, v);
+            float mx = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 128; ++i) { v[i] = fast_exp2(fmaf(v[i], p.scale_log2, -m)); psum += v[i]; }
+            for (int i = 0; i < 128; ++i) mx = fmaxf(mx, v[i]);
+            xch[g * 128 + row] = mx;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            const float m = fmaxf(xch[row], xch[128 + row]) * p.scale_log2;      // the scale is positive
+            float psum = 0.f;
 #pragma unroll
-        for (int piece = 0; piece < 16; ++piece) {
-            uint8_t* prow = gen + OFF_P + (2 * g + (piece >> 3)) * 16384 + row * 128;
-            *reinterpret_cast<uint4*>(prow + (((piece & 7) ^ (row & 7)) << 4)) =
-                make_uint4(pack_bf16x2(v[8 * piece], v[8 * piece + 1]), pack_bf16x2(v[8 * piece + 2], v[8 * piece + 3]),
-                           pack_bf16x2(v[8 * piece + 4], v[8 * piece + 5]), pack_bf16x2(v[8 * piece + 6], v[8 * piece + 7]));
+            for (int i = 0; i < 128; ++i) { v[i] = fast_exp2(fmaf(v[i], p.scale_log2, -m)); psum += v[i]; }
+            if (HALVES == 2 && h == 0) {                         // P lies over Q, which the other half's S reads
+                ok = mbar_wait(s_full(1), 0, abort_flag) && ok;
+                __syncwarp();
+            }
+#pragma unroll
+            for (int piece = 0; piece < 16; ++piece) {
+                uint8_t* prow = gen + C::off_p(h) + (2 * g + (piece >> 3)) * 16384 + row * 128;
+                *reinterpret_cast<uint4*>(prow + (((piece & 7) ^ (row & 7)) << 4)) =
+                    make_uint4(pack_bf16x2(v[8 * piece], v[8 * piece + 1]), pack_bf16x2(v[8 * piece + 2], v[8 * piece + 3]),
+                               pack_bf16x2(v[8 * piece + 4], v[8 * piece + 5]), pack_bf16x2(v[8 * piece + 6], v[8 * piece + 7]));
+            }
+            xch[256 + g * 128 + row] = psum;
+            tc5::tc_fence_before();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // P stores -> visible to the MMA
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (warp == 2 && lane == 0) mbar_arrive_local(p_full(h));
+            const float l = xch[256 + row] + xch[256 + 128 + row];
+            inv[h] = l > 0.f ? 1.0f / l : 0.f;
         }
-        xch[g * 128 + row] = psum;
-        tc5::tc_fence_before();
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // P stores -> visible to the MMA
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (warp == 2 && lane == 0) mbar_arrive_local(p_full);
-        const float l = xch[row] + xch[128 + row];
-        const float inv = l > 0.f ? 1.0f / l : 0.f;
-        ok = mbar_wait(o_full, 0, abort_flag) && ok;
-        __syncwarp();
-        tc5::tc_fence_after();
-        // group 0 stores dims 0..39, group 1 dims 40..71 (TMEM columns 32..63 and 64..79 are read in both)
-        float a[32], b[16];
-        tc5::tmem_ld32(tmem + t_lane + O_COL + (g == 0 ? 0 : 32), a);
-        tc5::tmem_ld16(tmem + t_lane + O_COL + (g == 0 ? 32 : 64), b);
-        if (ok) {
-            bf16* dst = p.out + ((size_t)(view * TOK + qh * 128 + row)) * width + head * HDIM;
-            auto pack8 = [&](const float* s) {
-                return make_uint4(pack_bf16x2(s[0] * inv, s[1] * inv), pack_bf16x2(s[2] * inv, s[3] * inv),
-                                  pack_bf16x2(s[4] * inv, s[5] * inv), pack_bf16x2(s[6] * inv, s[7] * inv));
-            };
-            if (g == 0) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dst + q * 8) = pack8(a + q * 8);
-                *reinterpret_cast<uint4*>(dst + 32) = pack8(b);
-            } else {
-                // a = dims 32..63, b = dims 64..79
+        for (int h = 0; h < HALVES; ++h) {
+            ok = mbar_wait(o_full(h), 0, abort_flag) && ok;
+            __syncwarp();
+            tc5::tc_fence_after();
+            // group 0 stores dims 0..39, group 1 dims 40..71 (TMEM columns 32..63 and 64..79 are read in both)
+            float a[32], b[16];
+            tc5::tmem_ld32(tmem + t_lane + C::o_col(h) + (g == 0 ? 0 : 32), a);
+            tc5::tmem_ld16(tmem + t_lane + C::o_col(h) + (g == 0 ? 32 : 64), b);
+            if (ok) {
+                bf16* dst = p.out + ((size_t)(view * TOK + (qh + h) * 128 + row)) * width + head * HDIM;
+                const float f = inv[h];
+                auto pack8 = [&](const float* s) {
+                    return make_uint4(pack_bf16x2(s[0] * f, s[1] * f), pack_bf16x2(s[2] * f, s[3] * f),
+                                      pack_bf16x2(s[4] * f, s[5] * f), pack_bf16x2(s[6] * f, s[7] * f));
+                };
+                if (g == 0) {
 #pragma unroll
-                for (int q = 1; q < 4; ++q) *reinterpret_cast<uint4*>(dst + 32 + q * 8) = pack8(a + q * 8);
-                *reinterpret_cast<uint4*>(dst + 64) = pack8(b);
+                    for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(dst + q * 8) = pack8(a + q * 8);
+                    *reinterpret_cast<uint4*>(dst + 32) = pack8(b);
+                } else {
+                    // a = dims 32..63, b = dims 64..79
+#pragma unroll
+                    for (int q = 1; q < 4; ++q) *reinterpret_cast<uint4*>(dst + 32 + q * 8) = pack8(a + q * 8);
+                    *reinterpret_cast<uint4*>(dst + 64) = pack8(b);
+                }
             }
         }
     }
@@ -640,15 +676,22 @@ vision_attention_tc5_kernel(const Args p, const __grid_constant__ CUtensorMap tm
     if (tid == 0 && *abort_flag && p.status) atomicExch(p.status, 5);
 }
 
-// qkv: [views * 256, 3 * heads * 72] bf16; out: [views * 256, heads * 72] bf16.
-inline int launch_vision_attention_tc5(const void* qkv, void* out, int views, int heads, int* status, cudaStream_t st) {
-    auto kern = vision_attention_tc5_kernel;
+template <int HALVES>
+inline int launch_vision_attention_halves(const Args& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, int views, cudaStream_t st) {
+    auto kern = vision_attention_tc5_kernel<HALVES>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<HALVES>::SMEM);
         if (e != cudaSuccess) { set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
         configured.set();
     }
+    cudaError_t e = launch_pdl(kern, dim3(2 / HALVES, a.heads, views), dim3(THREADS), Cfg<HALVES>::SMEM, st, a, tmQ, tmK, tmV);
+    if (e != cudaSuccess) { set_error("vision_attention_tc5_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
+    return check_launch("vision_attention_tc5_kernel");
+}
+
+// qkv: [views * 256, 3 * heads * 72] bf16; out: [views * 256, heads * 72] bf16.
+inline int launch_vision_attention_tc5(const void* qkv, void* out, int views, int heads, int* status, cudaStream_t st) {
     const uint64_t cols = (uint64_t)3 * heads * HDIM, rows = (uint64_t)views * TOK;
     CUtensorMap tmQ, tmK, tmV;
     int rc = tc5::make_map(&tmQ, qkv, cols, rows, cols, 64, 128);
@@ -658,9 +701,10 @@ inline int launch_vision_attention_tc5(const void* qkv, void* out, int views, in
     rc = tc5::make_map(&tmV, qkv, cols, rows, cols, 64, 64);
     if (rc) return rc;
     Args a{static_cast<bf16*>(out), heads, kLog2e / sqrtf((float)HDIM), status};
-    cudaError_t e = launch_pdl(kern, dim3(2, heads, views), dim3(THREADS), SMEM, st, a, tmQ, tmK, tmV);
-    if (e != cudaSuccess) { set_error("vision_attention_tc5_kernel: %s", cudaGetErrorString(e)); return FVLA_ERR_LAUNCH; }
-    return check_launch("vision_attention_tc5_kernel");
+    // Rounds of CTAs, one per SM, at 7.2 us with one half and 10.9 with both.
+    const int sms = tc5::num_sms(), items = heads * views;
+    if ((items + sms - 1) / sms * 10.9f < (2 * items + sms - 1) / sms * 7.2f) return launch_vision_attention_halves<2>(a, tmQ, tmK, tmV, views, st);
+    return launch_vision_attention_halves<1>(a, tmQ, tmK, tmV, views, st);
 }
 }  // namespace vis
 

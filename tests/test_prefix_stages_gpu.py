@@ -159,3 +159,23 @@ def test_frozen_pool_and_pinned_plans_go_op_by_op():
             assert not stages.vision_tower(w, b, 1)
         finally:
             _lib.call("fvla_gemm_plan_clear")
+
+
+@pytest.mark.parametrize("views", [4, 5, 9, 12, 24])
+def test_vision_attention_by_views(views):
+    """One query half per CTA (4 and 12 views) and both: a view's result does not depend on its neighbours or on the form."""
+    from flash_vla_b200 import op_table
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
+    gen = torch.Generator(device="cuda").manual_seed(views)
+    qkv = rnd(gen, views, 256, 3456)
+    qkv[:, :9] *= 25.0                                       # some rows whose softmax is all but one-hot
+    ops, out = op_table(True), torch.zeros(views, 256, 1152, dtype=bf16, device="cuda")
+    ops.vision_attention(qkv, out)
+    for v in (0, views // 2, views - 1):
+        alone = torch.zeros(1, 256, 1152, dtype=bf16, device="cuda")
+        ops.vision_attention(qkv[v:v + 1].contiguous(), alone)
+        assert torch.equal(out[v], alone[0]), f"view {v}"
+    ref = torch.zeros(2, 256, 1152)
+    O.op_table(False).vision_attention(qkv[-2:].float().cpu(), ref)
+    assert_close(out[-2:], ref, what="vision_attention")
+    assert _lib.load().fvla_device_status(None) == 0
