@@ -57,10 +57,11 @@ constexpr size_t smem_bytes(int tok, int x_rows, int slots) {
 }
 constexpr int slots_of(int tok, int x_rows, int kblocks) {
     int n = kblocks;
-    while (n > 1 && smem_bytes(tok, x_rows, n) > 232448) --n;
+    if (tok > 64)
+        while (n > 1 && smem_bytes(tok, x_rows, n) > 232448) --n;
     return n;
 }
-static_assert(slots_of(64, 64, MAX_KB) == MAX_KB && slots_of(128, 128, MAX_KB) == 5 && slots_of(96, 72, MAX_KB) == 7 && slots_of(128, 128, 2) == 2, "shared memory of one CTA");
+static_assert(smem_bytes(64, 64, MAX_KB) <= 232448 && slots_of(128, 128, MAX_KB) == 5 && slots_of(96, 72, MAX_KB) == 7 && slots_of(128, 128, 2) == 2, "shared memory of one CTA");
 
 enum Epi { EPI_QKV_ROPE = 0, EPI_RESIDUAL = 1, EPI_GEGLU = 2, EPI_BIAS = 3, EPI_RESIDUAL_SUMS = 4 };
 
@@ -522,13 +523,12 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-struct SkinnyPlan { int tok, splits, kblocks, tiles, slots, x_rows; size_t smem; bool ok; };
+struct SkinnyPlan { int tok, splits, kblocks, tiles; bool ok; int slots, x_rows; size_t smem; };      // the last three by place_skinny
 
 inline void place_skinny(SkinnyPlan& pl, int M, bool bf16_operand) {
     pl.x_rows = bf16_operand ? (M + 7) / 8 * 8 : pl.tok;      // (the in-kernel conversion of fp32 rows fills the whole tile)
     pl.slots = slots_of(pl.tok, pl.x_rows, pl.kblocks);
     pl.smem = smem_bytes(pl.tok, pl.x_rows, pl.slots);
-    pl.ok = true;
 }
 
 // bf16_operand: rows as bf16 (the activation itself or its shadow).
@@ -548,7 +548,7 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, bool bf16_operand
         if (s < (pl.tok <= 64 ? 1 : 2) || s > 8 || (s & (s - 1)) || kb_total % s || kb_total / s > MAX_KB || ((kb_total / s) & (kb_total / s - 1))) return pl;
         pl.splits = s;
         pl.kblocks = kb_total / s;
-        place_skinny(pl, M, bf16_operand);
+        pl.ok = true;
         return pl;
     }
     // largest cluster (<= 8) that divides the k-blocks, keeps <= 8 k-blocks per CTA and stays near one wave
@@ -574,7 +574,7 @@ inline SkinnyPlan plan_skinny(int M, int N, int K, bool geglu, bool bf16_operand
     }
     pl.splits = best;
     pl.kblocks = kb_total / best;
-    place_skinny(pl, M, bf16_operand);
+    pl.ok = true;
     return pl;
 }
 
@@ -646,8 +646,10 @@ inline int launch_skinny_tok(const SkinnyArgs& a, const SkinnyPlan& pl, const vo
 
 template <int EPI>
 inline int launch_skinny(const SkinnyArgs& a, const void* W, const void* W2, int ldw, cudaStream_t st) {
-    const SkinnyPlan pl = plan_skinny(a.M, a.N, a.K, EPI == EPI_GEGLU, !a.x_f32 || a.x_shadow != nullptr, a.groups > 1 ? a.groups : 1);
+    const bool bf16_operand = !a.x_f32 || a.x_shadow != nullptr;
+    SkinnyPlan pl = plan_skinny(a.M, a.N, a.K, EPI == EPI_GEGLU, bf16_operand, a.groups > 1 ? a.groups : 1);
     if (!pl.ok) { set_error("skinny gemm: shape %dx%dx%d not supported", a.M, a.N, a.K); return FVLA_ERR_UNSUPPORTED; }
+    place_skinny(pl, a.M, bf16_operand);
     switch (pl.tok) {
         case 32: return launch_skinny_tok<EPI, 32>(a, pl, W, W2, ldw, st);
         case 64: return launch_skinny_tok<EPI, 64>(a, pl, W, W2, ldw, st);
