@@ -290,9 +290,9 @@ inline int launch_attention(const AttnArgs& a, dim3 grid, cudaStream_t st) {
 // Two key tiles (KT = 2), where that keeps more clusters resident: equal parts of the prefix and of the step's own keys, four groups.
 // (With one maximum per CTA instead of per group fewer probabilities are exactly 1: 2.176e-3 from the 64-bit result at 65 tokens x 882
 // unit-variance keys, 2.087e-3 with groups of 64, 2.080e-3 on 8 CTAs with one tile each.)
-// Measured at 51 rows x 819 keys inside the decoder's chain: 6.4 us per launch, against 7.8 us for the warp-level form
+// Measured at 51 rows x 819 keys inside the decoder's chain: 6.1 us per launch, against 7.8 us for the warp-level form
 // (mma.sync on 8 warps, halves staged in shared memory, bulk copies). What bounds it is a chain of
-// latencies: dependency wait 0.9, Q 0.7, S^T 0.6, softmax and O^T 1.8, exchange 1.1 (28 KB per CTA; distributed shared memory
+// latencies: dependency wait 0.9, Q 0.7, S^T 0.6, softmax and O^T 1.5, exchange 1.1 (28 KB per CTA; distributed shared memory
 // moves 16 B/clk per SM when all SMs send), combine 0.5; DRAM and the tensor pipes idle.
 // ---------------------------------------------------------------------------------------------
 struct DecAttnArgs {
