@@ -92,9 +92,9 @@ def vision_tower(weights, buffers, num_views) -> bool:
              "o": ("vis_o_ws", (_lib.gemm_workspace_bytes(M, D, D, 0),), torch.uint8), "down": ("vis_down_ws", (_lib.gemm_workspace_bytes(M, D, F, 0),), torch.uint8)}
     if not all(_w.scratch_covers(role, shape, dtype, dev) for role, shape, dtype in roles.values()):
         return False
-    folded = [[_w._folded_layernorm(stacks[f"{lin}_w"][l], stacks[f"{norm}_w"][l], stacks[f"{norm}_b"][l], stacks[f"{lin}_b"][l]) for l in range(L)]
+    folded = [_w._folded_layers(stacks[f"{lin}_w"], stacks[f"{norm}_w"], stacks[f"{norm}_b"], stacks[f"{lin}_b"])
               for lin, norm in (("attn_qkv", "pre_attn_norm"), ("ffn_up", "pre_ffn_norm"))]
-    if any(f is None for side in folded for f in side):
+    if None in folded:
         return False
     bufs = {n: _w.scratch(role, shape, dtype, dev) for n, (role, shape, dtype) in roles.items()}
     arrays = [(ctypes.c_void_p * L)(*(f[i].data_ptr() for f in side)) for side in folded for i in range(3)]

@@ -224,6 +224,24 @@ def _folded_layernorm(weight, norm_w, norm_b, bias):
     return folded
 
 
+def _folded_layers(weight, norm_w, norm_b, bias):
+    """`_folded_layernorm` of every layer of stacked contiguous tensors, or None where one of them has to wait; a layer that is
+    folded already costs one look-up under the key and versions that its slices would have."""
+    owner = weight if weight._base is None else weight._base
+    table = getattr(owner, _FOLDED_ATTR, {})
+    stacks = (weight, norm_w, norm_b, bias)
+    versions = tuple(t._version for t in stacks)
+    (w0, ws), (n0, ns), (s0, ss), (b0, bs) = ((t.data_ptr(), t.stride(0) * t.element_size()) for t in stacks)
+    layers = []
+    for l in range(weight.shape[0]):
+        entry = table.get((w0 + l * ws, n0 + l * ns, s0 + l * ss, b0 + l * bs))
+        folded = entry[1] if entry is not None and entry[0] == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
+        if folded is None:
+            return None
+        layers.append(folded)
+    return layers
+
+
 def _folded_norm_linear(entry, act, x, norm_w, norm_b, weight, bias, out, x_norm):
     """The fused table's LayerNorm + linear: the norm happens inside the GEMM and `x_norm` stays untouched. Shapes
     outside the fused form (a CTA would own several tiles) and calls that would have to fold weights during

@@ -179,3 +179,20 @@ def test_vision_attention_by_views(views):
     O.op_table(False).vision_attention(qkv[-2:].float().cpu(), ref)
     assert_close(out[-2:], ref, what="vision_attention")
     assert _lib.load().fvla_device_status(None) == 0
+
+
+def test_folded_layers_follow_the_weights():
+    """The tower finds each layer's folded weights where the op keeps them, and folds again after an in-place update of any of the four stacks."""
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import wrappers
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    w, nw, nb, b = rnd(gen, 3, 1152, 64, scale=0.02), rnd(gen, 3, 1152) + 1, rnd(gen, 3, 1152), rnd(gen, 3, 64)
+    first = wrappers._folded_layers(w, nw, nb, b)
+    assert all(f is g for f, g in zip(first, wrappers._folded_layers(w, nw, nb, b)))
+    assert all(wrappers._folded_layernorm(w[l], nw[l], nb[l], b[l]) is first[l] for l in range(3))
+    for t in (w, nw, nb, b):
+        t[1].mul_(2.0)
+        again = wrappers._folded_layers(w, nw, nb, b)
+        for l in range(3):
+            folded = (nw[l].float()[:, None] * w[l].float()).to(bf16)
+            assert torch.equal(again[l][0], folded), "weight_folded"
+            torch.testing.assert_close(again[l][2], nb[l].float() @ w[l].float() + b[l].float(), rtol=1e-4, atol=1e-4)      # fp32 sums of 1 152 products
