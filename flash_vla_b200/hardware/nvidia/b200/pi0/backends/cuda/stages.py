@@ -107,6 +107,17 @@ def vision_tower(weights, buffers, num_views) -> bool:
     return _lib.offered("fvla_vision_tower_run", ctypes.byref(args), _w._stream())
 
 
+def vision_tower_as_by_op(weights, buffers, num_views) -> bool:
+    """`vision_tower` for as many views as the table's own ops read folded weights for (one to four). With more they read the weights
+    themselves, and a graph captured from them follows an in-place update, which one with folded copies cannot: those go op by op. (What that costs a
+    forward of ten steps: two episodes of three views 13.1 -> 13.3 ms, four 23.5 -> 23.65, eight nothing beyond noise.)"""
+    x = buffers["vision_x"]
+    if not isinstance(x, torch.Tensor) or x.ndim != 3:
+        return False
+    M = x.shape[0] * _w.VISION_TOKENS
+    return all(_lib.load().fvla_fused_norm_supported(M, N, _VIS, 0) for N in (3 * _VIS, _VIS_FFN)) and vision_tower(weights, buffers, num_views)
+
+
 def encoder_layers(weights, buffers, rows, sequences=1):
     """The prefix encoder behind its first QKV projection: a function that enqueues layers [first, last) up to layer `last`'s QKV
     projection, or None where the ops have to be called one by one (see `vision_tower`). Row norms come from sums that the
@@ -194,10 +205,10 @@ decoder_steps.stands_for = _own("decoder_action_in_proj", "decoder_action_mlp", 
                                 "decoder_norm_gated_ffn", "decoder_ffn_down_residual", "decoder_action_out_proj", "copy_rows")
 decoder_batch_layers.stands_for = _own("decoder_norm_qkv_rope", "decoder_attention", "decoder_out_proj_residual", "decoder_norm_gated_ffn",
                                        "decoder_ffn_down_residual")
-vision_tower.stands_for = _own("vision_patch_embed", "vision_norm_qkv", "vision_attention", "vision_out_proj_residual", "vision_norm_ffn_up",
-                               "vision_ffn_down_residual")
+vision_tower_as_by_op.stands_for = _own("vision_patch_embed", "vision_norm_qkv", "vision_attention", "vision_out_proj_residual", "vision_norm_ffn_up",
+                                        "vision_ffn_down_residual")
 encoder_layers.stands_for = _own("encoder_norm_qkv_rope", "encoder_attention", "encoder_out_proj_residual", "encoder_norm_gated_ffn",
                                  "encoder_ffn_down_residual")
 
-STAGES = {"decoder_steps": decoder_steps, "vision_tower": vision_tower, "encoder_layers": encoder_layers,
+STAGES = {"decoder_steps": decoder_steps, "vision_tower": vision_tower_as_by_op, "encoder_layers": encoder_layers,
           "decoder_batch_layers": decoder_batch_layers}
