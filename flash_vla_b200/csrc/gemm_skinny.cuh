@@ -81,7 +81,7 @@ struct SkinnyArgs {
     int group_rows, kv_skip;                  // rows per sequence, and rows of a sequence's cache that are not written (0, 0: one sequence)
     uint32_t inv_group;                       // sequence of a row = row * inv_group >> 20 (rows < 128); 0 for one sequence
     bf16* factor_out;                         // optional bf16 copy of the factors
-    float* row_sums; int sum_rows;            // RESIDUAL_SUMS: sums of squares of the rows as bf16, per 32 columns, [columns / 128][sum_rows][4]
+    float* row_sums; int sum_rows;            // RESIDUAL_SUMS: sums of squares of the rows as `out` holds them, per 32 columns, [columns / 128][sum_rows][4]
     int* status;
     uint32_t spin_limit;                       // polls before a wait gives up (0 = the default limit)
     uint32_t expect_extra_bytes;               // self-test only: bytes the owners wait for that no peer sends
@@ -495,7 +495,10 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
                     if (p.out_shadow) *reinterpret_cast<uint32_t*>(p.out_shadow + at[j][i]) = word;
                     if (p.out_f32) *reinterpret_cast<float2*>(static_cast<float*>(p.out) + at[j][i]) = make_float2(v0, v1);
                     else *reinterpret_cast<uint32_t*>(static_cast<bf16*>(p.out) + at[j][i]) = word;
-                    if (EPI == EPI_RESIDUAL_SUMS) { const float2 w = unpack_bf16x2(word); squares[i] = w.x * w.x + w.y * w.y; }
+                    if (EPI == EPI_RESIDUAL_SUMS) {
+                        const float2 w = p.out_f32 ? make_float2(v0, v1) : unpack_bf16x2(word);
+                        squares[i] = w.x * w.x + w.y * w.y;
+                    }
                 }
             }
             if (EPI == EPI_RESIDUAL_SUMS) {      // a warp has 32 columns of four tokens, even lanes the first two

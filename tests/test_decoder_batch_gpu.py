@@ -95,3 +95,31 @@ def test_up_to_128_rows_and_wide_episodes_go_op_by_op():
     from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
     lib = _lib.load()
     assert [lib.fvla_decoder_batch_supported(e, t) for e, t in ((1, 200), (2, 64), (2, 129), (0, 51), (3, 0), (3, 51))] == [0, 0, 0, 0, 0, 1]
+
+
+# row groups of 65, 51, 102, 128 and 23 rows; both projections, through the ring and without
+@pytest.mark.parametrize("episodes,tokens", [(2, 65), (3, 51), (8, 51), (4, 128), (7, 23)])
+@pytest.mark.parametrize("last", ["o", "down"])
+def test_handed_down_squares_are_those_of_the_fp32_rows(episodes, tokens, last):
+    """The residual stream is fp32, and so are the squares that the norms are made of: each partial sum against the 32 values it stands for."""
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import stages, wrappers
+    from flash_vla_b200.hardware.nvidia.b200.pi0.buffers import allocate_batched_decoder_buffers
+    from flash_vla_b200.runtime.cuda import ScratchPool
+    S, L, M = 256, 1, episodes * tokens
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    w = {"decoder_" + n: (torch.randn(L, *s, device="cuda", generator=gen) * 0.02).to(bf16) for n, s in (
+        ("attn_qkv_w", (1024, 2560)), ("attn_o_w", (2048, 1024)), ("ffn_gate_w", (1024, 4096)), ("ffn_up_w", (1024, 4096)), ("ffn_down_w", (4096, 1024)))}
+    if last == "o":
+        w["decoder_ffn_down_w"].zero_()                      # the rows stay those of the output projection, their squares are written again
+    d = allocate_batched_decoder_buffers(tokens - 1, episodes, S, "cuda")
+    d["decoder_x"].copy_(torch.randn(M, 1024, device="cuda", generator=gen) * 3)
+    d["decoder_x"][:5] *= 20
+    kv = {n: (torch.randn(episodes, L, S + tokens, 256, device="cuda", generator=gen) * 0.5).to(bf16) for n in ("encoder_K", "encoder_V")}
+    pool = ScratchPool()
+    with wrappers.use_pool(pool):
+        stages.decoder_batch_layers(w, kv, d, S, episodes, L)(0, L)
+    sums = pool.get("dec_row_sums", (M * 32,), torch.float32, d["decoder_x"].device).view(8, M, 4).permute(1, 0, 2).reshape(M, 32)
+    exact = d["decoder_x"].double().pow(2).view(M, 32, 32).sum(2)
+    # 32 squares and 31 additions in fp32, half an ulp each, pairwise: 7 roundings of 2^-24. (Squares of bf16 values: up to 2^-8.)
+    worst = ((sums.double() - exact).abs() / exact).max().item()
+    assert worst <= 7 * 2 ** -24, worst
