@@ -200,14 +200,15 @@ _FOLDED_ATTR = "_fvla_folded_layernorm"
 def _folded_layernorm(weight, norm_w, norm_b, bias):
     """(weight_folded, colsum, bias_folded) of `fvla_fold_layernorm` for this LayerNorm + linear pair, made on first
     use and kept ON the tensor that owns `weight`'s storage (found again through `view._base`, gone with it).
-    The entry also remembers the versions of the four tensors: an in-place update of any of them refolds.
-    None while a CUDA graph is being captured and nothing has been folded yet (folding allocates)."""
+    The entry also remembers the versions of the four tensors: an in-place update of any of them refolds, into the same
+    memory, which captured graphs go on reading. None while a CUDA graph is being captured and nothing has been folded yet
+    (folding allocates)."""
     owner = weight if weight._base is None else weight._base
     table = getattr(owner, _FOLDED_ATTR, None)
     if table is None:
         table = {}
         setattr(owner, _FOLDED_ATTR, table)
-    key = (weight.data_ptr(), norm_w.data_ptr(), norm_b.data_ptr(), bias.data_ptr())
+    key = (weight.data_ptr(), norm_w.data_ptr(), norm_b.data_ptr(), bias.data_ptr(), weight.shape)
     versions = (weight._version, norm_w._version, norm_b._version, bias._version)
     entry = table.get(key)
     if entry is not None and entry[0] == versions:
@@ -215,9 +216,9 @@ def _folded_layernorm(weight, norm_w, norm_b, bias):
     if torch.cuda.is_current_stream_capturing():
         return None
     K, N = weight.shape
-    folded = (torch.empty_like(weight, memory_format=torch.contiguous_format),
-              torch.empty(N, dtype=torch.float32, device=weight.device),
-              torch.empty(N, dtype=torch.float32, device=weight.device))
+    folded = entry[1] if entry is not None else (torch.empty_like(weight, memory_format=torch.contiguous_format),
+                                                 torch.empty(N, dtype=torch.float32, device=weight.device),
+                                                 torch.empty(N, dtype=torch.float32, device=weight.device))
     _lib.call("fvla_fold_layernorm", _chk("norm_w", norm_w, (K,)), _chk("norm_b", norm_b, (K,)), _chk("weight", weight),
               _chk("bias", bias, (N,)), folded[0].data_ptr(), folded[1].data_ptr(), folded[2].data_ptr(), N, K, _stream())
     table[key] = (versions, folded)
@@ -232,9 +233,9 @@ def _folded_layers(weight, norm_w, norm_b, bias):
     stacks = (weight, norm_w, norm_b, bias)
     versions = tuple(t._version for t in stacks)
     (w0, ws), (n0, ns), (s0, ss), (b0, bs) = ((t.data_ptr(), t.stride(0) * t.element_size()) for t in stacks)
-    layers = []
+    layers, shape = [], weight.shape[1:]
     for l in range(weight.shape[0]):
-        entry = table.get((w0 + l * ws, n0 + l * ns, s0 + l * ss, b0 + l * bs))
+        entry = table.get((w0 + l * ws, n0 + l * ns, s0 + l * ss, b0 + l * bs, shape))
         folded = entry[1] if entry is not None and entry[0] == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
         if folded is None:
             return None

@@ -19,6 +19,10 @@ episodes that share the weights:
 `batch_prefix=False` keeps the older form (E complete single-episode passes on E streams), whose
 per-episode results are bit-identical to the single-episode engine; the batched form runs the same
 per-row arithmetic but through differently shaped GEMM launches, so it agrees to rounding.
+
+The captured graph reads the tensors of `weights`, so an in-place update of one shows in the next `forward`. With up to four views in one
+SigLIP pass the exceptions are its QKV and FFN-up weights, biases and norms (five: QKV alone): there the graph reads copies with the norm
+folded in, which the next pass outside a graph over the same tensors, e.g. of a new engine, brings up to date in place.
 """
 from __future__ import annotations
 

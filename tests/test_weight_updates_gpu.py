@@ -37,3 +37,27 @@ def test_captured_batch_follows_updates_of_the_siglip_weights(views, episodes):
     for a, b, f in zip(after, before, fresh):
         assert not torch.equal(a, b), "the update does not show"
         assert torch.equal(a, f), "not what an engine captured after the update gives"
+
+
+def test_refolded_weights_reach_graphs_that_were_captured_before():
+    """Up to four views the graph reads folded copies: stale until a pass outside a graph folds again, then current, in the same memory."""
+    from flash_vla_b200 import Pi0Inference, random_checkpoint
+    weights = random_checkpoint(prompt_len=0, wscale=0.02, seed=0, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    inputs = ((torch.rand(1, 224, 224, 3, device="cuda", generator=gen) * 2 - 1).to(bf16),
+              torch.randn(32, device="cuda", generator=gen).to(bf16), torch.randn(10, 32, device="cuda", generator=gen).to(bf16))
+
+    def engine():
+        return Pi0Inference(weights, num_views=1, chunk_size=10, steps=1, layers=1)
+
+    def cache(e):
+        e.forward(*inputs)
+        return e.buffers["encoder_K"].clone()
+
+    captured = engine()
+    before = cache(captured)
+    for n in ("attn_qkv_w", "pre_attn_norm_b", "ffn_up_w", "pre_ffn_norm_w"):
+        weights["vision_" + n].mul_(1.25).add_(0.01)
+    fresh = cache(engine())                                  # its warm-up folds again
+    assert not torch.equal(fresh, before)
+    assert torch.equal(cache(captured), fresh)
