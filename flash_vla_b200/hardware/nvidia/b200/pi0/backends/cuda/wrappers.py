@@ -13,6 +13,7 @@ from __future__ import annotations
 import contextlib
 
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from flash_vla_b200.runtime.cuda import ScratchPool
 
@@ -197,31 +198,49 @@ def vision_norm_qkv(x, norm_w, norm_b, qkv_w, qkv_b, out, x_norm):
 _FOLDED_ATTR = "_fvla_folded_layernorm"
 
 
+class _Folded:
+    """Operands that `fvla_fold_layernorm` made of one LayerNorm + linear pair, and what they were made of."""
+    __slots__ = ("operands", "versions", "sources")
+
+    def __init__(self, operands, versions, sources):
+        self.operands, self.versions, self.sources = operands, versions, sources
+
+
+def _place(t: torch.Tensor):
+    """(storage, offset) of a tensor. Entries are found by these: while an entry holds a weak reference to a storage, no other can have its
+    number, whereas a freed tensor's address can be another tensor's the next moment."""
+    return t.untyped_storage()._cdata, t.storage_offset()
+
+
 def _folded_layernorm(weight, norm_w, norm_b, bias):
     """(weight_folded, colsum, bias_folded) of `fvla_fold_layernorm` for this LayerNorm + linear pair, made on first
-    use and kept ON the tensor that owns `weight`'s storage (found again through `view._base`, gone with it).
-    The entry also remembers the versions of the four tensors: an in-place update of any of them refolds, into the same
-    memory, which captured graphs go on reading. None while a CUDA graph is being captured and nothing has been folded yet
-    (folding allocates)."""
+    use and kept ON the tensor that owns `weight`'s storage (found again through `view._base`, gone with it or with the
+    norm's or the bias' storage). The entry also remembers the versions of the four tensors: an in-place update of any of them
+    refolds, into the same memory, which captured graphs go on reading. None while a CUDA graph is being captured and nothing has
+    been folded yet (folding allocates)."""
     owner = weight if weight._base is None else weight._base
     table = getattr(owner, _FOLDED_ATTR, None)
     if table is None:
         table = {}
         setattr(owner, _FOLDED_ATTR, table)
-    key = (weight.data_ptr(), norm_w.data_ptr(), norm_b.data_ptr(), bias.data_ptr(), weight.shape)
-    versions = (weight._version, norm_w._version, norm_b._version, bias._version)
+    sources = (weight, norm_w, norm_b, bias)
+    key = (*map(_place, sources), weight.shape)
+    versions = tuple(t._version for t in sources)
     entry = table.get(key)
-    if entry is not None and entry[0] == versions:
-        return entry[1]
+    if entry is not None and entry.versions == versions:
+        return entry.operands
     if torch.cuda.is_current_stream_capturing():
         return None
+    if entry is None:
+        for gone in [k for k, e in table.items() if any(ref.expired() for ref in e.sources)]:
+            del table[gone]
     K, N = weight.shape
-    folded = entry[1] if entry is not None else (torch.empty_like(weight, memory_format=torch.contiguous_format),
-                                                 torch.empty(N, dtype=torch.float32, device=weight.device),
-                                                 torch.empty(N, dtype=torch.float32, device=weight.device))
+    folded = entry.operands if entry is not None else (torch.empty_like(weight, memory_format=torch.contiguous_format),
+                                                       torch.empty(N, dtype=torch.float32, device=weight.device),
+                                                       torch.empty(N, dtype=torch.float32, device=weight.device))
     _lib.call("fvla_fold_layernorm", _chk("norm_w", norm_w, (K,)), _chk("norm_b", norm_b, (K,)), _chk("weight", weight),
               _chk("bias", bias, (N,)), folded[0].data_ptr(), folded[1].data_ptr(), folded[2].data_ptr(), N, K, _stream())
-    table[key] = (versions, folded)
+    table[key] = _Folded(folded, versions, tuple(StorageWeakRef(t.untyped_storage()) for t in sources))
     return folded
 
 
@@ -232,11 +251,11 @@ def _folded_layers(weight, norm_w, norm_b, bias):
     table = getattr(owner, _FOLDED_ATTR, {})
     stacks = (weight, norm_w, norm_b, bias)
     versions = tuple(t._version for t in stacks)
-    (w0, ws), (n0, ns), (s0, ss), (b0, bs) = ((t.data_ptr(), t.stride(0) * t.element_size()) for t in stacks)
+    (w0, ws), (n0, ns), (s0, ss), (b0, bs) = ((_place(t), t.stride(0)) for t in stacks)
     layers, shape = [], weight.shape[1:]
     for l in range(weight.shape[0]):
-        entry = table.get((w0 + l * ws, n0 + l * ns, s0 + l * ss, b0 + l * bs, shape))
-        folded = entry[1] if entry is not None and entry[0] == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
+        entry = table.get(((w0[0], w0[1] + l * ws), (n0[0], n0[1] + l * ns), (s0[0], s0[1] + l * ss), (b0[0], b0[1] + l * bs), shape))
+        folded = entry.operands if entry is not None and entry.versions == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
         if folded is None:
             return None
         layers.append(folded)

@@ -42,3 +42,41 @@ def test_refolding_writes_where_captured_graphs_read(folds, which):
     again = [wrappers._folded_layernorm(*single)] + wrappers._folded_layers(*stacked)
     assert [tuple(t.data_ptr() for t in f) for f in again] == held
     assert folds == held + held
+
+
+def test_a_norm_in_memory_that_an_earlier_one_had_is_folded(folds):
+    """Entries are not found by address: a tensor that took over a freed one's memory, at the same version, is another tensor."""
+    arena = torch.empty(1 << 16, dtype=torch.uint8)
+
+    def at(offset, value):                                   # a tensor of its own storage at a given address
+        import ctypes
+        t = torch.frombuffer((ctypes.c_char * (2 * K)).from_address(arena.data_ptr() + offset), dtype=bf16)
+        arena[offset:offset + 2 * K].view(bf16).fill_(value)
+        return t
+    w, _, nb, b = pair()
+    first = at(0, 1.0)
+    wrappers._folded_layernorm(w, first, nb, b)
+    wrappers._folded_layernorm(w, first, nb, b)
+    assert len(folds) == 1
+    address, version = first.data_ptr(), first._version
+    del first
+    second = at(0, 2.0)
+    assert (second.data_ptr(), second._version) == (address, version)
+    wrappers._folded_layernorm(w, second, nb, b)
+    assert len(folds) == 2
+
+
+def test_folds_of_norms_that_are_gone_are_given_back(folds):
+    w, _, nb, b = pair()
+    for _ in range(5):
+        wrappers._folded_layernorm(w, torch.randn(K).to(bf16), nb, b)
+    assert len(getattr(w, wrappers._FOLDED_ATTR)) == 1
+
+
+def test_folds_are_found_through_views_of_one_storage(folds):
+    """Slices made anew on every call, a stack's layers and its own slices, and `data` are the same weights."""
+    stacks = pair((L,))
+    first = wrappers._folded_layers(*stacks)
+    for l in range(L):
+        assert wrappers._folded_layernorm(*(t[l] for t in stacks)) is first[l]
+    assert all(a is f for a, f in zip(wrappers._folded_layers(*stacks), first)) and len(folds) == L
