@@ -200,10 +200,25 @@ _FOLDED_ATTR = "_fvla_folded_layernorm"
 
 class _Folded:
     """Operands that `fvla_fold_layernorm` made of one LayerNorm + linear pair, and what they were made of."""
-    __slots__ = ("operands", "versions", "sources")
+    __slots__ = ("operands", "versions", "sources", "stream", "recorded")
 
     def __init__(self, operands, versions, sources):
         self.operands, self.versions, self.sources = operands, versions, sources
+        self.stream, self.recorded = _stream(), _fold_recorded()
+
+    def ready(self):
+        """The operands, behind the fold on whichever stream is current. (A capture cannot wait for work outside it; what it reads has to have
+        run before it begins.)"""
+        if self.recorded is not None and _stream() != self.stream and not torch.cuda.is_current_stream_capturing():
+            if self.recorded.query():
+                self.recorded = None
+            else:
+                self.recorded.wait()
+        return self.operands
+
+
+def _fold_recorded():
+    return torch.cuda.current_stream().record_event()
 
 
 def _place(t: torch.Tensor):
@@ -228,7 +243,7 @@ def _folded_layernorm(weight, norm_w, norm_b, bias):
     versions = tuple(t._version for t in sources)
     entry = table.get(key)
     if entry is not None and entry.versions == versions:
-        return entry.operands
+        return entry.ready()
     if torch.cuda.is_current_stream_capturing():
         return None
     if entry is None:
@@ -255,7 +270,7 @@ def _folded_layers(weight, norm_w, norm_b, bias):
     layers, shape = [], weight.shape[1:]
     for l in range(weight.shape[0]):
         entry = table.get(((w0[0], w0[1] + l * ws), (n0[0], n0[1] + l * ns), (s0[0], s0[1] + l * ss), (b0[0], b0[1] + l * bs), shape))
-        folded = entry.operands if entry is not None and entry.versions == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
+        folded = entry.ready() if entry is not None and entry.versions == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
         if folded is None:
             return None
         layers.append(folded)
