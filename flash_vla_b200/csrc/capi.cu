@@ -838,16 +838,20 @@ int fvla_decoder_steps_run(const struct fvla_decoder_steps* d, void* stream) {
 // 8 or 4 bytes per 32 columns, which the next epilogue warps fetch while their MMAs run. Prefix pass, same kernels otherwise: one view 2.77 -> 2.57 ms,
 // three 4.35 -> 4.24, prompt 48 4.92 -> 4.81; two, four, eight episodes' forward 0.4, 0.5, 1.0 ms shorter (a batch's attention in one launch
 // among it). Error of the SigLIP QKV projection against 64 bits: 2.28e-3 with the sums, 2.35e-3 behind a row-norm kernel.
+// What a stage returns once it has launched anything: FVLA_ERR_UNSUPPORTED promises that nothing was.
+static int begun(int rc) { return rc == FVLA_ERR_UNSUPPORTED ? FVLA_ERR_LAUNCH : rc; }
+
 int fvla_row_sums_supported(int M) { return tc5_enabled() && M > 64 && g_plan_count.load(std::memory_order_acquire) == 0 ? 1 : 0; }
 
 int fvla_vision_tower_run(const struct fvla_vision_tower* t, void* stream) {
     constexpr int D = 1152, F = 4304, HEADS = 16, HD = 72, TOK = 256;
     FVLA_REQUIRE(t != nullptr && t->views >= 1 && t->views <= (1 << 16) && t->layers >= 0, "vision_tower: bad shape");
     const int M = t->views * TOK;
-    bool fits = fvla_row_sums_supported(M) && aligned16(t->x) && aligned16(t->qkv) && aligned16(t->attn) && aligned16(t->hidden) && aligned16(t->row_sums) &&
-                aligned16(t->ws_patch) && aligned16(t->patch_w) && aligned16(t->patch_b) && aligned16(t->pos_emb) && aligned16(t->o_w) && aligned16(t->o_b) &&
-                aligned16(t->down_w) && aligned16(t->down_b);
-    for (int l = 0; l < t->layers && fits; ++l) fits = aligned16(t->qkv_folded[l]) && aligned16(t->up_folded[l]);
+    const void* used[] = {t->images, t->patch_w, t->patch_b, t->pos_emb, t->o_w, t->o_b, t->down_w, t->down_b, t->x, t->qkv, t->attn, t->hidden, t->row_sums, t->ws_patch};
+    bool fits = fvla_row_sums_supported(M) && (t->layers == 0 || (t->qkv_folded && t->qkv_colsum && t->qkv_bias && t->up_folded && t->up_colsum && t->up_bias));
+    for (const void* p : used) fits = fits && p != nullptr && aligned16(p);
+    for (int l = 0; l < t->layers && fits; ++l)
+        fits = t->qkv_folded[l] && t->qkv_colsum[l] && t->qkv_bias[l] && t->up_folded[l] && t->up_colsum[l] && t->up_bias[l] && aligned16(t->qkv_folded[l]) && aligned16(t->up_folded[l]);
     if (!fits) { set_error("vision_tower: not with these kernels, plans or addresses"); return FVLA_ERR_UNSUPPORTED; }
     float* sums = static_cast<float*>(t->row_sums);
     int rc = patch_embed(t->images, t->patch_w, t->patch_b, t->pos_emb, t->x, sums, t->views, t->ws_patch, t->ws_patch_bytes, stream);
@@ -858,7 +862,7 @@ int fvla_vision_tower_run(const struct fvla_vision_tower* t, void* stream) {
         if (!rc) rc = folded_norm_linear(t->x, sums, t->up_folded[l], t->up_colsum[l], t->up_bias[l], t->hidden, M, F, D, 1, stream);
         if (!rc) rc = linear_with_sums(t->hidden, B(t->down_w) + (size_t)l * F * D, B(t->down_b) + (size_t)l * D, t->x, sums, 0, M, D, F, t->ws_down, t->ws_down_bytes, stream);
     }
-    return rc;
+    return begun(rc);
 }
 
 // A batch beyond 128 rows: QKV and gated FFN are general GEMMs, each behind a row-norm kernel of 4 us of the layer-step's 62 (eight episodes) until
@@ -906,7 +910,7 @@ int fvla_decoder_batch_layers_run(const struct fvla_decoder_batch_layers* d, voi
         }
         if (!rc) rc = linear_residual(d->hidden, B(d->down_w) + (size_t)l * FFN * W, d->x, 1, d->x_shadow, sums, M, W, FFN, d->tokens, nullptr, 0, stream);
     }
-    return rc;
+    return begun(rc);
 }
 
 int fvla_encoder_layers_run(const struct fvla_encoder_layers* e, void* stream) {
@@ -948,7 +952,7 @@ int fvla_encoder_layers_run(const struct fvla_encoder_layers* e, void* stream) {
             rc = tc5::launch_gemm_tc5_normed(a, device_status_ptr(), S(stream));
         }
     }
-    return rc;
+    return begun(rc);
 }
 
 int fvla_embed_rows(const void* table, const long long* ids, void* out, int rows, int dim, long long vocab, void* stream) {

@@ -236,7 +236,8 @@ int fvla_decoder_steps_run(const struct fvla_decoder_steps* args, void* stream);
  * attention, output projection + residual, LayerNorm + FFN up, FFN down + residual, in place on x (views * 256, 1152). The kernels
  * that write x leave their rows' sums and sums of squares in row_sums (views * 256 * 72 floats), from which the projections
  * behind them take the LayerNorm, folded into weights as by fvla_fold_layernorm: arrays of `layers` pointers each. Stacked
- * weights otherwise. FVLA_ERR_UNSUPPORTED, with nothing launched, where fvla_row_sums_supported(views * 256) is 0. */
+ * weights otherwise. FVLA_ERR_UNSUPPORTED, with nothing launched, where fvla_row_sums_supported(views * 256) is 0 and for null or misaligned
+ * pointers, those in the arrays among them. */
 struct fvla_vision_tower {
     const void *images, *patch_w, *patch_b, *pos_emb, *o_w, *o_b, *down_w, *down_b;
     const void* const* qkv_folded;

@@ -62,3 +62,29 @@ assert encoder() == 0
 @pytest.mark.parametrize("env,one,several", [({"FVLA_GEMM": "mma"}, -4, -4), ({"FVLA_ATTN": "mma"}, 0, -4)])
 def test_kernels_switched_off(env, one, several):
     probe(f"assert encoder() == {one} and encoder(sequences=2) == {several}", **env)
+
+
+LAYERS = """
+def arrays(layers=2, **change):
+    f = {n: (ctypes.c_void_p * layers)(*([P] * layers)) for n in ("qkv_folded", "qkv_colsum", "qkv_bias", "up_folded", "up_colsum", "up_bias")}
+    f.update(change)
+    return dict(layers=layers, **{n: a if a is None else ctypes.addressof(a) for n, a in f.items()}), f
+"""
+
+
+def test_tower_refuses_null_pointers():
+    """As the other two stages do: before anything is launched, let alone read through the pointer."""
+    probe(LAYERS + """
+given, keep = arrays()
+for n in ("images", "patch_w", "patch_b", "pos_emb", "o_w", "o_b", "down_w", "down_b", "x", "qkv", "attn", "hidden", "row_sums", "ws_patch"):
+    assert tower(**given, **{n: None}) == -4, n
+""")
+
+
+def test_tower_refuses_null_arrays_and_entries():
+    probe(LAYERS + """
+for n in ("qkv_folded", "qkv_colsum", "qkv_bias", "up_folded", "up_colsum", "up_bias"):
+    for broken in ((ctypes.c_void_p * 2)(P, None), None):
+        given, keep = arrays(**{n: broken})
+        assert tower(**given) == -4, n
+""")
