@@ -558,7 +558,7 @@ static ResidualPlan plan_residual(int M, int N, int K, int group_rows) {
     return {rows, groups, parts, tc5_enabled() && !general && skinny::skinny_supports(rows, N, K / parts, false, true, -1)};
 }
 
-// row_sums: sums of squares of the new rows, written where the cluster GEMM takes the shape.
+// row_sums: sums of squares of the new rows; an error where the cluster GEMM does not take the shape.
 static int linear_residual(const void* x, const void* weight, void* out, int out_is_f32, void* out_shadow, float* row_sums, int M,
                            int N, int K, int group_rows, void* ws, size_t ws_bytes, void* stream) {
     FVLA_REQUIRE(M > 0 && N > 0 && K > 0, "linear_residual: empty shape %dx%dx%d", M, N, K);
@@ -580,6 +580,7 @@ static int linear_residual(const void* x, const void* weight, void* out, int out
         }
         return FVLA_OK;
     }
+    if (row_sums != nullptr) { set_error("linear_residual: %dx%dx%d in groups of %d rows leaves no row sums", M, N, K, group_rows); return FVLA_ERR_UNSUPPORTED; }
     FVLA_REQUIRE(out_shadow == nullptr || out_is_f32, "linear_residual: a bf16 shadow only makes sense for an fp32 `out`");
     GemmArgs a;
     a.A = B(x); a.lda = K; a.B = B(weight); a.ldb = N; a.C = out; a.ldc = N; a.c_f32 = out_is_f32;

@@ -339,6 +339,7 @@ inline int launch_gemm_cfg(const GemmArgs& a, dim3 grid, cudaStream_t st) {
 
 // Validates, plans and launches. `ws` is only needed when the plan uses split-K.
 inline int launch_gemm_mma(GemmArgs a, void* ws, size_t ws_bytes, cudaStream_t st) {
+    if (a.row_sums != nullptr || a.in_sums != nullptr) { set_error("mma gemm: no row sums (%dx%dx%d)", a.M, a.N, a.K); return FVLA_ERR_UNSUPPORTED; }
     const bool dual = a.B2 != nullptr;
     if (a.Kb == 0) a.Kb = a.K;
     if (a.M <= 0 || a.N <= 0 || a.K <= 0) { set_error("gemm: empty shape %dx%dx%d", a.M, a.N, a.K); return FVLA_ERR_ARG; }

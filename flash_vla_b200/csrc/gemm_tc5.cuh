@@ -941,6 +941,11 @@ inline Tc5Plan plan_tc5(int M, int N, int K, bool ws_ok) {
 template <int BN, bool DUAL, int STAGES, bool ROPE, bool CLUSTER, int NORM, int EP>
 inline int launch_tc5_ep(const GemmArgs& g, int* status, cudaStream_t st, int splits, void* ws) {
     using Cfg = Tc5Cfg<BN, DUAL, STAGES>;
+    // Sums that this form does not write or take are an error: the next projection would go by those of another layer.
+    if ((g.row_sums != nullptr && (EP == EP_ANY || !(EP & EP_RES) || g.N % 32)) || (g.in_sums != nullptr && (NORM != 2 || g.K % (ROPE || DUAL ? 256 : 128)))) {
+        set_error("tc5 gemm: no row sums in this form (%dx%dx%d)", g.M, g.N, g.K);
+        return FVLA_ERR_UNSUPPORTED;
+    }
     auto kern = tc5_gemm_kernel<BN, DUAL, STAGES, ROPE, CLUSTER, NORM, EP>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
@@ -1122,7 +1127,6 @@ inline int normed_tile_width(int M, int N, int K, bool rope) {
 
 template <int BN, int STAGES>
 inline int launch_tc5_normed_width(const GemmArgs& g, int* status, cudaStream_t st) {
-    if (g.in_sums != nullptr && g.K % (g.rope != nullptr ? 256 : 128)) return FVLA_ERR_UNSUPPORTED;
     if (g.in_sums != nullptr)
         return g.rope != nullptr ? launch_tc5_cfg<BN, false, STAGES, true, false, 2>(g, status, st) : launch_tc5_cfg<BN, false, STAGES, false, false, 2>(g, status, st);
     return g.rope != nullptr ? launch_tc5_cfg<BN, false, STAGES, true, false, 1>(g, status, st) : launch_tc5_cfg<BN, false, STAGES, false, false, 1>(g, status, st);

@@ -426,6 +426,10 @@ inline PairPlan plan_pair_plain(int M, int N, int K, bool ws_ok) {
 
 template <bool DUAL, bool NORM = false>
 inline int launch_pair(const GemmArgs& g, int splits, void* ws, int* status, cudaStream_t st) {
+    if ((g.row_sums != nullptr && (DUAL || g.c_f32 || g.N % 32)) || (g.in_sums != nullptr && (!NORM || g.K % 128))) {      // (see the one-SM kernel)
+        set_error("pair gemm: no row sums in this form (%dx%dx%d)", g.M, g.N, g.K);
+        return FVLA_ERR_UNSUPPORTED;
+    }
     auto kern = tc5x2_gemm_kernel<DUAL, NORM>;
     static PerDeviceFlag configured;
     if (!configured.get()) {
