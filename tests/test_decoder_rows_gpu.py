@@ -176,3 +176,24 @@ def test_batched_decoder_attention_behind_the_kernel_that_writes_its_prefix(epis
             torch.cuda.synchronize()
         ops.decoder_attention(q, *caches, None, out, S)
     assert torch.equal(*results)
+
+
+# a batch's QKV projection behind its row-norm kernel: 128-wide tiles in one round (153 and 867 rows), 256-wide ones beyond 896 rows (918, a ragged last tile)
+@pytest.mark.parametrize("episodes,tokens", [(3, 51), (17, 51), (18, 51), (9, 127)])
+def test_batched_qkv_projection_by_tile_width(episodes, tokens):
+    from flash_vla_b200 import op_table
+    M, skip = episodes * tokens, 3
+    g = torch.Generator().manual_seed(M)
+    # Rows rounded to bf16: 1.1e-3 of the rms in a projection's result, and under a rotation, 5.3 standard deviations of it (6e-3) in the
+    # largest of two million, and half an ulp (4e-3 of the value) for the result's own rounding: inside the default bound. (A table of normal
+    # variates instead of a rotation stretches rows by up to five and does not meet it.)
+    x, w, rope = torch.randn(M, 1024, generator=g), rnd(g, 1024, 2560, scale=0.02), O.rope_table(tokens, 24)
+    Q, K, V = (torch.zeros(*s, 256, dtype=bf16, device="cuda") for s in ((M * 8,), (episodes, skip + tokens), (episodes, skip + tokens)))
+    op_table(True).decoder_norm_qkv_rope(x.cuda(), w.cuda(), rope.cuda(), Q, K[:, skip:], V[:, skip:], torch.zeros(M, dtype=bf16, device="cuda"))
+    for e in (0, episodes - 1):
+        r = slice(e * tokens, (e + 1) * tokens)
+        ref = torch.zeros(tokens * 8, 256), torch.zeros(tokens, 256), torch.zeros(tokens, 256)
+        O.op_table(False).decoder_norm_qkv_rope(x[r].clone(), w.float(), rope.float(), *ref, torch.zeros(tokens))
+        for got, want, what in zip((Q[r.start * 8:r.stop * 8], K[e, skip:], V[e, skip:]), ref, "QKV"):
+            assert_close(got, want, what=f"{what} of episode {e}")
+    assert not K[:, :skip].any() and not V[:, :skip].any()
