@@ -10,7 +10,7 @@ their static buffers and replays. Public surface and life cycle follow the refer
 episodes that share the weights:
   * SigLIP and the prefix encoder run ONCE over all episodes' tokens (M = E x S rows): every vision and
     prefix weight (4.8 of the 5.4 GB) is streamed once for the whole batch and the GEMMs have E times
-    the tiles to fill the GPU with; only the attention kernels, which mix tokens, run per episode;
+    the tiles to fill the GPU with; attention, which mixes tokens, keeps the episodes apart inside one launch;
   * each episode has its own KV cache; the action-expert decoder also runs over several episodes' rows at once: one
     or two groups of episodes (`decoder_groups`) on streams of their own, where they fill each other's idle SMs. Every
     projection runs once over a group's rows, attention for all its episodes in one launch. With `batch_decoder=False` the decoders
@@ -108,7 +108,7 @@ class Pi0Inference:
         if batch_decoder is None:
             batch_decoder = episodes >= 2
         self.batch_decoder = self.batch_prefix and bool(batch_decoder)
-        self.prefix_buffers, self.prefix_pool, self.decoder_groups, self.streams = None, None, [], []
+        self.prefix_buffers, self.prefix_pool, self.decoder_groups, self.streams, self.attention_streams = None, None, [], [], []
         if self.batch_prefix:
             self.prefix_buffers, self.episode_buffers, self.encoder_seq_len = allocate_batched_buffers(
                 num_views, chunk_size, self.prompt_len, episodes, device)
@@ -217,20 +217,20 @@ class Pi0Inference:
             main.wait_stream(side)
 
     def _attention_fork(self):
-        """`per_episode` hook of the batched prefix encoder: episode e's attention goes to a stream of its own,
-        forked from the current stream; the call with None joins them all back."""
+        """`per_episode` hook of the batched prefix encoder where it goes op by op: episode e's attention goes to a stream of its own,
+        made on first use and forked from the current stream; the call with None joins them all back."""
         import contextlib
         import os
         if "mma" in (os.environ.get("FVLA_ATTN"), os.environ.get("FVLA_GEMM")):
             return None      # the warp-level fallback shares one split-K scratch between the episodes: keep it serial
         main = torch.cuda.current_stream()
-        if not hasattr(self, "_attn_streams"):
-            self._attn_streams = [torch.cuda.Stream(device=main.device) for _ in range(self.episodes)]
         used = []
 
         @contextlib.contextmanager
         def on_stream(e):
-            stream = self._attn_streams[e]
+            if not self.attention_streams:
+                self.attention_streams = [torch.cuda.Stream(device=main.device) for _ in range(self.episodes)]
+            stream = self.attention_streams[e]
             stream.wait_stream(main)
             used.append(stream)
             with torch.cuda.stream(stream):

@@ -89,11 +89,11 @@ def transformer_encoder_batched(ops, weights, buffers, encoder_seq_len, num_view
                                 per_episode=None):
     """The prefix encoder over `episodes` sequences of `encoder_seq_len` tokens laid end to end in the batched
     buffers (`allocate_batched_buffers`): every projection runs once over all rows, so its weights are
-    streamed once for the whole batch; attention, which mixes tokens, runs per episode. K / V of layer L go
-    straight into rows [0, S) of every episode's cache. Same ops and call order per layer as
-    `transformer_encoder`. `per_episode(e)`, if given, returns a context manager under which episode e's
-    attention is enqueued (the engine uses it to put the episodes' attention launches, 48 CTAs each, side by
-    side on streams of their own) and `per_episode(None)` is called once after the last episode to join."""
+    streamed once for the whole batch. Attention, which mixes tokens, is one launch over the sequences in the native
+    layers (the table's `encoder_layers`) and one per episode where the ops go one by one. K / V of layer L go straight into rows [0, S) of every
+    episode's cache. Same ops and call order per layer as `transformer_encoder`. `per_episode(e)`, if given, returns a context
+    manager under which episode e's own attention launch is enqueued (the engine uses it to put these, 96 CTAs each, on
+    streams of their own) and `per_episode(None)` is called once after the last episode to join; neither is called by the native layers."""
     import contextlib
     w, b, S, E = weights, buffers, encoder_seq_len, episodes
     x = b["encoder_x"]

@@ -334,6 +334,29 @@ def test_episodes_in_one_decoder_group(full_checkpoint, episodes):
     torch.cuda.empty_cache()
 
 
+def test_batched_prefix_op_by_op(full_checkpoint):
+    """With a launch plan pinned, whatever its shape, the prefix stages go op by op: attention per episode on streams that no other engine
+    makes. Same bound as between one group and single episodes above."""
+    from flash_vla_b200 import Pi0Inference
+    from flash_vla_b200.hardware.nvidia.b200.pi0.backends.cuda import _lib
+    E = 3
+    inputs = [torch.stack([bench_inputs(seed=e)[i] for e in range(E)]) for i in range(3)]
+    results = []
+    for pinned in (False, True):
+        if pinned:
+            _lib.call("fvla_gemm_plan_set", 777, 2048, 2048, 0, 1, 128, 1)
+        try:
+            engine = Pi0Inference(full_checkpoint, num_views=3, chunk_size=50, steps=2, layers=2, episodes=E)
+        finally:
+            if pinned:
+                _lib.call("fvla_gemm_plan_clear")
+        results.append(engine.forward(*inputs).float().cpu())
+        assert len(engine.attention_streams) == (E if pinned else 0)
+        del engine
+        torch.cuda.empty_cache()
+    assert (results[0] - results[1]).abs().max().item() <= 2 * STEP_MAX_ABS + 2.0 ** -8 * results[0].abs().max().item()
+
+
 def test_two_devices_in_one_process(full_checkpoint):
     """One process driving two GPUs: kernel attributes, SM counts and the status word are per device, so
     the second engine must work as well as the first and both must match the fixture."""
