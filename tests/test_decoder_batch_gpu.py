@@ -67,8 +67,8 @@ def test_decoder_batch_layers(episodes, tokens):
         for c, before in zip((caches["encoder_K"], caches["encoder_V"]), kv):
             assert torch.equal(c[:, :, :S], before[:, :, :S]), "prefix rows are not written"
         results.append(seen)
-    # Operands rounded to bf16 on both sides (2^-9 / sqrt(3) = 1.1e-3 rms each, different values): up to twelve such roundings through
-    # three layers are 4e-3 per side, 5.5e-3 between them; twice that
+    # Operands rounded to bf16 on both sides (1.66e-3 each for normal variates, different values): up to twelve such roundings through
+    # three layers are 5.8e-3 per side, 8.1e-3 between them; a third more
     for n, got in results[0].items():
         assert_near(got, results[1][n], n, 1.1e-2)
 

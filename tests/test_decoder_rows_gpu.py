@@ -184,7 +184,7 @@ def test_batched_qkv_projection_by_tile_width(episodes, tokens):
     from flash_vla_b200 import op_table
     M, skip = episodes * tokens, 3
     g = torch.Generator().manual_seed(M)
-    # Rows rounded to bf16: 1.1e-3 of the rms in a projection's result, and under a rotation, 5.3 standard deviations of it (6e-3) in the
+    # Rows rounded to bf16: 1.7e-3 of the rms in a projection's result, and under a rotation, 5.3 standard deviations of it (9e-3) in the
     # largest of two million, and half an ulp (4e-3 of the value) for the result's own rounding: inside the default bound. (A table of normal
     # variates instead of a rotation stretches rows by up to five and does not meet it.)
     x, w, rope = torch.randn(M, 1024, generator=g), rnd(g, 1024, 2560, scale=0.02), O.rope_table(tokens, 24)

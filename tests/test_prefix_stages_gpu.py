@@ -20,8 +20,8 @@ def rnd(gen, *shape, scale=1.0):
 
 
 def assert_near(got, ref, what):
-    """Relative 2-norm. A result behind up to ten bf16 roundings (2^-9 / sqrt(3) = 1.13e-3 rms each, operands and stored activations) is
-    3.6e-3 from the exact one, two such results are 5e-3 from one another; twice that is allowed."""
+    """Relative 2-norm. A result behind up to ten bf16 roundings (1.66e-3 each for normal variates, operands and stored activations) is
+    5.2e-3 from the exact one, two such results are 7.4e-3 from one another; a third more is allowed."""
     got, ref = got.double(), ref.double().to(got.device)
     assert torch.isfinite(got).all(), what
     dist = ((got - ref).norm() / ref.norm()).item()
