@@ -179,9 +179,15 @@ def decoder_batch_layers(weights, caches, buffers, encoder_seq_len, episodes, la
     ws_bytes = _lib.gemm_workspace_bytes(M, _QKV, _WIDTH, 0)
     attn_bytes = _lib.load().fvla_decoder_attention_workspace_bytes(D * _w.DECODER_HEADS, S + D)
     roles = (("dec_row_sums", (M * (_WIDTH // 32),), torch.float32), ("dec_qkv_ws", (ws_bytes,), torch.uint8), ("dec_attn_ws", (attn_bytes,), torch.uint8))
+    # and what the ops take that these layers do not need: a pool warmed up by the stage serves the ops too, should a later pass go op by op
+    spare = tuple((f"dec_{n}_ws", (_lib.gemm_workspace_bytes(M, N, Kd, dual),), torch.uint8)
+                  for n, N, Kd, dual in (("o", _WIDTH, _Q, 0), ("gate", _FFN, _WIDTH, 1), ("down", _WIDTH, _FFN, 0)))
     if not all(_w.scratch_covers(*r, x.device) for r in roles):
         return None
     sums, ws, ws_attn = (_w.scratch(*r, x.device) for r in roles)
+    for role in spare:
+        if _w.scratch_covers(*role, x.device):
+            _w.scratch(*role, x.device)
     args = _lib.DecoderBatchLayers(
         x=x.data_ptr(), x_shadow=_w._shadow_of(x) or shadow.data_ptr(), k_cache=K.data_ptr(), v_cache=V.data_ptr(), row_sums=sums.data_ptr(),
         ws_qkv=ws.data_ptr(), ws_qkv_bytes=ws_bytes, ws_attn=ws_attn.data_ptr(), ws_attn_bytes=attn_bytes, layer_stride=(S + D) * hd, episode_stride=K.shape[1] * (S + D) * hd, episodes=episodes, tokens=D,

@@ -87,7 +87,7 @@ def test_tower(views, stay, monkeypatch):
 
 
 # ragged and whole row tiles of 128 and 256; K split in clusters, in pairs through scratch, not at all; one sequence and several
-@pytest.mark.parametrize("rows,sequences", [(257, 1), (273, 1), (768, 1), (817, 1), (1124, 1), (273, 3), (816, 4), (768, 8)])
+@pytest.mark.parametrize("rows,sequences", [(65, 1), (128, 1), (129, 1), (257, 1), (273, 1), (768, 1), (817, 1), (1124, 1), (273, 3), (816, 4), (768, 8)])
 @pytest.mark.parametrize("stay", [True, False])
 def test_encoder(rows, sequences, stay):
     from flash_vla_b200 import op_table
