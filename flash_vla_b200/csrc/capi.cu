@@ -170,6 +170,8 @@ static bool pair_enabled() {
 // K = 2 048, N = 16 384, row norm included, pairs against single SMs: 3 row tiles (257 to 384 rows) 53.4 / 50.3 to 56.3 / 52.7 us, 3 rounds instead
 // of 4; 5 row tiles 76.1 / 76.0 to 81.6 / 83.0, which stay on pairs; 2, 4, 6 and 7 row tiles 4 to 15 us in favour of pairs. (One
 // row tile is the single-SM kernel's whatever this says: the pair kernel takes more than 128 rows.)
+// With the norm from handed-down sums in place of the row-norm kernel, a whole prefix layer, pairs less single SMs: 2 row tiles -4.2 us, 3 +3.0 to +4.5, 4 -6.9 to
+// -10.0, 5 +1.4 to +2.7 (of 170), 6 -12.4, 7 -8.3 to -12.1, 8 -12.4, 9 -2.0 to -3.4, 10 -16.3: at five, 1 % behind, the other form would do better.
 static bool geglu_on_pairs(int M, int N, int K) {
     const int sms = tc5::num_sms(), tiles_n = (N + 127) / 128, k_iters = (K + 63) / 64;
     const int pair_rounds = ((M + 255) / 256 * tiles_n + sms / 2 - 1) / (sms / 2), rounds = ((M + 127) / 128 * tiles_n + sms - 1) / sms;
@@ -836,9 +838,10 @@ int fvla_decoder_steps_run(const struct fvla_decoder_steps* d, void* stream) {
 // Without the sums every projection behind a norm either re-reads its operand stages for them (16 KB more shared-memory traffic per
 // k step: SigLIP QKV 12.2 us at 768 rows against 10.9) or, where a CTA has several tiles and in the gated FFN, stands behind a row-norm kernel of its own
 // (4 to 13 us at 768 to 6 144 rows). The residual projections hold every value of a row in registers anyway; what they leave is
-// 8 or 4 bytes per 32 columns, which the next epilogue warps fetch while their MMAs run. Prefix pass, same kernels otherwise: one view 2.77 -> 2.57 ms,
-// three 4.35 -> 4.24, prompt 48 4.92 -> 4.81; two, four, eight episodes' forward 0.4, 0.5, 1.0 ms shorter (a batch's attention in one launch
-// among it). Error of the SigLIP QKV projection against 64 bits: 2.28e-3 with the sums, 2.35e-3 behind a row-norm kernel.
+// 8 or 4 bytes per 32 columns, which the next epilogue warps fetch while their MMAs run. Forwards, the ops one by one / as a stage: SigLIP, one view 6.96 / 6.84 ms, three
+// 8.34 / 8.25 (more views go by op: their weights are read live); prefix encoder, one view 6.91 / 6.84, four episodes of three views 22.26 / 21.98,
+// eight 35.78 / 35.49 (a batch's attention in one launch among it), two and five no difference. Error of the SigLIP QKV projection against 64 bits: 2.28e-3 with the sums, 2.35e-3
+// behind a row-norm kernel; of the prefix K / V caches at sixteen shapes of 1 to 8 episodes 1.01e-2 to 1.13e-2, 1.09e-2 to 1.21e-2 with normalised rows rounded.
 // What a stage returns once it has launched anything: FVLA_ERR_UNSUPPORTED promises that nothing was.
 static int begun(int rc) { return rc == FVLA_ERR_UNSUPPORTED ? FVLA_ERR_LAUNCH : rc; }
 
@@ -867,8 +870,8 @@ int fvla_vision_tower_run(const struct fvla_vision_tower* t, void* stream) {
 }
 
 // A batch beyond 128 rows: QKV and gated FFN are general GEMMs, each behind a row-norm kernel of 4 us of the layer-step's 62 (eight episodes) until
-// the residual projections, whose owners hold the new rows in registers, left their sums of squares for them. Forward of eight episodes 37.16 -> 36.24 ms,
-// of one camera each 18.64 -> 18.2, five episodes 25.5 -> 25.0.
+// the residual projections, whose owners hold the new fp32 rows in registers, left their sums of squares for them. Forwards, by op / as a stage: eight episodes
+// 35.76 / 35.49 ms, of one camera each 17.81 / 17.65, five episodes 25.83 / 24.76.
 int fvla_decoder_batch_supported(int episodes, int tokens) {
     if (episodes < 2 || tokens < 1 || tokens > 128 || (long long)episodes * tokens <= 128 || episodes > (1 << 16)) return 0;
     const int M = episodes * tokens;

@@ -320,11 +320,11 @@ skinny_gemm_kernel(const SkinnyArgs p, const __grid_constant__ CUtensorMap tmW, 
     };
     FVLA_STAMP(2);
 
-    // 64 slots: one thread adds up all k-blocks in order in one accumulator, so that a product is a single fp32 sum over the CTA's
+    // Up to 64 slots: one thread adds up all k-blocks in order in one accumulator, so that a product is a single fp32 sum over the CTA's
     // K slice from front to back, whatever issues it (decodes of several steps amplify a changed order of summation). Its warp
     // waits for all k-blocks at once, a lane each: they land within 0.1 us of one another, and waits in between take longer. MMAs
     // done after the X tile, at 51 rows: QKV 0.87 us, o 0.87, gate / up 1.9, down 1.3 (two threads with an accumulator each 0.92, 0.87, 2.4, 1.7).
-    // 128 slots: two threads issue the k-blocks in turn, each into an accumulator of its own.
+    // Beyond 64 slots: two threads issue the k-blocks in turn, each into an accumulator of its own.
     constexpr uint32_t idesc = skinny_idesc(TOK);
     const uint64_t ad = smem_desc(sW, 8192, 1024), bd = smem_desc(sX, 16, 1024);
     auto issue_block = [&](int slot, uint32_t acc, bool first) {
@@ -598,7 +598,7 @@ inline int launch_skinny_cfg(SkinnyArgs a, const SkinnyPlan& pl, const void* W, 
         set_error("skinny gemm: row groups are only built for the bias / residual forms with a bf16 operand");
         return FVLA_ERR_UNSUPPORTED;
     }
-    if (TOK != 64 && a.x_f32 && a.x_shadow == nullptr) { set_error("skinny gemm: more than 64 rows need a bf16 operand"); return FVLA_ERR_UNSUPPORTED; }
+    if (TOK != 64 && a.x_f32 && a.x_shadow == nullptr) { set_error("skinny gemm: fp32 rows without a bf16 copy take the 64-slot form only (%d slots)", TOK); return FVLA_ERR_UNSUPPORTED; }
     auto kern = skinny_gemm_kernel<EPI, TOK, S>;
     static PerDeviceFlag configured;
     if (!configured.get()) {

@@ -48,8 +48,8 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-// True in one lane of a converged warp. The compiler keeps a block behind it free of the moves to uniform registers that it puts
-// before every tcgen05 instruction behind `lane == 0`: 50 clk less per MMA in the decoder's cluster GEMM.
+// True in one lane of a converged warp. An issue loop behind it takes 50 clk less per MMA than behind `lane == 0` (decoder's cluster GEMM, 46
+// against 96).
 __device__ __forceinline__ bool elect_one() {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : : "memory");
@@ -717,8 +717,7 @@ tc5_gemm_kernel(const Tc5Args args, const __grid_constant__ CUtensorMap tmA,
                         }
                         __syncwarp();
                     }
-                    // the activation is chosen once per chunk, outside the element loop: inside it the compiler
-                    // evaluates every branch for every element and selects
+                    // the activation is chosen once per chunk: where it is a run-time choice (EP_ANY), 32 elements share it
                     const float* colc_chunk = colc + chalf * HALF + c * 32;
                     if (NORM) {
                         // the norm of this thread's row, applied to the raw product

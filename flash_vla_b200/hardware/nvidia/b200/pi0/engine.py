@@ -42,9 +42,10 @@ MAX_GROUP_ROWS = 128       # rows that the weight-streaming decoder GEMM takes
 
 def decoder_groups(episodes: int, rows: int):
     """Episodes whose decoders run as one batch, as (first, last + 1) pairs: one or two groups that the weight-streaming
-    GEMM takes, else one group on the general kernels. Measured, ms per replay of three views and ten steps: three episodes of 51
-    rows 19.2 / 17.8 / 18.7 in one, two and three groups, four 22.7 / 21.9, two of 65 rows 17.3 / 15.4; four of 65 rows 23.6 / 27.6 in
-    one and four, eight of 51 rows 37.8 / 43.1 in one and four: every group streams the weights for itself."""
+    GEMM takes, else one group on the general kernels. Measured, ms per replay of three views and ten steps: two episodes of 51 rows 13.2 / 13.4
+    in one and two groups, three 18.0 / 17.6 / 18.3 in one, two and three, two of 65 rows 15.2 / 14.7; three of 65 rows 17.7 / 20.1 in one and three, four
+    21.3 / 26.6 in one and four, five of 51 rows 24.7 / 29.9, eight 35.5 / 42.6: every group streams the weights for itself. Four of 51 rows
+    are at 21.2 / 21.5 in one and two: the two were chosen at 22.7 / 21.9, before one group's row norms and second down launch went."""
     count = -(-episodes // max(1, MAX_GROUP_ROWS // rows))
     if count > 2:
         count = 1

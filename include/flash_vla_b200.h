@@ -283,7 +283,9 @@ struct fvla_decoder_batch_layers {
 };
 int fvla_decoder_batch_layers_run(const struct fvla_decoder_batch_layers* args, void* stream);
 int fvla_decoder_batch_supported(int episodes, int tokens);
-/* 1 where the two prefix calls above take that many rows: tcgen05 kernels in use, more than 64 rows, no pinned launch plans. */
+/* 1 where the three calls above take that many rows in all: tcgen05 kernels in use, more than 64 rows, no pinned launch plans. (What else they ask
+ * for is in their own comments; fvla_encoder_layers_run also refuses several sequences under FVLA_ATTN=mma, and each refuses null or
+ * misaligned pointers.) */
 int fvla_row_sums_supported(int M);
 
 /* No counterpart in the reference, where these are torch `copy_` calls inside the pipeline (pipeline.py:103,
