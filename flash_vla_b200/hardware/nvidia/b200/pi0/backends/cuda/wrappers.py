@@ -200,20 +200,18 @@ _FOLDED_ATTR = "_fvla_folded_layernorm"
 
 class _Folded:
     """Operands that `fvla_fold_layernorm` made of one LayerNorm + linear pair, and what they were made of."""
-    __slots__ = ("operands", "versions", "sources", "stream", "recorded")
+    __slots__ = ("operands", "versions", "sources", "recorded", "ordered")
 
     def __init__(self, operands, versions, sources):
         self.operands, self.versions, self.sources = operands, versions, sources
-        self.stream, self.recorded = _stream(), _fold_recorded()
+        self.recorded, self.ordered = _fold_recorded(), {_stream()}
 
-    def ready(self):
-        """The operands, behind the fold on whichever stream is current. (A capture cannot wait for work outside it; what it reads has to have
-        run before it begins.)"""
-        if self.recorded is not None and _stream() != self.stream and not torch.cuda.is_current_stream_capturing():
-            if self.recorded.query():
-                self.recorded = None
-            else:
-                self.recorded.wait()
+    def ready(self, stream):
+        """The operands, for work behind the fold on the current stream: another stream than the fold's waits for it once. (A capture cannot wait
+        for work outside it; what it reads has to have run before it begins. And no event is queried, which a capture in another thread forbids.)"""
+        if stream not in self.ordered and not torch.cuda.is_current_stream_capturing():
+            self.recorded.wait()
+            self.ordered.add(stream)
         return self.operands
 
 
@@ -243,7 +241,7 @@ def _folded_layernorm(weight, norm_w, norm_b, bias):
     versions = tuple(t._version for t in sources)
     entry = table.get(key)
     if entry is not None and entry.versions == versions:
-        return entry.ready()
+        return entry.ready(_stream())
     if torch.cuda.is_current_stream_capturing():
         return None
     if entry is None:
@@ -267,10 +265,10 @@ def _folded_layers(weight, norm_w, norm_b, bias):
     stacks = (weight, norm_w, norm_b, bias)
     versions = tuple(t._version for t in stacks)
     (w0, ws), (n0, ns), (s0, ss), (b0, bs) = ((_place(t), t.stride(0)) for t in stacks)
-    layers, shape = [], weight.shape[1:]
+    layers, shape, stream = [], weight.shape[1:], _stream()
     for l in range(weight.shape[0]):
         entry = table.get(((w0[0], w0[1] + l * ws), (n0[0], n0[1] + l * ns), (s0[0], s0[1] + l * ss), (b0[0], b0[1] + l * bs), shape))
-        folded = entry.ready() if entry is not None and entry.versions == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
+        folded = entry.ready(stream) if entry is not None and entry.versions == versions else _folded_layernorm(weight[l], norm_w[l], norm_b[l], bias[l])
         if folded is None:
             return None
         layers.append(folded)

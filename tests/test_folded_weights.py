@@ -32,6 +32,34 @@ on = [0]                     # the current stream
 
 
 class Done:
+    """Stands for the event behind a fold. (No `query`: a capture in another thread forbids that.)"""
+    waits = 0
+
+    def wait(self):
+        Done.waits += 1
+
+
+@pytest.fixture
+def folds(monkeypatch):
+    """Destination addresses of the folds so far."""
+    made = []
+    on[0] = 0
+
+    def call(name, nw, nb, w, b, folded, colsum, bias, n, k, stream):
+        assert name == "fvla_fold_layernorm" and n == N and k == K
+        made.append((folded, colsum, bias))
+    monkeypatch.setattr(wrappers._lib, "call", call)
+    monkeypatch.setattr(wrappers, "_chk", lambda name, t, *a, **kw: t.data_ptr())
+    monkeypatch.setattr(wrappers, "_stream", lambda: on[0])
+    monkeypatch.setattr(wrappers, "_fold_recorded", lambda: Done(), raising=False)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    return made
+
+
+on = [0]                     # the current stream
+
+
+class Done:
     """Stands for the event behind a fold."""
     reached, waits = False, 0
 
@@ -103,18 +131,17 @@ def test_another_stream_waits_for_the_fold(folds, monkeypatch, stacked):
     """Engines that run their episodes on streams of their own fold on the first one's: the others must not read before that has run."""
     sources = pair((L,)) if stacked else pair()
     find, count = (wrappers._folded_layers, L) if stacked else (wrappers._folded_layernorm, 1)
-    monkeypatch.setattr(Done, "reached", False)
     monkeypatch.setattr(Done, "waits", 0)
     find(*sources)
     find(*sources)
     assert Done.waits == 0                                   # the same stream is in order anyway
-    on[0] = 1
-    find(*sources)
-    assert Done.waits == count
-    on[0] = 2
-    Done.reached = True
-    find(*sources)
+    for stream in (1, 2):
+        on[0], before = stream, Done.waits
+        find(*sources)
+        assert Done.waits == before + count
+        find(*sources)
+        assert Done.waits == before + count                  # and from then on
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
     on[0] = 3
-    Done.reached = False                                     # seen once, not asked again
     find(*sources)
-    assert Done.waits == count and len(folds) == count
+    assert Done.waits == 2 * count and len(folds) == count
